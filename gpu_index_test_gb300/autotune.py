@@ -4,14 +4,8 @@ Sweeps, over the C-ABI (gbsa_batcher_*):
   seed_variant   the persistent seeding + lookup kernel's shape: warps per block (reads
                  in flight per CTA), resident blocks per SM, and the shared-memory read
                  window (longest read seeded in shared memory: 512 or 256 bases)
-  lane_max_hits  the NAM merge's split between one lane per read and one warp per read
   sort_variant   the block size of the sort of rescued reads with many NAMs
-  lane_variant   the lane-per-read NAM merge: open NAMs in shared memory with a
-                 register budget of 96, 80 or 64, or open NAMs in registers
-  warp_variant   the register budget of the warp-per-read NAM merge (96, 80 or 64) and its
-                 blocks per SM (5, or 4 beside the sorts)
-(the first three as a grid, then the two register budgets as a grid at the best of
-the first) on the repeat-rich mid-size configuration (150 bp pairs), the uneven length configuration
+on the repeat-rich mid-size configuration (150 bp pairs), the uneven length configuration
 (50-500 bp, single-end and pairs mixed) and a tenth of the human-scale one (repeat
 families, 150 bp pairs), timing each shape's graph
 launches with CUDA events and checking its output byte for byte against the plain
@@ -36,10 +30,7 @@ import numpy as np
 from . import abi, native, synth
 from ._build_paths import GBSA_SO
 
-LANE_MAX_HITS = (64, 96, 128, 160)
 SORT_VARIANTS = (0, 1)
-REG_VARIANTS = (0, 1, 2, 3, 4)   # warp merge: 3, 4 launched four blocks per SM
-LANE_VARIANTS = (0, 1, 2, 3, 4, 5, 6)   # 3-6: the open NAMs in registers
 CHUNKS = (1 << 16, 1 << 17, 1 << 18, 1 << 19, 1 << 20)
 
 
@@ -104,17 +95,10 @@ def _same(a, b):
 
 
 def sweep(scale=1.0, reps=7, log=print):
-    """Shapes are (seed_variant, lane_max_hits, sort_variant, lane_variant, warp_variant)."""
-    grid = [(v, l, s, 0, 0) for v in range(abi.SEED_VARIANTS) for l in LANE_MAX_HITS for s in SORT_VARIANTS]
-    pick, rows, exact, score, plain_ms = _sweep(grid, scale, reps, log)
-    regs = [pick[:3] + (lv, wv) for lv in LANE_VARIANTS for wv in REG_VARIANTS]
-    pick2, rows2, exact2, _, _ = _sweep(regs, scale, reps, log)
-    rows.update(rows2)
-    exact.update(exact2)
-    names = list(plain_ms)
-    best = {nm: min(rows[sh][nm] for sh in rows if exact[sh]) for nm in names}
-    score = {sh: sum(rows[sh][nm] / best[nm] for nm in names) for sh in rows if exact[sh]}
-    return min(score, key=score.get), rows, exact, score, plain_ms
+    """Shapes are (seed_variant, lane_max_hits, sort_variant, lane_variant, warp_variant); the
+    configuration keeps the merge fields, which no longer select anything."""
+    grid = [(v, 128, s, 0, 0) for v in range(abi.SEED_VARIANTS) for s in SORT_VARIANTS]
+    return _sweep(grid, scale, reps, log)
 
 
 def _sweep(shapes, scale, reps, log):

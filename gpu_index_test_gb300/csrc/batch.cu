@@ -99,6 +99,8 @@ std::string library_dir() {
     return ".";
 }
 
+constexpr uint32_t kLaneMaxHitsCap = 160;   // largest lane_max_hits a configuration may name
+
 gbsa_batch_config builtin_config() {
     gbsa_batch_config c{};
     c.seed_variant = 0;
@@ -180,10 +182,7 @@ void lane_init(gbsa_batcher& b, Lane& L) {
     const int rc = gbsa_mapper_create(b.idx, &b.opt, b.max_reads, b.max_bases, &m);
     if (rc != GBSA_OK) throw Error(rc, std::string("batcher work areas: ") + gbsa_last_error());
     L.m = m;
-    L.m->cfg.lane_max_hits = b.cfg.lane_max_hits;
     L.m->cfg.sort_variant = b.cfg.sort_variant;
-    L.m->cfg.lane_variant = b.cfg.lane_variant;
-    L.m->cfg.warp_variant = b.cfg.warp_variant;
     L.m->cfg.rescue_block_hits = b.cfg.rescue_block_hits;
     if (b.profile && gbsa_mapper_set_profile(L.m, 1) != GBSA_OK) throw Error(GBSA_ERR_CUDA, gbsa_last_error());
     L.desc.resize(sizeof(BatchDesc));
@@ -539,6 +538,7 @@ void gbsa_batcher_free(gbsa_batcher* b) {
         if (L.m) {
             cudaStreamSynchronize(L.m->st);
             cudaStreamSynchronize(L.m->side);
+            cudaStreamSynchronize(L.m->side2);
         }
         drop_graph(L);
         for (cudaEvent_t e : {L.done, L.in_ready, L.out_free, L.wait_ev})
@@ -574,6 +574,7 @@ int gbsa_batcher_set_profile(gbsa_batcher* b, int on) {
             if (!L.m) continue;
             GBSA_CUDA(cudaStreamSynchronize(L.m->st));
             GBSA_CUDA(cudaStreamSynchronize(L.m->side));
+            GBSA_CUDA(cudaStreamSynchronize(L.m->side2));
             if (gbsa_mapper_set_profile(L.m, on) != GBSA_OK) throw Error(GBSA_ERR_CUDA, gbsa_last_error());
             drop_graph(L);   // the graph is captured anew, with (or without) the stage events
         }
@@ -767,6 +768,7 @@ int gbsa_batcher_map(gbsa_batcher* b, const char* seqs, const uint64_t* offsets,
                     if (L.m) {
                         cudaStreamSynchronize(L.m->st);
                         cudaStreamSynchronize(L.m->side);
+                        cudaStreamSynchronize(L.m->side2);
                         L.async = false;
                     }
                 cudaStreamSynchronize(b->copy_in);

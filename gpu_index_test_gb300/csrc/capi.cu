@@ -380,7 +380,6 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
     mark(2);
     if (fused) launch_lookup_long(I, C, n, m.rec.as<ReadRec>(), A, ctr, st);
     else launch_lookup(I, C, n, m.rec.as<ReadRec>(), A, ctr, st, desc);
-    launch_bucket_reads(n, C.lane_max_hits, m.rec.as<ReadRec>(), A, ctr, st, desc);
     if (early) {
         GBSA_CUDA(cudaEventRecord(m.early_ev, early));
         GBSA_CUDA(cudaStreamWaitEvent(main_st, m.early_ev, 0));
@@ -388,31 +387,39 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
     }
     mark(3);
     // The rescue chain works on the rescued reads only and the NAM kernels on the
-    // others: the rescue chain runs on the side stream (with its own scratch slots) so
-    // that its tail of reads with thousands of hits overlaps them.
+    // others: it runs on the side streams (with its own scratch slots) beside them.  The
+    // rescue kernel is submitted first: it holds one block an SM for as long as its
+    // heaviest read takes, and its sorts, which end the batch, wait for it (behind the group
+    // merge, which fills the SMs' registers, it started 2 ms late on the 2M-read batch).
     // (at the main stream's priority: a caller's stream has the lowest)
-    cudaStream_t side = m.side;
+    cudaStream_t side = m.side, side2 = m.side2;
     if (st != m.st) {
         int prio = 0, lo = 0, hi = 0;
         GBSA_CUDA(cudaStreamGetPriority(st, &prio));
         GBSA_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-        if (prio != hi) side = m.side_lo;
+        if (prio != hi) {
+            side = m.side_lo;
+            side2 = m.side2_lo;
+        }
     }
     GBSA_CUDA(cudaEventRecord(m.fork_ev, st));
-    // the lane merge is submitted ahead of the rescue kernel: the first of two kernels that
-    // become ready together takes the SMs first, and the rescue kernel ahead of the lane
-    // merge slowed the lane stage by a third
-    launch_nams(I, C, n, m.rec.as<ReadRec>(), A, ctr, st);
-    mark(4);
     GBSA_CUDA(cudaStreamWaitEvent(side, m.fork_ev, 0));
     Arenas As = A;
     As.slots = m.side_slots.as<uint8_t>();
     launch_rescue(I, C, n, m.rec.as<ReadRec>(), As, ctr, side);
     GBSA_CUDA(cudaEventRecord(m.rescue_ev, side));
     if (m.profile) record_stage(m.ev[6], side);
+    // the block sorts and the cluster sorts take different reads: beside each other
+    GBSA_CUDA(cudaStreamWaitEvent(side2, m.rescue_ev, 0));
     if (n) launch_sort_jobs(C, m.rec.as<ReadRec>(), As, ctr, side);
+    if (n) launch_sort_jobs_cluster(C, m.rec.as<ReadRec>(), As, ctr, side2);
+    GBSA_CUDA(cudaEventRecord(m.join2_ev, side2));
+    GBSA_CUDA(cudaStreamWaitEvent(side, m.join2_ev, 0));
     if (m.profile) record_stage(m.ev[7], side);
     GBSA_CUDA(cudaEventRecord(m.join_ev, side));
+    launch_bucket_reads(n, m.rec.as<ReadRec>(), A, ctr, st, desc);
+    launch_nams(C, n, m.rec.as<ReadRec>(), A, ctr, st);
+    mark(4);
     launch_nams_warp(C, n, m.rec.as<ReadRec>(), A, ctr, st);
     mark(5);
     // Every read's NAM count is known once the rescue kernel has ended (the sorts after
@@ -442,7 +449,7 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
 bool check_batch(gbsa_mapper& m, bool seeded) {
     const Counters h = *m.h_status.as<Counters>();
     if (m.profile) {
-        // seed, long seed, lookup, lane NAMs, warp NAMs (main stream); rescue, its
+        // seed, long seed, lookup, group NAMs, warp NAMs (main stream); rescue, its
         // block sorts (side stream, from the fork after the lookup)
         static const int from[7] = {0, 1, 2, 3, 4, 3, 6}, to[7] = {1, 2, 3, 4, 5, 6, 7};
         for (int i = 0; i < 7; ++i) GBSA_CUDA(cudaEventElapsedTime(&m.stage_ms[i], m.ev[from[i]], m.ev[to[i]]));
@@ -909,10 +916,7 @@ int gbsa_mapper_create(const gbsa_index* idx, const gbsa_map_options* opt, uint3
             gbsa_batch_config bc{};
             int from_file = 0;
             if (gbsa_batch_config_default(&bc, &from_file) == GBSA_OK) {
-                m->cfg.lane_max_hits = bc.lane_max_hits;
                 m->cfg.sort_variant = bc.sort_variant;
-                m->cfg.lane_variant = bc.lane_variant;
-                m->cfg.warp_variant = bc.warp_variant;
                 // heavy rescued reads of small batches merged a block each (10k-100k-read
                 // batches of 150 bp pairs: about 0.3 of the batch time less)
                 m->cfg.rescue_block_hits = bc.rescue_block_hits;
@@ -929,11 +933,14 @@ int gbsa_mapper_create(const gbsa_index* idx, const gbsa_map_options* opt, uint3
         GBSA_CUDA(cudaStreamCreateWithPriority(&m->st, cudaStreamNonBlocking, hi));
         GBSA_CUDA(cudaStreamCreateWithPriority(&m->side, cudaStreamNonBlocking, hi));
         GBSA_CUDA(cudaStreamCreateWithPriority(&m->side_lo, cudaStreamNonBlocking, lo));
+        GBSA_CUDA(cudaStreamCreateWithPriority(&m->side2, cudaStreamNonBlocking, hi));
+        GBSA_CUDA(cudaStreamCreateWithPriority(&m->side2_lo, cudaStreamNonBlocking, lo));
         GBSA_CUDA(cudaStreamCreateWithPriority(&m->early, cudaStreamNonBlocking, lo));
         GBSA_CUDA(cudaEventCreateWithFlags(&m->early_ev, cudaEventDisableTiming));
         GBSA_CUDA(cudaEventCreateWithFlags(&m->fork_ev, cudaEventDisableTiming));
         GBSA_CUDA(cudaEventCreateWithFlags(&m->join_ev, cudaEventDisableTiming));
         GBSA_CUDA(cudaEventCreateWithFlags(&m->rescue_ev, cudaEventDisableTiming));
+        GBSA_CUDA(cudaEventCreateWithFlags(&m->join2_ev, cudaEventDisableTiming));
         mapper_reserve(*m, m->max_reads, m->max_bases);
         *out = m.release();
     });
@@ -943,6 +950,7 @@ void gbsa_mapper_free(gbsa_mapper* m) {
     if (!m) return;
     gbsa_mapper_free(m->twin);
     if (m->side) cudaStreamSynchronize(m->side);
+    if (m->side2) cudaStreamSynchronize(m->side2);
     if (m->st) cudaStreamSynchronize(m->st);
     try {
         l2_window_attach(*m, false);
@@ -959,7 +967,8 @@ void gbsa_mapper_free(gbsa_mapper* m) {
     if (m->fork_ev) cudaEventDestroy(m->fork_ev);
     if (m->join_ev) cudaEventDestroy(m->join_ev);
     if (m->rescue_ev) cudaEventDestroy(m->rescue_ev);
-    for (cudaStream_t x : {m->early, m->side_lo})
+    if (m->join2_ev) cudaEventDestroy(m->join2_ev);
+    for (cudaStream_t x : {m->early, m->side_lo, m->side2, m->side2_lo})
         if (x) {
             cudaStreamSynchronize(x);
             cudaStreamDestroy(x);
@@ -1094,7 +1103,8 @@ int gbsa_map_reads(gbsa_mapper* m, const char* seqs, const uint64_t* offsets, co
             ~Drain() {
                 if (!armed) return;
                 for (int i = 0; i < 2; ++i)
-                    for (cudaStream_t x : {part[i]->early, part[i]->side, part[i]->st}) cudaStreamSynchronize(x);
+                    for (cudaStream_t x : {part[i]->early, part[i]->side, part[i]->side2, part[i]->st})
+                        cudaStreamSynchronize(x);
                 cudaStreamSynchronize(m->copy_in);
                 cudaStreamSynchronize(m->copy_out);
             }
@@ -1110,7 +1120,7 @@ int gbsa_map_reads(gbsa_mapper* m, const char* seqs, const uint64_t* offsets, co
             // a work area overflowed: let everything in flight end, then run the chunk again
             if (++retries > 8) throw Error(GBSA_ERR_DEVICE_STATUS, "work areas kept overflowing");
             for (gbsa_mapper* b : part)
-                for (cudaStream_t x : {b->early, b->side, b->st}) GBSA_CUDA(cudaStreamSynchronize(x));
+                for (cudaStream_t x : {b->early, b->side, b->side2, b->st}) GBSA_CUDA(cudaStreamSynchronize(x));
             GBSA_CUDA(cudaStreamSynchronize(m->copy_in));
             queued = finished;
         }
@@ -1258,6 +1268,7 @@ int gbsa_mapper_set_l2_window(gbsa_mapper* m, int on, uint64_t* window_bytes) {
             if (!x) continue;
             GBSA_CUDA(cudaStreamSynchronize(x->st));
             GBSA_CUDA(cudaStreamSynchronize(x->side));
+            GBSA_CUDA(cudaStreamSynchronize(x->side2));
             l2_window_attach(*x, false);
             x->use_l2_window = on != 0;
             l2_window_attach(*x, true);

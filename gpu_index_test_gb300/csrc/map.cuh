@@ -37,12 +37,14 @@ struct Counters {
     unsigned int n_rescue;        // rescued reads on the light end of the rescue list
     unsigned int n_long;
     unsigned int status;
-    unsigned int n_big;    // reads merged by the warp-cooperative NAM kernel
+    unsigned int n_big;    // reads with more NAMs than the group NAM kernel holds
     unsigned int n_heavy;  // rescued reads whose NAMs the block-per-read sort kernel orders (small tile)
     unsigned int n_rescue_heavy;  // rescued reads on the heavy end of the rescue list
     unsigned int n_huge;   // rescued reads whose NAMs the large-tile block sort orders
     unsigned int rescue_next;  // next rescue-list entry to take (k_rescue's work counter)
-    unsigned int lane_cnt[16]; // reads per hit-count bucket of the lane NAM kernel
+    unsigned int lane_cnt[16]; // reads per hit-count bucket of the register NAM merges
+    unsigned int group_next;   // next item of the group NAM kernel
+    unsigned int big_next;     // next read of the warp NAM kernel
     unsigned int queue_head;   // next read (work item) of the seeding (+ lookup) kernel
     unsigned int queue_head2;  // next read of the lookup kernel, when it runs on its own
     unsigned int rescue_block_next;  // next heavy rescued read to take a block (k_rescue)
@@ -67,7 +69,7 @@ struct BatchDesc {
     uint8_t* rescued;       // may be null
 };
 
-constexpr uint32_t kLaneBuckets = 13;   // hit-count buckets of the lane NAM kernel (<= 16)
+constexpr uint32_t kLaneBuckets = 13;    // hit-count buckets of the register NAM merge (<= 16)
 
 // A read whose NAMs are sorted by the block-per-read sort kernel.
 struct SortJob {
@@ -116,24 +118,13 @@ struct MapConfig {
     const void* l2_base;
     uint64_t l2_bytes;
     float l2_hit_ratio;
-    // NAM phase shape: reads with at most lane_max_hits hits (<= kLaneMaxHitsCap) are
-    // merged by one lane each, heavier ones by a warp each; sort_variant picks the block
-    // size of the sort of rescued reads with many NAMs (0: 256 threads, 1: 512)
-    uint32_t lane_max_hits;
+    // block size of the sort of rescued reads with many NAMs (0: 256 threads, 1: 512)
     int sort_variant;
-    // register budgets of the NAM merge kernels (resident blocks they must fit):
-    // lane_variant 0 none, 1 six blocks, 2 eight (3-6: the open NAMs in registers,
-    // k_nams_lane_r: 10 slots at 168 / 128 registers, 6 slots at 96 / 124); warp_variant
-    // 0 five, 1 six, 2 eight
-    // (3, 4: 96 / 80 registers launched four blocks per SM)
-    int lane_variant;
-    int warp_variant;
     // rescued reads whose estimated merge hits (their seeds' runs up to the count cap)
     // reach rescue_block_hits are merged by a whole block each, ahead of the others
     // (0: every rescued read by one warp, those above kRescueHeavyHits first)
     uint32_t rescue_block_hits;
 };
-constexpr uint32_t kLaneMaxHitsCap = 160;
 constexpr uint32_t kRescueBlockHitsDefault = 4000;   // a new mapper's rescue_block_hits
 
 // Reads shorter than this (and with at most kSmemSyncmers syncmers) are seeded
@@ -178,14 +169,14 @@ void launch_lookup_long(const IndexView& I, const MapConfig& C, uint32_t n, Read
                         cudaStream_t st);
 void launch_lookup(const IndexView& I, const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr,
                    cudaStream_t st, const BatchDesc* desc = nullptr);
-void launch_nams(const IndexView& I, const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr,
-                 cudaStream_t st);
-void launch_bucket_reads(uint32_t n, uint32_t lane_max_hits, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st,
+void launch_nams(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
+void launch_bucket_reads(uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st,
                          const BatchDesc* desc = nullptr);
 void launch_nams_warp(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 void launch_rescue(const IndexView& I, const MapConfig& C, uint32_t n_reads, ReadRec* rec, Arenas A, Counters* ctr,
                    cudaStream_t st);
 void launch_sort_jobs(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
+void launch_sort_jobs_cluster(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 // mode 0: every read; 1: the reads that were not rescued; 2: the rescued reads (A and
 // ctr give the rescue list; needed for mode 2 only).
 // With desc (batched form): n is the work areas' read capacity, the batch's read count,

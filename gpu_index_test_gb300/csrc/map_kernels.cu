@@ -10,6 +10,7 @@
 //   k_rescue                    find_nams_rescue (step2/nam.cu:927-985) + NAM sort
 #include <algorithm>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -487,82 +488,28 @@ __device__ void warp_finish_nams(const MapConfig& C, const NamLists& L, uint32_t
     __syncwarp();
 }
 
-constexpr uint32_t kLaneMaxHits = kLaneMaxHitsCap;   // the lane kernel's hit-count buckets cover this
-constexpr uint32_t kLaneOpen = 10;   // open NAMs a lane keeps in shared memory
-constexpr int kLaneWarps = 4;
-// The rescue chain runs beside the two NAM kernels on another stream; the persistent
-// grids are sized so that the rescue chain keeps room beside them: rescue 1 x 72 KB,
-// lane kernel 3 x 40 KB, then the warp kernel 5 x 32 KB (measured against 4, and against
-// 2-3 lane blocks: fewer main-stream blocks speed the rescue chain but slow the main
-// stream more).
-constexpr int kLaneBlocksPerSm = 3;
+// ---- the NAM merge in registers --------------------------------------------------------
+//
+// find_nams merge with the read's NAMs in registers: a group of G lanes (4 to 32 by hit
+// count) takes a read, 32 / G reads a warp, with R slots a lane: NAM i is slot (row) i / G
+// of lane i % G.  Slots are never given back (a read has at most as many NAMs as hits;
+// the few reads with more NAMs than slots go to a list in memory), so slot order is
+// creation order.  Same hit-major rule as warp_find_nams: hits in (orientation,
+// query_start, position) order, each joins the first NAM in creation order that accepts
+// it, found with one ballot a row; a NAM that the query start has passed, or of the other
+// orientation, accepts nothing, so it needs no closing (rows with no other NAM are
+// skipped).  The NAMs are then ranked by their keys through shared memory and written
+// once, in order.
+//
+// A lane a read (open NAMs in shared memory) ran 7.9 of 32 lanes an instruction at 15%
+// occupancy, waiting on shared memory, and its sort of many NAMs went through HBM: one
+// read of 128 hits took as long as a thousand reads.
+constexpr int kGroupWarps = 4;
+constexpr int kGroupBlocksPerSm = 8;     // 64 registers a thread
+// The rescue chain runs beside the NAM kernels on another stream; the persistent grids are
+// sized so that its block (72 KB) keeps room beside them.
 constexpr int kRescueBlocksPerSm = 1;
 
-__device__ __forceinline__ bool nam_key3_less(const NamKey& a, const NamKey& b) {
-    if (a.k1 != b.k1) return a.k1 < b.k1;
-    if (a.k2 != b.k2) return a.k2 < b.k2;
-    return a.k3 < b.k3;
-}
-
-// Open NAMs of the lanes of a block, one field per array ([slot][thread]) so that a
-// warp touching slot o reads 32 consecutive words.
-struct LaneOpen {
-    int32_t qs[kLaneOpen][32 * kLaneWarps], qe[kLaneOpen][32 * kLaneWarps], qprev[kLaneOpen][32 * kLaneWarps];
-    int32_t rs[kLaneOpen][32 * kLaneWarps], re[kLaneOpen][32 * kLaneWarps], rprev[kLaneOpen][32 * kLaneWarps];
-    int32_t nh[kLaneOpen][32 * kLaneWarps];
-    uint32_t ref[kLaneOpen][32 * kLaneWarps];
-    __device__ NamState get(uint32_t o, uint32_t t) const {
-        NamState n;
-        n.qs = qs[o][t];
-        n.qe = qe[o][t];
-        n.qprev = qprev[o][t];
-        n.rs = rs[o][t];
-        n.re = re[o][t];
-        n.rprev = rprev[o][t];
-        n.n_hits = nh[o][t];
-        n.ref_rc = ref[o][t];
-        return n;
-    }
-    __device__ void put(uint32_t o, uint32_t t, const NamState& n) {
-        qs[o][t] = n.qs;
-        qe[o][t] = n.qe;
-        qprev[o][t] = n.qprev;
-        rs[o][t] = n.rs;
-        re[o][t] = n.re;
-        rprev[o][t] = n.rprev;
-        nh[o][t] = n.n_hits;
-        ref[o][t] = n.ref_rc;
-    }
-    // After its merge a lane's 8 * kLaneOpen words (every 32 * kLaneWarps-th word of
-    // the struct, from its thread index on) are free: they hold the sort entries
-    // (first key word, NAM index; three words each) of up to kEntries of its NAMs.
-    // Only the lane touches them, and the lanes of a warp hit 32 different banks.
-    static constexpr uint32_t kEntries = 8 * kLaneOpen / 3;
-    static constexpr uint32_t kStride = 32 * kLaneWarps;
-    __device__ uint32_t* words() { return reinterpret_cast<uint32_t*>(this); }
-    __device__ uint64_t key(uint32_t e, uint32_t t) {
-        const uint32_t* w = words() + 3 * e * kStride + t;
-        return ((uint64_t)w[kStride] << 32) | w[0];
-    }
-    __device__ uint32_t index(uint32_t e, uint32_t t) { return words()[(3 * e + 2) * kStride + t]; }
-    __device__ void set_entry(uint32_t e, uint32_t t, uint64_t k, uint32_t i) {
-        uint32_t* w = words() + 3 * e * kStride + t;
-        w[0] = (uint32_t)k;
-        w[kStride] = (uint32_t)(k >> 32);
-        w[2 * kStride] = i;
-    }
-};
-static_assert(sizeof(LaneOpen) == 8 * kLaneOpen * 32 * kLaneWarps * 4, "LaneOpen is 8 word arrays");
-
-// find_nams merge with one lane per read, for reads with at most kLaneMaxHits hits
-// whose open-NAM list stays within kLaneOpen (the common case: one locus chain plus
-// scattered single hits).  Same hit-major rule as nam_merge_hit_major: hits in
-// (orientation, query_start, position) order, each joins the first open NAM in
-// creation order of its (orientation, ref id) that accepts it.  Open NAMs live in
-// shared memory; a NAM is closed (written to the read's slots in the NAM arena) when
-// the open list is full and the current query start has passed it, or at the end.
-// The read's NAMs are then sorted (through shared memory).  Reads that do not fit go
-// to the warp-cooperative kernel.
 __device__ __forceinline__ HitRec load_hit(const HitPacked* __restrict__ hits, uint32_t i, uint32_t H) {
     HitRec h;
     if (i < H) {
@@ -579,20 +526,19 @@ __device__ __forceinline__ HitRec load_hit(const HitPacked* __restrict__ hits, u
     return h;
 }
 
-// Hit-count bucket of a read for the lane kernel: 8 wide up to 64 hits, 16 wide up
-// to 128, then one bucket up to kLaneMaxHits.
+// Hit-count bucket of a read for the register merge: 8 wide up to 64 hits, 32 wide up to
+// 128, 64 wide up to 256, then one for all above.
 __device__ __forceinline__ uint32_t lane_bucket(uint32_t H) {
     if (H <= 64) return (H - 1) >> 3;
-    if (H <= 128) return 8 + ((H - 65) >> 4);
-    return 12;
+    if (H <= 128) return 8 + ((H - 65) >> 5);
+    return H <= 256 ? 10 + ((H - 129) >> 6) : kLaneBuckets - 1;
 }
 
-// Sorts the reads with hits for the NAM kernels: more than kLaneMaxHits hits to the
-// warp kernel's list, the others into lists by hit count, so that the lanes of a
-// warp of the lane kernel merge reads of similar size (a warp runs as long as its
-// longest read).  Appends are aggregated per warp and bucket.
-__global__ void k_bucket_reads(uint32_t n, uint32_t lane_max, const ReadRec* __restrict__ rec, Arenas A,
-                               Counters* ctr, const BatchDesc* desc) {
+// Sorts the reads with hits into lists by hit count for the register merge, so that the
+// groups of a warp merge reads of similar size (a warp runs as long as its longest read).
+// Appends are aggregated per warp and bucket.
+__global__ void k_bucket_reads(uint32_t n, const ReadRec* __restrict__ rec, Arenas A, Counters* ctr,
+                               const BatchDesc* desc) {
     if (desc) n = min(n, desc->n_reads);
     const uint32_t lane = lane_id();
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -602,358 +548,273 @@ __global__ void k_bucket_reads(uint32_t n, uint32_t lane_max, const ReadRec* __r
         if (r < n) {
             const uint32_t flags = rec[r].flags;
             const uint32_t H = rec[r].n_hits;
-            if (!(flags & (kReadFailed | kReadRescue)) && H > 0) key = H > lane_max ? 16u : lane_bucket(H);
+            if (!(flags & (kReadFailed | kReadRescue)) && H > 0) key = lane_bucket(H);
         }
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
         const uint32_t leader = __ffs(peers) - 1;
         uint32_t at = 0;
         if (key != 0xFFFFFFFFu && lane == leader)
-            at = atomicAdd(key == 16u ? &ctr->n_big : &ctr->lane_cnt[key], (unsigned)__popc(peers));
+            at = atomicAdd(&ctr->lane_cnt[key], (unsigned)__popc(peers));
         at = __shfl_sync(0xFFFFFFFFu, at, leader) + __popc(peers & lanemask_lt());
-        if (key == 16u) A.big_list[at] = r;
-        else if (key != 0xFFFFFFFFu) A.lane_lists[(size_t)key * A.lane_cap + at] = r;
+        if (key != 0xFFFFFFFFu) A.lane_lists[(size_t)key * A.lane_cap + at] = r;
     }
 }
 
-// Sorts a lane's n_closed NAMs (out[0..n_closed), written as they closed) by the NAM
-// order, stably, and returns the arena offset of the sorted list: for at most
-// Sort::kEntries NAMs on (first key word, index) entries in shared memory (full keys only
-// on a tie of the first word), then one pass writes the NAMs in order behind the unsorted
-// ones (out + H); more NAMs are insertion-sorted in place.  keys_ready: the entries were
-// written as the NAMs closed (else they are computed here from out).  The NAM loads of
-// the key pass and of the ordered copy are issued four at a time (each is a round trip
-// to L2: out was just written).
-template <class Sort>
-__device__ __forceinline__ uint64_t lane_sort_nams(const MapConfig& C, Sort& S, uint32_t t, NamState* out,
-                                                   uint32_t n_closed, uint32_t H, uint64_t noff, bool keys_ready) {
-    if (n_closed <= Sort::kEntries) {
-        if (!keys_ready) {
-            uint32_t i = 0;
-            for (; i + 4 <= n_closed; i += 4) {
-                const NamState a = out[i], b = out[i + 1], c = out[i + 2], d = out[i + 3];
-                S.set_entry(i, t, nam_key(a, 0, C.sort_mode).k1, i);
-                S.set_entry(i + 1, t, nam_key(b, 0, C.sort_mode).k1, i + 1);
-                S.set_entry(i + 2, t, nam_key(c, 0, C.sort_mode).k1, i + 2);
-                S.set_entry(i + 3, t, nam_key(d, 0, C.sort_mode).k1, i + 3);
-            }
-            for (; i < n_closed; ++i) S.set_entry(i, t, nam_key(out[i], 0, C.sort_mode).k1, i);
-        }
-        for (uint32_t i = 1; i < n_closed; ++i) {
-            const uint64_t kx = S.key(i, t);
-            if (kx > S.key(i - 1, t)) continue;   // already in place
-            const uint32_t ix = S.index(i, t);
-            NamKey fx;
-            bool have_fx = false;
-            uint32_t j = i;
-            while (j > 0) {
-                const uint64_t ky = S.key(j - 1, t);
-                const uint32_t iy = S.index(j - 1, t);
-                bool less = kx < ky;
-                if (kx == ky) {
-                    if (!have_fx) {
-                        fx = nam_key(out[ix], 0, C.sort_mode);
-                        have_fx = true;
-                    }
-                    less = nam_key3_less(fx, nam_key(out[iy], 0, C.sort_mode));
-                }
-                if (!less) break;
-                S.set_entry(j, t, ky, iy);
-                --j;
-            }
-            S.set_entry(j, t, kx, ix);
-        }
-        NamState* sorted = out + H;
-        uint32_t i = 0;
-        for (; i + 4 <= n_closed; i += 4) {
-            const NamState a = out[S.index(i, t)], b = out[S.index(i + 1, t)], c = out[S.index(i + 2, t)],
-                           d = out[S.index(i + 3, t)];
-            sorted[i] = a;
-            sorted[i + 1] = b;
-            sorted[i + 2] = c;
-            sorted[i + 3] = d;
-        }
-        for (; i < n_closed; ++i) sorted[i] = out[S.index(i, t)];
-        return noff + H;
-    }
-    for (uint32_t i = 1; i < n_closed; ++i) {
-        const NamState x = out[i];
-        const NamKey kx = nam_key(x, 0, C.sort_mode);
-        uint32_t j = i;
-        while (j > 0) {
-            const NamState y = out[j - 1];
-            if (!nam_key3_less(kx, nam_key(y, 0, C.sort_mode))) break;
-            out[j] = y;
-            --j;
-        }
-        out[j] = x;
-    }
-    return noff;
-}
-
-// kMinBlocks: resident blocks the compiler must leave room for (0: no bound); a smaller
-// register budget leaves room on the SM for the rescued reads' sorts beside it.
-template <int kMinBlocks>
-__global__ void __launch_bounds__(32 * kLaneWarps, kMinBlocks) k_nams_lane(MapConfig C, uint32_t n, ReadRec* __restrict__ rec,
-                                                               Arenas A, Counters* ctr) {
-    __shared__ LaneOpen S;
-    __shared__ uint32_t s_cnt[kLaneBuckets];
-    const uint32_t t = threadIdx.x;
-    if (t < kLaneBuckets) s_cnt[t] = *(volatile unsigned int*)&ctr->lane_cnt[t];
-    __syncthreads();
-    uint32_t total = 0;
-    for (uint32_t b = 0; b < kLaneBuckets; ++b) total += s_cnt[b];
-    // reads by bucket, the most hits first
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        uint32_t b = kLaneBuckets - 1, j = i;
-        while (j >= s_cnt[b]) j -= s_cnt[b--];
-        const uint32_t r = A.lane_lists[(size_t)b * A.lane_cap + j];
-        ReadRec& R = rec[r];
-        const uint32_t flags = R.flags;
-        const uint32_t H = R.n_hits;
-        // 2H slots: the NAMs as they close, then (for the sort through shared memory)
-        // the same NAMs in order
-        const uint64_t noff = atomicAdd(&ctr->nam_used, 2ull * H);
-        if (noff + 2ull * H > A.nam_cap) {
-            R.flags = flags | kReadFailed;
-            atomicOr(&ctr->status, kStatusNamOverflow);
-            continue;
-        }
-        const HitPacked* hits = A.hits + R.hit_off;
-        NamState* out = A.nams + noff;
-        uint32_t n_open = 0, n_closed = 0, cur_dir = 0;
-        bool overflow = false;
-        // the next two hits are loaded while one merges
-        HitRec nx0 = load_hit(hits, 0, H), nx1 = load_hit(hits, 1, H);
-        for (uint32_t i = 0; i < H; ++i) {
-            const HitRec x = nx0;
-            nx0 = nx1;
-            nx1 = load_hit(hits, i + 2, H);
-            const uint32_t dir = x.ref_rc >> 31;
-            if (dir != cur_dir) {   // the other orientation's NAMs can take no more hits
-                for (uint32_t o = 0; o < n_open; ++o) out[n_closed++] = S.get(o, t);
-                n_open = 0;
-                cur_dir = dir;
-            }
-            int found = -1;
-            for (uint32_t o = 0; o < n_open; ++o) {
-                if (S.ref[o][t] == x.ref_rc && S.qprev[o][t] < x.qs && x.qs <= S.qe[o][t] && S.rprev[o][t] < x.rs &&
-                    x.rs <= S.re[o][t]) {
-                    const bool ext = x.qe > S.qe[o][t] && x.re > S.re[o][t];
-                    if (ext || (x.qe <= S.qe[o][t] && x.re <= S.re[o][t])) {
-                        if (ext) {
-                            S.qe[o][t] = x.qe;
-                            S.re[o][t] = x.re;
-                        }
-                        S.qprev[o][t] = x.qs;
-                        S.rprev[o][t] = x.rs;
-                        S.nh[o][t] += 1;
-                        found = (int)o;
-                        break;
-                    }
-                }
-            }
-            if (found >= 0) continue;
-            if (n_open == kLaneOpen) {
-                // close NAMs the current query start has passed (order kept)
-                uint32_t k = 0;
-                for (uint32_t o = 0; o < n_open; ++o) {
-                    const NamState m = S.get(o, t);
-                    if (m.qe < x.qs) out[n_closed++] = m;
-                    else S.put(k++, t, m);
-                }
-                n_open = k;
-                if (n_open == kLaneOpen) {
-                    overflow = true;
-                    break;
-                }
-            }
-            S.put(n_open++, t, nam_from_hit(x));
-        }
-        if (overflow) {
-            A.big_list[atomicAdd(&ctr->n_big, 1u)] = r;
-            continue;
-        }
-        for (uint32_t o = 0; o < n_open; ++o) out[n_closed++] = S.get(o, t);
-        // the lane's open-list words are free now: they hold the sort entries
-        R.nam_off = lane_sort_nams(C, S, t, out, n_closed, H, noff, false);
-        R.n_nams = n_closed;
-    }
-}
-
-// The lane-per-read merge with the open NAMs in registers (lane_variant 3).  Same rule
-// as k_nams_lane: each hit joins the first open NAM in creation order that accepts it,
-// else opens one; when all kLaneOpen slots are in use, NAMs the current query start has
-// passed are closed, and a read that still has no free slot goes to the warp kernel.
-// A slot keeps its place while open: creation order is a per-slot sequence number, a
-// closed NAM frees its slot (the read's NAMs are sorted by their full key at the end,
-// so the order they close in does not matter).  Every slot access is unrolled over the
-// kLaneOpen slots, so the lanes of a warp stay together through a hit whatever their
-// open lists hold; shared memory holds only the final sort's entries.
-constexpr uint32_t kLaneEntriesR = 20;   // NAMs of a read sorted in shared memory (more: in place, in HBM)
-
-template <uint32_t kSlots>
-struct LaneSlots {
-    // query start | query end << 12 | creation number << 24 (query coordinates are below
-    // GBSA_MAX_READ_LEN = 4096, creation numbers below kLaneMaxHitsCap + 1); creation
-    // number kFree: the slot is free
-    uint32_t qse[kSlots];
-    uint32_t qpn[kSlots];   // previous hit's query start | n_hits << 16
-    int32_t rs[kSlots], re[kSlots], rprev[kSlots];
-    uint32_t ref[kSlots];
-    static constexpr uint32_t kFree = 0xFFu;
-    __device__ __forceinline__ uint32_t seq(uint32_t o) const { return qse[o] >> 24; }
-    __device__ __forceinline__ int32_t qe(uint32_t o) const { return (int32_t)((qse[o] >> 12) & 0xFFFu); }
-    __device__ __forceinline__ void free_slot(uint32_t o) { qse[o] |= kFree << 24; }
-    __device__ __forceinline__ NamState get(uint32_t o) const {
-        NamState n;
-        n.qs = (int32_t)(qse[o] & 0xFFFu);
-        n.qe = qe(o);
-        n.qprev = (int32_t)(qpn[o] & 0xFFFFu);
-        n.n_hits = (int32_t)(qpn[o] >> 16);
-        n.rs = rs[o];
-        n.re = re[o];
-        n.rprev = rprev[o];
-        n.ref_rc = ref[o];
-        return n;
-    }
-};
-static_assert(GBSA_MAX_READ_LEN <= 4096 && kLaneMaxHitsCap < 255, "lane slot packing");
-
-struct LaneSortR {
-    uint32_t w[3 * kLaneEntriesR][32 * kLaneWarps];
-    static constexpr uint32_t kEntries = kLaneEntriesR;
-    __device__ uint64_t key(uint32_t e, uint32_t t) const {
-        return ((uint64_t)w[3 * e + 1][t] << 32) | w[3 * e][t];
-    }
-    __device__ uint32_t index(uint32_t e, uint32_t t) const { return w[3 * e + 2][t]; }
-    __device__ void set_entry(uint32_t e, uint32_t t, uint64_t k, uint32_t i) {
-        w[3 * e][t] = (uint32_t)k;
-        w[3 * e + 1][t] = (uint32_t)(k >> 32);
-        w[3 * e + 2][t] = i;
-    }
+// Shared memory of a warp's register merge: the hits in flight, and the NAMs' sort keys by
+// slot (row * 32 + lane).
+template <int R>
+struct GroupShared {
+    uint4 hits[2][32];
+    uint64_t k1[32 * R], k2[32 * R], k3[32 * R];
+    uint8_t at[32 * R];   // slot that took a rank
 };
 
-// Writes a closing NAM to the lane's list and, while the list fits the shared-memory
-// sort, its sort entry (its first key word, computed from registers).
-__device__ __forceinline__ void lane_close_r(const MapConfig& C, LaneSortR& S, uint32_t t, NamState* out,
-                                             uint32_t& n_closed, const NamState& m) {
-    if (n_closed < LaneSortR::kEntries) S.set_entry(n_closed, t, nam_key(m, 0, C.sort_mode).k1, n_closed);
-    out[n_closed++] = m;
+// f(r) for every row, r a compile-time constant (the rows' state must stay in registers).
+template <class F, int... I>
+__device__ __forceinline__ void each_row_of(std::integer_sequence<int, I...>, F&& f) {
+    (f(std::integral_constant<int, I>{}), ...);
+}
+template <int R, class F>
+__device__ __forceinline__ void each_row(F&& f) {
+    each_row_of(std::make_integer_sequence<int, R>{}, f);
 }
 
-// kMinBlocks: the register budget (3: 168 registers, no spills; 4: 128 registers, which
-// leaves room beside two blocks per SM for the rescue kernel's block; 5 with 6 slots: 96
-// registers, three blocks per SM beside the rescue kernel's block).  kSlots: open NAMs
-// per lane (reads that need more go to the warp kernel).
-template <int kMinBlocks, uint32_t kSlots>
-__global__ void __launch_bounds__(32 * kLaneWarps, kMinBlocks)
-    k_nams_lane_r(MapConfig C, uint32_t n, ReadRec* __restrict__ rec, Arenas A, Counters* ctr) {
-    __shared__ LaneSortR S;
-    __shared__ uint32_t s_cnt[kLaneBuckets];
-    const uint32_t t = threadIdx.x;
-    if (t < kLaneBuckets) s_cnt[t] = *(volatile unsigned int*)&ctr->lane_cnt[t];
-    __syncthreads();
-    uint32_t total = 0;
-    for (uint32_t b = 0; b < kLaneBuckets; ++b) total += s_cnt[b];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        uint32_t b = kLaneBuckets - 1, j = i;
-        while (j >= s_cnt[b]) j -= s_cnt[b--];
-        const uint32_t r = A.lane_lists[(size_t)b * A.lane_cap + j];
-        ReadRec& R = rec[r];
-        const uint32_t flags = R.flags;
-        const uint32_t H = R.n_hits;
-        const uint64_t noff = atomicAdd(&ctr->nam_used, 2ull * H);
-        if (noff + 2ull * H > A.nam_cap) {
-            R.flags = flags | kReadFailed;
+// Merges the reads list[first ..] (one a group of G lanes, those below cnt) and writes
+// their sorted NAMs; S: the warp's shared memory.  Returns a group's read with more than
+// G * R NAMs in its lanes (its NAMs are not written), else kNoRead.
+constexpr uint32_t kNoRead = 0xFFFFFFFFu;
+template <int G, int R>
+__device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr,
+                                const uint32_t* __restrict__ list, uint32_t first, uint32_t cnt, GroupShared<R>& S) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    constexpr uint32_t kNoRef = 0xFFFFFFFFu;   // a hit's reference id has 24 bits
+    const uint32_t lane = lane_id();
+    const uint32_t sub = lane & (G - 1), base = lane & ~(uint32_t)(G - 1);
+    const uint32_t gmask = (G == 32 ? kFull : (1u << (G & 31)) - 1) << base;
+    const uint32_t at = first + lane / G;
+    const bool have = at < cnt;
+    const uint32_t rd = have ? list[at] : 0;
+    const uint32_t H = have ? rec[rd].n_hits : 0;
+    const uint4* hits = reinterpret_cast<const uint4*>(A.hits + (have ? rec[rd].hit_off : 0));
+    const uint32_t Hm = __reduce_max_sync(kFull, H);
+    int32_t rs[R], re[R], rp[R];
+    uint32_t ref[R], qep[R], qn[R];   // qep: query end << 16 | previous hit's start; qn: n_hits << 16 | query start
+    each_row<R>([&](auto row_c) {
+        constexpr int r = decltype(row_c)::value;
+        ref[r] = kNoRef;
+        qep[r] = qn[r] = 0;
+        rs[r] = re[r] = rp[r] = 0;
+    });
+    uint32_t n = 0;              // the group's NAMs
+    uint32_t rows = 0, live = 0; // rows in use by any group, and those that may still accept a hit (bits)
+    // the group's hits, G at a time through shared memory, the next G in flight
+    const uint4 none = make_uint4(kNoRef - 1, 0, 0, 0);
+    uint4 nx = sub < H ? __ldg(hits + sub) : none;
+    bool over = false;
+    for (uint32_t c = 0; c < Hm; c += G) {
+        uint4* buf = S.hits[(c / G) & 1];
+        buf[lane] = nx;
+        nx = c + G + sub < H ? __ldg(hits + c + G + sub) : none;
+        __syncwarp();
+        const uint32_t steps = min((uint32_t)G, Hm - c);
+        if (R <= 4 && rows > 1) {   // rows the query start has passed in every group
+            const uint4 v = buf[base];
+            const uint32_t xqs = v.y & 0xFFFFu;
+            live = 0;
+            each_row<R>([&](auto row_c) {
+                constexpr int r = decltype(row_c)::value;
+                if ((uint32_t)r < rows &&
+                    __any_sync(kFull, ref[r] != kNoRef && (int32_t)(ref[r] ^ v.x) >= 0 && (qep[r] >> 16) >= xqs))
+                    live |= 1u << r;
+            });
+        }
+        for (uint32_t j = 0; j < steps; ++j) {
+            const uint4 v = buf[base + j];
+            const uint32_t xqs = v.y & 0xFFFFu, xqe = v.y >> 16;
+            const int32_t xrs = (int32_t)v.z, xre = (int32_t)v.w;
+            bool done = c + j >= H;
+            // rows where some NAM could take the hit by its reference interval: most fail this
+            // (with 8 slots a lane the rows are tested without branches, so that their
+            // latencies overlap: that merge is a few long reads, each on one warp)
+            uint32_t may = 0;
+            auto in_ref = [&](int r) { return ref[r] == v.x && rp[r] < xrs && xrs <= re[r]; };
+            if (R > 4)
+                each_row<R>([&](auto row_c) {
+                    constexpr int r = decltype(row_c)::value;
+                    may |= __any_sync(kFull, in_ref(r)) ? 1u << r : 0u;
+                });
+            each_row<R>([&](auto row_c) {
+                constexpr int r = decltype(row_c)::value;
+                if (R > 4 ? !((may >> r) & 1u) : (!((live >> r) & 1u) || !__any_sync(kFull, in_ref(r)))) return;
+                const uint32_t qe = qep[r] >> 16;
+                const bool ok = !done && in_ref(r) && (qep[r] & 0xFFFFu) < xqs && xqs <= qe &&
+                                (xqe > qe) == (xre > re[r]);
+                const uint32_t b = __ballot_sync(kFull, ok) & gmask;
+                if (ok && (b & lanemask_lt()) == 0) {   // the first accepting NAM takes the hit
+                    qep[r] = (max(qe, xqe) << 16) | xqs;   // both ends grow or neither
+                    re[r] = max(re[r], xre);
+                    rp[r] = xrs;
+                    qn[r] += 1u << 16;
+                }
+                done = done || b != 0;
+            });
+            // a hit that no NAM took opens one in the group's next slot
+            if (__any_sync(kFull, !done)) {
+                if (n == G * R) {   // (never for reads of up to G * R hits)
+                    over = true;
+                    done = true;
+                }
+                const bool mine = !done && sub == (n & (G - 1));
+                each_row<R>([&](auto row_c) {
+                    constexpr int r = decltype(row_c)::value;
+                    if (mine && n / G == (uint32_t)r) {
+                        ref[r] = v.x;
+                        qep[r] = (xqe << 16) | xqs;
+                        rs[r] = xrs;
+                        re[r] = xre;
+                        rp[r] = xrs;
+                        qn[r] = (1u << 16) | xqs;
+                    }
+                });
+                const uint32_t row = done ? 0u : 1u << (n / G);
+                const uint32_t opened = G == 32 ? row : __reduce_or_sync(kFull, row);
+                if (!done) ++n;
+                live |= opened;
+                rows = max(rows, 32u - (uint32_t)__clz(opened));
+            }
+        }
+        if (G == 32 && over) return rd;
+    }
+    auto nam = [&](int r) {
+        NamState m;
+        m.qs = (int32_t)(qn[r] & 0xFFFFu);
+        m.qe = (int32_t)(qep[r] >> 16);
+        m.qprev = (int32_t)(qep[r] & 0xFFFFu);
+        m.rs = rs[r];
+        m.re = re[r];
+        m.rprev = rp[r];
+        m.n_hits = (int32_t)(qn[r] >> 16);
+        m.ref_rc = ref[r];
+        return m;
+    };
+    // ranks by the first key word (a NAM's is never all ones), one byte a row
+    uint64_t ranks = 0;
+    each_row<R>([&](auto row_c) {
+        constexpr int r = decltype(row_c)::value;
+        if ((uint32_t)r < rows) S.k1[32 * r + lane] = r * G + sub < n ? nam_key(nam(r), 0, C.sort_mode).k1 : ~0ULL;
+    });
+    __syncwarp();
+    const uint32_t nm = __reduce_max_sync(kFull, n);
+    for (uint32_t r = 0; r < rows; ++r) {   // (the keys are read by slot: no register array is indexed)
+        const uint64_t mine = S.k1[32 * r + lane];
+        uint32_t rank = 0;
+        for (uint32_t row = 0; row * G < nm; ++row) {
+            const uint64_t* k = S.k1 + 32 * row + base;
+            const uint32_t in_row = min((uint32_t)G, nm - row * G);
+#pragma unroll 4
+            for (uint32_t j = 0; j < in_row; ++j) rank += k[j] < mine ? 1u : 0u;
+        }
+        if (r * G + sub < n) S.at[R * base + rank] = (uint8_t)(r * G + sub);
+        ranks |= (uint64_t)(rank & 0xFFu) << (8 * r);
+    }
+    __syncwarp();
+    // NAMs whose first words tie took the same rank: then all three words and the
+    // creation order decide
+    bool tie = false;
+    each_row<R>([&](auto row_c) {
+        constexpr int r = decltype(row_c)::value;
+        if (r * G + sub < n) tie |= S.at[R * base + ((ranks >> (8 * r)) & 0xFFu)] != (uint8_t)(r * G + sub);
+    });
+    if (__any_sync(kFull, tie)) {
+        each_row<R>([&](auto row_c) {
+            constexpr int r = decltype(row_c)::value;
+            if (r * G + sub < n) {
+                const NamKey k = nam_key(nam(r), 0, C.sort_mode);
+                S.k2[32 * r + lane] = k.k2;
+                S.k3[32 * r + lane] = k.k3;
+            }
+        });
+        __syncwarp();
+        for (uint32_t f = lane; f < 32 * rows; f += 32) {   // the lane's slots again, by row
+            const uint32_t own = (f >> 5) * G + sub;
+            uint32_t more = 0;
+            for (uint32_t o = 0; own < n && o < n; ++o) {
+                const uint32_t e = 32 * (o / G) + base + (o & (G - 1));
+                if (S.k1[e] != S.k1[f] || o == own) continue;
+                const uint64_t a2 = S.k2[e], b2 = S.k2[f], a3 = S.k3[e], b3 = S.k3[f];
+                if (a2 != b2 ? a2 < b2 : (a3 != b3 ? a3 < b3 : o < own)) ++more;
+            }
+            ranks += (uint64_t)more << (8 * (f >> 5));
+        }
+    }
+    // NAM arena: one reservation a warp
+    const uint32_t count = sub == 0 ? n : 0;
+    const uint32_t inc = warp_inclusive_sum(count);
+    const uint32_t total = __shfl_sync(kFull, inc, 31);
+    const uint64_t off0 = warp_bump(&ctr->nam_used, total);
+    const uint64_t off = off0 + __shfl_sync(kFull, inc - count, base);
+    if (off0 + total > A.nam_cap) {
+        if (have && sub == 0) {
+            rec[rd].flags |= kReadFailed;
             atomicOr(&ctr->status, kStatusNamOverflow);
-            continue;
         }
-        const HitPacked* hits = A.hits + R.hit_off;
-        NamState* out = A.nams + noff;
-        LaneSlots<kSlots> L;
-#pragma unroll
-        for (uint32_t o = 0; o < kSlots; ++o) L.qse[o] = LaneSlots<kSlots>::kFree << 24;
-        uint32_t n_open = 0, n_closed = 0, cur_dir = 0, next_seq = 0;
-        bool overflow = false;
-        HitRec nx = load_hit(hits, 0, H);
-        for (uint32_t i = 0; i < H; ++i) {
-            const HitRec x = nx;
-            nx = load_hit(hits, i + 1, H);
-            const uint32_t dir = x.ref_rc >> 31;
-            if (dir != cur_dir) {   // the other orientation's NAMs can take no more hits
-#pragma unroll
-                for (uint32_t o = 0; o < kSlots; ++o)
-                    if (L.seq(o) != LaneSlots<kSlots>::kFree) {
-                        lane_close_r(C, S, t, out, n_closed, L.get(o));
-                        L.free_slot(o);
-                    }
-                n_open = 0;
-                cur_dir = dir;
-            }
-            // the accepting NAM created first (free slots have the largest number)
-            uint32_t best = kSlots, bseq = LaneSlots<kSlots>::kFree;
-#pragma unroll
-            for (uint32_t o = 0; o < kSlots; ++o) {
-                const int32_t sqe = L.qe(o);
-                const int32_t sqp = (int32_t)(L.qpn[o] & 0xFFFFu);
-                bool ok = L.ref[o] == x.ref_rc && sqp < x.qs && x.qs <= sqe && L.rprev[o] < x.rs && x.rs <= L.re[o];
-                ok = ok && ((x.qe > sqe && x.re > L.re[o]) || (x.qe <= sqe && x.re <= L.re[o]));
-                if (ok && L.seq(o) < bseq) {
-                    bseq = L.seq(o);
-                    best = o;
-                }
-            }
-            if (best < kSlots) {
-#pragma unroll
-                for (uint32_t o = 0; o < kSlots; ++o) {
-                    if (o != best) continue;
-                    if (x.qe > L.qe(o) && x.re > L.re[o]) {
-                        L.qse[o] = (L.qse[o] & 0xFF000FFFu) | ((uint32_t)x.qe << 12);
-                        L.re[o] = x.re;
-                    }
-                    L.qpn[o] = (uint32_t)x.qs | (((L.qpn[o] >> 16) + 1u) << 16);
-                    L.rprev[o] = x.rs;
-                }
-                continue;
-            }
-            if (n_open == kSlots) {
-                // close NAMs the current query start has passed
-#pragma unroll
-                for (uint32_t o = 0; o < kSlots; ++o)
-                    if (L.seq(o) != LaneSlots<kSlots>::kFree && L.qe(o) < x.qs) {
-                        lane_close_r(C, S, t, out, n_closed, L.get(o));
-                        L.free_slot(o);
-                        --n_open;
-                    }
-                if (n_open == kSlots) {
-                    overflow = true;
-                    break;
-                }
-            }
-            bool placed = false;
-#pragma unroll
-            for (uint32_t o = 0; o < kSlots; ++o) {
-                if (placed || L.seq(o) != LaneSlots<kSlots>::kFree) continue;
-                L.qse[o] = (uint32_t)x.qs | ((uint32_t)x.qe << 12) | (next_seq << 24);
-                L.qpn[o] = (uint32_t)x.qs | (1u << 16);
-                L.rs[o] = x.rs;
-                L.re[o] = x.re;
-                L.rprev[o] = x.rs;
-                L.ref[o] = x.ref_rc;
-                placed = true;
-            }
-            ++next_seq;
-            ++n_open;
+        __syncwarp();
+        return kNoRead;
+    }
+    each_row<R>([&](auto row_c) {
+        constexpr int r = decltype(row_c)::value;
+        if (r * G + sub < n) {
+            // the fields of NamState in order
+            uint4* to = reinterpret_cast<uint4*>(A.nams + off + ((ranks >> (8 * r)) & 0xFFu));
+            to[0] = make_uint4(qn[r] & 0xFFFFu, qep[r] >> 16, qep[r] & 0xFFFFu, (uint32_t)rs[r]);
+            to[1] = make_uint4((uint32_t)re[r], (uint32_t)rp[r], qn[r] >> 16, ref[r]);
         }
-        if (overflow) {
-            A.big_list[atomicAdd(&ctr->n_big, 1u)] = r;
-            continue;
+    });
+    if (have && sub == 0) {
+        rec[rd].nam_off = off;
+        rec[rd].n_nams = n;
+    }
+    __syncwarp();
+    return kNoRead;
+}
+
+// The register merge: persistent warps take the reads by bucket from a work counter, the
+// most hits first.  Groups of 4 lanes take reads of up to 16 hits, of 8 up to 32, of 16 up
+// to 64, a warp all others; a read with more than 128 NAMs (one in a thousand) goes to
+// k_nams.  4 slots a lane fit 64 registers, 32 warps an SM; with 8 slots (twice the reads
+// a warp for the same hits) they took 128 registers and three times as long a hit.
+__global__ void __launch_bounds__(32 * kGroupWarps, kGroupBlocksPerSm)
+    k_nams_group(MapConfig C, ReadRec* __restrict__ rec, Arenas A, Counters* ctr) {
+    __shared__ GroupShared<4> s_group[kGroupWarps];
+    __shared__ uint32_t s_cnt[kLaneBuckets];
+    if (threadIdx.x < kLaneBuckets) s_cnt[threadIdx.x] = *(volatile unsigned int*)&ctr->lane_cnt[threadIdx.x];
+    __syncthreads();
+    GroupShared<4>& S = s_group[threadIdx.x >> 5];
+    for (;;) {
+        uint32_t t = warp_next(&ctr->group_next);
+        int b = (int)kLaneBuckets - 1;
+        for (; b >= 0; --b) {
+            const uint32_t shift = b < 2 ? 3u : (b < 4 ? 2u : (b < 8 ? 1u : 0u));   // log2 of the reads a warp
+            const uint32_t items = (s_cnt[b] + (1u << shift) - 1) >> shift;
+            if (t < items) {
+                t <<= shift;
+                break;
+            }
+            t -= items;
         }
-#pragma unroll
-        for (uint32_t o = 0; o < kSlots; ++o)
-            if (L.seq(o) != LaneSlots<kSlots>::kFree) lane_close_r(C, S, t, out, n_closed, L.get(o));
-        R.nam_off = lane_sort_nams(C, S, t, out, n_closed, H, noff, n_closed <= LaneSortR::kEntries);
-        R.n_nams = n_closed;
+        if (b < 0) break;
+        const uint32_t* list = A.lane_lists + (size_t)b * A.lane_cap;
+        if (b < 2) {
+            group_merge<4, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+        } else if (b < 4) {
+            group_merge<8, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+        } else if (b < 8) {
+            group_merge<16, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+        } else {
+            const uint32_t r = group_merge<32, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+            if (r != kNoRead && lane_id() == 0) A.big_list[atomicAdd(&ctr->n_big, 1u)] = r;
+            __syncwarp();
+        }
     }
 }
 
@@ -1116,26 +977,33 @@ __device__ __forceinline__ bool warp_find_nams(const HitPacked* __restrict__ hit
 
 constexpr uint32_t kHeavyOpen = 256;   // open NAMs (and sort keys) a warp keeps in shared memory
 constexpr int kHeavyWarps = 4;
-constexpr int kHeavyBlocksPerSm = 5;   // register budget
-constexpr int kHeavyGridPerSm = 5;     // blocks launched per SM (32 KB each)
+constexpr int kHeavyBlocksPerSm = 4;   // 128 registers a thread
 
-// find_nams for the reads the lane kernel passed on (many hits, or many NAMs open
-// at once): a warp per read.  The open list lives in shared memory (in global
-// scratch for a read whose open list outgrows kHeavyOpen); closed NAMs go to the
-// warp's global scratch, which is only written until the sort.  The read's NAMs are
-// then sorted by key in shared memory (in scratch beyond kHeavyOpen NAMs) and
-// gathered to the NAM arena.
-// kMinBlocks: resident blocks the compiler must leave room for (its register budget);
-// the grid stays kHeavyGridPerSm blocks per SM, so a larger kMinBlocks leaves registers
-// free beside it for the rescued reads' sorts.
-template <int kMinBlocks>
-__global__ void __launch_bounds__(32 * kHeavyWarps, kMinBlocks)
+// find_nams for the reads with more NAMs than k_nams_group's slots: a warp a read, in
+// registers again with 8 slots a lane; a read with more than 256 NAMs once more with its
+// open list in shared memory (in global scratch when it outgrows kHeavyOpen); closed NAMs
+// then go to the warp's global scratch, which is only written until the sort, and the
+// NAMs are sorted by key in shared memory (in scratch beyond kHeavyOpen NAMs) and gathered
+// to the NAM arena.
+__global__ void __launch_bounds__(32 * kHeavyWarps, kHeavyBlocksPerSm)
     k_nams(MapConfig C, ReadRec* __restrict__ rec, Arenas A, Counters* ctr) {
     __shared__ __align__(16) int32_t s_open[kHeavyWarps][8 * kHeavyOpen];
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
     const uint32_t n_big = *(volatile unsigned int*)&ctr->n_big;
-    for (uint32_t b = warp_global_id(); b < n_big; b += warp_count()) {
+    static_assert(sizeof(GroupShared<8>) <= sizeof(s_open[0]), "a merge's shared memory fits the open-list buffer");
+    GroupShared<8>& S = *reinterpret_cast<GroupShared<8>*>(s_open[w]);
+    for (uint32_t b = warp_next(&ctr->big_next); b < n_big; b = warp_next(&ctr->big_next)) {
         const long long t0 = clock64();
+        if (group_merge<32, 8>(C, rec, A, ctr, A.big_list, b, n_big, S) == kNoRead) {
+            if (A.nam_cycles && lane == 0) {
+                uint64_t* note = A.nam_cycles + 4ull * b;   // cycles, hits, NAMs, merge cycles
+                note[0] = note[3] = (uint64_t)(clock64() - t0);
+                note[1] = rec[A.big_list[b]].n_hits;
+                note[2] = rec[A.big_list[b]].n_nams;
+            }
+            continue;
+        }
+        __syncwarp();
         const uint32_t r = A.big_list[b];
         ReadRec& R = rec[r];
         if (R.flags & (kReadFailed | kReadRescue)) continue;
@@ -2185,11 +2053,11 @@ void launch_lookup(const IndexView& I, const MapConfig& C, uint32_t n, ReadRec* 
 }
 
 // The NAM phase's kernels (lane and warp merges, rescue, NAM gather) run beside each
-// other and need most of an SM's shared memory together (rescue 73 KB + lane merge
-// 3 x 40 KB): they ask for the largest shared-memory carveout, so that the SM keeps that
+// other and need most of an SM's shared memory together (rescue 73 KB + group merge
+// 6 x 12 KB or warp merge 4 x 32 KB): they ask for the largest shared-memory carveout, so that the SM keeps that
 // configuration through the phase instead of switching it as each kernel's blocks
-// arrive (left to the driver, the lane merge took 5.0 instead of 3.3 ms on the C2 batch
-// inside the batch graph).  The seeding + lookup kernels keep the default: they use the
+// arrive (left to the driver, an earlier lane merge took 5.0 instead of 3.3 ms on the C2
+// batch inside the batch graph).  The seeding + lookup kernels keep the default: they use the
 // rest of the unified L1 to cache index entries.  Set once per device.
 void nam_phase_carveout() {
     static std::mutex mu;
@@ -2199,66 +2067,33 @@ void nam_phase_carveout() {
     std::lock_guard<std::mutex> g(mu);
     if ((int)done.size() <= dev) done.resize(dev + 1, 0);
     if (done[dev]) return;
-    const void* fs[] = {(const void*)k_nams_lane<0>, (const void*)k_nams_lane<6>, (const void*)k_nams_lane<8>,
-                        (const void*)k_nams_lane_r<3, kLaneOpen>, (const void*)k_nams_lane_r<4, kLaneOpen>,
-                        (const void*)k_nams_lane_r<5, 6>, (const void*)k_nams_lane_r<3, 6>,
-                        (const void*)k_nams<kHeavyBlocksPerSm>, (const void*)k_nams<6>, (const void*)k_nams<8>,
-                        (const void*)k_rescue, (const void*)k_gather_nams};
+    const void* fs[] = {(const void*)k_nams_group, (const void*)k_nams, (const void*)k_rescue, (const void*)k_gather_nams};
     for (const void* f : fs)
         GBSA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
     done[dev] = 1;
 }
 
-void launch_nams(const IndexView&, const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr,
-                 cudaStream_t st) {
+void launch_nams(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
     if (!n) return;
     nam_phase_carveout();
-    if (C.lane_variant >= 3) {
-        // 3: three blocks per SM at 168 registers (the SM's registers: the rescue kernel
-        // starts as they retire); 4: two blocks per SM at 128 registers, beside the
-        // rescue kernel's block; 5: six slots, three blocks per SM at 96 registers, beside it
-        // 6: six slots at 124 registers, two blocks per SM beside the rescue kernel's block
-        const unsigned per_sm = C.lane_variant == 4 || C.lane_variant == 6 ? 2u : 3u;
-        const unsigned blocks = grid_for(n, 32 * kLaneWarps, (unsigned)device_sm_count() * per_sm);
-        if (C.lane_variant == 4) k_nams_lane_r<4, kLaneOpen><<<blocks, 32 * kLaneWarps, 0, st>>>(C, n, rec, A, ctr);
-        else if (C.lane_variant == 5) k_nams_lane_r<5, 6><<<blocks, 32 * kLaneWarps, 0, st>>>(C, n, rec, A, ctr);
-        else if (C.lane_variant == 6) k_nams_lane_r<3, 6><<<blocks, 32 * kLaneWarps, 0, st>>>(C, n, rec, A, ctr);
-        else k_nams_lane_r<3, kLaneOpen><<<blocks, 32 * kLaneWarps, 0, st>>>(C, n, rec, A, ctr);
-        GBSA_LAUNCHED();
-        return;
-    }
-    const unsigned blocks = grid_for(n, 32 * kLaneWarps, (unsigned)device_sm_count() * kLaneBlocksPerSm);
-    switch (C.lane_variant) {
-        case 1: k_nams_lane<6><<<blocks, 32 * kLaneWarps, 0, st>>>(C, n, rec, A, ctr); break;
-        case 2: k_nams_lane<8><<<blocks, 32 * kLaneWarps, 0, st>>>(C, n, rec, A, ctr); break;
-        default: k_nams_lane<0><<<blocks, 32 * kLaneWarps, 0, st>>>(C, n, rec, A, ctr); break;
-    }
+    const unsigned blocks = grid_for(n, kGroupWarps, (unsigned)device_sm_count() * kGroupBlocksPerSm);
+    k_nams_group<<<blocks, 32 * kGroupWarps, 0, st>>>(C, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 
-void launch_bucket_reads(uint32_t n, uint32_t lane_max_hits, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st,
-                         const BatchDesc* desc) {
+void launch_bucket_reads(uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st, const BatchDesc* desc) {
     if (!n) return;
-    const uint32_t lane_max = lane_max_hits == 0 ? kLaneMaxHits : std::min(lane_max_hits, kLaneMaxHits);
-    k_bucket_reads<<<grid_for(n, 256, (unsigned)device_sm_count() * 8), 256, 0, st>>>(n, lane_max, rec, A, ctr,
-                                                                                      desc);
+    k_bucket_reads<<<grid_for(n, 256, (unsigned)device_sm_count() * 8), 256, 0, st>>>(n, rec, A, ctr, desc);
     GBSA_LAUNCHED();
 }
 
 void launch_nams_warp(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
     if (!n) return;
-    // at most nam_kernel_warps(n) warps: one scratch slot each.  Variants 3 and 4 launch
-    // 4 blocks per SM (96 / 80 registers), leaving registers for the rescued reads' sorts
-    // beside them.
-    const unsigned per_sm = C.warp_variant >= 3 ? 4u : (unsigned)kHeavyGridPerSm;
-    const unsigned blocks = (unsigned)std::min<uint64_t>((uint64_t)device_sm_count() * per_sm,
+    // at most nam_kernel_warps(n) warps: one scratch slot each
+    const unsigned blocks = (unsigned)std::min<uint64_t>((uint64_t)device_sm_count() * kHeavyBlocksPerSm,
                                                          (n + kHeavyWarps - 1) / kHeavyWarps);
-    switch (C.warp_variant) {
-        case 1: case 4: k_nams<6><<<blocks, 32 * kHeavyWarps, 0, st>>>(C, rec, A, ctr); break;
-        case 2: k_nams<8><<<blocks, 32 * kHeavyWarps, 0, st>>>(C, rec, A, ctr); break;
-        default: k_nams<kHeavyBlocksPerSm><<<blocks, 32 * kHeavyWarps, 0, st>>>(C, rec, A, ctr); break;
-    }
+    k_nams<<<blocks, 32 * kHeavyWarps, 0, st>>>(C, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 
@@ -2273,34 +2108,40 @@ void launch_rescue(const IndexView& I, const MapConfig& C, uint32_t n_reads, Rea
     GBSA_LAUNCHED();
 }
 
+// The sorts' dynamic shared memory: a tile of kSortTile keys; their limit is set once per
+// device (mappers may launch from several threads at once).
+constexpr int kSortThreads = 256;
+constexpr size_t kSortSmem = kSortTile * 28;
+
+static void sort_smem_limit() {
+    static std::mutex mu;
+    static std::vector<char> done;
+    int dev = 0;
+    GBSA_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> g(mu);
+    if ((int)done.size() <= dev) done.resize(dev + 1, 0);
+    if (done[dev]) return;
+    for (const void* f : {(const void*)k_sort_jobs<kSortThreads, kSortTile>,
+                          (const void*)k_sort_jobs<2 * kSortThreads, kSortTile>, (const void*)k_sort_jobs_cluster})
+        GBSA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortSmem));
+    done[dev] = 1;
+}
+
 void launch_sort_jobs(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
-    constexpr int kSmall = 256;
-    constexpr size_t smem = kSortTile * 28;
-    {
-        // the kernels' dynamic shared-memory limit, set once per device (mappers may
-        // launch from several threads at once)
-        static std::mutex mu;
-        static std::vector<char> done;
-        int dev = 0;
-        GBSA_CUDA(cudaGetDevice(&dev));
-        std::lock_guard<std::mutex> g(mu);
-        if ((int)done.size() <= dev) done.resize(dev + 1, 0);
-        if (!done[dev]) {
-            GBSA_CUDA(cudaFuncSetAttribute(k_sort_jobs<kSmall, kSortTile>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            GBSA_CUDA(cudaFuncSetAttribute(k_sort_jobs<2 * kSmall, kSortTile>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            GBSA_CUDA(cudaFuncSetAttribute(k_sort_jobs_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
-            done[dev] = 1;
-        }
-    }
+    sort_smem_limit();
     const unsigned sms = (unsigned)device_sm_count();
-    if (C.sort_variant == 1) k_sort_jobs<2 * kSmall, kSortTile><<<sms * 3, 2 * kSmall, smem, st>>>(C, rec, A, ctr);
-    else k_sort_jobs<kSmall, kSortTile><<<sms * 4, kSmall, smem, st>>>(C, rec, A, ctr);
+    if (C.sort_variant == 1)
+        k_sort_jobs<2 * kSortThreads, kSortTile><<<sms * 3, 2 * kSortThreads, kSortSmem, st>>>(C, rec, A, ctr);
+    else
+        k_sort_jobs<kSortThreads, kSortTile><<<sms * 4, kSortThreads, kSortSmem, st>>>(C, rec, A, ctr);
     GBSA_LAUNCHED();
-    // sms / 2 clusters of kClusterCtas CTAs
-    k_sort_jobs_cluster<<<std::max(1u, sms / 2) * kClusterCtas, 256, smem, st>>>(C, rec, A, ctr);
+}
+
+void launch_sort_jobs_cluster(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
+    sort_smem_limit();
+    // SMs / 2 clusters of kClusterCtas CTAs
+    const unsigned clusters = std::max(1u, (unsigned)device_sm_count() / 2);
+    k_sort_jobs_cluster<<<clusters * kClusterCtas, 256, kSortSmem, st>>>(C, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 

@@ -16,6 +16,8 @@ struct gbsa_mapper {
     cudaStream_t side = nullptr;                           // rescue chain, beside the NAM kernels
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr, rescue_ev = nullptr;
     cudaStream_t side_lo = nullptr;                        // rescue chain of a batch on a caller's stream
+    cudaStream_t side2 = nullptr, side2_lo = nullptr;      // cluster sorts, beside the chain's block sorts
+    cudaEvent_t join2_ev = nullptr;
     cudaStream_t early = nullptr;                          // seeding + lookup of pipelined chunks
     cudaEvent_t early_ev = nullptr;
     uint32_t max_reads = 0;

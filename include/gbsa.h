@@ -255,20 +255,11 @@ typedef struct gbsa_batch_config {
     int32_t  seed_variant;   /* persistent seeding + lookup kernel: 0 8 warps x 6 blocks/SM, reads up to
                                 512 bases in shared memory; 1 8 x 5; 2 4 x 12; 3 8 x 7, 256 bases;
                                 4 16 x 3; 5 8 x 6, 256 bases (longer reads take the long-read path) */
-    uint32_t lane_max_hits;  /* reads with at most this many hits (1-160) are merged by one lane,
-                                heavier ones by a warp */
+    uint32_t lane_max_hits;  /* 1-160; without effect (one NAM merge serves every value) */
     int32_t  sort_variant;   /* block size of the sort of rescued reads with many NAMs: 0 256, 1 512 */
     uint32_t chunk_reads;    /* reads per batch of the host entry point (three batches in flight) */
-    int32_t  lane_variant;   /* the lane-per-read NAM merge: open NAMs in shared memory with a register
-                                budget of 0 no bound (96 registers), 1 six blocks (80), 2 eight (64); or
-                                3 open NAMs in registers (168 registers, three blocks per SM), 4 the same
-                                at 128 registers and two blocks per SM (room for the rescue kernel);
-                                5, 6 six open NAMs per lane in registers (reads needing more go to the warp
-                                merge) at 96 registers and three blocks per SM, or 124 and two */
-    int32_t  warp_variant;   /* register budget of the warp-per-read NAM merge: 0 five blocks (96 registers),
-                                1 six (80), 2 eight (64), launched 5 blocks per SM; 3 (96) and 4 (80)
-                                launched 4 blocks per SM; fewer registers leave room for the rescued
-                                reads' sorts beside it */
+    int32_t  lane_variant;   /* 0-6; without effect, as lane_max_hits */
+    int32_t  warp_variant;   /* 0-4; without effect, as lane_max_hits */
     uint32_t rescue_block_hits;  /* as gbsa_mapper_set_rescue_block (0: every rescued read by one warp) */
     uint32_t _reserved;          /* 0 */
 } gbsa_batch_config;
