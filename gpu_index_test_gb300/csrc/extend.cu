@@ -9,7 +9,7 @@
 // reference runs the best-segment scan only when the Hamming distance admits the ungapped
 // path, which leaves a handful of mismatches: the scan steps over the runs between them.
 // A thread per NAM walking bytes waited on its loads (0.70 ms for 1M NAMs of 150 bp reads
-// against KERNEL_MS here, 0.06 ms being what the bytes take).
+// against 0.23 here; 0.06 ms is what the bytes take).
 #include "common.cuh"
 #include "runtime.h"
 
@@ -73,32 +73,31 @@ __device__ __forceinline__ uint32_t complement4(uint32_t w) {
 }
 
 // 8 bytes from p on, as two words in memory order; only aligned words that hold a byte of
-// [lo, hi) are read (the others' bytes are 0).
-__device__ __forceinline__ uint2 load8(const uint8_t* p, const uint8_t* lo, const uint8_t* hi) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p) & ~uintptr_t(3);
-    const uint32_t mis = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
-    auto word = [&](int i) {
-        const uintptr_t x = a + 4 * i;
-        return x + 4 > reinterpret_cast<uintptr_t>(lo) && x < reinterpret_cast<uintptr_t>(hi)
-                   ? __ldg(reinterpret_cast<const uint32_t*>(x))
-                   : 0u;
-    };
-    const uint32_t w0 = word(0), w1 = word(1), w2 = mis ? word(2) : 0u;
+// the sequence are read (the others' bytes are 0): `off` bytes of it lie before p (negative:
+// it starts behind p), `rem` bytes from p on.
+__device__ __forceinline__ uint2 load8(const uint8_t* p, int off, int rem) {
+    const int mis = (int)(reinterpret_cast<uintptr_t>(p) & 3);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - mis);
+    const uint32_t w0 = off + 4 - mis > 0 ? __ldg(w) : 0u;
+    const uint32_t w1 = off + 8 - mis > 0 && 4 - mis < rem ? __ldg(w + 1) : 0u;
+    const uint32_t w2 = mis != 0 && 8 - mis < rem ? __ldg(w + 2) : 0u;
     return make_uint2(__funnelshift_r(w0, w1, 8 * mis), __funnelshift_r(w1, w2, 8 * mis));
 }
-
-// A comparison of n bases: the contig's from ref on with the read's (in the orientation
-// rc) from position q on.
-struct Compare {
-    const uint8_t* ref;
-    const uint8_t* fwd;   // the read as given, L bases
-    int L, q, n;
-    uint32_t rc;
-};
 
 constexpr int kExtendWarps = 4;
 constexpr int kMaskBases = 512;                  // longest comparison of the warp
 constexpr int kMaskWords = kMaskBases / 32 + 1;  // (odd: the lanes' words lie in different banks)
+constexpr int kMaxKmer = 32;                     // longest k-mer of the warp's checks
+
+// What a lane has the warp compare: n bases of the contig with the read's in the orientation
+// rc, from (ref, q) on; and for the k-mer checks a second pair of the same length.
+struct Compare {
+    const uint8_t* ref;
+    const uint8_t* fwd;   // the read as given, L bases
+    int L, n;
+    int q, q2, ref2;      // ref2: the second stretch's place after ref
+    uint32_t rc;
+};
 
 struct ExtendShared {
     Compare task[32];
@@ -106,9 +105,26 @@ struct ExtendShared {
     uint8_t list[32];
 };
 
+// Mismatch bits of the n (1 to 8 counted, more allowed) bases from ref + j and q + j on.
+__device__ __forceinline__ uint32_t compare8(const Compare& t, const uint8_t* ref, int q, int j) {
+    const int n = t.n - j;
+    const uint2 r = load8(ref + j, 0, n);
+    // the read's bases q + j on, or L - 1 - q - j downwards and complemented
+    const int at = t.rc ? t.L - 8 - q - j : q + j;
+    uint2 x = load8(t.fwd + at, at, t.L - at);
+    if (t.rc)
+        x = make_uint2(complement4(__byte_perm(x.y, 0u, 0x0123)), complement4(__byte_perm(x.x, 0u, 0x0123)));
+    // a one in each differing byte, then side by side
+    const uint32_t d0 = __vcmpne4(r.x, x.x) & 0x01010101u, d1 = __vcmpne4(r.y, x.y) & 0x01010101u;
+    const uint32_t bits = ((d0 * 0x01020408u) >> 24) | (((d1 * 0x01020408u) >> 24) << 4);
+    return n < 8 ? bits & ((1u << n) - 1) : bits;
+}
+
 // Runs the comparisons of the lanes with `want` (n <= kMaskBases): afterwards bit j of
-// S.mask[lane] says that base j differs (bits from n on are 0).
-__device__ __forceinline__ void warp_compare(ExtendShared& S, bool want, const Compare& c) {
+// S.mask[lane] says that base j differs (bits from n on are 0); kKmers: both stretches
+// (n <= kMaxKmer), the first's bits in word 0 and the second's in word 1.
+template <bool kKmers>
+__device__ __noinline__ void warp_compare(ExtendShared& S, bool want, const Compare& c) {
     const uint32_t lane = lane_id();
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, want);
     if (want) {
@@ -121,23 +137,13 @@ __device__ __forceinline__ void warp_compare(ExtendShared& S, bool want, const C
         const uint32_t owner = S.list[g];
         const Compare t = S.task[owner];
         uint8_t* out = reinterpret_cast<uint8_t*>(S.mask[owner]);
-        for (int j = 8 * (int)sub; j < ((t.n + 31) & ~31); j += 64) {
-            uint32_t bits = 0;
-            if (j < t.n) {
-                const uint2 r = load8(t.ref + j, t.ref, t.ref + t.n);
-                uint2 x;
-                if (t.rc) {   // bases L-1-q-j downwards, complemented
-                    const uint2 y = load8(t.fwd + (t.L - 8 - t.q - j), t.fwd, t.fwd + t.L);
-                    x = make_uint2(complement4(__byte_perm(y.y, 0u, 0x0123)), complement4(__byte_perm(y.x, 0u, 0x0123)));
-                } else {
-                    x = load8(t.fwd + t.q + j, t.fwd, t.fwd + t.L);
-                }
-                // a byte of ones for each differing byte, then one bit each
-                const uint32_t d0 = __vcmpne4(r.x, x.x) & 0x01010101u, d1 = __vcmpne4(r.y, x.y) & 0x01010101u;
-                bits = ((d0 * 0x01020408u) >> 24) | (((d1 * 0x01020408u) >> 24) << 4);
-                if (j + 8 > t.n) bits &= (1u << (t.n - j)) - 1;
-            }
-            out[j >> 3] = (uint8_t)bits;
+        if (kKmers) {
+            const int j = 8 * (int)(sub & 3u);
+            const bool second = sub >= 4;
+            out[sub] = j < t.n ? (uint8_t)compare8(t, second ? t.ref + t.ref2 : t.ref, second ? t.q2 : t.q, j) : 0;
+        } else {
+            for (int j = 8 * (int)sub; j < ((t.n + 31) & ~31); j += 64)
+                out[j >> 3] = j < t.n ? (uint8_t)compare8(t, t.ref, t.q, j) : 0;
         }
     }
     __syncwarp();
@@ -214,7 +220,8 @@ __device__ __forceinline__ bool hamming_admits(int mismatches, int L) {
     return hamming_dist >= 0 && ((float)hamming_dist / L) < 0.05;
 }
 
-// The whole step for one NAM by one thread, base by base: reads longer than kMaskBases.
+// The whole step for one NAM by one thread, base by base: reads longer than kMaskBases, k
+// above kMaxKmer.
 __device__ __noinline__ void extend_long(gbsa_nam nam, const uint8_t* fwd, const uint8_t* ref, int L, int rlen, int k,
                                          const gbsa_align_params& ap, gbsa_seed_alignment& o) {
     bool consistent = kmer_equal(ref + nam.ref_start, ReadView{fwd, L, nam.is_rc != 0}, nam.query_start, k) &&
@@ -277,7 +284,7 @@ __global__ void __launch_bounds__(32 * kExtendWarps)
         const uint8_t* fwd = ok ? read_seqs + read_offs[r] : nullptr;
         const uint8_t* ref = ok ? ref_seqs + ref_offs[nam.ref_id] : nullptr;
         if (ok) o.ref_id = nam.ref_id;
-        if (ok && L > kMaskBases) {
+        if (ok && (L > kMaskBases || k > kMaxKmer)) {
             gbsa_seed_alignment x = o;   // (o itself stays in registers)
             extend_long(nam, fwd, ref, L, rlen, k, ap, x);
             o = x;
@@ -295,43 +302,40 @@ __global__ void __launch_bounds__(32 * kExtendWarps)
         Compare c;
         c.fwd = fwd;
         c.L = L;
-        c.ref = ref + pstart;
-        c.q = 0;
-        c.n = L;
-        c.rc = nam.is_rc != 0;
-        warp_compare(S, diag, c);
-        bool consistent = diag && mask_clear(mask, nam.query_start, k) && mask_clear(mask, nam.query_end - k, k);
-        bool compared = consistent;   // the mask is the window's in the NAM's orientation
-        auto kmers = [&](bool want, bool rc, int qs, int qe) {   // the two k-mer checks
-            c.rc = rc;
-            c.n = k;
-            c.ref = ref + nam.ref_start;
-            c.q = qs;
-            warp_compare(S, want, c);
-            want = want && mask_clear(mask, 0, k);
-            c.ref = ref + nam.ref_end - k;
-            c.q = qe - k;
-            warp_compare(S, want, c);
-            return want && mask_clear(mask, 0, k);
-        };
-        if (__any_sync(0xFFFFFFFFu, ok && !consistent)) {
-            // off the diagonal: the k-mers themselves; then the other orientation
-            if (kmers(ok && !diag, nam.is_rc != 0, nam.query_start, nam.query_end)) consistent = true;
-            const int qs2 = L - nam.query_end, qe2 = L - nam.query_start;
-            if (kmers(ok && !consistent, nam.is_rc == 0, qs2, qe2)) {
-                nam.is_rc = nam.is_rc ? 0 : 1;
-                nam.query_start = qs2;
-                nam.query_end = qe2;
-                consistent = true;
-            }
-            // extend_seed_part's window (step2/main.cu:582-643) of those
-            const bool more = ok && consistent && !compared && window(pstart);
+        bool consistent = false, compared = false;   // compared: the mask is the window's, in the NAM's orientation
+        for (int pass = 0; pass < 2; ++pass) {
+            // extend_seed_part's window (step2/main.cu:582-643); in the second pass of the
+            // NAMs whose k-mers were checked apart
+            const bool want = pass == 0 ? diag : ok && consistent && !compared && window(pstart);
             c.ref = ref + pstart;
             c.q = 0;
             c.n = L;
             c.rc = nam.is_rc != 0;
-            warp_compare(S, more, c);
-            compared = compared || more;
+            warp_compare<false>(S, want, c);
+            if (pass == 0 && diag)
+                consistent = mask_clear(mask, nam.query_start, k) && mask_clear(mask, nam.query_end - k, k);
+            compared = compared || (want && consistent);
+            if (pass == 1 || !__any_sync(0xFFFFFFFFu, ok && !consistent)) break;
+            // off the diagonal: the k-mers themselves; then the other orientation
+            const int qs2 = L - nam.query_end, qe2 = L - nam.query_start;
+            c.ref = ref + nam.ref_start;
+            c.ref2 = nam.ref_end - k - nam.ref_start;
+            c.n = k;
+            for (int flip = 0; flip < 2; ++flip) {
+                const bool check = ok && !consistent && (flip || !diag);
+                c.rc = (nam.is_rc != 0) != (flip != 0);
+                c.q = flip ? qs2 : nam.query_start;
+                c.q2 = (flip ? qe2 : nam.query_end) - k;
+                warp_compare<true>(S, check, c);
+                if (check && mask[0] == 0 && mask[1] == 0) {
+                    consistent = true;
+                    if (flip) {
+                        nam.is_rc = nam.is_rc ? 0 : 1;
+                        nam.query_start = qs2;
+                        nam.query_end = qe2;
+                    }
+                }
+            }
         }
         if (ok) {
             o.query_start = nam.query_start;
@@ -404,7 +408,7 @@ __device__ __forceinline__ uint32_t pack4(uint32_t c) { return (c * 0x40100401u)
 // with all of them.  Any match answers the question, so the window's 128-position blocks
 // are taken from where the insert size puts the mate outwards: most mates are found in the
 // first.  Scanned from the window's start, with 13 byte loads and 23 compares a position,
-// 1M NAMs of 150 bp pairs took 4.16 ms against KERNEL_MS here.
+// 1M NAMs of 150 bp pairs took 4.16 ms against 0.68 here (bound by integer issue).
 __global__ void __launch_bounds__(32 * kRescueWarps)
     k_rescue_mates(const uint8_t* __restrict__ ref_seqs, const uint64_t* __restrict__ ref_offs,
                    const uint64_t* __restrict__ ref_lens, uint32_t n_refs, const uint8_t* __restrict__ read_seqs,
