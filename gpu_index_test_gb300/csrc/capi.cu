@@ -291,6 +291,7 @@ static Arenas arenas_of(gbsa_mapper& m) {
     A.rescue_cap = (uint32_t)per;
     A.long_list = m.lists.as<uint32_t>() + per;
     A.big_list = m.lists.as<uint32_t>() + 2 * per;
+    A.slow_list = m.lists.as<uint32_t>() + 3 * per;
     A.lane_lists = m.lane_lists.as<uint32_t>();
     A.lane_cap = (uint32_t)(m.lane_lists.size() / (4ull * kLaneBuckets));
     A.sort_jobs = m.jobs.as<SortJob>();
@@ -409,8 +410,11 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
     launch_rescue(I, C, n, m.rec.as<ReadRec>(), As, ctr, side);
     GBSA_CUDA(cudaEventRecord(m.rescue_ev, side));
     if (m.profile) record_stage(m.ev[6], side);
-    // the block sorts and the cluster sorts take different reads: beside each other
-    GBSA_CUDA(cudaStreamWaitEvent(side2, m.rescue_ev, 0));
+    // what the packed sort passes on: the block sorts and the cluster sorts take different
+    // reads, beside each other
+    if (n) launch_sort_packed(C, m.rec.as<ReadRec>(), As, ctr, side);
+    GBSA_CUDA(cudaEventRecord(m.join2_ev, side));
+    GBSA_CUDA(cudaStreamWaitEvent(side2, m.join2_ev, 0));
     if (n) launch_sort_jobs(C, m.rec.as<ReadRec>(), As, ctr, side);
     if (n) launch_sort_jobs_cluster(C, m.rec.as<ReadRec>(), As, ctr, side2);
     GBSA_CUDA(cudaEventRecord(m.join2_ev, side2));

@@ -48,6 +48,9 @@ struct Counters {
     unsigned int queue_head;   // next read (work item) of the seeding (+ lookup) kernel
     unsigned int queue_head2;  // next read of the lookup kernel, when it runs on its own
     unsigned int rescue_block_next;  // next heavy rescued read to take a block (k_rescue)
+    unsigned int sort_next;    // next job of the packed sort
+    unsigned int n_slow;       // jobs that it passed on to the block sort
+    unsigned int n_slow_huge;  // and to the cluster sort
 };
 
 // A batch of the batched form, in device memory: the kernels of a captured batch graph
@@ -98,6 +101,7 @@ struct Arenas {
     uint32_t rescue_cap;
     uint32_t* long_list;
     uint32_t* big_list;
+    uint32_t* slow_list;     // sort jobs the packed sort passed on: block sort's from the front, cluster sort's from the back
     uint32_t* lane_lists;    // kLaneBuckets lists of lane_cap reads each
     uint32_t lane_cap;
     SortJob* sort_jobs;      // small-tile jobs from the front, large-tile ones from the back
@@ -175,6 +179,7 @@ void launch_bucket_reads(uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cuda
 void launch_nams_warp(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 void launch_rescue(const IndexView& I, const MapConfig& C, uint32_t n_reads, ReadRec* rec, Arenas A, Counters* ctr,
                    cudaStream_t st);
+void launch_sort_packed(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 void launch_sort_jobs(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 void launch_sort_jobs_cluster(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 // mode 0: every read; 1: the reads that were not rescued; 2: the rescued reads (A and

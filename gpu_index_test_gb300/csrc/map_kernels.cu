@@ -450,21 +450,20 @@ __device__ void warp_sort_idx(uint64_t* k1, uint32_t* ix, const uint64_t* k2, co
     }
 }
 
-// Sorts a rescued read's NAMs (at most kWarpSortMax) with the warp in its shared
-// buffers sa / sb (4 KB each, free after the merge) and writes them to the NAM arena.
-__device__ void warp_finish_nams(const MapConfig& C, const NamLists& L, uint32_t* sa, uint32_t* sb, ReadRec& R,
+// Sorts a rescued read's NN <= kWarpSortMax NAMs with the warp in its shared buffer (7 KB,
+// free after the merge) and writes them to the NAM arena.
+__device__ void warp_finish_nams(const MapConfig& C, const NamState* closed, uint32_t NN, uint32_t* buf, ReadRec& R,
                                  const Arenas& A, Counters* ctr) {
     const uint32_t lane = lane_id();
-    const uint32_t NN = L.n_closed;
     const uint32_t P = next_pow2(NN);
-    uint64_t* k1 = reinterpret_cast<uint64_t*>(sa);       // P <= 256: 2 KB
-    uint32_t* ix = sa + 512;                              // 1 KB
-    uint64_t* k2 = reinterpret_cast<uint64_t*>(sb);       // 2 KB
+    uint64_t* k1 = reinterpret_cast<uint64_t*>(buf);      // P <= 256: 2 KB
+    uint64_t* k2 = k1 + 256;                              // 2 KB
     uint64_t* k3 = k2 + 256;                              // 2 KB
+    uint32_t* ix = reinterpret_cast<uint32_t*>(k3 + 256); // 1 KB
     for (uint32_t t = lane; t < P; t += 32) {
         NamKey k;
         if (t < NN) {
-            k = nam_key(L.closed[t], t, C.sort_mode);
+            k = nam_key(closed[t], t, C.sort_mode);
         } else {   // padding sorts last (a NAM's first key word is never all ones)
             k.k1 = k.k2 = k.k3 = ~0ULL;
         }
@@ -480,7 +479,7 @@ __device__ void warp_finish_nams(const MapConfig& C, const NamLists& L, uint32_t
         warp_fail(R, ctr, kStatusNamOverflow);
         return;
     }
-    for (uint32_t t = lane; t < NN; t += 32) A.nams[noff + t] = L.closed[ix[t]];
+    for (uint32_t t = lane; t < NN; t += 32) A.nams[noff + t] = closed[ix[t]];
     if (lane == 0) {
         R.nam_off = noff;
         R.n_nams = NN;
@@ -508,7 +507,7 @@ constexpr int kGroupWarps = 4;
 constexpr int kGroupBlocksPerSm = 8;     // 64 registers a thread
 // The rescue chain runs beside the NAM kernels on another stream; the persistent grids are
 // sized so that its block (72 KB) keeps room beside them.
-constexpr int kRescueBlocksPerSm = 1;
+constexpr int kRescueBlocksPerSm = 2;
 
 __device__ __forceinline__ HitRec load_hit(const HitPacked* __restrict__ hits, uint32_t i, uint32_t H) {
     HitRec h;
@@ -1095,7 +1094,7 @@ struct RescuePlan {
     uint32_t maxrun;
 };
 
-// One orientation d of rescue_prepare: adds its taken prefix to plan.
+// One orientation d: adds its taken prefix to plan.
 __device__ void rescue_prepare_dir(const IndexView& I, const MapConfig& C, const Query* const* Qd,
                                    const uint64_t* const* Pd, const uint32_t* nqd, uint32_t Pq, uint64_t* buf, int d,
                                    RescuePlan& plan) {
@@ -1158,68 +1157,297 @@ __device__ void rescue_prepare_dir(const IndexView& I, const MapConfig& C, const
     }
 }
 
-__device__ RescuePlan rescue_prepare(const IndexView& I, const MapConfig& C, const Query* const* Qd,
-                                     const uint64_t* const* Pd, const uint32_t* nqd, uint32_t Pq, uint64_t* buf) {
-    RescuePlan plan{};
-    rescue_prepare_dir(I, C, Qd, Pd, nqd, Pq, buf, 0, plan);
-    rescue_prepare_dir(I, C, Qd, Pd, nqd, Pq, buf, 1, plan);
-    return plan;
-}
-
-// Phase 2 (warp): walk the runs of the taken rescue hits in (orientation,
-// query_start) order and merge them NAM-major; all NAMs end in L.closed.  The hits
-// of the current query are held in compact form in hrs/hpk/tb (room for
-// plan.maxrun hits).
-__device__ uint64_t rescue_merge(const IndexView& I, const Query* const* Qd, const uint64_t* const* Pd,
-                                 const RescuePlan& plan, const uint64_t* tkbuf, uint32_t Pq, NamLists& L, uint32_t* hrs,
-                                 uint32_t* hpk, uint8_t* tb) {
-    uint64_t walk_cycles = 0;
-    const uint64_t* tk[2] = {tkbuf + 2 * Pq, tkbuf + 3 * Pq};
-    for (int d = 0; d < 2; ++d) {
-        for (uint32_t j = 0; j < plan.m[d]; ++j) {
-            const uint32_t qi = (uint32_t)(tk[d][j] >> 32) & 0xFFFF;
-            const uint32_t cnt = (uint32_t)tk[d][j];
-            const Query q = Qd[d][qi];
-            QueryHits Q;
-            Q.rs = hrs;
-            Q.packed = hpk;
-            Q.qs = (int)q.start;
-            Q.qe = (int)q.end;
-            Q.dir = (uint32_t)d;
-            Q.k = I.k;
-            const long long tw = clock64();
-            Q.n = warp_walk_run_n(I, Q.qs, Q.qe, Pd[d][qi], cnt, hrs, hpk, plan.maxrun);
-            walk_cycles += (uint64_t)(clock64() - tw);
-            nam_close_merge_q(L, Q, tb);
-        }
-        nam_close_passed(L, 0x7FFFFFFF);
-    }
-    return walk_cycles;
-}
-
 constexpr uint32_t kWarpSortMax = 256;   // rescued reads with more NAMs are sorted by k_sort_jobs
 constexpr uint32_t kSortTile = 2048;      // keys per shared-memory tile of the small block sort (56 KB)
+constexpr int kClusterCtas = 8;           // CTAs of a cluster sort
+constexpr uint32_t kRescueSmemHits = 1024;// per-warp shared buffer for one query's hits
 
-// find_nams_rescue for the reads on the rescue list (a warp per read).  Reads that
-// end with more than kWarpSortMax NAMs leave the sort to k_sort_jobs.
-constexpr uint32_t kRescueSmemHits = 1024;   // per-warp shared buffer for one query's hits
+// Words a merge needs for queries of up to n hits: their positions, packed words and the
+// NAM that claims each, and a bit each for the ones claimed by earlier NAMs.
+__host__ __device__ constexpr uint32_t rescue_hit_words(uint32_t n) { return 3 * n + (n + 31) / 32; }
 
-// Hands a rescued read's NAMs to the block sort (more than kWarpSortMax) and returns
-// true, or returns false (the caller's warp sorts them).
-__device__ __forceinline__ bool rescue_sort_job(const Arenas& A, Counters* ctr, ReadRec& R, const NamLists& L,
-                                                NamKey* keys, uint32_t r, uint32_t t) {
-    if (L.n_closed <= kWarpSortMax) return false;
+// Shared memory of the rescue kernel: a buffer a warp (a block's merge uses all warps'
+// buffers as one).
+struct RescueShared {
+    uint32_t buf[kWarpsPerBlock][rescue_hit_words(kRescueSmemHits)];
+    uint32_t cnt[kWarpsPerBlock];   // block merge: kept or untaken hits per warp
+    int least[kWarpsPerBlock];      // block walk: least length difference per warp
+    uint32_t item;
+    uint8_t* scratch;
+    RescuePlan plan[2];
+};
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// warp_walk_run_n by the block: 128 entries a warp at a time (a run of up to 1024 in one
+// pass); the running minimum and the kept hits' places cross the warps through S.
+__device__ __forceinline__ uint32_t block_walk_run(const IndexView& I, int qs, int qe, uint64_t pos, uint32_t cnt,
+                                                   uint32_t* rs_out, uint32_t* pk_out, RescueShared& S,
+                                                   uint32_t& min_span, uint32_t& max_span) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    const uint2* ent = reinterpret_cast<const uint2*>(I.rs + pos);   // (position, packed) at offset 8
+    int carry = 0x7FFFFFFF;   // least difference of the passes before
+    uint32_t n = 0, mn = 0xFFu, mx = 0;
+    for (uint32_t pass = 0; pass < cnt; pass += 128 * kWarpsPerBlock) {
+        const uint32_t base = pass + 128 * w;
+        uint2 e[4];
+        int before[4];   // least difference ahead of the entry, within the warp's 128
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t j = base + 32 * u + lane;
+            e[u] = j < cnt ? __ldg(&ent[2 * (size_t)j + 1]) : make_uint2(0, 0);
+        }
+        int least = 0x7FFFFFFF;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int x = (qe - qs) - ((int)(e[u].y & 0xFF) + I.k);
+            const int diff = base + 32 * u + lane < cnt ? (x < 0 ? -x : x) : 0x7FFFFFFF;
+            int pm = diff;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(kFull, pm, o);
+                if (lane >= (uint32_t)o) pm = min(pm, v);
+            }
+            const int ex = __shfl_up_sync(kFull, pm, 1);
+            before[u] = lane ? min(ex, least) : least;
+            least = min(least, __shfl_sync(kFull, pm, 31));
+        }
+        if (lane == 0) S.least[w] = least;
+        __syncthreads();
+        int ahead = carry;
+        for (uint32_t v = 0; v < kWarpsPerBlock; ++v) {
+            if (v < w) ahead = min(ahead, S.least[v]);
+            carry = min(carry, S.least[v]);
+        }
+        uint32_t keep = 0, kept = 0;
+        uint32_t km[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t j = base + 32 * u + lane;
+            const int x = (qe - qs) - ((int)(e[u].y & 0xFF) + I.k);
+            const bool take = j < cnt && (x < 0 ? -x : x) <= min(before[u], ahead);
+            keep |= take ? 1u << u : 0u;
+            km[u] = __ballot_sync(kFull, take);
+            kept += __popc(km[u]);
+        }
+        if (lane == 0) S.cnt[w] = kept;
+        __syncthreads();
+        uint32_t to = n;
+        for (uint32_t v = 0; v < kWarpsPerBlock; ++v) {
+            if (v < w) to += S.cnt[v];
+            n += S.cnt[v];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if ((keep >> u) & 1u) {
+                const uint32_t k = to + __popc(km[u] & lanemask_lt());
+                rs_out[k] = e[u].x;
+                pk_out[k] = e[u].y;
+                mn = min(mn, e[u].y & 0xFFu);
+                mx = max(mx, e[u].y & 0xFFu);
+            }
+            to += __popc(km[u]);
+        }
+        __syncthreads();
+    }
+    mn = __reduce_min_sync(kFull, mn);
+    mx = __reduce_max_sync(kFull, mx);
+    if (lane == 0) {
+        S.least[w] = (int)mn;
+        S.cnt[w] = mx;
+    }
+    __syncthreads();
+    for (uint32_t v = 0; v < kWarpsPerBlock; ++v) {
+        mn = min(mn, (uint32_t)S.least[v]);
+        mx = max(mx, S.cnt[v]);
+    }
+    min_span = mn + (uint32_t)I.k;
+    max_span = mx + (uint32_t)I.k;
+    return n;   // (the caller synchronises before the hits are read or S is written again)
+}
+
+// Phase 2 of find_nams_rescue: walks the runs of the taken rescue hits in (orientation,
+// query_start) order and merges them NAM-major into O (struct of arrays, in creation
+// order); returns the number of NAMs.  kBlock: by the block, else by the warp alone.
+//
+// NAM-major rule (merge_hits_into_nams_fast, step2/nam.cu:94-343): for each open NAM in
+// creation order, the first hit of the query that it accepts and that no NAM before it
+// took.  The threads take a round of NAMs (one each) at a time.  Within a round that is the
+// outcome of all its NAMs proposing at once, each to its first acceptable hit, a hit
+// keeping the NAM created first and a NAM that loses its hit going on to its next one, in
+// whatever order the proposals come: hits are claimed with an atomic minimum of the NAM's
+// number, and the thread that displaces a NAM goes on with that one.  Hits claimed in
+// earlier rounds are gone for good: a bit each lets a NAM step over any number of them at
+// once.  A hit lies where a NAM can accept it only near the NAM's end, as its length is
+// known to within the query's shortest and longest hit.  A NAM that the query has passed
+// (query_end < query_start) accepts nothing and stays where it is, so nothing is moved
+// between lists; then a thread a hit updates the NAM that holds it, and unclaimed hits open
+// NAMs in ref_start order.  (A warp resolving 32 NAMs after the other, testing every hit
+// between a NAM's last hit and its end and moving every NAM of the list for every query,
+// took 2.7M cycles for a read of 8550 hits, 1.5 ms of a batch.)
+//
+// buf: rescue_hit_words(cap) words, plan.maxrun <= cap.
+template <bool kBlock>
+__device__ __forceinline__ uint32_t rescue_merge(const IndexView& I, const Query* const* Qd, const uint64_t* const* Pd,
+                                                 const RescuePlan& plan, const uint64_t* tkbuf, uint32_t Pq,
+                                                 const OpenSoA& O, uint32_t* buf, uint32_t cap, RescueShared& S,
+                                                 uint64_t& walk_cycles) {
+    constexpr uint32_t kFree = 0xFFFFFFFFu;
+    const uint32_t lane = lane_id(), w = kBlock ? threadIdx.x >> 5 : 0;
+    const uint32_t tid = kBlock ? threadIdx.x : lane, nt = kBlock ? blockDim.x : 32u;
+    const uint32_t nw = kBlock ? kWarpsPerBlock : 1u;
+    auto sync = [] {
+        if (kBlock) __syncthreads();
+        else __syncwarp();
+    };
+    uint32_t *hrs = buf, *hpk = buf + cap, *claim = buf + 2 * (size_t)cap, *gone = buf + 3 * (size_t)cap;
+    int32_t *fqe = O.f(1), *fqprev = O.f(2), *fre = O.f(4), *frprev = O.f(5), *fnh = O.f(6);
+    const uint32_t* fref = reinterpret_cast<const uint32_t*>(O.f(7));
+    const volatile uint32_t* held = claim;
+    uint32_t n = 0;
+    for (int d = 0; d < 2; ++d) {
+        const uint64_t* tk = tkbuf + (2 + d) * Pq;
+        const uint32_t lo = n;   // the other orientation's NAMs can take no hit
+        for (uint32_t j = 0; j < plan.m[d]; ++j) {
+            const uint32_t qi = (uint32_t)(tk[j] >> 32) & 0xFFFF;
+            const uint32_t cnt = (uint32_t)tk[j];
+            const int qs = (int)Qd[d][qi].start, qe = (int)Qd[d][qi].end;
+            uint32_t nh = 0, min_span = 0, max_span = 0;
+            const long long tw = clock64();
+            if constexpr (kBlock) nh = block_walk_run(I, qs, qe, Pd[d][qi], cnt, hrs, hpk, S, min_span, max_span);
+            else nh = warp_walk_run_n(I, qs, qe, Pd[d][qi], cnt, hrs, hpk, cap, min_span, max_span);
+            walk_cycles += (uint64_t)(clock64() - tw);
+            for (uint32_t t = tid; t < cnt; t += nt) claim[t] = kFree;
+            for (uint32_t t = tid; 32 * t < cnt; t += nt) gone[t] = 0;
+            // the next query's run (its first entries), on its way while this one merges
+            if (!kBlock && j + 1 < plan.m[d] && 8 * lane < (uint32_t)tk[j + 1])
+                prefetch_l2(I.rs + Pd[d][(uint32_t)(tk[j + 1] >> 32) & 0xFFFF] + 8 * lane);
+            sync();
+            // proposals, a round of nt NAMs at a time (the next round's fields on their way)
+            auto fields = [&](uint32_t i) {
+                return i < n ? make_int4(fqe[i], fre[i], frprev[i], (int)fref[i]) : make_int4(-1, 0, 0, 0);
+            };
+            int4 nx = fields(lo + tid);
+            for (uint32_t r0 = lo; r0 < n; r0 += nt) {
+                const int4 f = nx;
+                nx = fields(r0 + nt + tid);
+                uint32_t i = r0 + tid, fresh = kFree;
+                if (f.x >= qs) {
+                    int nqe = f.x, nre = f.y, from = f.z + 1, last = nre;
+                    uint32_t want = (uint32_t)f.w & 0x7FFFFFFFu;
+                    // a hit is accepted when both its ends lie beyond the NAM's or neither does
+                    if (qe > nqe) from = max(from, nre - (int)max_span + 1);
+                    else last = nre - (int)min_span;
+                    uint32_t at = 0, hi = nh;
+                    while (at < hi) {   // hits are sorted by ref_start
+                        const uint32_t mid = (at + hi) >> 1;
+                        if ((int)hrs[mid] < from) at = mid + 1;
+                        else hi = mid;
+                    }
+                    for (; at < nh; ++at) {
+                        // the next hit that no NAM of an earlier round took
+                        uint32_t free = ~gone[at >> 5] & (0xFFFFFFFFu << (at & 31));
+                        if (!free) {
+                            at |= 31u;
+                            if (at + 1 >= nh || (int)hrs[at + 1] > last) break;
+                            continue;
+                        }
+                        at = (at & ~31u) + (uint32_t)__ffs(free) - 1;
+                        if (at >= nh) break;
+                        const int rs = (int)hrs[at];
+                        if (rs > last) break;
+                        const uint32_t pk = hpk[at];
+                        const int re = rs + (int)(pk & 0xFF) + I.k;
+                        if ((pk >> 8) != want || held[at] < i || (qe > nqe) != (re > nre)) continue;
+                        const uint32_t old = atomicMin(&claim[at], i);
+                        if (old < i) continue;
+                        if (old == kFree) {
+                            fresh = at;
+                            break;
+                        }
+                        i = old;   // displaced: on with its next hit
+                        nqe = fqe[i];
+                        nre = fre[i];
+                        last = qe > nqe ? nre : nre - (int)min_span;
+                        want = fref[i] & 0x7FFFFFFFu;
+                    }
+                }
+                if (r0 + nt >= n) break;   // the last round: its claims need no bits
+                sync();
+                if (fresh != kFree) atomicOr(&gone[fresh >> 5], 1u << (fresh & 31));
+                sync();
+            }
+            sync();
+            // hits to their NAMs; the others open NAMs in order
+            const uint32_t per = ((nh + nw - 1) / nw + 31) & ~31u;
+            const uint32_t h0 = min(w * per, nh), h1 = min(h0 + per, nh);
+            uint32_t mine = 0;
+            for (uint32_t b = h0; b < h1; b += 32)
+                mine += __popc(__ballot_sync(0xFFFFFFFFu, b + lane < h1 && held[b + lane] == kFree));
+            uint32_t to = n, opened = mine;
+            if constexpr (kBlock) {
+                if (lane == 0) S.cnt[w] = mine;
+                __syncthreads();
+                opened = 0;
+                for (uint32_t v = 0; v < nw; ++v) {
+                    if (v < w) to += S.cnt[v];
+                    opened += S.cnt[v];
+                }
+            }
+            for (uint32_t b = h0; b < h1; b += 32) {
+                const uint32_t h = b + lane;
+                const bool in = h < h1;
+                const uint32_t i = in ? held[h] : 0u;
+                const bool open = in && i == kFree;
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, open);
+                if (in) {
+                    const int rs = (int)hrs[h];
+                    const uint32_t pk = hpk[h];
+                    const int re = rs + (int)(pk & 0xFF) + I.k;
+                    if (open) {
+                        HitRec x;
+                        x.ref_rc = ((uint32_t)d << 31) | (pk >> 8);
+                        x.qs = qs;
+                        x.qe = qe;
+                        x.rs = rs;
+                        x.re = re;
+                        O.put(to + __popc(m & lanemask_lt()), nam_from_hit(x));
+                    } else {
+                        if (qe > fqe[i] && re > fre[i]) {
+                            fqe[i] = qe;
+                            fre[i] = re;
+                        }
+                        fqprev[i] = qs;
+                        frprev[i] = rs;
+                        fnh[i] += 1;
+                    }
+                }
+                to += __popc(m);
+            }
+            n += opened;
+            sync();
+        }
+    }
+    return n;
+}
+
+// Hands a rescued read's NAMs to the block sort when they are more than kWarpSortMax and
+// returns true, else false (the caller's warp sorts them).
+__device__ __forceinline__ bool rescue_sort_job(const Arenas& A, Counters* ctr, ReadRec& R, NamState* closed,
+                                                uint32_t n, NamKey* keys, uint32_t r, uint32_t t) {
+    if (n <= kWarpSortMax) return false;
     // many NAMs: the block-per-read sort kernel orders them.  The count is known now
     // (the sort only orders them), so the NAM offsets of the batch can be computed
     // while the sorts run; the sort sets nam_off.
     if (lane_id() == 0) {
-        R.n_nams = L.n_closed;
-        const uint32_t j = L.n_closed > kSortTile ? A.jobs_cap - 1 - atomicAdd(&ctr->n_huge, 1u)
-                                                  : atomicAdd(&ctr->n_heavy, 1u);
+        R.n_nams = n;
+        const uint32_t j = n > kSortTile ? A.jobs_cap - 1 - atomicAdd(&ctr->n_huge, 1u)
+                                         : atomicAdd(&ctr->n_heavy, 1u);
         SortJob job;
-        job.closed = L.closed;
+        job.closed = closed;
         job.keys = keys;
-        job.n = L.n_closed;
+        job.n = n;
         job.read = r;
         job.note = t;
         job.pad = 0;
@@ -1228,240 +1456,310 @@ __device__ __forceinline__ bool rescue_sort_job(const Arenas& A, Counters* ctr, 
     return true;
 }
 
-// find_nams_rescue for one heavy read (entry t of the rescue list) with the whole
-// block: the two orientations' plans on warps 0 and 1, each query's hit run walked by
-// warp 0 and merged by block_close_merge_q.  The shared buffers of the block's warps
-// serve as one: the candidates (hrs), the query's hits (hpk: positions, then packed
-// words) and its taken flags (tb).
-__device__ void rescue_read_block(const IndexView& I, const MapConfig& C, ReadRec* __restrict__ rec,
-                                  const Arenas& A, Counters* ctr, uint32_t t, uint32_t* s_hrs, uint32_t* s_hpk,
-                                  uint8_t* s_tb) {
-    __shared__ uint8_t* s_sc;
-    __shared__ RescuePlan s_plan[2];
-    __shared__ uint32_t s_n;
-    __shared__ uint32_t s_bcnt[kBlockSeg / 32];
-    __shared__ uint32_t s_tot[3];
-    constexpr uint32_t kBlockHits = kWarpsPerBlock * kRescueSmemHits / 2;   // hits of one query in s_hpk
-    static_assert(kWarpsPerBlock * kRescueSmemHits >= kBlockSeg, "the candidates fit the shared buffers");
+// find_nams_rescue for the rescued read r (entry t of the rescue list) by the calling warp
+// or, kBlock, by the block (a heavy read: the two orientations' plans on two warps, each
+// query's run walked by one).
+template <bool kBlock>
+__device__ __forceinline__ void rescue_read(const IndexView& I, const MapConfig& C, ReadRec* __restrict__ rec,
+                                            const Arenas& A, Counters* ctr, uint32_t t, uint32_t r, RescueShared& S) {
     const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+    const bool first = !kBlock || w == 0;   // the warp that takes scratch and writes the result
+    const uint32_t tid = kBlock ? threadIdx.x : lane, nt = kBlock ? blockDim.x : 32u;
     const long long t0 = clock64();
-    const uint32_t r = A.rescue_list[A.rescue_cap - 1 - t];
     ReadRec& R = rec[r];
+    uint64_t* note = A.rescue_cycles && first && lane == 0 ? A.rescue_cycles + 8ull * t : nullptr;
+    // scratch for the team (nullptr, with the read marked failed, when there is none)
+    auto scratch = [&](uint64_t slot_off, uint64_t bytes) {
+        uint8_t* p = nullptr;
+        if (first) {
+            p = warp_scratch(A, ctr, slot_off, bytes);
+            if (!p) warp_fail(R, ctr, kStatusScratchOverflow);
+        }
+        if (kBlock) {
+            if (threadIdx.x == 0) S.scratch = p;
+            __syncthreads();
+            p = S.scratch;
+            __syncthreads();
+        }
+        return p;
+    };
     const uint32_t nqd[2] = {R.nq, R.nq2 - R.nq};
     const Query* Qd[2] = {A.q + R.q_off, A.q + R.q_off + R.nq};
     const uint64_t* Pd[2] = {A.q_pos + R.q_off, A.q_pos + R.q_off + R.nq};
-    const uint32_t nqm = nqd[0] > nqd[1] ? nqd[0] : nqd[1];
-    const uint32_t Pq = next_pow2(nqm > 0 ? nqm : 1);
+    const uint32_t Pq = next_pow2(max(max(nqd[0], nqd[1]), 1u));
     const uint64_t b1 = 4ull * 8 * Pq + 64;
-    if (w == 0) {
-        uint8_t* sc1 = warp_scratch(A, ctr, 0, b1);
-        if (!sc1) warp_fail(R, ctr, kStatusScratchOverflow);
-        if (lane == 0) s_sc = sc1;
-    }
-    __syncthreads();
-    uint64_t* buf = reinterpret_cast<uint64_t*>(s_sc);
-    __syncthreads();
+    uint64_t* buf = reinterpret_cast<uint64_t*>(scratch(0, b1));
     if (!buf) return;
-    if (w < 2) {
-        RescuePlan p{};
-        rescue_prepare_dir(I, C, Qd, Pd, nqd, Pq, buf, (int)w, p);
-        if (lane == 0) s_plan[w] = p;
+    RescuePlan plan{};
+    if (kBlock) {
+        if (w < 2) {
+            RescuePlan p{};
+            rescue_prepare_dir(I, C, Qd, Pd, nqd, Pq, buf, (int)w, p);
+            if (lane == 0) S.plan[w] = p;
+        }
+        __syncthreads();
+        plan.m[0] = S.plan[0].m[0];
+        plan.m[1] = S.plan[1].m[1];
+        plan.bound = S.plan[0].bound + S.plan[1].bound;
+        plan.maxrun = max(S.plan[0].maxrun, S.plan[1].maxrun);
+    } else {
+        rescue_prepare_dir(I, C, Qd, Pd, nqd, Pq, buf, 0, plan);
+        rescue_prepare_dir(I, C, Qd, Pd, nqd, Pq, buf, 1, plan);
     }
-    __syncthreads();
-    RescuePlan plan;
-    plan.m[0] = s_plan[0].m[0];
-    plan.m[1] = s_plan[1].m[1];
-    plan.bound = s_plan[0].bound + s_plan[1].bound;
-    plan.maxrun = s_plan[0].maxrun > s_plan[1].maxrun ? s_plan[0].maxrun : s_plan[1].maxrun;
-    const bool notes = A.rescue_cycles && threadIdx.x == 0;
-    uint64_t* note = A.rescue_cycles ? A.rescue_cycles + 8ull * t : nullptr;
-    if (notes) {
-        note[1] = (uint64_t)(clock64() - t0);
+    if (note) {
+        note[0] = note[1] = (uint64_t)(clock64() - t0);
         note[4] = plan.bound;
         note[7] = plan.maxrun;
     }
     if (plan.bound == 0) {
-        if (threadIdx.x == 0) {
-            R.n_nams = 0;
-            if (notes) note[0] = (uint64_t)(clock64() - t0);
-        }
-        __syncthreads();
+        if (first && lane == 0) R.n_nams = 0;
+        if (kBlock) __syncthreads();
         return;
     }
+    // the NAMs (as many as hits), sort keys only for more than the cluster sort's tiles
+    // hold, and a long run's hits
     const uint32_t H = (uint32_t)plan.bound;
-    const uint64_t P2 = next_pow2(H);
-    const bool big_run = plan.maxrun > kBlockHits;
-    // open, closed and spare lists (H each) and the sort keys; big runs' hits after them
-    const uint64_t b2 = 96ull * H + 32ull * P2 + (big_run ? 9ull * plan.maxrun + 64 : 0) + 256;
-    if (w == 0) {
-        uint8_t* sc2 = warp_scratch(A, ctr, (b1 + 255) & ~255ull, b2);
-        if (!sc2) warp_fail(R, ctr, kStatusScratchOverflow);
-        if (lane == 0) s_sc = sc2;
-    }
-    __syncthreads();
-    uint8_t* sc2 = s_sc;
-    __syncthreads();
+    const uint32_t smem_hits = kBlock ? kWarpsPerBlock * kRescueSmemHits : kRescueSmemHits;
+    const bool big_run = plan.maxrun > smem_hits;
+    const uint64_t key_bytes = H > kClusterCtas * kSortTile ? 32ull * next_pow2(H) : 0;
+    const uint64_t off2 = (b1 + 255) & ~255ull;
+    const uint64_t b2 = 32ull * H + key_bytes + (big_run ? 4ull * rescue_hit_words(plan.maxrun) : 0) + 64;
+    uint8_t* sc2 = scratch(off2, b2);
     if (!sc2) return;
-    NamLists L;
-    L.open = reinterpret_cast<NamState*>(sc2);
-    L.closed = L.open + H;
-    NamKey* keys = reinterpret_cast<NamKey*>(L.closed + H);
-    NamState* spare = reinterpret_cast<NamState*>(keys + P2);
-    uint32_t* hrs = s_hpk;
-    uint32_t* hpk = s_hpk + kBlockHits;
-    uint8_t* tb = s_tb;
-    if (big_run) {
-        hrs = reinterpret_cast<uint32_t*>(spare + H);
-        hpk = hrs + plan.maxrun;
-        tb = reinterpret_cast<uint8_t*>(hpk + plan.maxrun);
-    }
-    L.n_open = L.n_closed = 0;
-    L.cap = H;
+    NamKey* keys = reinterpret_cast<NamKey*>(sc2);
+    const OpenSoA O{reinterpret_cast<int32_t*>(sc2 + key_bytes), H};
+    uint32_t* hits = big_run ? reinterpret_cast<uint32_t*>(sc2 + key_bytes + 32ull * H)
+                             : (kBlock ? &S.buf[0][0] : S.buf[w]);
     const long long t_merge = clock64();
     uint64_t walk_cycles = 0;
-    const uint64_t* tk[2] = {buf + 2 * Pq, buf + 3 * Pq};
-    for (int d = 0; d < 2; ++d) {
-        for (uint32_t j = 0; j < plan.m[d]; ++j) {
-            const uint32_t qi = (uint32_t)(tk[d][j] >> 32) & 0xFFFF;
-            const uint32_t cnt = (uint32_t)tk[d][j];
-            const Query q = Qd[d][qi];
-            QueryHits Q;
-            Q.rs = hrs;
-            Q.packed = hpk;
-            Q.qs = (int)q.start;
-            Q.qe = (int)q.end;
-            Q.dir = (uint32_t)d;
-            Q.k = I.k;
-            if (w == 0) {
-                const long long tw = clock64();
-                const uint32_t n = warp_walk_run_n(I, Q.qs, Q.qe, Pd[d][qi], cnt, hrs, hpk, plan.maxrun);
-                walk_cycles += (uint64_t)(clock64() - tw);
-                if (lane == 0) s_n = n;
-            }
-            __syncthreads();
-            Q.n = s_n;
-            block_close_merge_q(L, spare, Q, tb, s_hrs, s_bcnt, s_tot);
-        }
-        block_close_all(L);
-    }
-    if (notes) {
+    const uint32_t n = rescue_merge<kBlock>(I, Qd, Pd, plan, buf, Pq, O, hits, big_run ? plan.maxrun : smem_hits, S,
+                                            walk_cycles);
+    if (note) {
         note[2] = (uint64_t)(clock64() - t_merge);
-        note[5] = L.n_closed;
+        note[5] = n;
         note[6] = walk_cycles;
     }
-    if (w == 0 && !rescue_sort_job(A, ctr, R, L, keys, r, t)) {
+    // the NAMs as records; those of a sort job outlive this read, so not in the warp's slot
+    NamState* closed = reinterpret_cast<NamState*>(
+        scratch(n > kWarpSortMax ? A.slot_bytes : off2 + ((b2 + 255) & ~255ull), 32ull * n + 32));
+    if (!closed) return;
+    for (uint32_t i = tid; i < n; i += nt) closed[i] = O.get(i);
+    if (kBlock) __syncthreads();
+    else __syncwarp();
+    if (first && !rescue_sort_job(A, ctr, R, closed, n, key_bytes ? keys : nullptr, r, t)) {
         const long long t_fin = clock64();
-        warp_finish_nams(C, L, s_hrs, s_hpk, R, A, ctr);
-        if (notes) note[3] = (uint64_t)(clock64() - t_fin);
+        warp_finish_nams(C, closed, n, S.buf[w], R, A, ctr);
+        if (note) note[3] = (uint64_t)(clock64() - t_fin);
     }
-    if (notes) note[0] = (uint64_t)(clock64() - t0);
-    __syncthreads();
+    if (note) note[0] = (uint64_t)(clock64() - t0);
+    if (kBlock) __syncthreads();
+    else __syncwarp();
 }
 
-// find_nams_rescue for the reads on the rescue list.  With C.rescue_block_hits set and
-// no more rescued reads than the grid has warps (a small batch, whose heavy reads
-// would otherwise set the kernel's time while most warps idle), the heavy end of the
-// list (reads whose estimated merge hits reach rescue_block_hits) is taken first, a
-// block per read, then the rest a warp per read; otherwise every read a warp, heavy
-// ones first.
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_rescue(IndexView I, MapConfig C, ReadRec* __restrict__ rec,
-                                                                 Arenas A, Counters* ctr) {
-    __shared__ __align__(16) uint32_t s_hrs[kWarpsPerBlock][kRescueSmemHits];
-    __shared__ __align__(16) uint32_t s_hpk[kWarpsPerBlock][kRescueSmemHits];
-    __shared__ uint8_t s_tb[kWarpsPerBlock][kRescueSmemHits];
-    __shared__ uint32_t s_item;
-    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
+// find_nams_rescue for the reads on the rescue list, heavy ones (at the list's heavy end)
+// first, a warp a read; with C.rescue_block_hits set, and few heavy reads for the grid or
+// few rescued reads for its warps, the heavy ones a block each, which ends a read in a third
+// of a warp's time but takes eight warps for it: 22900 rescued reads of 2M, 1742 of them
+// heavy, took 1.95 ms with blocks and 1.05 with warps (1.54 before this merge); the 10 of
+// 1000 reads 0.09 ms with blocks (0.23 before).
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, 3)
+    k_rescue(IndexView I, MapConfig C, ReadRec* __restrict__ rec, Arenas A, Counters* ctr) {
+    extern __shared__ __align__(16) uint8_t s_dyn[];
+    RescueShared& S = *reinterpret_cast<RescueShared*>(s_dyn);
+    static_assert(sizeof(S.buf[0]) >= 7168 && kWarpSortMax <= 256, "the sort entries fit a warp's buffer");
     const uint32_t n_heavy = *(volatile unsigned int*)&ctr->n_rescue_heavy;
     const uint32_t n_rescue = n_heavy + *(volatile unsigned int*)&ctr->n_rescue;
     uint32_t first = 0;
-    if (C.rescue_block_hits && n_rescue <= warp_count()) {
+    if (C.rescue_block_hits && (n_rescue <= warp_count() || n_heavy <= 3 * gridDim.x)) {
         for (;;) {
-            if (threadIdx.x == 0) s_item = atomicAdd(&ctr->rescue_block_next, 1u);
+            if (threadIdx.x == 0) S.item = atomicAdd(&ctr->rescue_block_next, 1u);
             __syncthreads();
-            const uint32_t t = s_item;
+            const uint32_t t = S.item;
             __syncthreads();
             if (t >= n_heavy) break;
-            rescue_read_block(I, C, rec, A, ctr, t, &s_hrs[0][0], &s_hpk[0][0], &s_tb[0][0]);
+            rescue_read<true>(I, C, rec, A, ctr, t, A.rescue_list[A.rescue_cap - 1 - t], S);
         }
         first = n_heavy;
     }
     // resident warps take reads in list order, heavy ones first
     for (;;) {
-        uint32_t t = 0;
-        if (lane == 0) t = atomicAdd(&ctr->rescue_next, 1u);
-        t = __shfl_sync(0xFFFFFFFFu, t, 0) + first;
+        const uint32_t t = warp_next(&ctr->rescue_next) + first;
         if (t >= n_rescue) break;
-        const long long t_start = clock64();
-        const uint32_t r = t < n_heavy ? A.rescue_list[A.rescue_cap - 1 - t] : A.rescue_list[t - n_heavy];
-        ReadRec& R = rec[r];
-        struct CycleNote {
-            const Arenas& A;
-            uint32_t t;
-            long long t0;
-            __device__ ~CycleNote() {
-                if (A.rescue_cycles && lane_id() == 0) A.rescue_cycles[8ull * t] = (uint64_t)(clock64() - t0);
+        rescue_read<false>(I, C, rec, A, ctr, t,
+                           t < n_heavy ? A.rescue_list[A.rescue_cap - 1 - t] : A.rescue_list[t - n_heavy], S);
+    }
+}
+
+// ---- sort of rescued reads with packed keys --------------------------------------------
+//
+// In the score order (score descending, orientation, reference id, query start, query end,
+// reference start, ...) the NAMs of one read need few bits a field, and they are created in
+// (orientation, query start, reference start) order, so their number stands for what comes
+// after the query end: score | orientation | reference | query start | query end | number
+// makes one 64-bit word without ties.  Up to 8192 such words sort in a block's registers
+// (bitonic; partners in other lanes by shuffles, in other warps through shared memory),
+// with nothing but the word to move; a read whose fields do not fit, or whose NAMs are not
+// in that order, goes to the sorts below.  Those move a key word and an index through
+// shared memory at every stage and read two more words on ties: 0.96 + 1.29 ms for the
+// 5629 reads of a batch of 2M, against 0.47.
+constexpr int kPackThreads = 512;
+constexpr uint32_t kPackMax = 16 * kPackThreads;   // NAMs
+
+// Bitonic stages (k, j), j = j0, j0 / 2, .., 1, of the words x of a block, word
+// t * kKeys + r at x[r] of thread t.
+template <int kKeys>
+__device__ __forceinline__ void pack_merge(uint64_t (&x)[kKeys], uint32_t k, uint32_t j0, uint64_t* sm) {
+    const uint32_t t = threadIdx.x;
+    const bool asc = ((t * kKeys) & k) == 0;   // (k >= kKeys: alike for the thread's words)
+    for (uint32_t j = j0; j >= kKeys; j >>= 1) {
+        const uint32_t m = j / kKeys;   // partner thread t ^ m
+        const bool keep_min = ((t & m) == 0) == asc;
+        if (m < 32) {
+#pragma unroll
+            for (int r = 0; r < kKeys; ++r) {
+                const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, x[r], m);
+                if ((x[r] > y) == keep_min) x[r] = y;
             }
-            __device__ void phase(int k, long long since) const {
-                if (A.rescue_cycles && lane_id() == 0) A.rescue_cycles[8ull * t + k] = (uint64_t)(clock64() - since);
+        } else {
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < kKeys; ++r) sm[r * kPackThreads + t] = x[r];
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < kKeys; ++r) {
+                const uint64_t y = sm[r * kPackThreads + (t ^ m)];
+                if ((x[r] > y) == keep_min) x[r] = y;
             }
-            __device__ void set(int k, uint64_t v) const {
-                if (A.rescue_cycles && lane_id() == 0) A.rescue_cycles[8ull * t + k] = v;
+        }
+    }
+    if (j0 >= kKeys) j0 = kKeys / 2;
+#pragma unroll
+    for (int j = kKeys / 2; j > 0; j >>= 1) {
+        if ((uint32_t)j > j0) continue;
+#pragma unroll
+        for (int r = 0; r < kKeys; ++r) {
+            if (r & j) continue;
+            const bool up = ((t * kKeys + r) & k) == 0;
+            const uint64_t u = x[r], v = x[r | j];
+            if ((u > v) == up) {
+                x[r] = v;
+                x[r | j] = u;
             }
-        } note{A, t, t_start};
-        const uint32_t nqd[2] = {R.nq, R.nq2 - R.nq};
-        const Query* Qd[2] = {A.q + R.q_off, A.q + R.q_off + R.nq};
-        const uint64_t* Pd[2] = {A.q_pos + R.q_off, A.q_pos + R.q_off + R.nq};
-        const uint32_t nqm = nqd[0] > nqd[1] ? nqd[0] : nqd[1];
-        const uint32_t Pq = next_pow2(nqm > 0 ? nqm : 1);
-        const uint64_t b1 = 4ull * 8 * Pq + 64;
-        uint8_t* sc1 = warp_scratch(A, ctr, 0, b1);
-        if (!sc1) {
-            warp_fail(R, ctr, kStatusScratchOverflow);
-            continue;
         }
-        uint64_t* buf = reinterpret_cast<uint64_t*>(sc1);
-        const RescuePlan plan = rescue_prepare(I, C, Qd, Pd, nqd, Pq, buf);
-        note.phase(1, t_start);
-        note.set(4, plan.bound);
-        note.set(7, plan.maxrun);
-        if (plan.bound == 0) {
-            if (lane == 0) R.n_nams = 0;
-            continue;
+    }
+}
+
+// Sorts one job of at most kKeys * kPackThreads NAMs; false when its keys cannot be packed.
+template <int kKeys>
+__device__ __noinline__ bool pack_sort(const SortJob& job, ReadRec& R, const Arenas& A, Counters* ctr, uint64_t* sm) {
+    __shared__ uint32_t s_max[3];   // score, reference id, query end
+    __shared__ uint64_t s_noff;
+    const uint32_t t = threadIdx.x, n = job.n;
+    const NamState* closed = job.closed;
+    if (t < 3) s_max[t] = 0;
+    __syncthreads();
+    uint32_t ms = 0, mr = 0, mq = 0;
+    bool ok = true;
+    for (uint32_t i = t; i < n; i += kPackThreads) {
+        const NamState a = closed[i];
+        ms = max(ms, (uint32_t)nam_score_int(a));
+        mr = max(mr, a.ref_rc & 0x7FFFFFFFu);
+        mq = max(mq, (uint32_t)a.qe);
+        if (i + 1 < n) {   // created in (orientation, query start, reference start) order
+            const NamState b = closed[i + 1];
+            const uint32_t oa = a.ref_rc >> 31, ob = b.ref_rc >> 31;
+            ok &= oa != ob ? oa < ob : (a.qs != b.qs ? a.qs < b.qs : a.rs <= b.rs);
         }
-        const uint32_t H = (uint32_t)plan.bound;
-        const uint64_t P2 = next_pow2(H);
-        const bool big_run = plan.maxrun > kRescueSmemHits;
-        const uint64_t b2 = 64ull * H + 32ull * P2 + (big_run ? 9ull * plan.maxrun + 64 : 0) + 256;
-        uint8_t* sc2 = warp_scratch(A, ctr, (b1 + 255) & ~255ull, b2);
-        if (!sc2) {
-            warp_fail(R, ctr, kStatusScratchOverflow);
-            continue;
+    }
+    ms = __reduce_max_sync(0xFFFFFFFFu, ms);
+    mr = __reduce_max_sync(0xFFFFFFFFu, mr);
+    mq = __reduce_max_sync(0xFFFFFFFFu, mq);
+    if (lane_id() == 0) {
+        atomicMax(&s_max[0], ms);
+        atomicMax(&s_max[1], mr);
+        atomicMax(&s_max[2], mq);
+    }
+    if (!__syncthreads_and(ok)) return false;
+    ms = s_max[0];
+    mr = s_max[1];
+    mq = s_max[2];
+    const uint32_t br = 32 - __clz(mr), bq = 32 - __clz(mq), bn = 32 - __clz(n - 1);
+    if (32 - __clz(ms) + 1 + br + 2 * bq + bn > 63) return false;   // (padding is all ones)
+    uint64_t x[kKeys];
+#pragma unroll
+    for (int r = 0; r < kKeys; ++r) {
+        const uint32_t i = r * kPackThreads + t;
+        x[r] = ~0ULL;
+        if (i < n) {
+            const NamState a = closed[i];
+            uint64_t v = ((uint64_t)(ms - (uint32_t)nam_score_int(a)) << 1) | (a.ref_rc >> 31);
+            v = (v << br) | (a.ref_rc & 0x7FFFFFFFu);
+            v = (v << bq) | (uint32_t)a.qs;
+            v = (v << bq) | (uint32_t)a.qe;
+            x[r] = (v << bn) | i;
         }
-        NamLists L;
-        L.open = reinterpret_cast<NamState*>(sc2);
-        L.closed = L.open + H;
-        NamKey* keys = reinterpret_cast<NamKey*>(L.closed + H);
-        uint32_t* hrs = s_hrs[w];
-        uint32_t* hpk = s_hpk[w];
-        uint8_t* tb = s_tb[w];
-        if (big_run) {
-            hrs = reinterpret_cast<uint32_t*>(keys + P2);
-            hpk = hrs + plan.maxrun;
-            tb = reinterpret_cast<uint8_t*>(hpk + plan.maxrun);
+    }
+    for (uint32_t k = 2; k <= kKeys * kPackThreads; k <<= 1) pack_merge<kKeys>(x, k, k >> 1, sm);
+    if (t == 0) {
+        const uint64_t noff = atomicAdd(&ctr->nam_used, (unsigned long long)n);
+        if (noff + n > A.nam_cap) {
+            R.flags |= kReadFailed;
+            R.n_nams = 0;   // the rescue kernel set the count ahead of the sort
+            atomicOr(&ctr->status, kStatusNamOverflow);
+            s_noff = ~0ULL;
+        } else {
+            R.nam_off = noff;
+            s_noff = noff;
         }
-        L.n_open = L.n_closed = 0;
-        L.cap = H;
-        const long long t_merge = clock64();
-        const uint64_t walk = rescue_merge(I, Qd, Pd, plan, buf, Pq, L, hrs, hpk, tb);
-        note.phase(2, t_merge);
-        note.set(6, walk);
-        note.set(5, L.n_closed);
-        if (rescue_sort_job(A, ctr, R, L, keys, r, t)) continue;
-        const long long t_fin = clock64();
-        static_assert(kWarpSortMax <= 256 && kRescueSmemHits >= 1024, "the sort entries fit the hit buffers");
-        warp_finish_nams(C, L, s_hrs[w], s_hpk[w], R, A, ctr);
-        note.phase(3, t_fin);
-        __syncwarp();
+    }
+    // the order to shared memory, so that consecutive threads write consecutive NAMs
+    __syncthreads();
+    uint32_t* order = reinterpret_cast<uint32_t*>(sm);
+#pragma unroll
+    for (int r = 0; r < kKeys; ++r) order[t * kKeys + r] = (uint32_t)x[r] & ((1u << bn) - 1);
+    __syncthreads();
+    const uint64_t noff = s_noff;
+    if (noff != ~0ULL)
+        for (uint32_t i = t; i < n; i += kPackThreads) A.nams[noff + i] = closed[order[i]];
+    return true;
+}
+
+// The packed sort of the rescued reads with more than kWarpSortMax NAMs, the ones with more
+// than kSortTile first; jobs that it passes on go to the slow list (those above kSortTile
+// from its back).
+__global__ void __launch_bounds__(kPackThreads, 2)
+    k_sort_packed(MapConfig C, ReadRec* __restrict__ rec, Arenas A, Counters* ctr) {
+    extern __shared__ __align__(16) uint8_t s_dyn[];   // kPackMax words
+    uint64_t* sm = reinterpret_cast<uint64_t*>(s_dyn);
+    __shared__ uint32_t s_next;
+    const uint32_t n_huge = *(volatile unsigned int*)&ctr->n_huge;
+    const uint32_t n_jobs = n_huge + *(volatile unsigned int*)&ctr->n_heavy;
+    for (;;) {
+        if (threadIdx.x == 0) s_next = atomicAdd(&ctr->sort_next, 1u);
+        __syncthreads();
+        const uint32_t h = s_next;
+        if (h >= n_jobs) break;
+        const long long t0 = clock64();
+        const uint32_t at = h < n_huge ? A.jobs_cap - 1 - h : h - n_huge;
+        const SortJob job = A.sort_jobs[at];
+        ReadRec& R = rec[job.read];
+        bool done = false;
+        if (C.sort_mode == GBSA_SORT_SCORE && job.n <= kPackMax) {
+            if (job.n <= kPackThreads) done = pack_sort<1>(job, R, A, ctr, sm);
+            else if (job.n <= 2 * kPackThreads) done = pack_sort<2>(job, R, A, ctr, sm);
+            else if (job.n <= 4 * kPackThreads) done = pack_sort<4>(job, R, A, ctr, sm);
+            else if (job.n <= 8 * kPackThreads) done = pack_sort<8>(job, R, A, ctr, sm);
+            else done = pack_sort<16>(job, R, A, ctr, sm);
+        }
+        if (threadIdx.x == 0) {
+            if (!done) {
+                if (h < n_huge) A.slow_list[A.rescue_cap - 1 - atomicAdd(&ctr->n_slow_huge, 1u)] = at;
+                else A.slow_list[atomicAdd(&ctr->n_slow, 1u)] = at;
+            } else if (A.rescue_cycles) {
+                A.rescue_cycles[8ull * job.note + 3] = (uint64_t)(clock64() - t0);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -1607,10 +1905,9 @@ __device__ void idx_tile_sort(IdxSortTile tile, uint32_t P) {
     }
 }
 
-// Sorts the NAMs of the rescued reads with kWarpSortMax < NAMs <= kSortTile
-// (typically reads inside short tandem repeats): one block per read, bitonic sort in
-// a shared-memory tile, then the read's NAMs are written to the NAM arena in order.
-// The jobs are at the front of the job list.
+// Sorts the NAMs of the rescued reads with kWarpSortMax < NAMs <= kSortTile that the packed
+// sort passed on: one block per read, bitonic sort in a shared-memory tile, then the
+// read's NAMs are written to the NAM arena in order.
 template <int kThreads, uint32_t kTile>
 __global__ void __launch_bounds__(kThreads) k_sort_jobs(MapConfig C, ReadRec* __restrict__ rec, Arenas A,
                                                          Counters* ctr) {
@@ -1626,10 +1923,10 @@ __global__ void __launch_bounds__(kThreads) k_sort_jobs(MapConfig C, ReadRec* __
     itile.k2 = tile.k2;
     itile.k3 = tile.k3;
     itile.ix = tile.idx;
-    const uint32_t n_jobs = *(volatile unsigned int*)&ctr->n_heavy;
+    const uint32_t n_jobs = *(volatile unsigned int*)&ctr->n_slow;
     for (uint32_t h = blockIdx.x; h < n_jobs; h += gridDim.x) {
         const long long t0 = clock64();
-        const SortJob job = A.sort_jobs[h];
+        const SortJob job = A.sort_jobs[A.slow_list[h]];
         ReadRec& R = rec[job.read];
         const NamState* closed = job.closed;
         const uint32_t NN = job.n;
@@ -1678,7 +1975,7 @@ __global__ void __launch_bounds__(kThreads) k_sort_jobs(MapConfig C, ReadRec* __
     }
 }
 
-// ---- cluster sort of the rescued reads with more than kSortTile NAMs ------------------
+// ---- cluster sort of the other rescued reads with more than kSortTile NAMs -------------
 //
 // A cluster of kClusterCtas CTAs sorts one read's keys: each CTA holds T = P /
 // kClusterCtas of the P (next power of two) keys in its shared-memory tile, so up to
@@ -1687,8 +1984,6 @@ __global__ void __launch_bounds__(kThreads) k_sort_jobs(MapConfig C, ReadRec* __
 // few with larger distances compare and swap across the CTAs' tiles through
 // distributed shared memory (cluster barrier).  Each CTA needs only kSortTile keys of
 // shared memory, so the clusters run beside the NAM kernels of the other stream.
-constexpr int kClusterCtas = 8;
-
 // Tie break of the index-moving cluster sort: NAM indices ib and ia whose first key
 // words are equal, by their second and third words (fixed, NAM e in CTA e / T at e % T)
 // and then the index.
@@ -1714,11 +2009,11 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(256)
     tile.k2 = tile.k1 + kSortTile;
     tile.k3 = tile.k2 + kSortTile;
     tile.idx = reinterpret_cast<uint32_t*>(tile.k3 + kSortTile);
-    const uint32_t n_jobs = *(volatile unsigned int*)&ctr->n_huge;
+    const uint32_t n_jobs = *(volatile unsigned int*)&ctr->n_slow_huge;
     const uint32_t n_clusters = gridDim.x / kClusterCtas;
     for (uint32_t h = blockIdx.x / kClusterCtas; h < n_jobs; h += n_clusters) {
         const long long t0 = clock64();
-        const SortJob job = A.sort_jobs[A.jobs_cap - 1 - h];
+        const SortJob job = A.sort_jobs[A.slow_list[A.rescue_cap - 1 - h]];
         const NamState* closed = job.closed;
         const uint32_t NN = job.n;
         const uint32_t P = next_pow2(NN);
@@ -2071,6 +2366,7 @@ void nam_phase_carveout() {
     for (const void* f : fs)
         GBSA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
+    GBSA_CUDA(cudaFuncSetAttribute(k_rescue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RescueShared)));
     done[dev] = 1;
 }
 
@@ -2104,7 +2400,7 @@ void launch_rescue(const IndexView& I, const MapConfig& C, uint32_t n_reads, Rea
     // persistent, kRescueBlocksPerSm per SM (at most one scratch slot per warp)
     const unsigned blocks =
         std::min<unsigned>(warp_grid(n_reads, kWarpsPerBlock), (unsigned)device_sm_count() * kRescueBlocksPerSm);
-    launch_probe(k_rescue, blocks, 32 * kWarpsPerBlock, 0, st, C, I, C, rec, A, ctr);
+    launch_probe(k_rescue, blocks, 32 * kWarpsPerBlock, sizeof(RescueShared), st, C, I, C, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 
@@ -2124,7 +2420,14 @@ static void sort_smem_limit() {
     for (const void* f : {(const void*)k_sort_jobs<kSortThreads, kSortTile>,
                           (const void*)k_sort_jobs<2 * kSortThreads, kSortTile>, (const void*)k_sort_jobs_cluster})
         GBSA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSortSmem));
+    GBSA_CUDA(cudaFuncSetAttribute(k_sort_packed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(8 * kPackMax)));
     done[dev] = 1;
+}
+
+void launch_sort_packed(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
+    sort_smem_limit();
+    k_sort_packed<<<(unsigned)device_sm_count() * 2, kPackThreads, 8 * kPackMax, st>>>(C, rec, A, ctr);
+    GBSA_LAUNCHED();
 }
 
 void launch_sort_jobs(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {

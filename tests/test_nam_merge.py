@@ -92,3 +92,62 @@ def test_merge_at_group_and_slot_bounds(merged, mode):
     for i in (0, len(HITS) + 5, 2 * len(HITS) - 1, 3 * len(HITS) - 2, 4 * len(HITS) - 1):
         one, _, _ = m.find_nams(q[int(offs[i]): int(offs[i + 1])], offs[i: i + 2] - offs[i])
         assert (one == nams[int(noff[i]): int(noff[i + 1])]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [abi.GBSA_SORT_SCORE, abi.GBSA_SORT_REF_MATE2])
+@pytest.mark.parametrize("block", [0, 1])
+def test_rescue_merge_and_sort_bounds(mode, block):
+    """find_nams_rescue of reads whose NAM counts lie around the sorts' sizes (a warp's, a
+    block's registers, a cluster's tiles, memory), with a warp and with a block a read: NAMs
+    that join hits of many queries, NAMs that compete for hits, reference ids and query ends
+    too wide for one key word, and two queries with the same start."""
+    rng = np.random.default_rng(23)
+    p = native.params_from_read_length(150)
+    rs, reads = [(1, 0, 0)], []
+    counts = (3, 31, 255, 256, 257, 511, 512, 513, 1000, 1025, 2047, 2048, 2049, 4096, 4097, 8192, 8193, 16384, 16500)
+
+    def read(n, near, refs, wide, same_start):
+        out, left, qs = [], n, 0
+        while left:
+            m = int(min(left, rng.integers(1, 1001)))
+            left -= m
+            span = int(rng.integers(p.k, p.k + 40))
+            h = int(rng.integers(1 << 20, (1 << 62) - 1))
+            pos = (np.sort(rng.choice(200_000_000, m, replace=False)) if not near
+                   else 5000 + qs + near * np.arange(m) + rng.integers(0, 2))
+            ref = rng.integers(0, refs, m)
+            for x, r, s in zip(pos, ref, rng.integers(0, 3, m) + span):
+                rs.append((h, int(x), (int(r) << 8) | (int(s) - p.k)))
+            out.append((h, qs, qs + span, int(rng.integers(2))))
+            qs += 0 if same_start and len(out) == 2 else int(rng.integers(1, 200 if wide else 9))
+        reads.append(out)
+
+    for n in counts:
+        read(n, 0, 3, False, False)
+    for near in (1, 2, 3, 6):
+        for refs in (1, 2, 20):
+            read(int(rng.integers(2000, 9000)), near, refs, False, False)
+            read(int(rng.integers(40, 700)), near, refs, False, False)
+    read(3000, 0, 1 << 24, True, False)
+    read(700, 0, 1 << 24, True, False)
+    read(3000, 2, 2, False, True)
+    ent = np.sort(np.array(rs, abi.REF_RANDSTROBE), order=["hash", "position", "packed"])
+    bits = 10
+    starts = np.searchsorted(ent["hash"] >> np.uint64(64 - bits), np.arange((1 << bits) + 1, dtype=np.uint64)).astype(
+        np.uint64)
+    q = np.zeros(sum(len(r) for r in reads), abi.QUERY_RANDSTROBE)
+    flat = [x for r in reads for x in r]
+    for i, f in enumerate(("hash", "start", "end", "is_reverse")):
+        q[f] = [x[i] for x in flat]
+    offs = np.concatenate([[0], np.cumsum([len(r) for r in reads])]).astype(np.uint64)
+    o = oracle_py.Index.load(p, ent, starts, bits, 100)
+    m = native.Mapper(native.Index.load(p, ent, starts, bits, 100), abi.map_options(sort_mode=mode), max_reads=256)
+    m.set_rescue_block(block)
+    nams, noff, _ = m.find_nams(q, offs, rescue=True, rescue_cutoff=1500)
+    for i in range(len(reads)):
+        want = oracle_py.sort_nams(o.find_nams_rescue(q[int(offs[i]): int(offs[i + 1])], 1500), mode)
+        got = nams[int(noff[i]): int(noff[i + 1])]
+        assert len(got) == len(want), i
+        for f in abi.NAM_COMPARED:
+            assert (got[f] == want[f]).all(), (i, f)
