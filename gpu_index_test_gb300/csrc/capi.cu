@@ -424,7 +424,7 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
     launch_bucket_reads(n, m.rec.as<ReadRec>(), A, ctr, st, desc);
     launch_nams(C, n, m.rec.as<ReadRec>(), A, ctr, st);
     mark(4);
-    launch_nams_warp(C, n, m.rec.as<ReadRec>(), A, ctr, st);
+    launch_nams_warp(C, I.k, n, m.rec.as<ReadRec>(), A, ctr, st);
     mark(5);
     // Every read's NAM count is known once the rescue kernel has ended (the sorts after
     // it only order NAMs): per-read counts → offsets, and the records of the reads that

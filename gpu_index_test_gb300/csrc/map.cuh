@@ -176,7 +176,7 @@ void launch_lookup(const IndexView& I, const MapConfig& C, uint32_t n, ReadRec* 
 void launch_nams(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 void launch_bucket_reads(uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st,
                          const BatchDesc* desc = nullptr);
-void launch_nams_warp(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
+void launch_nams_warp(const MapConfig& C, int k, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 void launch_rescue(const IndexView& I, const MapConfig& C, uint32_t n_reads, ReadRec* rec, Arenas A, Counters* ctr,
                    cudaStream_t st);
 void launch_sort_packed(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);

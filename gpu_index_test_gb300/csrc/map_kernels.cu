@@ -817,9 +817,8 @@ __global__ void __launch_bounds__(32 * kGroupWarps, kGroupBlocksPerSm)
     }
 }
 
-// Open NAM list of one warp in struct-of-arrays form (field f of NAM o at
-// b[f * stride + o]), so that 32 lanes reading one field of 32 NAMs touch 32
-// consecutive words.
+// A NAM list in struct-of-arrays form (field f of NAM o at b[f * stride + o]), so that 32
+// lanes reading one field of 32 NAMs touch 32 consecutive words.
 struct OpenSoA {
     int32_t* b;
     uint32_t stride;
@@ -847,239 +846,6 @@ struct OpenSoA {
         b[7 * stride + o] = (int32_t)n.ref_rc;
     }
 };
-
-// Moves the open NAMs with query_end < qs (all of them when qs == INT_MAX) to the
-// closed list, keeping the order of both lists.
-__device__ __forceinline__ void soa_close_passed(const OpenSoA& O, uint32_t& n_open, NamState* closed,
-                                                 uint32_t& n_closed, int qs) {
-    const uint32_t lane = lane_id();
-    if (qs != 0x7FFFFFFF) {
-        bool any = false;
-        for (uint32_t base = 0; base < n_open && !any; base += 32) {
-            const uint32_t o = base + lane;
-            any = __any_sync(0xFFFFFFFFu, o < n_open && O.b[O.stride + o] < qs);
-        }
-        if (!any) return;
-    }
-    uint32_t keep = 0, done = 0;
-    for (uint32_t base = 0; base < n_open; base += 32) {
-        const uint32_t o = base + lane;
-        const bool valid = o < n_open;
-        NamState n;
-        if (valid) n = O.get(o);
-        const bool stay = valid && n.qe >= qs;
-        const uint32_t ms = __ballot_sync(0xFFFFFFFFu, stay);
-        const uint32_t mc = __ballot_sync(0xFFFFFFFFu, valid && !stay);
-        __syncwarp();
-        if (stay) O.put(keep + __popc(ms & lanemask_lt()), n);
-        else if (valid) closed[n_closed + done + __popc(mc & lanemask_lt())] = n;
-        keep += __popc(ms);
-        done += __popc(mc);
-        __syncwarp();
-    }
-    n_open = keep;
-    n_closed += done;
-}
-
-// Hit-major merge of nh <= 32 hits of one query randstrobe, held one per lane in
-// registers (lane j holds hit j, in ref_start order), against the NAMs [0, nn) that
-// were open when the query started: each hit joins the first of them in creation
-// order that accepts it, else opens a new NAM.  Returns false (with the list
-// unchanged from the failing hit on) when a new NAM would not fit in cap.
-__device__ __forceinline__ bool soa_merge_hits(const OpenSoA& O, uint32_t nn, uint32_t& n_open, uint32_t cap,
-                                               const HitRec& xl, uint32_t nh) {
-    const uint32_t lane = lane_id();
-    const int32_t* fqe = O.f(1);
-    const int32_t* fqprev = O.f(2);
-    const int32_t* fre = O.f(4);
-    const int32_t* frprev = O.f(5);
-    const int32_t* fref = O.f(7);
-    for (uint32_t j = 0; j < nh; ++j) {
-        HitRec x;
-        x.ref_rc = __shfl_sync(0xFFFFFFFFu, xl.ref_rc, j);
-        x.qs = __shfl_sync(0xFFFFFFFFu, xl.qs, j);
-        x.qe = __shfl_sync(0xFFFFFFFFu, xl.qe, j);
-        x.rs = __shfl_sync(0xFFFFFFFFu, xl.rs, j);
-        x.re = __shfl_sync(0xFFFFFFFFu, xl.re, j);
-        bool found = false;
-        for (uint32_t base = 0; base < nn; base += 32) {
-            const uint32_t o = base + lane;
-            bool ok = false;
-            int qe = 0, re = 0;
-            if (o < nn) {
-                qe = fqe[o];
-                re = fre[o];
-                ok = (uint32_t)fref[o] == x.ref_rc && fqprev[o] < x.qs && x.qs <= qe && frprev[o] < x.rs &&
-                     x.rs <= re && ((x.qe > qe && x.re > re) || (x.qe <= qe && x.re <= re));
-            }
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
-            if (m) {
-                if (lane == (uint32_t)(__ffs(m) - 1)) {   // the first accepting NAM takes the hit
-                    if (x.qe > qe && x.re > re) {
-                        O.f(1)[o] = x.qe;
-                        O.f(4)[o] = x.re;
-                    }
-                    O.f(2)[o] = x.qs;
-                    O.f(5)[o] = x.rs;
-                    O.f(6)[o] += 1;
-                }
-                found = true;
-                break;
-            }
-        }
-        if (!found) {
-            if (n_open == cap) return false;
-            if (lane == 0) O.put(n_open, nam_from_hit(x));
-            ++n_open;
-        }
-        __syncwarp();
-    }
-    return true;
-}
-
-
-// find_nams merge of one read's hits (in (orientation, query_start, position)
-// order) with the open list O (capacity cap); closed NAMs are appended to closed.
-// Each query randstrobe's hits are loaded 32 at a time, one per lane, and the next
-// chunk is fetched while the current one merges.  Returns false when the open list
-// outgrew cap.
-__device__ __forceinline__ bool warp_find_nams(const HitPacked* __restrict__ hits, uint32_t H, const OpenSoA& O,
-                                               uint32_t cap, NamState* closed, uint32_t& n_closed) {
-    const uint32_t lane = lane_id();
-    uint32_t n_open = 0, cur_dir = 0;
-    n_closed = 0;
-    uint32_t i = 0;
-    HitRec xl = load_hit(hits, lane, H);
-    while (i < H) {
-        const uint32_t dir = __shfl_sync(0xFFFFFFFFu, xl.ref_rc, 0) >> 31;
-        const int qs = __shfl_sync(0xFFFFFFFFu, xl.qs, 0);
-        if (dir != cur_dir) {   // the other orientation's NAMs can take no more hits
-            soa_close_passed(O, n_open, closed, n_closed, 0x7FFFFFFF);
-            cur_dir = dir;
-        }
-        soa_close_passed(O, n_open, closed, n_closed, qs);
-        const uint32_t nn = n_open;   // NAMs made by this query cannot take its other hits
-        for (;;) {
-            const bool same = i + lane < H && (xl.ref_rc >> 31) == dir && xl.qs == qs;
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, same);
-            const uint32_t cnt = m == 0xFFFFFFFFu ? 32u : (uint32_t)(__ffs(~m) - 1);
-            const HitRec nx = load_hit(hits, i + cnt + lane, H);
-            if (!soa_merge_hits(O, nn, n_open, cap, xl, cnt)) return false;
-            i += cnt;
-            xl = nx;
-            if (cnt < 32) break;
-        }
-    }
-    soa_close_passed(O, n_open, closed, n_closed, 0x7FFFFFFF);
-    return true;
-}
-
-constexpr uint32_t kHeavyOpen = 256;   // open NAMs (and sort keys) a warp keeps in shared memory
-constexpr int kHeavyWarps = 4;
-constexpr int kHeavyBlocksPerSm = 4;   // 128 registers a thread
-
-// find_nams for the reads with more NAMs than k_nams_group's slots: a warp a read, in
-// registers again with 8 slots a lane; a read with more than 256 NAMs once more with its
-// open list in shared memory (in global scratch when it outgrows kHeavyOpen); closed NAMs
-// then go to the warp's global scratch, which is only written until the sort, and the
-// NAMs are sorted by key in shared memory (in scratch beyond kHeavyOpen NAMs) and gathered
-// to the NAM arena.
-__global__ void __launch_bounds__(32 * kHeavyWarps, kHeavyBlocksPerSm)
-    k_nams(MapConfig C, ReadRec* __restrict__ rec, Arenas A, Counters* ctr) {
-    __shared__ __align__(16) int32_t s_open[kHeavyWarps][8 * kHeavyOpen];
-    const uint32_t lane = lane_id(), w = threadIdx.x >> 5;
-    const uint32_t n_big = *(volatile unsigned int*)&ctr->n_big;
-    static_assert(sizeof(GroupShared<8>) <= sizeof(s_open[0]), "a merge's shared memory fits the open-list buffer");
-    GroupShared<8>& S = *reinterpret_cast<GroupShared<8>*>(s_open[w]);
-    for (uint32_t b = warp_next(&ctr->big_next); b < n_big; b = warp_next(&ctr->big_next)) {
-        const long long t0 = clock64();
-        if (group_merge<32, 8>(C, rec, A, ctr, A.big_list, b, n_big, S) == kNoRead) {
-            if (A.nam_cycles && lane == 0) {
-                uint64_t* note = A.nam_cycles + 4ull * b;   // cycles, hits, NAMs, merge cycles
-                note[0] = note[3] = (uint64_t)(clock64() - t0);
-                note[1] = rec[A.big_list[b]].n_hits;
-                note[2] = rec[A.big_list[b]].n_nams;
-            }
-            continue;
-        }
-        __syncwarp();
-        const uint32_t r = A.big_list[b];
-        ReadRec& R = rec[r];
-        if (R.flags & (kReadFailed | kReadRescue)) continue;
-        const uint32_t H = R.n_hits;
-        if (H == 0) continue;
-        const HitPacked* hits = A.hits + R.hit_off;
-        const uint32_t P2 = next_pow2(H);
-        const bool big = H > kHeavyOpen;
-        uint8_t* sc = warp_scratch(A, ctr, 0, 32ull * H + (big ? 32ull * P2 : 0) + 64);
-        if (!sc) {
-            warp_fail(R, ctr, kStatusScratchOverflow);
-            continue;
-        }
-        NamState* closed = reinterpret_cast<NamState*>(sc);
-        uint32_t NN = 0;
-        OpenSoA O{s_open[w], kHeavyOpen};
-        if (!warp_find_nams(hits, H, O, kHeavyOpen, closed, NN)) {
-            // the open list outgrew shared memory: again with it in scratch
-            __syncwarp();
-            const OpenSoA G{reinterpret_cast<int32_t*>(closed + H), P2};
-            warp_find_nams(hits, H, G, H, closed, NN);
-        }
-        const long long t_merge = clock64();
-        __syncwarp();
-        // sort: up to kHeavyOpen NAMs in the warp's shared open-list buffer (now free),
-        // moving only the first key word and the NAM index; more in global scratch
-        const bool small = NN <= kHeavyOpen;
-        uint32_t* order = nullptr;   // sorted NAM indices
-        NamKey* keys = reinterpret_cast<NamKey*>(closed + H);
-        if (small) {
-            static_assert(kHeavyOpen <= 256, "the sort entries fit the open-list buffer");
-            int32_t* so = s_open[w];
-            uint64_t* k1 = reinterpret_cast<uint64_t*>(so);         // 2 KB
-            uint32_t* ix = reinterpret_cast<uint32_t*>(so + 512);   // 1 KB
-            uint64_t* k2 = reinterpret_cast<uint64_t*>(so + 768);   // 2 KB
-            uint64_t* k3 = k2 + 256;                                // 2 KB
-            const uint32_t P = next_pow2(NN);
-            for (uint32_t t = lane; t < P; t += 32) {
-                NamKey k;
-                if (t < NN) {
-                    k = nam_key(closed[t], t, C.sort_mode);
-                } else {   // padding sorts last (a NAM's first key word is never all ones)
-                    k.k1 = k.k2 = k.k3 = ~0ULL;
-                }
-                k1[t] = k.k1;
-                ix[t] = t;
-                k2[t] = k.k2;
-                k3[t] = k.k3;
-            }
-            __syncwarp();
-            warp_sort_idx(k1, ix, k2, k3, P);
-            order = ix;
-        } else {
-            for (uint32_t t = lane; t < NN; t += 32) keys[t] = nam_key(closed[t], t, C.sort_mode);
-            __syncwarp();
-            warp_sort_keys(keys, NN);
-        }
-        const uint64_t noff = warp_bump(&ctr->nam_used, NN);
-        if (noff + NN > A.nam_cap) {
-            warp_fail(R, ctr, kStatusNamOverflow);
-            continue;
-        }
-        for (uint32_t t = lane; t < NN; t += 32) A.nams[noff + t] = closed[small ? order[t] : keys[t].idx];
-        if (lane == 0) {
-            R.nam_off = noff;
-            R.n_nams = NN;
-            if (A.nam_cycles) {
-                uint64_t* note = A.nam_cycles + 4ull * b;   // cycles, hits, NAMs, merge cycles
-                note[0] = (uint64_t)(clock64() - t0);
-                note[1] = H;
-                note[2] = NN;
-                note[3] = (uint64_t)(t_merge - t0);
-            }
-        }
-        __syncwarp();
-    }
-}
 
 // Phase 1 of find_nams_rescue for one read (warp): RescueHit{position, count, qs,
 // qe} of every found query of each orientation, sorted by (count, query_start) —
@@ -1267,44 +1033,168 @@ __device__ __forceinline__ uint32_t block_walk_run(const IndexView& I, int qs, i
     return n;   // (the caller synchronises before the hits are read or S is written again)
 }
 
+// Merges one query's hits into the NAMs [lo, n) of its orientation d in O (struct of
+// arrays, in creation order) and returns the new number of NAMs: hits h of nh (positions
+// hrs, packed words hpk as in the index, sorted by position, all from query_start qs to
+// query_end qe, of spans min_span to max_span).  claim: kFree for every hit, gone: their bits
+// 0; the team (kBlock: the block, else the warp) has synchronised since they were written,
+// and has again on return.  cnt: a word a warp (kBlock).
+//
+// Which hit joins which NAM.  NAM-major (merge_hits_into_nams_fast, step2/nam.cu:94-343):
+// for each open NAM in creation order, the first hit that it accepts and that no NAM before
+// it took.  Hit-major (merge_hits_into_nams, step2/nam.cu:347-513): for each hit in order,
+// the first NAM in creation order that accepts it (a NAM takes one hit of a query, as the
+// next must start behind it).  Both give the one pairing that no NAM and hit would leave
+// for each other, NAMs preferring earlier hits and hits earlier NAMs, and that is what all
+// proposing at once comes to, each NAM to its first acceptable hit, a hit keeping the NAM
+// created first and a NAM that loses its hit going on to its next one, in whatever order
+// the proposals come.  The threads take a round of NAMs (one each) at a time: hits are
+// claimed with an atomic minimum of the NAM's number, and the thread that displaces a NAM
+// goes on with that one.  Hits claimed in earlier rounds are gone for good: a bit each lets
+// a NAM step over any number of them at once.  A hit lies where a NAM can accept it only
+// near the NAM's end, as its length is known to within the query's shortest and longest
+// hit.  A NAM that the query has passed (query_end < query_start) accepts nothing and stays
+// where it is, so nothing is moved between lists; then a thread a hit updates the NAM that
+// holds it, and unclaimed hits open NAMs in ref_start order.  (A warp resolving 32 NAMs
+// after the other, testing every hit between a NAM's last hit and its end and moving every
+// NAM of the list for every query, took 2.7M cycles for a read of 8550 hits, 1.5 ms of a
+// batch.)
+//
+// kPrev: queries may share their start, and a NAM takes one hit of all of them.
+constexpr uint32_t kFree = 0xFFFFFFFFu;
+
+template <bool kBlock, bool kPrev>
+__device__ __forceinline__ uint32_t merge_query(const OpenSoA& O, uint32_t lo, uint32_t n, int qs, int qe, uint32_t d,
+                                                int k, uint32_t nh, uint32_t min_span, uint32_t max_span,
+                                                const uint32_t* hrs, const uint32_t* hpk, uint32_t* claim,
+                                                uint32_t* gone, uint32_t* cnt) {
+    const uint32_t lane = lane_id(), w = kBlock ? threadIdx.x >> 5 : 0;
+    const uint32_t tid = kBlock ? threadIdx.x : lane, nt = kBlock ? blockDim.x : 32u;
+    const uint32_t nw = kBlock ? blockDim.x >> 5 : 1u;
+    auto sync = [] {
+        if (kBlock) __syncthreads();
+        else __syncwarp();
+    };
+    int32_t *fqe = O.f(1), *fqprev = O.f(2), *fre = O.f(4), *frprev = O.f(5), *fnh = O.f(6);
+    const uint32_t* fref = reinterpret_cast<const uint32_t*>(O.f(7));
+    const volatile uint32_t* held = claim;
+    // proposals, a round of nt NAMs at a time (the next round's fields on their way)
+    auto fields = [&](uint32_t i) {   // (a NAM the query has passed, or that took one of its hits: none)
+        if (i >= n || (kPrev && fqprev[i] >= qs)) return make_int4(-1, 0, 0, 0);
+        return make_int4(fqe[i], fre[i], frprev[i], (int)fref[i]);
+    };
+    int4 nx = fields(lo + tid);
+    for (uint32_t r0 = lo; r0 < n; r0 += nt) {
+        const int4 f = nx;
+        nx = fields(r0 + nt + tid);
+        uint32_t i = r0 + tid, fresh = kFree;
+        if (f.x >= qs) {
+            int nqe = f.x, nre = f.y, from = f.z + 1, last = nre;
+            uint32_t want = (uint32_t)f.w & 0x7FFFFFFFu;
+            // a hit is accepted when both its ends lie beyond the NAM's or neither does
+            if (qe > nqe) from = max(from, nre - (int)max_span + 1);
+            else last = nre - (int)min_span;
+            uint32_t at = 0, hi = nh;
+            while (at < hi) {   // hits are sorted by ref_start
+                const uint32_t mid = (at + hi) >> 1;
+                if ((int)hrs[mid] < from) at = mid + 1;
+                else hi = mid;
+            }
+            for (; at < nh; ++at) {
+                // the next hit that no NAM of an earlier round took
+                uint32_t free = ~gone[at >> 5] & (0xFFFFFFFFu << (at & 31));
+                if (!free) {
+                    at |= 31u;
+                    if (at + 1 >= nh || (int)hrs[at + 1] > last) break;
+                    continue;
+                }
+                at = (at & ~31u) + (uint32_t)__ffs(free) - 1;
+                if (at >= nh) break;
+                const int rs = (int)hrs[at];
+                if (rs > last) break;
+                const uint32_t pk = hpk[at];
+                const int re = rs + (int)(pk & 0xFF) + k;
+                if ((pk >> 8) != want || held[at] < i || (qe > nqe) != (re > nre)) continue;
+                const uint32_t old = atomicMin(&claim[at], i);
+                if (old < i) continue;
+                if (old == kFree) {
+                    fresh = at;
+                    break;
+                }
+                i = old;   // displaced: on with its next hit
+                nqe = fqe[i];
+                nre = fre[i];
+                last = qe > nqe ? nre : nre - (int)min_span;
+                want = fref[i] & 0x7FFFFFFFu;
+            }
+        }
+        if (r0 + nt >= n) break;   // the last round: its claims need no bits
+        sync();
+        if (fresh != kFree) atomicOr(&gone[fresh >> 5], 1u << (fresh & 31));
+        sync();
+    }
+    sync();
+    // hits to their NAMs; the others open NAMs in order
+    const uint32_t per = ((nh + nw - 1) / nw + 31) & ~31u;
+    const uint32_t h0 = min(w * per, nh), h1 = min(h0 + per, nh);
+    uint32_t mine = 0;
+    for (uint32_t b = h0; b < h1; b += 32)
+        mine += __popc(__ballot_sync(0xFFFFFFFFu, b + lane < h1 && held[b + lane] == kFree));
+    uint32_t to = n, opened = mine;
+    if constexpr (kBlock) {
+        if (lane == 0) cnt[w] = mine;
+        __syncthreads();
+        opened = 0;
+        for (uint32_t v = 0; v < nw; ++v) {
+            if (v < w) to += cnt[v];
+            opened += cnt[v];
+        }
+    }
+    for (uint32_t b = h0; b < h1; b += 32) {
+        const uint32_t h = b + lane;
+        const bool in = h < h1;
+        const uint32_t i = in ? held[h] : 0u;
+        const bool open = in && i == kFree;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, open);
+        if (in) {
+            const int rs = (int)hrs[h];
+            const uint32_t pk = hpk[h];
+            const int re = rs + (int)(pk & 0xFF) + k;
+            if (open) {
+                HitRec x;
+                x.ref_rc = (d << 31) | (pk >> 8);
+                x.qs = qs;
+                x.qe = qe;
+                x.rs = rs;
+                x.re = re;
+                O.put(to + __popc(m & lanemask_lt()), nam_from_hit(x));
+            } else {
+                if (qe > fqe[i] && re > fre[i]) {
+                    fqe[i] = qe;
+                    fre[i] = re;
+                }
+                fqprev[i] = qs;
+                frprev[i] = rs;
+                fnh[i] += 1;
+            }
+        }
+        to += __popc(m);
+    }
+    sync();
+    return n + opened;
+}
+
 // Phase 2 of find_nams_rescue: walks the runs of the taken rescue hits in (orientation,
-// query_start) order and merges them NAM-major into O (struct of arrays, in creation
-// order); returns the number of NAMs.  kBlock: by the block, else by the warp alone.
-//
-// NAM-major rule (merge_hits_into_nams_fast, step2/nam.cu:94-343): for each open NAM in
-// creation order, the first hit of the query that it accepts and that no NAM before it
-// took.  The threads take a round of NAMs (one each) at a time.  Within a round that is the
-// outcome of all its NAMs proposing at once, each to its first acceptable hit, a hit
-// keeping the NAM created first and a NAM that loses its hit going on to its next one, in
-// whatever order the proposals come: hits are claimed with an atomic minimum of the NAM's
-// number, and the thread that displaces a NAM goes on with that one.  Hits claimed in
-// earlier rounds are gone for good: a bit each lets a NAM step over any number of them at
-// once.  A hit lies where a NAM can accept it only near the NAM's end, as its length is
-// known to within the query's shortest and longest hit.  A NAM that the query has passed
-// (query_end < query_start) accepts nothing and stays where it is, so nothing is moved
-// between lists; then a thread a hit updates the NAM that holds it, and unclaimed hits open
-// NAMs in ref_start order.  (A warp resolving 32 NAMs after the other, testing every hit
-// between a NAM's last hit and its end and moving every NAM of the list for every query,
-// took 2.7M cycles for a read of 8550 hits, 1.5 ms of a batch.)
-//
+// query_start) order and merges them into O (merge_query); returns the number of NAMs.
+// kBlock: by the block, else by the warp alone.
 // buf: rescue_hit_words(cap) words, plan.maxrun <= cap.
 template <bool kBlock>
 __device__ __forceinline__ uint32_t rescue_merge(const IndexView& I, const Query* const* Qd, const uint64_t* const* Pd,
                                                  const RescuePlan& plan, const uint64_t* tkbuf, uint32_t Pq,
                                                  const OpenSoA& O, uint32_t* buf, uint32_t cap, RescueShared& S,
                                                  uint64_t& walk_cycles) {
-    constexpr uint32_t kFree = 0xFFFFFFFFu;
-    const uint32_t lane = lane_id(), w = kBlock ? threadIdx.x >> 5 : 0;
-    const uint32_t tid = kBlock ? threadIdx.x : lane, nt = kBlock ? blockDim.x : 32u;
-    const uint32_t nw = kBlock ? kWarpsPerBlock : 1u;
-    auto sync = [] {
-        if (kBlock) __syncthreads();
-        else __syncwarp();
-    };
+    const uint32_t tid = kBlock ? threadIdx.x : lane_id(), nt = kBlock ? blockDim.x : 32u;
     uint32_t *hrs = buf, *hpk = buf + cap, *claim = buf + 2 * (size_t)cap, *gone = buf + 3 * (size_t)cap;
-    int32_t *fqe = O.f(1), *fqprev = O.f(2), *fre = O.f(4), *frprev = O.f(5), *fnh = O.f(6);
-    const uint32_t* fref = reinterpret_cast<const uint32_t*>(O.f(7));
-    const volatile uint32_t* held = claim;
     uint32_t n = 0;
     for (int d = 0; d < 2; ++d) {
         const uint64_t* tk = tkbuf + (2 + d) * Pq;
@@ -1321,112 +1211,12 @@ __device__ __forceinline__ uint32_t rescue_merge(const IndexView& I, const Query
             for (uint32_t t = tid; t < cnt; t += nt) claim[t] = kFree;
             for (uint32_t t = tid; 32 * t < cnt; t += nt) gone[t] = 0;
             // the next query's run (its first entries), on its way while this one merges
-            if (!kBlock && j + 1 < plan.m[d] && 8 * lane < (uint32_t)tk[j + 1])
-                prefetch_l2(I.rs + Pd[d][(uint32_t)(tk[j + 1] >> 32) & 0xFFFF] + 8 * lane);
-            sync();
-            // proposals, a round of nt NAMs at a time (the next round's fields on their way)
-            auto fields = [&](uint32_t i) {
-                return i < n ? make_int4(fqe[i], fre[i], frprev[i], (int)fref[i]) : make_int4(-1, 0, 0, 0);
-            };
-            int4 nx = fields(lo + tid);
-            for (uint32_t r0 = lo; r0 < n; r0 += nt) {
-                const int4 f = nx;
-                nx = fields(r0 + nt + tid);
-                uint32_t i = r0 + tid, fresh = kFree;
-                if (f.x >= qs) {
-                    int nqe = f.x, nre = f.y, from = f.z + 1, last = nre;
-                    uint32_t want = (uint32_t)f.w & 0x7FFFFFFFu;
-                    // a hit is accepted when both its ends lie beyond the NAM's or neither does
-                    if (qe > nqe) from = max(from, nre - (int)max_span + 1);
-                    else last = nre - (int)min_span;
-                    uint32_t at = 0, hi = nh;
-                    while (at < hi) {   // hits are sorted by ref_start
-                        const uint32_t mid = (at + hi) >> 1;
-                        if ((int)hrs[mid] < from) at = mid + 1;
-                        else hi = mid;
-                    }
-                    for (; at < nh; ++at) {
-                        // the next hit that no NAM of an earlier round took
-                        uint32_t free = ~gone[at >> 5] & (0xFFFFFFFFu << (at & 31));
-                        if (!free) {
-                            at |= 31u;
-                            if (at + 1 >= nh || (int)hrs[at + 1] > last) break;
-                            continue;
-                        }
-                        at = (at & ~31u) + (uint32_t)__ffs(free) - 1;
-                        if (at >= nh) break;
-                        const int rs = (int)hrs[at];
-                        if (rs > last) break;
-                        const uint32_t pk = hpk[at];
-                        const int re = rs + (int)(pk & 0xFF) + I.k;
-                        if ((pk >> 8) != want || held[at] < i || (qe > nqe) != (re > nre)) continue;
-                        const uint32_t old = atomicMin(&claim[at], i);
-                        if (old < i) continue;
-                        if (old == kFree) {
-                            fresh = at;
-                            break;
-                        }
-                        i = old;   // displaced: on with its next hit
-                        nqe = fqe[i];
-                        nre = fre[i];
-                        last = qe > nqe ? nre : nre - (int)min_span;
-                        want = fref[i] & 0x7FFFFFFFu;
-                    }
-                }
-                if (r0 + nt >= n) break;   // the last round: its claims need no bits
-                sync();
-                if (fresh != kFree) atomicOr(&gone[fresh >> 5], 1u << (fresh & 31));
-                sync();
-            }
-            sync();
-            // hits to their NAMs; the others open NAMs in order
-            const uint32_t per = ((nh + nw - 1) / nw + 31) & ~31u;
-            const uint32_t h0 = min(w * per, nh), h1 = min(h0 + per, nh);
-            uint32_t mine = 0;
-            for (uint32_t b = h0; b < h1; b += 32)
-                mine += __popc(__ballot_sync(0xFFFFFFFFu, b + lane < h1 && held[b + lane] == kFree));
-            uint32_t to = n, opened = mine;
-            if constexpr (kBlock) {
-                if (lane == 0) S.cnt[w] = mine;
-                __syncthreads();
-                opened = 0;
-                for (uint32_t v = 0; v < nw; ++v) {
-                    if (v < w) to += S.cnt[v];
-                    opened += S.cnt[v];
-                }
-            }
-            for (uint32_t b = h0; b < h1; b += 32) {
-                const uint32_t h = b + lane;
-                const bool in = h < h1;
-                const uint32_t i = in ? held[h] : 0u;
-                const bool open = in && i == kFree;
-                const uint32_t m = __ballot_sync(0xFFFFFFFFu, open);
-                if (in) {
-                    const int rs = (int)hrs[h];
-                    const uint32_t pk = hpk[h];
-                    const int re = rs + (int)(pk & 0xFF) + I.k;
-                    if (open) {
-                        HitRec x;
-                        x.ref_rc = ((uint32_t)d << 31) | (pk >> 8);
-                        x.qs = qs;
-                        x.qe = qe;
-                        x.rs = rs;
-                        x.re = re;
-                        O.put(to + __popc(m & lanemask_lt()), nam_from_hit(x));
-                    } else {
-                        if (qe > fqe[i] && re > fre[i]) {
-                            fqe[i] = qe;
-                            fre[i] = re;
-                        }
-                        fqprev[i] = qs;
-                        frprev[i] = rs;
-                        fnh[i] += 1;
-                    }
-                }
-                to += __popc(m);
-            }
-            n += opened;
-            sync();
+            if (!kBlock && j + 1 < plan.m[d] && 8 * tid < (uint32_t)tk[j + 1])
+                prefetch_l2(I.rs + Pd[d][(uint32_t)(tk[j + 1] >> 32) & 0xFFFF] + 8 * tid);
+            if (kBlock) __syncthreads();
+            else __syncwarp();
+            n = merge_query<kBlock, false>(O, lo, n, qs, qe, (uint32_t)d, I.k, nh, min_span, max_span, hrs, hpk, claim,
+                                           gone, S.cnt);
         }
     }
     return n;
@@ -1758,6 +1548,137 @@ __global__ void __launch_bounds__(kPackThreads, 2)
             } else if (A.rescue_cycles) {
                 A.rescue_cycles[8ull * job.note + 3] = (uint64_t)(clock64() - t0);
             }
+        }
+        __syncthreads();
+    }
+}
+
+// find_nams for the reads with more NAMs than k_nams_group's slots (reads in repeats, with
+// queries of dozens of hits): a block a read, a query's hits merged at once (merge_query).
+// A warp a read, hit by hit with 8 slots a lane, took 0.36 ms for the longest of 81 such
+// reads of 100k, 0.95 ms where some of 250 bp had more than 256 NAMs; here 0.12 and 0.17.
+constexpr int kBigThreads = kPackThreads;
+constexpr uint32_t kBigHits = 512;   // hits of one query in shared memory
+
+__global__ void __launch_bounds__(kBigThreads, 2) k_nams(MapConfig C, int k, ReadRec* __restrict__ rec, Arenas A,
+                                                         Counters* ctr) {
+    __shared__ union {
+        uint32_t hits[rescue_hit_words(kBigHits)];
+        uint64_t sort[4 * kPackThreads];   // also the warp sort's buffer
+    } s;
+    __shared__ uint32_t s_cnt[kBigThreads / 32];
+    __shared__ uint32_t s_item, s_run, s_min, s_max;
+    __shared__ uint8_t* s_scratch;
+    static_assert(sizeof(s) >= 7168 && kWarpSortMax <= 256, "a warp's sort entries fit");
+    const uint32_t tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
+    const uint32_t n_big = *(volatile unsigned int*)&ctr->n_big;
+    for (;;) {
+        if (tid == 0) s_item = atomicAdd(&ctr->big_next, 1u);
+        __syncthreads();
+        const uint32_t b = s_item;
+        if (b >= n_big) break;
+        const long long t0 = clock64();
+        const uint32_t r = A.big_list[b];
+        ReadRec& R = rec[r];
+        const uint32_t H = R.n_hits;
+        const HitPacked* hits = A.hits + R.hit_off;
+        // the NAMs (at most H), their records, sort keys, and the hits of a query with more
+        // than kBigHits
+        const uint32_t P2 = next_pow2(H);
+        const uint64_t b_soa = 32ull * H, b_keys = 32ull * P2;
+        if (w == 0) {
+            uint8_t* p = warp_scratch(A, ctr, 0, b_soa + 32ull * H + b_keys + 4ull * rescue_hit_words(H) + 64);
+            if (!p) warp_fail(R, ctr, kStatusScratchOverflow);
+            if (lane == 0) s_scratch = p;
+        }
+        __syncthreads();
+        uint8_t* sc = s_scratch;
+        if (!sc) continue;
+        const OpenSoA O{reinterpret_cast<int32_t*>(sc), H};
+        NamState* closed = reinterpret_cast<NamState*>(sc + b_soa);
+        NamKey* keys = reinterpret_cast<NamKey*>(closed + H);
+        uint32_t* big_buf = reinterpret_cast<uint32_t*>(sc + b_soa + 32ull * H + b_keys);
+        uint32_t n = 0, lo = 0, cur_dir = 0;
+        for (uint32_t i = 0; i < H;) {
+            // hits [i, i + nh) of one query
+            const HitRec x = load_hit(hits, i, H);
+            const uint32_t dir = x.ref_rc >> 31;
+            if (tid == 0) {
+                s_run = 0xFFFFFFFFu;
+                s_min = 0xFFFFFFFFu;
+                s_max = 0;
+            }
+            if (dir != cur_dir) {   // the other orientation's NAMs can take no more hits
+                lo = n;
+                cur_dir = dir;
+            }
+            __syncthreads();
+            uint32_t nh = 0;
+            for (uint32_t c = 0;; c += kBigThreads) {
+                const HitRec y = load_hit(hits, i + c + tid, H);
+                const bool same = i + c + tid < H && (y.ref_rc >> 31) == dir && y.qs == x.qs && y.qe == x.qe;
+                if (!same) atomicMin(&s_run, c + tid);
+                if (__syncthreads_and(same)) continue;
+                nh = s_run;
+                break;
+            }
+            const uint32_t cap = nh <= kBigHits ? kBigHits : H;
+            uint32_t* buf = nh <= kBigHits ? s.hits : big_buf;
+            uint32_t *hrs = buf, *hpk = buf + cap, *claim = buf + 2 * (size_t)cap, *gone = buf + 3 * (size_t)cap;
+            bool bad = false;
+            for (uint32_t t = tid; t < nh; t += kBigThreads) {
+                const HitRec y = load_hit(hits, i + t, H);
+                const uint32_t span = (uint32_t)(y.re - y.rs);
+                bad |= t > 0 && load_hit(hits, i + t - 1, H).rs > y.rs;
+                hrs[t] = (uint32_t)y.rs;
+                hpk[t] = (y.ref_rc << 8) | (span - (uint32_t)k);   // as in the index
+                claim[t] = kFree;
+                atomicMin(&s_min, span);
+                atomicMax(&s_max, span);
+            }
+            for (uint32_t t = tid; 32 * t < nh; t += kBigThreads) gone[t] = 0;
+            // (an index whose runs are not in position order: hit by hit)
+            if (__syncthreads_or(bad)) nh = 1;
+            n = merge_query<true, true>(O, lo, n, x.qs, x.qe, dir, k, nh, s_min, s_max, hrs, hpk, claim, gone, s_cnt);
+            i += nh;
+        }
+        for (uint32_t i = tid; i < n; i += kBigThreads) closed[i] = O.get(i);
+        if (tid == 0) R.n_nams = n;
+        __syncthreads();
+        const long long t_merge = clock64();
+        SortJob job;
+        job.closed = closed;
+        job.n = n;
+        bool done = false;
+        if (C.sort_mode == GBSA_SORT_SCORE && n <= 4 * kPackThreads) {
+            if (n <= kPackThreads) done = pack_sort<1>(job, R, A, ctr, s.sort);
+            else if (n <= 2 * kPackThreads) done = pack_sort<2>(job, R, A, ctr, s.sort);
+            else done = pack_sort<4>(job, R, A, ctr, s.sort);
+        }
+        __syncthreads();
+        if (!done && w == 0) {
+            if (n <= kWarpSortMax) {
+                warp_finish_nams(C, closed, n, reinterpret_cast<uint32_t*>(&s), R, A, ctr);
+            } else {
+                for (uint32_t t = lane; t < n; t += 32) keys[t] = nam_key(closed[t], t, C.sort_mode);
+                __syncwarp();
+                warp_sort_keys(keys, n);
+                const uint64_t noff = warp_bump(&ctr->nam_used, n);
+                if (noff + n > A.nam_cap) {
+                    warp_fail(R, ctr, kStatusNamOverflow);
+                    if (lane == 0) R.n_nams = 0;
+                } else {
+                    for (uint32_t t = lane; t < n; t += 32) A.nams[noff + t] = closed[keys[t].idx];
+                    if (lane == 0) R.nam_off = noff;
+                }
+            }
+        }
+        if (A.nam_cycles && tid == 0) {
+            uint64_t* note = A.nam_cycles + 4ull * b;   // cycles, hits, NAMs, merge cycles
+            note[0] = (uint64_t)(clock64() - t0);
+            note[1] = H;
+            note[2] = n;
+            note[3] = (uint64_t)(t_merge - t0);
         }
         __syncthreads();
     }
@@ -2347,12 +2268,12 @@ void launch_lookup(const IndexView& I, const MapConfig& C, uint32_t n, ReadRec* 
     GBSA_LAUNCHED();
 }
 
-// The NAM phase's kernels (lane and warp merges, rescue, NAM gather) run beside each
-// other and need most of an SM's shared memory together (rescue 73 KB + group merge
-// 6 x 12 KB or warp merge 4 x 32 KB): they ask for the largest shared-memory carveout, so that the SM keeps that
-// configuration through the phase instead of switching it as each kernel's blocks
-// arrive (left to the driver, an earlier lane merge took 5.0 instead of 3.3 ms on the C2
-// batch inside the batch graph).  The seeding + lookup kernels keep the default: they use the
+// The NAM phase's kernels (group and block merges, rescue, NAM gather) run beside each
+// other and need most of an SM's shared memory together (rescue 2 x 97 KB, group merge
+// 17 KB a block): they ask for the largest shared-memory carveout, so that the SM keeps
+// that configuration through the phase instead of switching it as each kernel's blocks
+// arrive (left to the driver, an earlier merge took 5.0 instead of 3.3 ms on the C2 batch
+// inside the batch graph).  The seeding + lookup kernels keep the default: they use the
 // rest of the unified L1 to cache index entries.  Set once per device.
 void nam_phase_carveout() {
     static std::mutex mu;
@@ -2384,12 +2305,12 @@ void launch_bucket_reads(uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cuda
     GBSA_LAUNCHED();
 }
 
-void launch_nams_warp(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
+void launch_nams_warp(const MapConfig& C, int k, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
     if (!n) return;
-    // at most nam_kernel_warps(n) warps: one scratch slot each
-    const unsigned blocks = (unsigned)std::min<uint64_t>((uint64_t)device_sm_count() * kHeavyBlocksPerSm,
-                                                         (n + kHeavyWarps - 1) / kHeavyWarps);
-    k_nams<<<blocks, 32 * kHeavyWarps, 0, st>>>(C, rec, A, ctr);
+    // a scratch slot a block (its first warp's; at most nam_kernel_warps(n) warps)
+    const unsigned blocks = (unsigned)std::min<uint64_t>((uint64_t)device_sm_count() * 2,
+                                                         (n + kBigThreads / 32 - 1) / (kBigThreads / 32));
+    k_nams<<<blocks, kBigThreads, 0, st>>>(C, k, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 
