@@ -2051,7 +2051,6 @@ __global__ void k_gather_nams(uint32_t n, const ReadRec* __restrict__ rec, const
                               const uint64_t* __restrict__ out_off, gbsa_nam* __restrict__ out, uint64_t out_cap,
                               float* frac, uint8_t* rescued, int mode, Arenas A, const Counters* ctr,
                               const BatchDesc* desc) {
-    const uint32_t lane = lane_id();
     uint64_t* copy_off = nullptr;
     if (desc) {
         const uint32_t cap = n;
@@ -2066,28 +2065,48 @@ __global__ void k_gather_nams(uint32_t n, const ReadRec* __restrict__ rec, const
             if (blockIdx.x == 0 && threadIdx.x == 0) copy_off[n] = out_off[cap];
         }
     }
+    // a rescued read by the block (it may hold thousands of NAMs: by a warp, the longest took
+    // 30 us of a batch of 1000 reads)
     if (mode == 2) {
         const uint32_t n_light = ctr->n_rescue, n_heavy = ctr->n_rescue_heavy;
-        for (uint32_t t = warp_global_id(); t < n_light + n_heavy; t += warp_count()) {
+        for (uint32_t t = blockIdx.x; t < n_light + n_heavy; t += gridDim.x) {
             const uint32_t r = t < n_light ? A.rescue_list[t] : A.rescue_list[A.rescue_cap - 1 - (t - n_light)];
             const ReadRec R = rec[r];
             const uint64_t o = out_off[r];
-            for (uint32_t j = lane; j < R.n_nams; j += 32)
+            for (uint32_t j = threadIdx.x; j < R.n_nams; j += blockDim.x)
                 if (o + j < out_cap) to_gbsa_nam(arena[R.nam_off + j], (int)j, out[o + j]);
         }
         return;
     }
-    for (uint32_t r = warp_global_id(); r < n; r += warp_count()) {
-        const ReadRec R = rec[r];
-        const uint64_t o = out_off[r];
+    // 16 lanes a read (most hold about ten NAMs), the next read's record on its way
+    const uint32_t sub = threadIdx.x & 15u;
+    const uint32_t stride = 2 * warp_count();
+    uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+    ReadRec R{};
+    uint64_t o = 0;
+    if (r < n) {
+        R = rec[r];
+        o = out_off[r];
+    }
+    while (r < n) {
+        const uint32_t rn = r + stride;
+        ReadRec Rn{};
+        uint64_t on = 0;
+        if (rn < n) {
+            Rn = rec[rn];
+            on = out_off[rn];
+        }
         const bool skip = mode == 1 && (R.flags & kReadRescue);
-        for (uint32_t j = lane; j < (skip ? 0u : R.n_nams); j += 32)
+        for (uint32_t j = sub; j < (skip ? 0u : R.n_nams); j += 16)
             if (o + j < out_cap) to_gbsa_nam(arena[R.nam_off + j], (int)j, out[o + j]);
-        if (lane == 0) {
+        if (sub == 0) {
             if (frac) frac[r] = R.frac;
             if (rescued) rescued[r] = (R.flags & kReadRescue) ? 1 : 0;
             if (copy_off) copy_off[r] = o;
         }
+        r = rn;
+        R = Rn;
+        o = on;
     }
 }
 
