@@ -361,17 +361,21 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
     auto mark = [&](int i) {
         if (m.profile) record_stage(m.ev[i], st);
     };
-    // Seeding and lookup run as one kernel (a warp seeds a read, then looks it up:
-    // hashing overlaps the gathers) unless the index's entries exceed fuse_index_bytes:
-    // gathers from an entry array beyond the GPU's TLB reach (3.1 Gbp: 9.9 GB) run
-    // faster in a lookup kernel of their own (measured: 56.1 ms fused against 22.7 +
-    // 27.8 ms for 10M reads).
+    // Seeding and lookup run as one kernel (a warp seeds a read, then looks it up: hashing
+    // overlaps the gathers) where the reads take its fast path, or the index's entries stay
+    // below 2 GiB (1M reads of 150 bp against 3.1 Gbp, 9.9 GB of entries: the fast path
+    // 4.8 ms, in two kernels 3.6 + 4.1 ms; the general path is equal in both forms there:
+    // 10.8 against 3.6 + 7.4 ms).  A limit that the caller set (gbsa_mapper_set_fuse_limit)
+    // counts alone.
     // (the batched form runs its persistent work-queue kernel, with the lookup fused
-    // under the same limit)
-    const bool fused = !seeded && I.n * sizeof(gbsa_ref_randstrobe) <= m.fuse_index_bytes;
+    // under the same rule)
+    const uint64_t entry_bytes = I.n * sizeof(gbsa_ref_randstrobe);
+    const bool fused = !seeded && (m.fuse_index_bytes != kFuseAuto ? entry_bytes <= m.fuse_index_bytes
+                                                                   : entry_bytes <= (2ull << 30) ||
+                                                                         seeds_fast(m.idx->dp, I, C));
     m.fused = fused;
     mark(0);
-    if (desc) launch_seed_lookup_queue(m.idx->dp, I, C, desc, m.rec.as<ReadRec>(), A, ctr, bm->variant, fused, st);
+    if (desc) launch_seed_lookup_queue(m.idx->dp, I, C, desc, m.rec.as<ReadRec>(), A, ctr, bm->variant, fused, n, st);
     else if (fused) launch_seed_lookup(m.idx->dp, I, C, d_seqs, d_offs, d_lens, n, m.rec.as<ReadRec>(), A, ctr, st);
     else if (!seeded) launch_seed(m.idx->dp, d_seqs, d_offs, d_lens, n, m.rec.as<ReadRec>(), A, ctr, st);
     mark(1);
@@ -511,8 +515,7 @@ static uint64_t run_pipeline(gbsa_mapper& m, const uint8_t* d_seqs, const uint64
     throw Error(GBSA_ERR_DEVICE_STATUS, "work areas kept overflowing");
 }
 
-// L2 access-policy window over the index's bucket table (the 32-bit copy when there
-// is one: 32 MB for 2^23 buckets), read by every probe of the lookup: held persisting
+// L2 access-policy window over the index's bucket table (64 MB for 2^23 buckets), read by every probe of the lookup: held persisting
 // in L2 so that the entry gathers do not evict it.  Used when the table fits the
 // device's largest window; the hit ratio is the part of the table the persisting L2
 // set-aside can hold.  The set-aside (cudaLimitPersistingL2CacheSize) is a limit of
@@ -538,8 +541,8 @@ void l2_window_attach(gbsa_mapper& m, bool on) {
         return;
     }
     const gbsa_index& ix = *m.idx;
-    const void* base = ix.starts32.size() ? ix.starts32.as<void>() : ix.starts.as<void>();
-    const uint64_t bytes = ((1ull << ix.bits) + 1) * (ix.starts32.size() ? 4 : 8);
+    const void* base = ix.buckets.size() ? ix.buckets.as<void>() : ix.starts.as<void>();
+    const uint64_t bytes = ((1ull << ix.bits) + 1) * 8;
     int max_window = 0, persist_max = 0;
     GBSA_CUDA(cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, dev));
     GBSA_CUDA(cudaDeviceGetAttribute(&persist_max, cudaDevAttrMaxPersistingL2CacheSize, dev));
@@ -727,7 +730,7 @@ int gbsa_index_load(const gbsa_params* p, const gbsa_ref_randstrobe* randstrobes
         ix->starts.resize(8 * nb);
         if (n) GBSA_CUDA(cudaMemcpy(ix->rs.as<void>(), randstrobes, 16 * n, cudaMemcpyHostToDevice));
         GBSA_CUDA(cudaMemcpy(ix->starts.as<void>(), start_indices, 8 * nb, cudaMemcpyHostToDevice));
-        make_compact_starts(*ix, 0);
+        make_buckets(*ix, 0);
         ix->info.size = n;
         ix->info.bits = bits;
         ix->info.filter_cutoff = filter_cutoff;
@@ -1252,9 +1255,9 @@ int gbsa_mapper_set_profile(gbsa_mapper* m, int on) {
 }
 
 int gbsa_mapper_last_counts(const gbsa_mapper* m, uint64_t* out) {
-    out[0] = m->last.q_used;
-    out[1] = m->last.hit_used;
-    out[2] = m->last.nam_used;
+    out[0] = m->last.q_used - m->last.q_spare + m->last.q_direct;
+    out[1] = m->last.hit_used - m->last.hit_spare;
+    out[2] = m->last.nam_used - m->last.nam_spare;
     out[3] = m->last.n_rescue + m->last.n_rescue_heavy;
     out[4] = m->last.n_long;
     out[5] = m->last.scratch_used;

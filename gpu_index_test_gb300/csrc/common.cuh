@@ -50,6 +50,10 @@ __host__ __device__ __forceinline__ uint32_t nt4(uint8_t c) {
     return 4;
 }
 
+// The 8 bits of an entry's hash that the bucket table keeps: below the bucket number's (at
+// most 31 bits of 64), and not the low bits, which the choice of the second strobe biases.
+__host__ __device__ __forceinline__ uint32_t hash_tag(uint64_t hash) { return (uint32_t)(hash >> 24) & 0xFFu; }
+
 // Device copy of the index parameters actually used by the kernels.
 struct DevParams {
     int k, s, t;        // t = t_syncmer (1-based offset of the s-mer minimum)

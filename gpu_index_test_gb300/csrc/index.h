@@ -23,16 +23,25 @@ struct gbsa_index {
     int device = 0;
     gbsa::DeviceBuffer rs;       // gbsa_ref_randstrobe[n]
     gbsa::DeviceBuffer starts;   // uint64_t[2^bits + 1]
-    gbsa::DeviceBuffer starts32; // uint32_t[2^bits + 1] copy read by the kernels when n < 2^32
+    gbsa::DeviceBuffer buckets;  // Bucket[2^bits + 1] read by the kernels when n < 2^32
 };
 
 namespace gbsa {
+
+// A bucket as the lookup reads it: its start, and a tag (8 bits of the hash, hash_tag) of
+// each of its first four entries.  Two thirds of a read's queries are not in the index (its
+// other strand, and seeds with a sequencing error): the tags answer nearly all of those
+// from the bucket's own sector, without the dependent fetch of an entry.
+struct Bucket {
+    uint32_t start;
+    uint32_t tags;   // entry i's in byte i (0 past the bucket's end)
+};
 
 // Read-only view of the index used by device code.
 struct IndexView {
     const gbsa_ref_randstrobe* rs;
     const uint64_t* starts;
-    const uint32_t* starts32;   // half-size table (half the L2 footprint), or null
+    const Bucket* buckets;      // or null (2^32 entries or more, or a loaded table out of order)
     uint64_t n;
     int bits;
     uint32_t filter_cutoff;
@@ -41,12 +50,13 @@ struct IndexView {
 
 inline IndexView view_of(const gbsa_index& ix) {
     return IndexView{ix.rs.as<gbsa_ref_randstrobe>(), ix.starts.as<uint64_t>(),
-                     ix.starts32.size() ? ix.starts32.as<uint32_t>() : nullptr, ix.n, ix.bits, ix.filter_cutoff,
+                     ix.buckets.size() ? ix.buckets.as<Bucket>() : nullptr, ix.n, ix.bits, ix.filter_cutoff,
                      ix.params.k};
 }
 
-// Builds the 32-bit copy of the bucket table when every start fits (n < 2^32).
-void make_compact_starts(gbsa_index& ix, cudaStream_t st);
+// Builds the lookup's bucket table of a loaded index, when every start fits 32 bits
+// (n < 2^32) and the entries lie in their buckets in order.
+void make_buckets(gbsa_index& ix, cudaStream_t st);
 
 // Validates parameters like the reference constructors (step2/indexparameters.hpp:24-68).
 bool params_valid(const gbsa_params& p);

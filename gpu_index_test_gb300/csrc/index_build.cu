@@ -117,32 +117,55 @@ __global__ void k_ref_randstrobes(DevParams P, const uint64_t* __restrict__ sh, 
     }
 }
 
-__global__ void k_first_distinct(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n,
-                                 unsigned long long* __restrict__ p1) {
+// First entry whose hash is not rs[0]'s (n when there is none): doubling steps, then a
+// binary search; nearly always entry 1.
+__device__ __forceinline__ uint64_t second_run(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n) {
     const uint64_t h0 = rs[0].hash;
-    for (uint64_t i = 1 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (rs[i].hash != h0) {
-            atomicMin(p1, (unsigned long long)i);
-            return;
-        }
+    uint64_t lo = 0, step = 1;   // rs[lo] is of the first run
+    while (lo + step < n && rs[lo + step].hash == h0) {
+        lo += step;
+        step *= 2;
     }
+    uint64_t hi = lo + step < n ? lo + step : n;
+    while (hi - lo > 1) {
+        const uint64_t mid = lo + (hi - lo) / 2;
+        if (rs[mid].hash == h0) lo = mid;
+        else hi = mid;
+    }
+    return hi;
 }
 
+// Bucket b's start and tags, its first entry being `at`.
+__device__ __forceinline__ Bucket bucket_at(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, int bits,
+                                            uint64_t b, uint64_t at) {
+    Bucket k;
+    k.start = (uint32_t)at;
+    k.tags = 0;
+    for (int j = 0; j < 4 && at + j < n; ++j) {
+        const uint64_t h = rs[at + j].hash;
+        if ((h >> (64 - bits)) != b) break;
+        k.tags |= hash_tag(h) << (8 * j);
+    }
+    return k;
+}
+
+// The bucket table (the reference's first-bucket rule: the buckets up to the first entry's
+// start at the second run) and, where `buckets` is set, the lookup's form of it, in one
+// pass: an entry that opens a bucket writes it and the empty ones before it.
 __global__ void k_bucket_starts(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, int bits,
-                                const unsigned long long* __restrict__ p1, uint64_t* __restrict__ starts) {
+                                uint64_t* __restrict__ starts, Bucket* __restrict__ buckets) {
     const uint64_t nb = 1ULL << bits;
+    auto put = [&](uint64_t b0, uint64_t b1, uint64_t at, uint64_t own) {   // [b0, b1), `own`: where at's entries lie
+        for (uint64_t b = b0; b < b1; ++b) {
+            starts[b] = at;
+            if (buckets) buckets[b] = b == own ? bucket_at(rs, n, bits, b, at) : Bucket{(uint32_t)at, 0u};
+        }
+    };
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t t = rs[i].hash >> (64 - bits);
-        if (i == 0) {
-            const uint64_t v = *p1;
-            for (uint64_t b = 0; b <= t; ++b) starts[b] = v;
-        } else {
-            const uint64_t tp = rs[i - 1].hash >> (64 - bits);
-            for (uint64_t b = tp + 1; b <= t; ++b) starts[b] = i;
-        }
-        if (i == n - 1) {
-            for (uint64_t b = t + 1; b <= nb; ++b) starts[b] = n;
-        }
+        if (i == 0) put(0, t + 1, second_run(rs, n), t);
+        else put((rs[i - 1].hash >> (64 - bits)) + 1, t + 1, i, t);
+        if (i == n - 1) put(t + 1, nb + 1, n, nb + 1);
     }
 }
 
@@ -355,16 +378,15 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     // ---- bucket table ------------------------------------------------------------
     const uint64_t nb = (1ULL << ix.bits) + 1;
     ix.starts.resize(8 * nb);
+    const bool tagged = n_rs < (1ull << 32);
+    if (tagged) ix.buckets.resize(sizeof(Bucket) * nb);
     const gbsa_ref_randstrobe* rs = ix.rs.as<gbsa_ref_randstrobe>();
     if (n_rs == 0) {
         GBSA_CUDA(cudaMemsetAsync(ix.starts.as<void>(), 0, 8 * nb, st));
+        GBSA_CUDA(cudaMemsetAsync(ix.buckets.as<void>(), 0, sizeof(Bucket) * nb, st));
     } else {
-        unsigned long long* d_p1 = ws.get<unsigned long long>(1);
-        GBSA_CUDA(cudaMemcpyAsync(d_p1, &n_rs, 8, cudaMemcpyHostToDevice, st));
-        k_first_distinct<<<grid_for(n_rs, 256, 1u << 16), 256, 0, st>>>(rs, n_rs, d_p1);
-        GBSA_LAUNCHED();
-        k_bucket_starts<<<grid_for(n_rs, 256, 1u << 20), 256, 0, st>>>(rs, n_rs, ix.bits, d_p1,
-                                                                       ix.starts.as<uint64_t>());
+        k_bucket_starts<<<grid_for(n_rs, 256, 1u << 20), 256, 0, st>>>(
+            rs, n_rs, ix.bits, ix.starts.as<uint64_t>(), tagged ? ix.buckets.as<Bucket>() : nullptr);
         GBSA_LAUNCHED();
     }
 
@@ -393,22 +415,39 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     finish_stats(ix, H, unique, f);
     ix.info.size = ix.n;
     ix.info.bits = ix.bits;
-    make_compact_starts(ix, st);
 }
 
-__global__ void k_narrow_starts(const uint64_t* __restrict__ in, uint32_t* __restrict__ out, uint64_t n) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = (uint32_t)in[i];
+// As bucket_at, for a table that was not built here: `odd` is set when the entries are
+// not in order or a bucket holds one that belongs elsewhere, for then a tag could answer
+// differently from the search in order.
+__global__ void k_make_buckets(const uint64_t* __restrict__ starts, const gbsa_ref_randstrobe* __restrict__ rs,
+                               uint64_t n, int bits, Bucket* __restrict__ out, uint32_t* __restrict__ odd) {
+    const uint64_t nb = 1ULL << bits;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i <= nb; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t a = starts[i], e = i < nb ? starts[i + 1] : a;
+        const bool good = a <= n && e <= n &&
+                          (a >= e || ((rs[a].hash >> (64 - bits)) == i && (rs[e - 1].hash >> (64 - bits)) == i));
+        if (!good) *odd = 1;
+        out[i] = good && a < e ? bucket_at(rs, e, bits, i, a) : Bucket{(uint32_t)a, 0u};
+    }
+    for (uint64_t i = 1 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        if (rs[i - 1].hash > rs[i].hash) *odd = 1;
 }
 
-void make_compact_starts(gbsa_index& ix, cudaStream_t st) {
+void make_buckets(gbsa_index& ix, cudaStream_t st) {
     if (ix.n >= (1ull << 32)) return;
-    const uint64_t nb = (1ULL << ix.bits) + 1;
-    ix.starts32.resize(4 * nb);
-    k_narrow_starts<<<grid_for(nb, 256, 1u << 16), 256, 0, st>>>(ix.starts.as<uint64_t>(), ix.starts32.as<uint32_t>(),
-                                                                 nb);
+    const uint64_t nb = 1ULL << ix.bits;
+    ix.buckets.resize(sizeof(Bucket) * (nb + 1));
+    DeviceBuffer d_odd(4);
+    uint32_t odd = 0;
+    GBSA_CUDA(cudaMemsetAsync(d_odd.as<void>(), 0, 4, st));
+    k_make_buckets<<<grid_for(nb + 1, 256, 1u << 20), 256, 0, st>>>(ix.starts.as<uint64_t>(),
+                                                                    ix.rs.as<gbsa_ref_randstrobe>(), ix.n, ix.bits,
+                                                                    ix.buckets.as<Bucket>(), d_odd.as<uint32_t>());
     GBSA_LAUNCHED();
+    GBSA_CUDA(cudaMemcpyAsync(&odd, d_odd.as<void>(), 4, cudaMemcpyDeviceToHost, st));
     GBSA_CUDA(cudaStreamSynchronize(st));
+    if (odd) ix.buckets.release();
 }
 
 }  // namespace gbsa

@@ -35,26 +35,17 @@ __device__ __forceinline__ uint64_t get_hash(const IndexView& I, uint64_t pos) {
     return pos < I.n ? __ldg(&I.rs[pos].hash) : ~0ULL;
 }
 
-// Entry i of the bucket table (the 32-bit copy when the index has one).
+// Start of bucket i.
 __device__ __forceinline__ uint64_t bucket_start(const IndexView& I, uint64_t i) {
-    return I.starts32 ? (uint64_t)__ldg(&I.starts32[i]) : __ldg(&I.starts[i]);
+    return I.buckets ? (uint64_t)__ldg(&I.buckets[i].start) : __ldg(&I.starts[i]);
 }
 
-// StrobemerIndex::find (step2/index.hpp:57-81): first entry of the key's bucket
-// whose hash equals the key, or kNotFound.  The in-bucket search examines entries
-// in order until one is >= key (buckets hold ~2 entries on average) and switches to
-// a binary search for long buckets; both give the reference's answer.  ex receives
-// the number of entries examined by the linear rule (for the byte count).
-__device__ __forceinline__ uint64_t index_find(const IndexView& I, uint64_t key, uint32_t* ex = nullptr,
-                                               uint64_t* bucket_end = nullptr) {
-    const uint64_t top = key >> (64 - I.bits);
-    const uint64_t a = bucket_start(I, top);
-    const uint64_t b = bucket_start(I, top + 1);
-    if (bucket_end) *bucket_end = b;
-    if (a >= b) {
-        if (ex) *ex = 0;
-        return kNotFound;
-    }
+// First entry of [a, b), sorted by hash, whose hash equals the key, or kNotFound: entries in
+// order until one is >= key (buckets hold ~2 entries on average), or a binary search for a
+// long range; both give the reference's answer.  ex receives the number of entries
+// examined by the linear rule (for the byte count).
+__device__ __forceinline__ uint64_t find_in(const IndexView& I, uint64_t key, uint64_t a, uint64_t b,
+                                            uint32_t* ex = nullptr) {
     if (b - a <= 16) {
         for (uint64_t x = a; x < b; ++x) {
             const uint64_t h = __ldg(&I.rs[x].hash);
@@ -74,6 +65,100 @@ __device__ __forceinline__ uint64_t index_find(const IndexView& I, uint64_t key,
     }
     if (ex) *ex = (uint32_t)(lo - a + 1 < b - a ? lo - a + 1 : b - a);
     return (lo < b && __ldg(&I.rs[lo].hash) == key) ? lo : kNotFound;
+}
+
+// StrobemerIndex::find (step2/index.hpp:57-81): first entry of the key's bucket
+// whose hash equals the key, or kNotFound.
+__device__ __forceinline__ uint64_t index_find(const IndexView& I, uint64_t key, uint32_t* ex = nullptr,
+                                               uint64_t* bucket_end = nullptr) {
+    const uint64_t top = key >> (64 - I.bits);
+    const uint64_t a = bucket_start(I, top);
+    const uint64_t b = bucket_start(I, top + 1);
+    if (bucket_end) *bucket_end = b;
+    if (a >= b) {
+        if (ex) *ex = 0;
+        return kNotFound;
+    }
+    return find_in(I, key, a, b, ex);
+}
+
+// An index entry as one 16-byte load.
+struct Entry {
+    uint64_t hash;
+    uint32_t position, packed;
+};
+__device__ __forceinline__ Entry load_entry(const IndexView& I, uint32_t pos) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(I.rs) + pos);
+    return Entry{((uint64_t)v.y << 32) | v.x, v.z, v.w};
+}
+
+// A query's answer from the tagged buckets (I.buckets set): the position of its hash
+// (kMissing: not in the index), whether it is filtered, and for one that is not the hits
+// that add_to_hits_per_ref keeps and the first of them (the run's first entry, which is
+// always kept).
+constexpr uint32_t kMissing = 0xFFFFFFFFu;   // fewer than 2^32 entries: no entry's position
+struct Probe {
+    uint32_t pos;
+    bool filtered;
+    uint32_t n_hits;
+    uint32_t position, packed;
+};
+
+// Candidates are the entries of the bucket whose tag matches; a bucket of more than four is
+// searched as a whole.  `len` is the query's length.
+__device__ __forceinline__ Probe index_probe(const IndexView& I, uint64_t key, int len) {
+    Probe p;
+    p.pos = kMissing;
+    p.filtered = false;
+    p.n_hits = 0;
+    p.position = p.packed = 0;
+    const uint32_t top = (uint32_t)(key >> (64 - I.bits));
+    const uint2 bk = __ldg(reinterpret_cast<const uint2*>(I.buckets) + top);
+    const uint32_t end = __ldg(&I.buckets[top + 1].start);
+    const uint32_t a = bk.x, cnt = end > a ? end - a : 0u;
+    if (cnt == 0) return p;
+    Entry e;
+    // bit 8 i: entry i's tag matches (of a bucket of up to four)
+    const uint32_t match = __vcmpeq4(bk.y, hash_tag(key) * 0x01010101u) & (cnt < 4 ? (1u << (8 * cnt)) - 1 : 0xFFFFFFFFu) &
+                           0x01010101u;
+    if (cnt <= 4) {
+        for (uint32_t m = match;; m &= m - 1) {
+            if (!m) return p;
+            const uint32_t i = (uint32_t)(__ffs(m) - 1) >> 3;
+            e = load_entry(I, a + i);
+            if (e.hash == key) {
+                p.pos = a + i;
+                break;
+            }
+        }
+    } else {
+        const uint64_t x = find_in(I, key, a, end);
+        if (x == kNotFound) return p;
+        p.pos = (uint32_t)x;
+        e = load_entry(I, p.pos);
+    }
+    // an entry at or past the bucket's end has other top bits, so it cannot equal key; past
+    // the table's end the reference reads all ones
+    const uint64_t far = (uint64_t)p.pos + I.filter_cutoff;
+    p.filtered = far >= end ? far >= I.n && key == ~0ULL : __ldg(&I.rs[far].hash) == key;
+    if (p.filtered) return p;
+    p.position = e.position;
+    p.packed = e.packed;
+    p.n_hits = 1;
+    int least = len - ((int)(e.packed & 0xFF) + I.k);
+    least = least < 0 ? -least : least;
+    for (uint32_t x = p.pos + 1; x < end; ++x) {
+        if (cnt <= 4 && !((match >> (8 * (x - a))) & 1u)) break;
+        const Entry f = load_entry(I, x);
+        if (f.hash != key) break;
+        int diff = len - ((int)(f.packed & 0xFF) + I.k);
+        diff = diff < 0 ? -diff : diff;
+        if (diff <= least) {
+            least = diff;
+            ++p.n_hits;
+        }
+    }
+    return p;
 }
 
 __device__ __forceinline__ bool index_is_filtered(const IndexView& I, uint64_t pos) {   // index.hpp:91-93

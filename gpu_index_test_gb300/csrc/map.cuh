@@ -29,8 +29,10 @@ constexpr uint32_t kReadFailed = 1u << 2;   // a capacity limit was hit
 // Device counters of one batch (bump allocators, work lists, status).
 struct Counters {
     unsigned long long q_used;
+    unsigned long long q_direct;    // query randstrobes looked up without a place in the arena
     unsigned long long hit_used;
     unsigned long long nam_used;
+    unsigned long long q_spare, hit_spare, nam_spare;   // taken ahead by a warp and not used
     unsigned long long scratch_used;
     unsigned long long alg_bytes;   // roofline numerator (see k_lookup)
     unsigned long long alg_sectors; // distinct 32 B sectors of the lookup's gathers (see k_lookup)
@@ -161,9 +163,13 @@ struct SeedVariant {
 };
 constexpr int kSeedVariants = 6;
 SeedVariant seed_variant(int v);
-// lookup false: seeding alone (the lookup then runs as launch_lookup with desc).
+// Whether the reads of such a batch mostly take the fused kernel's fast path.
+bool seeds_fast(const DevParams& P, const IndexView& I, const MapConfig& C);
+// lookup false: seeding alone (the lookup then runs as launch_lookup with desc).  cap: the
+// work areas' read capacity.
 void launch_seed_lookup_queue(const DevParams& P, const IndexView& I, const MapConfig& C, const BatchDesc* desc,
-                              ReadRec* rec, Arenas A, Counters* ctr, int variant, bool lookup, cudaStream_t st);
+                              ReadRec* rec, Arenas A, Counters* ctr, int variant, bool lookup, uint32_t cap,
+                              cudaStream_t st);
 // Main path: seeding and lookup fused (a warp per read); reads too long for the
 // shared-memory buffers are seeded by launch_seed_long and looked up by launch_lookup_long.
 void launch_seed_lookup(const DevParams& P, const IndexView& I, const MapConfig& C, const uint8_t* seqs,

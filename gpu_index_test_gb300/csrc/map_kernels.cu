@@ -37,10 +37,44 @@ __device__ __forceinline__ uint64_t warp_bump(unsigned long long* ctr, uint64_t 
 // The next read for the calling warp from a device work counter: warps pull reads one
 // at a time, so reads of uneven cost (lengths, repeats) balance over a grid of resident
 // warps instead of each warp owning a fixed stride of them.
-__device__ __forceinline__ uint32_t warp_next(unsigned int* head) {
+__device__ __forceinline__ uint32_t warp_take(unsigned int* head, uint32_t n) {
     uint32_t r = 0;
-    if (lane_id() == 0) r = atomicAdd(head, 1u);
+    if (lane_id() == 0) r = atomicAdd(head, n);
     return __shfl_sync(0xFFFFFFFFu, r, 0);
+}
+__device__ __forceinline__ uint32_t warp_next(unsigned int* head) { return warp_take(head, 1); }
+
+// Work items a warp takes at a time from a counter that all warps share (each take is a
+// round trip, and they queue at one address): four while there are many for each warp.
+__device__ __forceinline__ uint32_t items_per_take(uint32_t n) { return n >= 32 * warp_count() ? 4u : 1u; }
+
+// Room in an arena whose bump counter all warps share, taken ahead in pieces of up to
+// `piece` entries: a warp's requests come from its piece while they fit.  What is left
+// unused of the pieces is counted (`spare`), so that the counters still tell what was used.
+struct WarpRoom {
+    uint64_t at = 0;
+    uint32_t left = 0, spare = 0;
+    __device__ __forceinline__ uint64_t take(unsigned long long* used, uint64_t n, uint32_t piece) {
+        if (n > left) {
+            spare += left;
+            const uint64_t want = n > piece ? n : piece;
+            at = warp_bump(used, want);
+            left = (uint32_t)(want - n);
+        } else {
+            left -= (uint32_t)n;
+        }
+        const uint64_t r = at;
+        at += n;
+        return r;
+    }
+    __device__ __forceinline__ void done(unsigned long long* total) const {
+        if (lane_id() == 0 && spare + left) atomicAdd(total, (unsigned long long)(spare + left));
+    }
+};
+// The pieces of all warps of the grid together take at most an eighth of the arena.
+__device__ __forceinline__ uint32_t arena_piece(uint64_t cap) {
+    const uint64_t p = cap / (8ull * warp_count());
+    return p < 512 ? (uint32_t)p : 512u;
 }
 
 __device__ __forceinline__ void warp_fail(ReadRec& rec, Counters* ctr, uint32_t bit) {
@@ -53,9 +87,9 @@ __device__ __forceinline__ void warp_fail(ReadRec& rec, Counters* ctr, uint32_t 
 // Writes the query randstrobes of read r from its syncmers.
 __device__ __forceinline__ void emit_read_queries(const DevParams& P, const uint64_t* sh, const uint32_t* sp,
                                                   uint32_t ns, uint32_t L, ReadRec& rec, const Arenas& A,
-                                                  Counters* ctr) {
+                                                  Counters* ctr, WarpRoom& room) {
     const uint32_t nq = n_query_per_dir(P, ns, L);
-    const uint64_t off = warp_bump(&ctr->q_used, 2ull * nq);
+    const uint64_t off = room.take(&ctr->q_used, 2 * nq, arena_piece(A.q_cap));
     if (off + 2ull * nq > A.q_cap) {
         warp_fail(rec, ctr, kStatusQueryOverflow);
         if (lane_id() == 0) rec.nq = rec.nq2 = 0;
@@ -79,7 +113,15 @@ __global__ void __launch_bounds__(32 * kSeedWarps, 5) k_seed_smem(DevParams P, c
     __shared__ uint64_t s_sh[kSeedWarps][kSmemSyncmers];
     __shared__ uint32_t s_sp[kSeedWarps][kSmemSyncmers];
     const uint32_t w = threadIdx.x >> 5;
-    for (uint32_t r = warp_next(&ctr->queue_head); r < n; r = warp_next(&ctr->queue_head)) {
+    const uint32_t per = items_per_take(n);
+    WarpRoom room;
+    uint32_t left = 0, r = 0;
+    for (;; ++r, --left) {
+        if (left == 0) {
+            r = warp_take(&ctr->queue_head, per);
+            left = per;
+        }
+        if (r >= n) break;
         const uint32_t L = lens[r];
         ReadRec& R = rec[r];
         if (L > GBSA_MAX_READ_LEN) {
@@ -96,9 +138,10 @@ __global__ void __launch_bounds__(32 * kSeedWarps, 5) k_seed_smem(DevParams P, c
             }
             continue;
         }
-        emit_read_queries(P, s_sh[w], s_sp[w], ns, L, R, A, ctr);
+        emit_read_queries(P, s_sh[w], s_sp[w], ns, L, R, A, ctr, room);
         __syncwarp();
     }
+    room.done(&ctr->q_spare);
 }
 
 // Reads that did not fit the shared-memory buffers: same code on a per-warp slot of
@@ -120,6 +163,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_seed_long(DevParams P, 
     uint64_t* hb = reinterpret_cast<uint64_t*>(nm + kLongWords);
     uint64_t* sh = hb + 64;
     uint32_t* sp = reinterpret_cast<uint32_t*>(sh + GBSA_MAX_READ_LEN);
+    WarpRoom room;
     for (uint32_t t = warp_global_id(); t < n_long; t += warp_count()) {
         const uint32_t r = A.long_list[t];
         const uint32_t L = lens[r];
@@ -129,9 +173,10 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_seed_long(DevParams P, 
             warp_fail(R, ctr, kStatusSyncmerOverflow);
             continue;
         }
-        emit_read_queries(P, sh, sp, ns, L, R, A, ctr);
+        emit_read_queries(P, sh, sp, ns, L, R, A, ctr, room);
         __syncwarp();
     }
+    room.done(&ctr->q_spare);
 }
 
 // Distinct 32 B sectors of [lo, hi) bytes.
@@ -146,9 +191,9 @@ __device__ __forceinline__ uint64_t sector_span(uintptr_t lo, uintptr_t hi) {
 __device__ __forceinline__ uint64_t lookup_sectors(const IndexView& I, uint64_t key, uint32_t ex, uint64_t pos,
                                                    uint32_t run) {
     const uint64_t top = key >> (64 - I.bits);
-    const uintptr_t sb = I.starts32 ? reinterpret_cast<uintptr_t>(I.starts32 + top)
-                                    : reinterpret_cast<uintptr_t>(I.starts + top);
-    uint64_t n = sector_span(sb, sb + (I.starts32 ? 8 : 16));
+    const uintptr_t sb = I.buckets ? reinterpret_cast<uintptr_t>(I.buckets + top)
+                                   : reinterpret_cast<uintptr_t>(I.starts + top);
+    uint64_t n = sector_span(sb, sb + 16);
     const uint64_t a = bucket_start(I, top);
     uint64_t end = a + ex;   // entries [a, end) touched
     if (pos != kNotFound) {
@@ -164,6 +209,33 @@ __device__ __forceinline__ uint64_t lookup_sectors(const IndexView& I, uint64_t 
 
 constexpr uint32_t kRescueHeavyHits = 2000;   // estimated merge hits of a heavy rescued read
 
+// Puts read r, whose queries' positions are in the arena, on the rescue list.  Reads inside
+// short tandem repeats merge thousands of hits: their seeds' runs (up to the count cap)
+// estimate the merge's hits; reads above kRescueHeavyHits (C.rescue_block_hits when set) go
+// to the heavy end of the list, which the rescue kernel takes first.  filtered: some found
+// query is filtered (else none has a long run).
+__device__ __forceinline__ void enlist_rescue(const IndexView& I, const MapConfig& C, uint32_t r, ReadRec& R,
+                                              const Arenas& A, Counters* ctr, bool filtered) {
+    const uint32_t lane = lane_id();
+    uint32_t w = 0;
+    if (filtered) {
+        for (uint32_t i = lane; i < R.nq2; i += 32) {
+            const uint64_t pos = A.q_pos[R.q_off + i];
+            if (pos == kNotFound) continue;
+            const uint32_t c = index_get_count(I, pos);
+            w += c <= C.count_cap ? c : 0u;
+        }
+        w = warp_sum(w);
+    }
+    const bool heavy = w >= (C.rescue_block_hits ? C.rescue_block_hits : kRescueHeavyHits);
+    if (lane == 0) {
+        R.flags |= kReadRescue;
+        if (heavy) A.rescue_list[A.rescue_cap - 1 - atomicAdd(&ctr->n_rescue_heavy, 1u)] = r;
+        else A.rescue_list[atomicAdd(&ctr->n_rescue, 1u)] = r;
+        R.n_hits = 0;
+    }
+}
+
 // kCount: also count the reference's algorithmic bytes and gather sectors (a
 // separate instance, so that the counting code costs the mapping kernel nothing).
 // find / is_filtered / walk for the queries of read r (warp): per-query index
@@ -172,7 +244,7 @@ constexpr uint32_t kRescueHeavyHits = 2000;   // estimated merge hits of a heavy
 // The query loop of find_nams (step2/nam.cu:748-790).
 template <bool kCount>
 __device__ __forceinline__ void lookup_read(const IndexView& I, const MapConfig& C, uint32_t r, ReadRec* __restrict__ rec,
-                                            const Arenas& A, Counters* ctr) {
+                                            const Arenas& A, Counters* ctr, WarpRoom& room) {
     const uint32_t lane = lane_id();
     ReadRec& R = rec[r];
     if (R.flags & kReadFailed) return;
@@ -183,6 +255,16 @@ __device__ __forceinline__ void lookup_read(const IndexView& I, const MapConfig&
     uint64_t bytes = 0, sectors = 0;
     for (uint32_t i = lane; i < nq2; i += 32) {
         const Query q = Q[i];
+        if (!kCount && I.buckets) {
+            const Probe p = index_probe(I, q.hash, (int)(q.end - q.start));
+            if (p.pos != kMissing) {
+                ++tot;
+                good += p.filtered ? 0u : 1u;
+            }
+            A.q_pos[R.q_off + i] = p.pos == kMissing ? kNotFound : (uint64_t)p.pos;
+            aux[i] = p.n_hits;
+            continue;
+        }
         uint32_t ex = 0;
         uint64_t bend = 0;
         const uint64_t pos = index_find(I, q.hash, &ex, &bend);
@@ -220,27 +302,7 @@ __device__ __forceinline__ void lookup_read(const IndexView& I, const MapConfig&
         R.n_found = tot;
     }
     if (rescue) {
-        // Reads inside short tandem repeats merge thousands of hits: their seeds'
-        // runs (up to the count cap) estimate the merge's hits; reads above
-        // kRescueHeavyHits (C.rescue_block_hits when set) go to the heavy end of the
-        // list, which the rescue kernel takes first.
-        uint32_t w = 0;
-        if (good < tot) {
-            for (uint32_t i = lane; i < nq2; i += 32) {
-                const uint64_t pos = A.q_pos[R.q_off + i];
-                if (pos == kNotFound) continue;
-                const uint32_t c = index_get_count(I, pos);
-                w += c <= C.count_cap ? c : 0u;
-            }
-            w = warp_sum(w);
-        }
-        const bool heavy = w >= (C.rescue_block_hits ? C.rescue_block_hits : kRescueHeavyHits);
-        if (lane == 0) {
-            R.flags |= kReadRescue;
-            if (heavy) A.rescue_list[A.rescue_cap - 1 - atomicAdd(&ctr->n_rescue_heavy, 1u)] = r;
-            else A.rescue_list[atomicAdd(&ctr->n_rescue, 1u)] = r;
-            R.n_hits = 0;
-        }
+        enlist_rescue(I, C, r, R, A, ctr, good < tot);
         return;
     }
     // hit offsets in generation order (query order, then run order)
@@ -254,7 +316,7 @@ __device__ __forceinline__ void lookup_read(const IndexView& I, const MapConfig&
     }
     __syncwarp();
     const uint64_t H = running;
-    const uint64_t hoff = warp_bump(&ctr->hit_used, H);
+    const uint64_t hoff = room.take(&ctr->hit_used, H, arena_piece(A.hit_cap));
     if (hoff + H > A.hit_cap) {
         warp_fail(R, ctr, kStatusHitOverflow);
         return;
@@ -284,8 +346,18 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_lookup(IndexView I, Map
                                                                  ReadRec* __restrict__ rec, Arenas A, Counters* ctr,
                                                                  const BatchDesc* desc) {
     if (desc) n = min(n, desc->n_reads);   // batched form: n is the work areas' capacity
-    for (uint32_t r = warp_next(&ctr->queue_head2); r < n; r = warp_next(&ctr->queue_head2))
-        lookup_read<kCount>(I, C, r, rec, A, ctr);
+    const uint32_t per = items_per_take(n);
+    WarpRoom room;
+    uint32_t left = 0, r = 0;
+    for (;; ++r, --left) {
+        if (left == 0) {
+            r = warp_take(&ctr->queue_head2, per);
+            left = per;
+        }
+        if (r >= n) break;
+        lookup_read<kCount>(I, C, r, rec, A, ctr, room);
+    }
+    room.done(&ctr->hit_spare);
 }
 
 // The lookup of the reads seeded by k_seed_long (the long list).
@@ -294,8 +366,207 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_lookup_long(IndexView I
                                                                       ReadRec* __restrict__ rec, Arenas A,
                                                                       Counters* ctr) {
     const uint32_t n_long = *(volatile unsigned int*)&ctr->n_long;
+    WarpRoom room;
     for (uint32_t t = warp_global_id(); t < n_long; t += warp_count())
-        lookup_read<kCount>(I, C, A.long_list[t], rec, A, ctr);
+        lookup_read<kCount>(I, C, A.long_list[t], rec, A, ctr, room);
+    room.done(&ctr->hit_spare);
+}
+
+// Seeding and lookup of a read in one go, for the reads nearly all batches are made of: only
+// A, C, G and T, no tied syncmer window, at most kFastQueries queries, and parameters and
+// an index for which fast_seed() holds (all profiles of read lengths).  Returns false, with
+// nothing written, for any other read (the caller then takes the steps one by one).
+//
+// Both orientations' randstrobes run through one loop (the reverse ones walk the syncmers
+// downwards; the distance between two syncmers is the same either way), a query goes from
+// the lane that selects it straight into the index, and what is left of it for the hits (its
+// interval, the run's place and first entry) lies in the warp's scratch slot, which stays in
+// L2, instead of passing query, position and count through the arena: 2,290 warp
+// instructions a read of 150 bp (2,710 by the steps), both bound by integer issue; with the
+// tags and with one atomic a piece (WarpRoom, items_per_take) 2M reads 6.05 -> 4.5 ms, 100k
+// reads of 300 bp 1.12 -> 1.00 ms, of 400 bp 1.36 -> 1.10 ms.
+constexpr uint32_t kFastQueries = 256;
+
+__host__ __device__ __forceinline__ bool fast_seed(const DevParams& P, const IndexView& I, const MapConfig& C) {
+    return P.q <= 0xFF && P.W <= 32 && I.buckets != nullptr && I.filter_cutoff <= 255 && !C.force_rescue && !C.count_bytes;
+}
+
+__device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I, const MapConfig& C,
+                                          const uint8_t* __restrict__ seq, uint32_t L, uint32_t r,
+                                          ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr, uint64_t* pk,
+                                          uint32_t* ring, uint64_t* sh, uint32_t* sp, uint32_t cap, WarpRoom& room,
+                                          uint32_t& direct) {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
+    const uint32_t lane = lane_id();
+    if (L < (uint32_t)P.k || !warp_pack_clean(seq, L, pk)) return false;
+    const uint32_t nwin = L - (uint32_t)P.k + 1;
+    const uint32_t n = P.W == 5 && P.t == 3 && P.s <= 16 ? warp_clean_syncmers<5>(P, pk, nwin, ring, sp, cap)
+                                                         : warp_clean_syncmers<0>(P, pk, nwin, ring, sp, cap);
+    if (n > cap) return false;   // (ties too)
+    const uint32_t nq = n_query_per_dir(P, n, L), nq2 = 2 * nq;
+    if (nq2 > kFastQueries) return false;
+    // the syncmers' hashes; their positions and the hash bits that the selection compares
+    for (uint32_t i = lane; i < n; i += 32) {
+        const uint32_t w = sp[i];
+        const uint64_t h = kmer_hash(P, pk, w);
+        sh[i] = h;
+        sp[i] = (w << 8) | ((uint32_t)h & 0xFFu);
+    }
+    __syncwarp();
+    const uint32_t q8 = (uint32_t)P.q, k = (uint32_t)P.k;
+    // per found query: its interval, the run's place, the run's first entry
+    uint4* found = reinterpret_cast<uint4*>(A.slots + (uint64_t)warp_global_id() * A.slot_bytes);
+    uint64_t hits = 0;   // a byte a round
+    uint32_t tot = 0, good = 0, sum = 0, is_found = 0;   // is_found: a bit a round
+    for (uint32_t round = 0; 32 * round < nq2; ++round) {
+        const uint32_t i = 32 * round + lane;
+        Probe p;
+        p.pos = kMissing;
+        p.filtered = false;
+        p.n_hits = 0;
+        if (i < nq2) {
+            const bool rev = i >= nq;
+            const uint32_t j = rev ? i - nq : i;
+            const int i1 = (int)(rev ? n - 1 - j : j), dir = rev ? -1 : 1;
+            const uint32_t v1 = sp[i1], p1 = v1 >> 8;
+            const uint32_t last = min(P.w_max, n - 1 - j);
+            uint32_t best = 0xFFFFFFFFu;
+            for (uint32_t x = P.w_min; x <= last; ++x) {
+                const uint32_t v = sp[i1 + dir * (int)x];
+                const uint32_t dist = rev ? p1 - (v >> 8) : (v >> 8) - p1;
+                if (dist > P.max_dist) break;
+                best = min(best, ((uint32_t)__popc((v ^ v1) & q8) << 16) | x);   // the first of the least
+            }
+            const int i2 = best == 0xFFFFFFFFu ? i1 : i1 + dir * (int)(best & 0xFFFFu);
+            const uint32_t p2 = sp[i2] >> 8;
+            const uint32_t s1 = rev ? L - p1 - k : p1, e2 = rev ? L - p2 : p2 + k;
+            p = index_probe(I, sh[i1] + sh[i2], (int)(e2 - s1));
+            if (p.pos != kMissing) {
+                found[i] = make_uint4(s1 | (e2 << 16), p.pos, p.position, p.packed);
+                is_found |= 1u << round;
+                hits |= (uint64_t)p.n_hits << (8 * round);
+                sum += p.n_hits;
+            }
+        }
+        tot += __popc(__ballot_sync(kFull, p.pos != kMissing));
+        good += __popc(__ballot_sync(kFull, p.pos != kMissing && !p.filtered));
+    }
+    ReadRec& R = rec[r];
+    // nonrepetitive_fraction (step2/nam.cu:892) and the rescue trigger, as in lookup_read
+    const float frac = tot > 0 ? ((float)good) / ((float)tot) : 1.0f;
+    const bool rescue = C.rescue_level > 1 && (good == 0 || (double)frac < 0.7);
+    if (lane == 0) {
+        R.frac = frac;
+        R.n_found = tot;
+    }
+    if (rescue) {
+        // the rescue kernel reads the found queries from the arena
+        const uint64_t off = warp_bump(&ctr->q_used, nq2);
+        if (off + nq2 > A.q_cap) {
+            warp_fail(R, ctr, kStatusQueryOverflow);
+            if (lane == 0) R.nq = R.nq2 = 0;
+            return true;
+        }
+        if (lane == 0) {
+            R.q_off = off;
+            R.nq = nq;
+            R.nq2 = nq2;
+        }
+        for (uint32_t round = 0; 32 * round < nq2; ++round) {
+            const uint32_t i = 32 * round + lane;
+            if (i >= nq2) continue;
+            uint64_t pos = kNotFound;
+            if ((is_found >> round) & 1u) {
+                const uint4 f = found[i];
+                pos = f.y;
+                A.q[off + i] = Query{0, f.x & 0xFFFFu, f.x >> 16};
+            }
+            A.q_pos[off + i] = pos;
+        }
+        __syncwarp();
+        enlist_rescue(I, C, r, R, A, ctr, good < tot);
+        __syncwarp();
+        return true;
+    }
+    const uint32_t H = __reduce_add_sync(kFull, sum);
+    direct += nq2;
+    const uint64_t hoff = room.take(&ctr->hit_used, H, arena_piece(A.hit_cap));
+    if (hoff + H > A.hit_cap) {
+        warp_fail(R, ctr, kStatusHitOverflow);
+        return true;
+    }
+    // the hits in generation order (query order, then run order)
+    HitPacked* out = A.hits + hoff;
+    uint32_t at = 0;
+    for (uint32_t round = 0; 32 * round < nq2; ++round) {
+        const uint32_t i = 32 * round + lane;
+        const uint32_t nh = (uint32_t)(hits >> (8 * round)) & 0xFFu;
+        const uint32_t any = __ballot_sync(kFull, nh != 0);
+        if (!any) continue;
+        uint32_t to = at + __popc(any & lanemask_lt());
+        if (__any_sync(kFull, nh > 1)) {
+            const uint32_t inc = warp_inclusive_sum(nh);
+            to = at + inc - nh;
+            at += __shfl_sync(kFull, inc, 31);
+        } else {
+            at += __popc(any);
+        }
+        if (nh) {
+            const uint4 f = found[i];
+            const uint32_t rc = i >= nq ? 0x80000000u : 0u;
+            const int qs = (int)(f.x & 0xFFFFu), qe = (int)(f.x >> 16);
+            if (nh == 1) {
+                out[to] = pack_hit(rc | (f.w >> 8), qs, qe, (int)f.z, (int)(f.z + (f.w & 0xFFu) + k));
+            } else {
+                walk_hit_run(I, qs, qe, f.y, [&](uint32_t ref, int rs, int re) {
+                    out[to++] = pack_hit(rc | ref, qs, qe, rs, re);
+                });
+            }
+        }
+    }
+    if (lane == 0) {
+        R.hit_off = hoff;
+        R.n_hits = H;
+    }
+    __syncwarp();
+    return true;
+}
+
+// The same read by the steps: seeding into the query arena, then lookup_read.  Reads that do
+// not fit the shared-memory buffers go to the long list.
+template <bool kCount, bool kLookup>
+__device__ __forceinline__ void step_read(const DevParams& P, const IndexView& I, const MapConfig& C,
+                                          const uint8_t* seq, uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A,
+                                          Counters* ctr, uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh,
+                                          uint32_t* sp, uint32_t max_len, uint32_t cap, WarpRoom& queries,
+                                          WarpRoom& hits) {
+    ReadRec& R = rec[r];
+    uint32_t ns = 0xFFFFFFFFu;
+    if (L <= max_len) ns = warp_read_syncmers(P, seq, L, pk, nm, hb, sh, sp, cap);
+    if (ns == 0xFFFFFFFFu) {
+        if (lane_id() == 0) {
+            R.flags |= kReadLong;
+            A.long_list[atomicAdd(&ctr->n_long, 1u)] = r;
+        }
+        return;
+    }
+    emit_read_queries(P, sh, sp, ns, L, R, A, ctr, queries);
+    __syncwarp();
+    if (kLookup) {
+        lookup_read<kCount>(I, C, r, rec, A, ctr, hits);
+        __syncwarp();
+    }
+}
+
+// step_read beside the fast path: out of line, for the few reads that need it.
+__device__ __noinline__ void slow_read(const DevParams& P, const IndexView& I, const MapConfig& C, const uint8_t* seq,
+                                       uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A, Counters* ctr,
+                                       uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh, uint32_t* sp,
+                                       uint32_t max_len, uint32_t cap) {
+    WarpRoom queries, hits;
+    step_read<false, true>(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, max_len, cap, queries, hits);
+    queries.done(&ctr->q_spare);
+    hits.done(&ctr->hit_spare);
 }
 
 // Seeding and lookup of a read by one warp (the main path): randstrobes_query, then
@@ -312,7 +583,7 @@ constexpr int kFusedBlocksPerSm = 6;
 constexpr uint32_t kFusedMaxLen = 512;
 constexpr uint32_t kFusedSyncmers = 160;
 
-template <bool kCount>
+template <bool kCount, bool kFast>
 __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
     k_seed_lookup(DevParams P, IndexView I, MapConfig C, const uint8_t* __restrict__ seqs,
                   const uint64_t* __restrict__ offs, const uint32_t* __restrict__ lens, uint32_t n,
@@ -323,28 +594,34 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
     __shared__ uint64_t s_sh[kSeedWarps][kFusedSyncmers];
     __shared__ uint32_t s_sp[kSeedWarps][kFusedSyncmers];
     const uint32_t w = threadIdx.x >> 5;
-    for (uint32_t r = warp_next(&ctr->queue_head); r < n; r = warp_next(&ctr->queue_head)) {
+    const uint32_t per = items_per_take(n);
+    WarpRoom room, queries;
+    uint32_t direct = 0, left = 0, r = 0;
+    for (;; ++r, --left) {
+        if (left == 0) {
+            r = warp_take(&ctr->queue_head, per);
+            left = per;
+        }
+        if (r >= n) break;
         const uint32_t L = lens[r];
-        ReadRec& R = rec[r];
         if (L > GBSA_MAX_READ_LEN) {
-            warp_fail(R, ctr, kStatusReadTooLong);
+            warp_fail(rec[r], ctr, kStatusReadTooLong);
             continue;
         }
-        uint32_t ns = 0xFFFFFFFFu;
-        if (L <= kFusedMaxLen)
-            ns = warp_read_syncmers(P, seqs + offs[r], L, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w], kFusedSyncmers);
-        if (ns == 0xFFFFFFFFu) {
-            if (lane_id() == 0) {
-                R.flags |= kReadLong;
-                A.long_list[atomicAdd(&ctr->n_long, 1u)] = r;
-            }
-            continue;
+        if (kFast) {
+            if (L > kFusedMaxLen ||
+                !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], reinterpret_cast<uint32_t*>(s_hb[w]),
+                           s_sh[w], s_sp[w], kFusedSyncmers, room, direct))
+                slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
+                          kFusedMaxLen, kFusedSyncmers);
+        } else {
+            step_read<kCount, true>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w],
+                                    s_sp[w], kFusedMaxLen, kFusedSyncmers, queries, room);
         }
-        emit_read_queries(P, s_sh[w], s_sp[w], ns, L, R, A, ctr);
-        __syncwarp();
-        lookup_read<kCount>(I, C, r, rec, A, ctr);
-        __syncwarp();
     }
+    room.done(&ctr->hit_spare);
+    if (!kFast) queries.done(&ctr->q_spare);
+    if (direct && lane_id() == 0) atomicAdd(&ctr->q_direct, (unsigned long long)direct);
 }
 
 // The batched form's seeding + lookup: the body of k_seed_lookup, but each warp pulls
@@ -355,7 +632,7 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
 // template of its own per variant, picked at run time.
 // kLookup false: seeding alone (indexes whose entries exceed the fuse limit are looked
 // up by k_lookup afterwards, as in the plain form).
-template <bool kCount, bool kLookup, int kWarps, int kBlocks, uint32_t kMaxLen, uint32_t kSyncmers>
+template <bool kCount, bool kLookup, bool kFast, int kWarps, int kBlocks, uint32_t kMaxLen, uint32_t kSyncmers>
 __global__ void __launch_bounds__(32 * kWarps, kBlocks)
     k_seed_lookup_q(DevParams P, IndexView I, MapConfig C, const BatchDesc* __restrict__ desc,
                     ReadRec* __restrict__ rec, Arenas A, Counters* ctr) {
@@ -370,8 +647,14 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
     const uint32_t* __restrict__ lens = desc->lens;
     const uint32_t* __restrict__ items = desc->items;
     const uint32_t n_items = items ? desc->n_items : desc->n_reads;
-    for (;;) {
-        const uint32_t it = warp_next(&ctr->queue_head);
+    const uint32_t per = items_per_take(n_items);
+    WarpRoom room, queries;
+    uint32_t direct = 0, left = 0, it = 0;
+    for (;; ++it, --left) {
+        if (left == 0) {
+            it = warp_take(&ctr->queue_head, per);
+            left = per;
+        }
         if (it >= n_items) break;
         // item bounds outside [0, n_reads] are clamped (reads no item covers stay empty)
         const uint32_t n_reads = desc->n_reads;
@@ -379,29 +662,25 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
         const uint32_t r1 = min(items ? items[it + 1] : it + 1, n_reads);
         for (uint32_t r = r0; r < r1; ++r) {
             const uint32_t L = lens[r];
-            ReadRec& R = rec[r];
             if (L > GBSA_MAX_READ_LEN) {
-                warp_fail(R, ctr, kStatusReadTooLong);
+                warp_fail(rec[r], ctr, kStatusReadTooLong);
                 continue;
             }
-            uint32_t ns = 0xFFFFFFFFu;
-            if (L <= kMaxLen)
-                ns = warp_read_syncmers(P, seqs + offs[r], L, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w], kSyncmers);
-            if (ns == 0xFFFFFFFFu) {
-                if (lane_id() == 0) {
-                    R.flags |= kReadLong;
-                    A.long_list[atomicAdd(&ctr->n_long, 1u)] = r;
-                }
-                continue;
-            }
-            emit_read_queries(P, s_sh[w], s_sp[w], ns, L, R, A, ctr);
-            __syncwarp();
-            if (kLookup) {
-                lookup_read<kCount>(I, C, r, rec, A, ctr);
-                __syncwarp();
+            if (kFast) {
+                if (L > kMaxLen ||
+                    !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w],
+                               reinterpret_cast<uint32_t*>(s_hb[w]), s_sh[w], s_sp[w], kSyncmers, room, direct))
+                    slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
+                              kMaxLen, kSyncmers);
+            } else {
+                step_read<kCount, kLookup>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w],
+                                           s_sh[w], s_sp[w], kMaxLen, kSyncmers, queries, room);
             }
         }
     }
+    room.done(&ctr->hit_spare);
+    if (!kFast) queries.done(&ctr->q_spare);
+    if (direct && lane_id() == 0) atomicAdd(&ctr->q_direct, (unsigned long long)direct);
 }
 
 // Scratch of `bytes` for the calling warp: its own slot from byte `slot_off` on when
@@ -584,7 +863,8 @@ __device__ __forceinline__ void each_row(F&& f) {
 constexpr uint32_t kNoRead = 0xFFFFFFFFu;
 template <int G, int R>
 __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr,
-                                const uint32_t* __restrict__ list, uint32_t first, uint32_t cnt, GroupShared<R>& S) {
+                                const uint32_t* __restrict__ list, uint32_t first, uint32_t cnt, GroupShared<R>& S,
+                                WarpRoom& room) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     constexpr uint32_t kNoRef = 0xFFFFFFFFu;   // a hit's reference id has 24 bits
     const uint32_t lane = lane_id();
@@ -746,11 +1026,11 @@ __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, c
             ranks += (uint64_t)more << (8 * (f >> 5));
         }
     }
-    // NAM arena: one reservation a warp
+    // NAM arena
     const uint32_t count = sub == 0 ? n : 0;
     const uint32_t inc = warp_inclusive_sum(count);
     const uint32_t total = __shfl_sync(kFull, inc, 31);
-    const uint64_t off0 = warp_bump(&ctr->nam_used, total);
+    const uint64_t off0 = room.take(&ctr->nam_used, total, arena_piece(A.nam_cap));
     const uint64_t off = off0 + __shfl_sync(kFull, inc - count, base);
     if (off0 + total > A.nam_cap) {
         if (have && sub == 0) {
@@ -789,8 +1069,17 @@ __global__ void __launch_bounds__(32 * kGroupWarps, kGroupBlocksPerSm)
     if (threadIdx.x < kLaneBuckets) s_cnt[threadIdx.x] = *(volatile unsigned int*)&ctr->lane_cnt[threadIdx.x];
     __syncthreads();
     GroupShared<4>& S = s_group[threadIdx.x >> 5];
-    for (;;) {
-        uint32_t t = warp_next(&ctr->group_next);
+    uint32_t all = 0;
+    for (uint32_t b = 0; b < kLaneBuckets; ++b) all += s_cnt[b];
+    const uint32_t per = items_per_take(all / 4);
+    WarpRoom room;
+    uint32_t next = 0, left = 0;
+    for (;; ++next, --left) {
+        if (left == 0) {
+            next = warp_take(&ctr->group_next, per);
+            left = per;
+        }
+        uint32_t t = next;
         int b = (int)kLaneBuckets - 1;
         for (; b >= 0; --b) {
             const uint32_t shift = b < 2 ? 3u : (b < 4 ? 2u : (b < 8 ? 1u : 0u));   // log2 of the reads a warp
@@ -804,17 +1093,18 @@ __global__ void __launch_bounds__(32 * kGroupWarps, kGroupBlocksPerSm)
         if (b < 0) break;
         const uint32_t* list = A.lane_lists + (size_t)b * A.lane_cap;
         if (b < 2) {
-            group_merge<4, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+            group_merge<4, 4>(C, rec, A, ctr, list, t, s_cnt[b], S, room);
         } else if (b < 4) {
-            group_merge<8, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+            group_merge<8, 4>(C, rec, A, ctr, list, t, s_cnt[b], S, room);
         } else if (b < 8) {
-            group_merge<16, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+            group_merge<16, 4>(C, rec, A, ctr, list, t, s_cnt[b], S, room);
         } else {
-            const uint32_t r = group_merge<32, 4>(C, rec, A, ctr, list, t, s_cnt[b], S);
+            const uint32_t r = group_merge<32, 4>(C, rec, A, ctr, list, t, s_cnt[b], S, room);
             if (r != kNoRead && lane_id() == 0) A.big_list[atomicAdd(&ctr->n_big, 1u)] = r;
             __syncwarp();
         }
     }
+    room.done(&ctr->nam_spare);
 }
 
 // A NAM list in struct-of-arrays form (field f of NAM o at b[f * stride + o]), so that 32
@@ -2228,32 +2518,38 @@ SeedVariant seed_variant(int v) {
     return table[v < 0 || v >= kSeedVariants ? 0 : v];
 }
 
-template <bool kCount, bool kLookup, int kWarps, int kBlocks, uint32_t kMaxLen, uint32_t kSyncmers>
+template <bool kCount, bool kLookup, bool kFast, int kWarps, int kBlocks, uint32_t kMaxLen, uint32_t kSyncmers>
 static void launch_q(const DevParams& P, const IndexView& I, const MapConfig& C, const BatchDesc* desc, ReadRec* rec,
-                     Arenas A, Counters* ctr, cudaStream_t st) {
-    const unsigned grid = (unsigned)device_sm_count() * kBlocks;
-    launch_probe(k_seed_lookup_q<kCount, kLookup, kWarps, kBlocks, kMaxLen, kSyncmers>, grid, 32 * kWarps, 0, st, C,
+                     Arenas A, Counters* ctr, uint32_t cap, cudaStream_t st) {
+    // resident blocks, and a scratch slot a warp (the work areas hold nam_kernel_warps(cap))
+    const unsigned grid = std::min<unsigned>((unsigned)device_sm_count() * kBlocks,
+                                             std::max(1u, nam_kernel_warps(cap) / kWarps));
+    launch_probe(k_seed_lookup_q<kCount, kLookup, kFast, kWarps, kBlocks, kMaxLen, kSyncmers>, grid, 32 * kWarps, 0, st, C,
                  P, I, C, desc, rec, A, ctr);
 }
 
-template <bool kCount, bool kLookup>
+template <bool kCount, bool kLookup, bool kFast>
 static void launch_q_variant(int v, const DevParams& P, const IndexView& I, const MapConfig& C, const BatchDesc* desc,
-                             ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
+                             ReadRec* rec, Arenas A, Counters* ctr, uint32_t cap, cudaStream_t st) {
     switch (v) {
-        case 1: launch_q<kCount, kLookup, 8, 5, 512, 160>(P, I, C, desc, rec, A, ctr, st); break;
-        case 2: launch_q<kCount, kLookup, 4, 12, 512, 160>(P, I, C, desc, rec, A, ctr, st); break;
-        case 3: launch_q<kCount, kLookup, 8, 7, 256, 96>(P, I, C, desc, rec, A, ctr, st); break;
-        case 4: launch_q<kCount, kLookup, 16, 3, 512, 160>(P, I, C, desc, rec, A, ctr, st); break;
-        case 5: launch_q<kCount, kLookup, 8, 6, 256, 96>(P, I, C, desc, rec, A, ctr, st); break;
-        default: launch_q<kCount, kLookup, 8, 6, 512, 160>(P, I, C, desc, rec, A, ctr, st); break;
+        case 1: launch_q<kCount, kLookup, kFast, 8, 5, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
+        case 2: launch_q<kCount, kLookup, kFast, 4, 12, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
+        case 3: launch_q<kCount, kLookup, kFast, 8, 7, 256, 96>(P, I, C, desc, rec, A, ctr, cap, st); break;
+        case 4: launch_q<kCount, kLookup, kFast, 16, 3, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
+        case 5: launch_q<kCount, kLookup, kFast, 8, 6, 256, 96>(P, I, C, desc, rec, A, ctr, cap, st); break;
+        default: launch_q<kCount, kLookup, kFast, 8, 6, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
     }
 }
 
+bool seeds_fast(const DevParams& P, const IndexView& I, const MapConfig& C) { return fast_seed(P, I, C); }
+
 void launch_seed_lookup_queue(const DevParams& P, const IndexView& I, const MapConfig& C, const BatchDesc* desc,
-                              ReadRec* rec, Arenas A, Counters* ctr, int variant, bool lookup, cudaStream_t st) {
-    if (!lookup) launch_q_variant<false, false>(variant, P, I, C, desc, rec, A, ctr, st);
-    else if (C.count_bytes) launch_q_variant<true, true>(variant, P, I, C, desc, rec, A, ctr, st);
-    else launch_q_variant<false, true>(variant, P, I, C, desc, rec, A, ctr, st);
+                              ReadRec* rec, Arenas A, Counters* ctr, int variant, bool lookup, uint32_t cap,
+                              cudaStream_t st) {
+    if (!lookup) launch_q_variant<false, false, false>(variant, P, I, C, desc, rec, A, ctr, cap, st);
+    else if (C.count_bytes) launch_q_variant<true, true, false>(variant, P, I, C, desc, rec, A, ctr, cap, st);
+    else if (fast_seed(P, I, C)) launch_q_variant<false, true, true>(variant, P, I, C, desc, rec, A, ctr, cap, st);
+    else launch_q_variant<false, true, false>(variant, P, I, C, desc, rec, A, ctr, cap, st);
     GBSA_LAUNCHED();
 }
 
@@ -2263,7 +2559,8 @@ void launch_seed_lookup(const DevParams& P, const IndexView& I, const MapConfig&
     if (!n) return;
     // resident blocks only: the warps pull reads from the work counter until none is left
     const unsigned grid = std::min<unsigned>(warp_grid(n, kSeedWarps), (unsigned)device_sm_count() * kFusedBlocksPerSm);
-    launch_probe(C.count_bytes ? k_seed_lookup<true> : k_seed_lookup<false>, grid, 32 * kSeedWarps, 0, st, C, P, I, C,
+    launch_probe(C.count_bytes ? k_seed_lookup<true, false>
+                               : (fast_seed(P, I, C) ? k_seed_lookup<false, true> : k_seed_lookup<false, false>), grid, 32 * kSeedWarps, 0, st, C, P, I, C,
                  seqs, offs, lens, n, rec, A, ctr);
     GBSA_LAUNCHED();
 }

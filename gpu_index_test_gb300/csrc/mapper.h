@@ -8,6 +8,9 @@
 
 struct gbsa_batcher;
 
+// gbsa_mapper::fuse_index_bytes while the caller has set no limit
+constexpr uint64_t kFuseAuto = ~0ull - 1;
+
 struct gbsa_mapper {
     const gbsa_index* idx = nullptr;
     gbsa_map_options opt{};
@@ -42,7 +45,7 @@ struct gbsa_mapper {
     double nams_per_read = 16.0;
     uint64_t retries = 0;   // batches run again after a work area grew
     bool fused = false;     // the last batch ran seeding and lookup as one kernel
-    uint64_t fuse_index_bytes = 2ull << 30;   // largest index (entry bytes) seeded and looked up in one kernel
+    uint64_t fuse_index_bytes = kFuseAuto;   // largest index (entry bytes) seeded and looked up in one kernel
     uint32_t pipe_chunks = 2;   // full chunks a large gbsa_map_reads call is cut into
     gbsa::Workspace ws;       // temporary device buffers of the prefix scans
     uint64_t alg_bytes = 0;   // algorithmic bytes of the last batch (when counting)

@@ -103,6 +103,37 @@ __device__ __forceinline__ bool warp_pack_read(const uint8_t* seq, uint32_t L, u
     return __any_sync(0xFFFFFFFFu, has_n);
 }
 
+// warp_pack_read for a read of only A, C, G and T (either case): false when it holds
+// anything else (packed is then incomplete).  A lane's 4 bases are one byte of a word, so
+// the lanes store bytes and nothing is exchanged.
+__device__ __forceinline__ bool warp_pack_clean(const uint8_t* seq, uint32_t L, uint64_t* packed) {
+    const uint32_t lane = lane_id();
+    const uint32_t nw = (L + 31) / 32 + 2;
+    const uintptr_t a0 = reinterpret_cast<uintptr_t>(seq);
+    const uint32_t mis = (uint32_t)(a0 & 3);
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(a0 - mis);
+    uint8_t* out = reinterpret_cast<uint8_t*>(packed);
+    bool clean = true;
+    for (uint32_t g = lane; g < 8 * nw; g += 32) {   // group g: bases 4 g .. 4 g + 3
+        const uint32_t p0 = 4 * g;
+        uint32_t code8 = 0;
+        if (p0 < L) {
+            const uint32_t lo = words[g];
+            const uint32_t hi = (mis != 0 && (g + 1) * 4 - mis < L) ? words[g + 1] : 0u;
+            const uint32_t w = __funnelshift_r(lo, hi, 8 * mis);   // base p0 in the low byte
+            const uint32_t c4 = ((w >> 1) ^ (w >> 2)) & 0x03030303u;
+            const uint32_t t = (c4 | (c4 >> 4)) & 0x00FF00FFu;
+            const uint32_t nv = min(L - p0, 4u);   // bases of the read among the 4
+            const uint32_t vmask = nv == 4 ? 0xFFFFFFFFu : (1u << (8 * nv)) - 1;
+            clean &= (((w & 0xDFDFDFDFu) ^ __byte_perm(0x54474341u, 0u, (t | (t >> 8)) & 0xFFFFu)) & vmask) == 0;
+            code8 = ((c4 & vmask) * 0x40100401u) >> 24;   // the first base highest
+        }
+        out[g ^ 7] = (uint8_t)code8;
+    }
+    __syncwarp();
+    return __all_sync(0xFFFFFFFFu, clean);
+}
+
 // n (<= 33) bits of an LSB-first u32 bitmask stream starting at bit p (two words
 // always cover them: the shift within the first word is at most 31).
 __device__ __forceinline__ uint64_t nbits33(const uint32_t* m, uint64_t p, int n) {
@@ -112,22 +143,23 @@ __device__ __forceinline__ uint64_t nbits33(const uint32_t* m, uint64_t p, int n
     return v & ((1ULL << n) - 1);
 }
 
+// The canonical s-mer at p, s <= 16, in the low 2 s bits.
+__device__ __forceinline__ uint32_t smer16(const DevParams& P, const uint64_t* packed, uint32_t p) {
+    // s-mers of up to 16 bases in 32 bits: the stream seen as 32-bit groups of 16
+    // bases (group g is the high half of word g/2 for even g, the low half for odd
+    // g; little-endian halves sit at u32 index g ^ 1)
+    const uint32_t* w32 = reinterpret_cast<const uint32_t*>(packed);
+    const uint32_t g = p >> 4;
+    uint32_t f = __funnelshift_l(w32[(g + 1) ^ 1], w32[g ^ 1], (p & 15) * 2);
+    f >>= 32 - 2 * P.s;   // P.s >= 1
+    uint32_t r = __brev(~f);
+    r = ((r >> 1) & 0x55555555u) | ((r & 0x55555555u) << 1);
+    r >>= 32 - 2 * P.s;
+    return f < r ? f : r;
+}
+
 __device__ __forceinline__ uint64_t smer_hash(const DevParams& P, const uint64_t* packed, uint64_t p) {
-    if (P.s <= 16) {
-        // s-mers of up to 16 bases in 32 bits: the stream seen as 32-bit groups of 16
-        // bases (group g is the high half of word g/2 for even g, the low half for odd
-        // g; little-endian halves sit at u32 index g ^ 1)
-        const uint32_t* w32 = reinterpret_cast<const uint32_t*>(packed);
-        const uint64_t g = p >> 4;
-        const uint32_t sh = (uint32_t)(p & 15) * 2;
-        const uint32_t hi = w32[g ^ 1], lo = w32[(g + 1) ^ 1];
-        uint32_t f = __funnelshift_l(lo, hi, sh);
-        f >>= 32 - 2 * P.s;   // P.s >= 1
-        uint32_t r = __brev(~f);
-        r = ((r >> 1) & 0x55555555u) | ((r & 0x55555555u) << 1);
-        r >>= 32 - 2 * P.s;
-        return xxh64((uint64_t)(f < r ? f : r));
-    }
+    if (P.s <= 16) return xxh64((uint64_t)smer16(P, packed, (uint32_t)p));
     const uint64_t f = extract_bases(packed, p, P.s);
     const uint64_t r = revcomp_bits(f, P.s);
     return xxh64(f < r ? f : r);
@@ -406,6 +438,43 @@ __device__ __forceinline__ uint32_t n_query_per_dir(const DevParams& P, uint32_t
     return n > P.w_min ? n - P.w_min : 0;
 }
 
+// Syncmers of a clean read (packed by warp_pack_clean).  A window is a syncmer when its s-mer
+// number t - 1 has the least hash of the W, decided on the hashes' high words, so that a
+// window costs W words of a ring of high words and a few minima.  Where that s-mer ties
+// with the least of the others the state machine's history may count: returns 0xFFFFFFFF,
+// and the caller takes the full scan.  kW: W when known at compile time (0: P.W).  sp: the
+// first `cap` syncmers' windows; ring: 64 words (32 + W - 1 <= 64).
+template <int kW>
+__device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, const uint64_t* packed, uint32_t nwin,
+                                                        uint32_t* ring, uint32_t* sp, uint32_t cap) {
+    const uint32_t lane = lane_id();
+    const uint32_t W = kW ? kW : (uint32_t)P.W, t = kW ? kW / 2 : (uint32_t)(P.t - 1);
+    uint32_t n = 0;
+    auto high = [&](uint32_t p) {
+        return (uint32_t)((kW ? xxh64((uint64_t)smer16(P, packed, p)) : smer_hash(P, packed, p)) >> 32);
+    };
+    if (lane < W - 1) ring[lane] = high(lane);
+    for (uint32_t c = 0; c < nwin; c += 32) {
+        const uint32_t w = c + lane;
+        ring[(w + W - 1) & 63] = high(w + W - 1);
+        __syncwarp();
+        const uint32_t mid = ring[(w + t) & 63];
+        uint32_t least = 0xFFFFFFFFu;
+#pragma unroll 4
+        for (uint32_t d = 0; d < W; ++d)
+            if (d != t) least = min(least, ring[(w + d) & 63]);
+        const bool in = w < nwin;
+        if (__any_sync(0xFFFFFFFFu, in && mid == least)) return 0xFFFFFFFFu;
+        const bool sync = in && mid < least;
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, sync);
+        const uint32_t idx = n + __popc(b & lanemask_lt());
+        if (sync && idx < cap) sp[idx] = w;
+        n += __popc(b);
+        __syncwarp();
+    }
+    return n;
+}
+
 // Writes the 2*nq query randstrobes of a read (forward, then reverse complement).
 // The two orientations take passes of their own: a pass that mixed them would run
 // both selection loops one after the other.
@@ -427,3 +496,4 @@ __device__ __forceinline__ void warp_write_queries(const DevParams& P, const uin
 }
 
 }  // namespace gbsa
+

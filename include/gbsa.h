@@ -612,15 +612,16 @@ int gbsa_bench_gather_index(const gbsa_index* idx, double* probes_per_s, double*
  * returns the last batch's milliseconds for: seeding + lookup (one kernel, a warp
  * per read; seeding alone when gbsa_mapper_fused_lookup is 0), long-read seeding,
  * long-read lookup + read bucketing (the whole lookup + bucketing when not fused),
- * NAM merge + sort (lane per read), NAM merge + sort (warp per read), rescue,
+ * NAM merge + sort (a group of lanes per read), NAM merge + sort (a warp or a block
+ * per read), rescue,
  * sorting of the rescued reads with many NAMs.  The last two run on a second stream
  * beside the two NAM stages and are timed from the end of the lookup.  No reference
  * counterpart. */
 int gbsa_mapper_set_profile(gbsa_mapper* m, int on);
 int gbsa_mapper_stage_ms(const gbsa_mapper* m, float* ms, int n);
 /* Work counts of the last batch: out[0] query randstrobes, [1] hits of the normal
- * path, [2] NAM-state arena slots taken by the merges (the room they reserve: two per hit
- * of a lane-merged read; not the NAMs output, which the call returns), [3] rescued reads,
+ * path, [2] NAM-state arena slots taken by the merges (the room they reserve, not the NAMs
+ * output, which the call returns), [3] rescued reads,
  * [4] reads seeded by the long-read kernel,
  * [5] overflow scratch bytes, [6] reads merged by the warp-cooperative NAM kernel.
  * out must hold 7 values.  No reference counterpart. */
@@ -629,13 +630,14 @@ int gbsa_mapper_last_counts(const gbsa_mapper* m, uint64_t* out);
  * scratch) was too small and has grown, since it was created.  No reference
  * counterpart. */
 uint64_t gbsa_mapper_retries(const gbsa_mapper* m);
-/* 1 when the last batch ran seeding and lookup as one kernel (indexes of up to 2 GiB
- * of entries), 0 when it ran them as two kernels (larger indexes); selects the
- * meaning of the first and third gbsa_mapper_stage_ms values.  No reference
- * counterpart. */
+/* 1 when the last batch ran seeding and lookup as one kernel, 0 when it ran them as
+ * two kernels (gbsa_mapper_set_fuse_limit); selects the meaning of the first and third
+ * gbsa_mapper_stage_ms values.  No reference counterpart. */
 int gbsa_mapper_fused_lookup(const gbsa_mapper* m);
 /* Largest index (bytes of entries, 16 per entry) whose batches run seeding and lookup
- * as one kernel; default 2 GiB.  0 runs them as two kernels for every index.  The
+ * as one kernel; until it is set, all where the reads take that kernel's fast path
+ * (selection masks of up to 8 bits, a filter cutoff of up to 255, no forced rescue), and
+ * those of up to 2 GiB otherwise.  0 runs them as two kernels for every index.  The
  * results are the same either way.  No reference counterpart. */
 int gbsa_mapper_set_fuse_limit(gbsa_mapper* m, uint64_t index_bytes);
 /* Hold the index's bucket table in L2 during the probing kernels (on = 1, the
