@@ -4,17 +4,17 @@
 // commented out in the reference) with the RandstrobeGenerator of
 // step2/randstrobes.cu:161-190:
 //   1. pack the contigs into a 2-bit stream + N bitmask (one pass over the bases);
-//   2. canonical syncmers of every contig, a warp per 2048-window segment (count
-//      pass, exclusive scan, write pass); a segment starts at an "anchor" window
-//      whose syncmer state does not depend on earlier windows;
+//   2. canonical syncmers of every contig, a warp per 2048-window segment (a bit a
+//      window and a count, exclusive scan, write pass); where the state machine is needed
+//      a segment starts at an "anchor" window whose syncmer state does not depend on
+//      earlier windows;
 //   3. one forward randstrobe per syncmer with at least w_min successors in its
 //      contig, packed = (ref_index << 8) + (strobe2 - strobe1); contigs shorter than
 //      w_max keep zeroed entries (counted, never assigned, as in the reference);
-//   4. stable LSD radix sort by (hash, position) — ties keep generation order, which
-//      is (ref_index, position), i.e. the table ends up sorted by (hash, position,
-//      packed);
-//   5. bucket start table with the reference's first-bucket rule, and the run-length
-//      statistics that give filter_cutoff (float product unique_mers * f).
+//   4. stable sort by (hash, position) — ties keep generation order, which is
+//      (ref_index, position), i.e. the table ends up sorted by (hash, position, packed);
+//   5. bucket tables with the reference's first-bucket rule, and the run-length
+//      statistics that give filter_cutoff (float product unique_mers * f), in one pass.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -59,33 +59,93 @@ struct SegTables {
     const uint32_t* contig_nwin;
 };
 
-template <bool kWrite>
-__global__ void __launch_bounds__(32 * kSegWarps) k_contig_syncmers(DevParams P, const uint64_t* __restrict__ packed,
-                                                                    const uint32_t* __restrict__ nmask, SegTables T,
-                                                                    uint32_t n_seg, uint64_t* __restrict__ seg_count,
-                                                                    const uint64_t* __restrict__ seg_off,
-                                                                    uint64_t* __restrict__ sh, uint32_t* __restrict__ sp) {
+constexpr uint32_t kSegWords = kSegWindows / 32;
+
+// The syncmers of each segment as a bit a window, and their number.  Bound by integer issue
+// (a 64-bit hash a window); segments of A, C, G and T without a tied window take the scan
+// that needs no state, the others the state machine from their anchor.
+__global__ void __launch_bounds__(32 * kSegWarps) k_mark_syncmers(DevParams P, const uint64_t* __restrict__ packed,
+                                                                  const uint32_t* __restrict__ nmask, SegTables T,
+                                                                  uint32_t n_seg, uint64_t* __restrict__ seg_count,
+                                                                  uint32_t* __restrict__ bits) {
     __shared__ uint64_t s_h[kSegWarps][64];
-    const uint32_t wid = threadIdx.x >> 5;
+    __shared__ uint32_t s_bits[kSegWarps][kSegWords];
+    const uint32_t wid = threadIdx.x >> 5, lane = lane_id();
     uint64_t* hbuf = s_h[wid];
+    uint32_t* own = s_bits[wid];
     for (uint32_t s = blockIdx.x * kSegWarps + wid; s < n_seg; s += gridDim.x * kSegWarps) {
         const uint32_t c = T.seg_contig[s];
         const uint32_t w0 = T.seg_w0[s], w1 = T.seg_w1[s];
         const uint64_t base = T.contig_base[c];
-        const uint32_t nwin = T.contig_nwin[c];
-        const uint32_t anchor = warp_find_anchor(P, packed, nmask, base, nwin, w0, hbuf);
-        if (kWrite) {
-            const uint64_t o = seg_off[s];
-            const uint32_t n = warp_syncmer_scan(P, packed, nmask, base, nwin, anchor, w1, w0, hbuf,
-                                                 [&](uint32_t idx, uint32_t w) { sp[o + idx] = w; });
+        const uint64_t g = base + w0;   // the segment's first base
+        const uint32_t words = ((uint32_t)(g & 31) + (w1 - w0) + (uint32_t)P.k - 1 + 31) / 32;
+        uint32_t any_n = P.W > 32 ? 1u : 0u;
+        for (uint32_t i = lane; i < words; i += 32) any_n |= nmask[(g >> 5) + i];
+        uint32_t n = 0;
+        auto put = [&](uint32_t at, uint32_t b) {
+            if (lane == 0) own[at >> 5] = b;
+            n += __popc(b);
+        };
+        bool ok = !__any_sync(0xFFFFFFFFu, any_n != 0);
+        if (ok) {
+            uint32_t* ring = reinterpret_cast<uint32_t*>(hbuf);
+            const uint64_t* pk = packed + (g >> 5);
+            const uint32_t p0 = (uint32_t)(g & 31);
+            ok = clean_scan5(P) ? warp_clean_scan<5>(P, pk, p0, w1 - w0, ring, put)
+                                : warp_clean_scan<0>(P, pk, p0, w1 - w0, ring, put);
             __syncwarp();
-            for (uint32_t i = lane_id(); i < n; i += 32) sh[o + i] = kmer_hash(P, packed, base + sp[o + i]);
-        } else {
-            const uint32_t n = warp_syncmer_scan(P, packed, nmask, base, nwin, anchor, w1, w0, hbuf,
-                                                 [](uint32_t, uint32_t) {});
-            if (lane_id() == 0) seg_count[s] = n;
         }
+        if (!ok) {
+            for (uint32_t i = lane; i < kSegWords; i += 32) own[i] = 0;
+            __syncwarp();
+            const uint32_t nwin = T.contig_nwin[c];
+            const uint32_t anchor = warp_find_anchor(P, packed, nmask, base, nwin, w0, hbuf);
+            n = warp_syncmer_scan(P, packed, nmask, base, nwin, anchor, w1, w0, hbuf,
+                                  [&](uint32_t, uint32_t w) { atomicOr(&own[(w - w0) >> 5], 1u << ((w - w0) & 31)); });
+        }
+        __syncwarp();
+        for (uint32_t i = lane; 32 * i < w1 - w0; i += 32) bits[(uint64_t)s * kSegWords + i] = own[i];
+        if (lane == 0) seg_count[s] = n;
+        __syncwarp();
     }
+}
+
+// The marked windows' k-mer hashes and positions, in order.
+__global__ void __launch_bounds__(32 * kSegWarps) k_write_syncmers(DevParams P, const uint64_t* __restrict__ packed,
+                                                                   SegTables T, uint32_t n_seg,
+                                                                   const uint64_t* __restrict__ seg_off,
+                                                                   const uint32_t* __restrict__ bits,
+                                                                   uint64_t* __restrict__ sh,
+                                                                   uint32_t* __restrict__ sp) {
+    __shared__ uint16_t s_w[kSegWarps][kSegWindows];
+    const uint32_t wid = threadIdx.x >> 5, lane = lane_id();
+    for (uint32_t s = blockIdx.x * kSegWarps + wid; s < n_seg; s += gridDim.x * kSegWarps) {
+        const uint32_t w0 = T.seg_w0[s], w1 = T.seg_w1[s];
+        const uint64_t g = T.contig_base[T.seg_contig[s]] + w0;
+        uint32_t n = 0;
+        for (uint32_t i = 0; 32 * i < w1 - w0; i += 32) {
+            uint32_t b = 32 * (i + lane) < w1 - w0 ? bits[(uint64_t)s * kSegWords + i + lane] : 0u;
+            const uint32_t cnt = __popc(b), inc = warp_inclusive_sum(cnt);
+            for (uint32_t at = n + inc - cnt; b; b &= b - 1) s_w[wid][at++] = (uint16_t)(32 * (i + lane) + __ffs(b) - 1);
+            n += __shfl_sync(0xFFFFFFFFu, inc, 31);
+        }
+        __syncwarp();
+        const uint64_t o = seg_off[s];
+        for (uint32_t i = lane; i < n; i += 32) {
+            const uint32_t w = s_w[wid][i];
+            sp[o + i] = w0 + w;
+            sh[o + i] = kmer_hash(P, packed, g + w);
+        }
+        __syncwarp();
+    }
+}
+
+// The first syncmer of every contig, and their number at the end.
+__global__ void k_contig_starts(const uint64_t* __restrict__ seg_off, const uint64_t* __restrict__ first_seg,
+                                uint32_t n_contigs, uint32_t n_seg, const uint64_t* __restrict__ total,
+                                uint64_t* __restrict__ out) {
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c <= n_contigs; c += gridDim.x * blockDim.x)
+        out[c] = first_seg[c] < n_seg ? seg_off[first_seg[c]] : *total;
 }
 
 __global__ void k_ref_randstrobes(DevParams P, const uint64_t* __restrict__ sh, const uint32_t* __restrict__ sp,
@@ -150,10 +210,16 @@ __device__ __forceinline__ Bucket bucket_at(const gbsa_ref_randstrobe* __restric
 }
 
 // The bucket table (the reference's first-bucket rule: the buckets up to the first entry's
-// start at the second run) and, where `buckets` is set, the lookup's form of it, in one
-// pass: an entry that opens a bucket writes it and the empty ones before it.
-__global__ void k_bucket_starts(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, int bits,
-                                uint64_t* __restrict__ starts, Bucket* __restrict__ buckets) {
+// start at the second run), where `buckets` is set the lookup's form of it, and the
+// histogram of the runs' lengths (bins 1..100 exact, bin 101: longer), in one pass: an entry
+// that opens a bucket writes it and the empty ones before it, one that opens a run walks it
+// (102 entries at most).
+__global__ void __launch_bounds__(256) k_tables(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, int bits,
+                                                uint64_t* __restrict__ starts, Bucket* __restrict__ buckets,
+                                                unsigned long long* __restrict__ hist) {
+    __shared__ unsigned int h[102];
+    for (int i = threadIdx.x; i < 102; i += blockDim.x) h[i] = 0;
+    __syncthreads();
     const uint64_t nb = 1ULL << bits;
     auto put = [&](uint64_t b0, uint64_t b1, uint64_t at, uint64_t own) {   // [b0, b1), `own`: where at's entries lie
         for (uint64_t b = b0; b < b1; ++b) {
@@ -161,36 +227,22 @@ __global__ void k_bucket_starts(const gbsa_ref_randstrobe* __restrict__ rs, uint
             if (buckets) buckets[b] = b == own ? bucket_at(rs, n, bits, b, at) : Bucket{(uint32_t)at, 0u};
         }
     };
+    uint32_t once = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t t = rs[i].hash >> (64 - bits);
+        const uint64_t hash = rs[i].hash, t = hash >> (64 - bits);
+        const uint64_t before = i ? rs[i - 1].hash : ~hash;
         if (i == 0) put(0, t + 1, second_run(rs, n), t);
-        else put((rs[i - 1].hash >> (64 - bits)) + 1, t + 1, i, t);
+        else put((before >> (64 - bits)) + 1, t + 1, i, t);
         if (i == n - 1) put(t + 1, nb + 1, n, nb + 1);
+        if (hash != before) {
+            uint32_t len = 1;
+            while (len < 101 && i + len < n && rs[i + len].hash == hash) ++len;
+            if (len == 1) ++once;
+            else atomicAdd(&h[len], 1u);
+        }
     }
-}
-
-__global__ void k_run_flags(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, uint64_t* __restrict__ flags) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        flags[i] = (i == 0 || rs[i].hash != rs[i - 1].hash) ? 1 : 0;
-}
-
-__global__ void k_run_starts(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, const uint64_t* __restrict__ idx,
-                             uint64_t* __restrict__ run_start) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        if (i == 0 || rs[i].hash != rs[i - 1].hash) run_start[idx[i]] = i;
-}
-
-// histogram of run lengths: bins 1..100 exact, bin 101 = longer
-__global__ void k_run_hist(const uint64_t* __restrict__ run_start, uint64_t n_runs, uint64_t n,
-                           unsigned long long* __restrict__ hist) {
-    __shared__ unsigned int h[102];
-    for (int i = threadIdx.x; i < 102; i += blockDim.x) h[i] = 0;
-    __syncthreads();
-    for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n_runs; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t e = (j + 1 < n_runs) ? run_start[j + 1] : n;
-        const uint64_t len = e - run_start[j];
-        atomicAdd(&h[len > 101 ? 101 : len], 1u);
-    }
+    once = __reduce_add_sync(0xFFFFFFFFu, once);
+    if (lane_id() == 0 && once) atomicAdd(&h[1], once);
     __syncthreads();
     for (int i = threadIdx.x; i < 102; i += blockDim.x)
         if (h[i]) atomicAdd(&hist[i], (unsigned long long)h[i]);
@@ -307,39 +359,39 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     SegTables T{d_segc.as<uint32_t>(), d_segw0.as<uint32_t>(), d_segw1.as<uint32_t>(), d_cbase.as<uint64_t>(),
                 d_cnwin.as<uint32_t>()};
 
-    DeviceBuffer d_segcnt(8 * (n_seg + 1)), d_segoff(8 * (n_seg + 1));
-    uint64_t n_sm = 0;
+    DeviceBuffer d_segcnt(8 * (n_seg + 1)), d_segoff(8 * (n_seg + 1)), d_cseg(8 * (n_contigs + 1));
+    DeviceBuffer d_bits(4ull * kSegWords * (n_seg + 1)), d_csm(8 * (n_contigs + 1));
     const unsigned seg_blocks = grid_for(n_seg, kSegWarps, 1u << 20);
+    std::vector<uint64_t> csm(n_contigs + 1, 0);   // first syncmer of every contig, and their number
     if (n_seg) {
-        k_contig_syncmers<false><<<seg_blocks, 32 * kSegWarps, 0, st>>>(P, d_packed.as<uint64_t>(),
-                                                                        d_nmask.as<uint32_t>(), T, n_seg,
-                                                                        d_segcnt.as<uint64_t>(), nullptr, nullptr,
-                                                                        nullptr);
+        GBSA_CUDA(cudaMemcpyAsync(d_cseg.as<void>(), cfirst_seg.data(), 8 * (n_contigs + 1), cudaMemcpyHostToDevice, st));
+        k_mark_syncmers<<<seg_blocks, 32 * kSegWarps, 0, st>>>(P, d_packed.as<uint64_t>(), d_nmask.as<uint32_t>(), T,
+                                                               n_seg, d_segcnt.as<uint64_t>(), d_bits.as<uint32_t>());
         GBSA_LAUNCHED();
         uint64_t* d_tot = ws.get<uint64_t>(1);
         scan_exclusive_u64(d_segcnt.as<uint64_t>(), d_segoff.as<uint64_t>(), n_seg, d_tot, ws, st);
-        GBSA_CUDA(cudaMemcpyAsync(&n_sm, d_tot, 8, cudaMemcpyDeviceToHost, st));
+        k_contig_starts<<<grid_for(n_contigs + 1, 256, 4096), 256, 0, st>>>(
+            d_segoff.as<uint64_t>(), d_cseg.as<uint64_t>(), n_contigs, n_seg, d_tot, d_csm.as<uint64_t>());
+        GBSA_LAUNCHED();
+        GBSA_CUDA(cudaMemcpyAsync(csm.data(), d_csm.as<uint64_t>(), 8 * (n_contigs + 1), cudaMemcpyDeviceToHost, st));
         GBSA_CUDA(cudaStreamSynchronize(st));
     }
+    const uint64_t n_sm = csm[n_contigs];
     DeviceBuffer d_sh(8 * (n_sm + 1)), d_sp(4 * (n_sm + 1));
     if (n_seg) {
-        k_contig_syncmers<true><<<seg_blocks, 32 * kSegWarps, 0, st>>>(P, d_packed.as<uint64_t>(),
-                                                                       d_nmask.as<uint32_t>(), T, n_seg, nullptr,
-                                                                       d_segoff.as<uint64_t>(), d_sh.as<uint64_t>(),
-                                                                       d_sp.as<uint32_t>());
+        k_write_syncmers<<<seg_blocks, 32 * kSegWarps, 0, st>>>(P, d_packed.as<uint64_t>(), T, n_seg,
+                                                                d_segoff.as<uint64_t>(), d_bits.as<uint32_t>(),
+                                                                d_sh.as<uint64_t>(), d_sp.as<uint32_t>());
         GBSA_LAUNCHED();
     }
     d_g.release();
 
-    // ---- per-contig syncmer ranges and randstrobe offsets (count_randstrobes) ---
-    std::vector<uint64_t> segoff(n_seg + 1, 0);
-    if (n_seg) GBSA_CUDA(cudaMemcpyAsync(segoff.data(), d_segoff.as<uint64_t>(), 8 * n_seg, cudaMemcpyDeviceToHost, st));
-    GBSA_CUDA(cudaStreamSynchronize(st));
-    segoff[n_seg] = n_sm;
-    std::vector<uint64_t> csm(n_contigs + 1), cref(n_contigs + 1, 0), clen(n_contigs + 1, 0);
-    for (uint32_t c = 0; c <= n_contigs; ++c) csm[c] = segoff[cfirst_seg[c]];
+    // ---- per-contig randstrobe offsets (count_randstrobes) ----------------------
+    std::vector<uint64_t> cref(n_contigs + 1, 0), clen(n_contigs + 1, 0);
     uint64_t n_rs = 0;
+    uint32_t max_position = 0;
     for (uint32_t c = 0; c < n_contigs; ++c) {
+        max_position = std::max(max_position, (uint32_t)lengths[c]);
         const uint64_t nc = csm[c + 1] - csm[c];
         cref[c] = n_rs;
         n_rs += nc < P.w_min ? 0 : nc - P.w_min;
@@ -348,8 +400,7 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     cref[n_contigs] = n_rs;
     ix.n = n_rs;
     ix.info.tot_strobemer_count = n_rs;
-    DeviceBuffer d_csm(8 * (n_contigs + 1)), d_cref(8 * (n_contigs + 1)), d_clen(8 * (n_contigs + 1));
-    GBSA_CUDA(cudaMemcpyAsync(d_csm.as<void>(), csm.data(), 8 * (n_contigs + 1), cudaMemcpyHostToDevice, st));
+    DeviceBuffer d_cref(8 * (n_contigs + 1)), d_clen(8 * (n_contigs + 1));
     GBSA_CUDA(cudaMemcpyAsync(d_cref.as<void>(), cref.data(), 8 * (n_contigs + 1), cudaMemcpyHostToDevice, st));
     GBSA_CUDA(cudaMemcpyAsync(d_clen.as<void>(), clen.data(), 8 * (n_contigs + 1), cudaMemcpyHostToDevice, st));
 
@@ -368,50 +419,34 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
 
     // ---- sort --------------------------------------------------------------------
     gbsa_ref_randstrobe* sorted =
-        radix_sort_ref_randstrobes(d_a.as<gbsa_ref_randstrobe>(), d_b.as<gbsa_ref_randstrobe>(), n_rs, ws, st);
+        sort_ref_randstrobes(d_a.as<gbsa_ref_randstrobe>(), d_b.as<gbsa_ref_randstrobe>(), n_rs, max_position, ws, st);
     if (sorted == d_a.as<gbsa_ref_randstrobe>()) {
         ix.rs = std::move(d_a);
     } else {
         ix.rs = std::move(d_b);
     }
 
-    // ---- bucket table ------------------------------------------------------------
+    // ---- bucket tables, run-length statistics → filter_cutoff -----------------------
     const uint64_t nb = (1ULL << ix.bits) + 1;
     ix.starts.resize(8 * nb);
     const bool tagged = n_rs < (1ull << 32);
     if (tagged) ix.buckets.resize(sizeof(Bucket) * nb);
     const gbsa_ref_randstrobe* rs = ix.rs.as<gbsa_ref_randstrobe>();
+    std::vector<unsigned long long> H(102, 0);
     if (n_rs == 0) {
         GBSA_CUDA(cudaMemsetAsync(ix.starts.as<void>(), 0, 8 * nb, st));
         GBSA_CUDA(cudaMemsetAsync(ix.buckets.as<void>(), 0, sizeof(Bucket) * nb, st));
     } else {
-        k_bucket_starts<<<grid_for(n_rs, 256, 1u << 20), 256, 0, st>>>(
-            rs, n_rs, ix.bits, ix.starts.as<uint64_t>(), tagged ? ix.buckets.as<Bucket>() : nullptr);
-        GBSA_LAUNCHED();
-    }
-
-    // ---- run-length statistics → filter_cutoff ---------------------------------------
-    std::vector<unsigned long long> H(102, 0);
-    uint64_t unique = 0;
-    if (n_rs) {
-        uint64_t* flags = ws.get<uint64_t>(n_rs);
-        uint64_t* idx = ws.get<uint64_t>(n_rs);
-        uint64_t* d_runs = ws.get<uint64_t>(1);
-        k_run_flags<<<grid_for(n_rs, 256, 1u << 20), 256, 0, st>>>(rs, n_rs, flags);
-        GBSA_LAUNCHED();
-        scan_exclusive_u64(flags, idx, n_rs, d_runs, ws, st);
-        GBSA_CUDA(cudaMemcpyAsync(&unique, d_runs, 8, cudaMemcpyDeviceToHost, st));
-        GBSA_CUDA(cudaStreamSynchronize(st));
-        uint64_t* run_start = flags;   // reuse
-        k_run_starts<<<grid_for(n_rs, 256, 1u << 20), 256, 0, st>>>(rs, n_rs, idx, run_start);
-        GBSA_LAUNCHED();
         unsigned long long* d_h = ws.get<unsigned long long>(102);
         GBSA_CUDA(cudaMemsetAsync(d_h, 0, 102 * 8, st));
-        k_run_hist<<<grid_for(unique, 256, 4096), 256, 0, st>>>(run_start, unique, n_rs, d_h);
+        k_tables<<<grid_for(n_rs, 256, 16 * device_sm_count()), 256, 0, st>>>(rs, n_rs, ix.bits, ix.starts.as<uint64_t>(),
+                                                                tagged ? ix.buckets.as<Bucket>() : nullptr, d_h);
         GBSA_LAUNCHED();
         GBSA_CUDA(cudaMemcpyAsync(H.data(), d_h, 102 * 8, cudaMemcpyDeviceToHost, st));
     }
     GBSA_CUDA(cudaStreamSynchronize(st));
+    uint64_t unique = 0;
+    for (const unsigned long long runs : H) unique += runs;
     finish_stats(ix, H, unique, f);
     ix.info.size = ix.n;
     ix.info.bits = ix.bits;

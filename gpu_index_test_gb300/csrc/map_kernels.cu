@@ -399,9 +399,7 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = lane_id();
     if (L < (uint32_t)P.k || !warp_pack_clean(seq, L, pk)) return false;
-    const uint32_t nwin = L - (uint32_t)P.k + 1;
-    const uint32_t n = P.W == 5 && P.t == 3 && P.s <= 16 ? warp_clean_syncmers<5>(P, pk, nwin, ring, sp, cap)
-                                                         : warp_clean_syncmers<0>(P, pk, nwin, ring, sp, cap);
+    const uint32_t n = warp_clean_syncmers(P, pk, L - (uint32_t)P.k + 1, ring, sp, cap);
     if (n > cap) return false;   // (ties too)
     const uint32_t nq = n_query_per_dir(P, n, L), nq2 = 2 * nq;
     if (nq2 > kFastQueries) return false;

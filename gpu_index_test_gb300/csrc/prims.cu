@@ -1,4 +1,4 @@
-// prims.cu — exclusive scan and stable LSD radix sort (see prims.cuh).
+// prims.cu — exclusive scan and stable sort of the index's records (see prims.cuh).
 #include "prims.cuh"
 
 namespace gbsa {
@@ -78,8 +78,7 @@ __device__ __forceinline__ uint32_t digit_of(const gbsa_ref_randstrobe& r, int p
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const gbsa_ref_randstrobe* in, size_t n, int pass,
-                                                              uint64_t* block_hist, size_t nblocks,
-                                                              unsigned long long* global_hist) {
+                                                              uint64_t* block_hist, size_t nblocks) {
     __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -89,9 +88,7 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const gbsa_ref_rand
         if (idx < n) atomicAdd(&h[digit_of(in[idx], pass)], 1u);
     }
     __syncthreads();
-    const uint32_t c = h[threadIdx.x];
-    block_hist[(size_t)threadIdx.x * nblocks + blockIdx.x] = c;
-    if (c) atomicAdd(&global_hist[threadIdx.x], (unsigned long long)c);
+    block_hist[(size_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const gbsa_ref_randstrobe* in,
@@ -135,6 +132,199 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const gbsa_ref_r
     }
 }
 
+// ---- groups of the top hash bits ------------------------------------------------
+constexpr size_t kGroupMean = 160;     // largest mean size of a group
+constexpr uint32_t kGroupMax = 256;    // records a warp sorts in shared memory
+constexpr int kGroupWarps = 8;
+constexpr uint32_t kBlockGroupMax = 2048;   // records a block sorts in shared memory
+constexpr uint32_t kBlockGroupThreads = 512;
+
+__global__ void k_group_starts(const gbsa_ref_randstrobe* __restrict__ rs, size_t n, int bits,
+                               uint64_t* __restrict__ start) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uint64_t t = rs[i].hash >> (64 - bits);
+        for (uint64_t g = i ? (rs[i - 1].hash >> (64 - bits)) + 1 : 0; g <= t; ++g) start[g] = i;
+        if (i == n - 1)
+            for (uint64_t g = t + 1; g <= (1ULL << bits); ++g) start[g] = n;
+    }
+}
+
+// A warp sorts each group of up to kGroupMax records by rank in shared memory: 61 records a
+// group at 4M records, 122 comparisons a lane instead of six more passes over memory
+// (186 us against 105 a pass).  The
+// comparisons are of 32 bits, the first that the group does not share: a record comes after
+// those with smaller bits and after those with the same that precede it in place.  That is
+// right where those are in order already (copies of one seed, in a contig); a group where
+// two neighbours among them are not is ranked by all bits.  Groups of up to kBlockGroupMax go
+// to the list for a block each, the size of larger ones (repeats) into `large`.
+__global__ void __launch_bounds__(32 * kGroupWarps) k_sort_groups(gbsa_ref_randstrobe* __restrict__ rs,
+                                                                  const uint64_t* __restrict__ start, uint64_t n_groups,
+                                                                  int bits, uint64_t* __restrict__ large,
+                                                                  uint32_t* __restrict__ n_medium,
+                                                                  uint32_t* __restrict__ medium) {
+    __shared__ uint64_t s_hash[kGroupWarps][kGroupMax];
+    __shared__ uint32_t s_pos[kGroupWarps][kGroupMax];
+    __shared__ __align__(16) uint32_t s_key[kGroupWarps][kGroupMax];
+    constexpr uint32_t kRows = kGroupMax / 32, kNone = 0xFFFFFFFFu;
+    const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
+    uint64_t* hash = s_hash[wid];
+    uint32_t* pos = s_pos[wid];
+    uint32_t* key = s_key[wid];
+    for (uint64_t g = blockIdx.x * (uint64_t)kGroupWarps + wid; g < n_groups; g += (uint64_t)gridDim.x * kGroupWarps) {
+        const uint64_t a = start[g], size = start[g + 1] - a;
+        if (lane == 0) {
+            large[g] = size > kBlockGroupMax ? size : 0;
+            if (size > kGroupMax && size <= kBlockGroupMax) medium[atomicAdd(n_medium, 1u)] = (uint32_t)g;
+        }
+        if (size < 2 || size > kGroupMax) continue;
+        const uint32_t m = (uint32_t)size;
+        uint4 v[kRows];
+        uint4* rec = reinterpret_cast<uint4*>(rs) + a;
+#pragma unroll
+        for (uint32_t j = 0; j < kRows; ++j) {
+            const uint32_t i = 32 * j + lane;
+            if (32 * j < m) {
+                v[j] = i < m ? rec[i] : make_uint4(~0u, ~0u, ~0u, ~0u);
+                const uint64_t h = ((uint64_t)v[j].y << 32) | v[j].x;
+                hash[i] = h;
+                pos[i] = v[j].z;
+                key[i] = i < m ? (uint32_t)(h >> (32 - bits)) : kNone;
+            }
+        }
+        __syncwarp();
+        uint32_t rank[kRows];
+        bool wrong = false;
+#pragma unroll
+        for (uint32_t j = 0; j < kRows; ++j) {
+            const uint32_t i = 32 * j + lane;
+            rank[j] = 0;
+            if (32 * j < m) {
+                const uint32_t mine = key[i];
+                uint32_t r = 0, prev = kNone;
+                auto upto = [&](uint32_t x, uint32_t k) {
+                    r += k <= mine;
+                    if (k == mine) prev = x;
+                };
+                uint32_t x = 0;
+                for (; x < 32 * j; x += 4) {   // records before the row
+                    const uint4 k = *reinterpret_cast<const uint4*>(key + x);
+                    upto(x, k.x);
+                    upto(x + 1, k.y);
+                    upto(x + 2, k.z);
+                    upto(x + 3, k.w);
+                }
+                const uint32_t row = min(m, 32 * j + 32);
+                for (; x < row; ++x) {
+                    const uint32_t k = key[x];
+                    if (x < i) upto(x, k);
+                    else r += k < mine;
+                }
+                for (; x < m; x += 4) {   // behind it (past m all ones: below none)
+                    const uint4 k = *reinterpret_cast<const uint4*>(key + x);
+                    r += (k.x < mine) + (k.y < mine) + (k.z < mine) + (k.w < mine);
+                }
+                rank[j] = r;
+                if (prev != kNone && i < m)
+                    wrong |= hash[prev] > hash[i] || (hash[prev] == hash[i] && pos[prev] > pos[i]);
+            }
+        }
+        if (__any_sync(0xFFFFFFFFu, wrong)) {
+#pragma unroll
+            for (uint32_t j = 0; j < kRows; ++j) {
+                const uint32_t i = 32 * j + lane;
+                if (i < m) {
+                    const uint64_t h = hash[i];
+                    const uint32_t p = pos[i];
+                    rank[j] = 0;
+                    for (uint32_t x = 0; x < m; ++x) {
+                        const uint64_t o = hash[x];
+                        rank[j] += o < h || (o == h && (pos[x] < p || (pos[x] == p && x < i)));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kRows; ++j)
+            if (32 * j + lane < m) rec[rank[j]] = v[j];
+        __syncwarp();
+    }
+}
+
+// The listed groups, a block each: a bitonic sort by (hash, position, place) in shared memory
+// (a group of 2,000 equal hashes took 400 us by rank).
+__global__ void __launch_bounds__(kBlockGroupThreads) k_sort_medium(gbsa_ref_randstrobe* __restrict__ rs,
+                                                                    const uint64_t* __restrict__ start,
+                                                                    const uint32_t* __restrict__ n_medium,
+                                                                    const uint32_t* __restrict__ medium) {
+    __shared__ uint64_t s_hash[kBlockGroupMax];
+    __shared__ uint32_t s_pos[kBlockGroupMax];
+    __shared__ uint16_t s_at[kBlockGroupMax];
+    constexpr uint32_t kRows = kBlockGroupMax / kBlockGroupThreads;
+    for (uint32_t t = blockIdx.x; t < *n_medium; t += gridDim.x) {
+        const uint64_t g = medium[t], a = start[g];
+        const uint32_t m = (uint32_t)(start[g + 1] - a);
+        uint32_t size = 2 * kGroupMax;
+        while (size < m) size *= 2;
+        uint4* rec = reinterpret_cast<uint4*>(rs) + a;
+        for (uint32_t i = threadIdx.x; i < size; i += kBlockGroupThreads) {
+            const uint4 v = i < m ? rec[i] : make_uint4(~0u, ~0u, ~0u, ~0u);
+            s_hash[i] = ((uint64_t)v.y << 32) | v.x;
+            s_pos[i] = v.z;
+            s_at[i] = (uint16_t)i;
+        }
+        __syncthreads();
+        for (uint32_t k = 2; k <= size; k *= 2)
+            for (uint32_t d = k / 2; d; d /= 2) {
+                for (uint32_t x = threadIdx.x; x < size / 2; x += kBlockGroupThreads) {
+                    const uint32_t i = 2 * x - (x & (d - 1)), l = i + d;
+                    const uint64_t hi = s_hash[i], hl = s_hash[l];
+                    const uint32_t pi = s_pos[i], pl = s_pos[l];
+                    const uint16_t ai = s_at[i], al = s_at[l];
+                    const bool after = hi > hl || (hi == hl && (pi > pl || (pi == pl && ai > al)));
+                    if (after == ((i & k) == 0)) {
+                        s_hash[i] = hl;
+                        s_hash[l] = hi;
+                        s_pos[i] = pl;
+                        s_pos[l] = pi;
+                        s_at[i] = al;
+                        s_at[l] = ai;
+                    }
+                }
+                __syncthreads();
+            }
+        uint4 v[kRows];
+#pragma unroll
+        for (uint32_t j = 0; j < kRows; ++j) {
+            const uint32_t i = kBlockGroupThreads * j + threadIdx.x;
+            if (i < m) v[j] = rec[s_at[i]];
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < kRows; ++j) {
+            const uint32_t i = kBlockGroupThreads * j + threadIdx.x;
+            if (i < m) rec[i] = v[j];
+        }
+    }
+}
+
+// The records of the large groups (those with room of their own in `off`) between their
+// places in rs and the packed list, a warp a group.
+template <bool kOut>
+__global__ void k_move_groups(gbsa_ref_randstrobe* __restrict__ rs, gbsa_ref_randstrobe* __restrict__ list,
+                              const uint64_t* __restrict__ start, const uint64_t* __restrict__ off, uint64_t n_groups) {
+    const uint32_t lane = lane_id();
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
+    for (uint64_t g = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32; g < n_groups; g += warps) {
+        const uint64_t o = off[g], m = off[g + 1] - o;
+        uint4* place = reinterpret_cast<uint4*>(rs) + start[g];
+        uint4* packed = reinterpret_cast<uint4*>(list) + o;
+        for (uint64_t i = lane; i < m; i += 32) {
+            if (kOut) packed[i] = place[i];
+            else place[i] = packed[i];
+        }
+    }
+}
+
 }  // namespace
 
 void scan_exclusive_u64(const uint64_t* in, uint64_t* out, size_t n, uint64_t* d_total, Workspace& ws,
@@ -157,29 +347,70 @@ void scan_exclusive_u64(const uint64_t* in, uint64_t* out, size_t n, uint64_t* d
     GBSA_LAUNCHED();
 }
 
-gbsa_ref_randstrobe* radix_sort_ref_randstrobes(gbsa_ref_randstrobe* a, gbsa_ref_randstrobe* b, size_t n,
-                                                Workspace& ws, cudaStream_t st) {
-    if (n <= 1) return a;
+// One stable pass over the digit `pass` of n records, src to dst.
+static void radix_pass(const gbsa_ref_randstrobe* src, gbsa_ref_randstrobe* dst, size_t n, int pass, uint64_t* bh,
+                       Workspace& ws, cudaStream_t st) {
     const size_t nb = (n + kSortTile - 1) / kSortTile;
-    uint64_t* bh = ws.get<uint64_t>(256 * nb);
-    unsigned long long* gh = ws.get<unsigned long long>(256);
-    std::vector<unsigned long long> hgh(256);
+    k_radix_hist<<<(unsigned)nb, kSortThreads, 0, st>>>(src, n, pass, bh, nb);
+    GBSA_LAUNCHED();
+    const size_t at = ws.mark();
+    scan_exclusive_u64(bh, bh, 256 * nb, nullptr, ws, st);
+    ws.rewind(at);   // the next pass follows in the stream
+    k_radix_scatter<<<(unsigned)nb, kSortThreads, 0, st>>>(src, dst, n, pass, bh, nb);
+    GBSA_LAUNCHED();
+}
+
+gbsa_ref_randstrobe* sort_ref_randstrobes(gbsa_ref_randstrobe* a, gbsa_ref_randstrobe* b, size_t n, uint32_t max_position,
+                                          Workspace& ws, cudaStream_t st) {
+    if (n <= 1) return a;
+    uint64_t* bh = ws.get<uint64_t>(256 * ((n + kSortTile - 1) / kSortTile));
+    // passes over the position's used bytes, then the hash's
+    auto all_passes = [&](gbsa_ref_randstrobe* src, gbsa_ref_randstrobe* dst, size_t m) {
+        for (int pass = 0; pass < 12; ++pass) {
+            if (pass < 4 && (max_position >> (8 * pass)) == 0) continue;
+            radix_pass(src, dst, m, pass, bh, ws, st);
+            std::swap(src, dst);
+        }
+        return src;
+    };
+    // groups by the hash's top bits: of up to kGroupMean records on average while that saves
+    // a pass, else of 24 to 48
+    int bytes = 1;
+    while (bytes < 3 && (n >> (8 * bytes)) >= kGroupMean) ++bytes;
+    int bits = 8 * bytes;
+    while (bits > 8 && (n >> bits) < 24) --bits;
     gbsa_ref_randstrobe* src = a;
     gbsa_ref_randstrobe* dst = b;
-    for (int pass = 0; pass < 12; ++pass) {
-        GBSA_CUDA(cudaMemsetAsync(gh, 0, 256 * sizeof(unsigned long long), st));
-        k_radix_hist<<<(unsigned)nb, kSortThreads, 0, st>>>(src, n, pass, bh, nb, gh);
-        GBSA_LAUNCHED();
-        GBSA_CUDA(cudaMemcpyAsync(hgh.data(), gh, 256 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-        GBSA_CUDA(cudaStreamSynchronize(st));
-        bool trivial = false;
-        for (int d = 0; d < 256; ++d) trivial |= (hgh[d] == n);
-        if (trivial) continue;
-        scan_exclusive_u64(bh, bh, 256 * nb, nullptr, ws, st);
-        k_radix_scatter<<<(unsigned)nb, kSortThreads, 0, st>>>(src, dst, n, pass, bh, nb);
-        GBSA_LAUNCHED();
+    for (int pass = 12 - bytes; pass < 12; ++pass) {
+        radix_pass(src, dst, n, pass, bh, ws, st);
         std::swap(src, dst);
     }
+    const uint64_t n_groups = 1ULL << bits;
+    uint64_t* start = ws.get<uint64_t>(n_groups + 1);
+    k_group_starts<<<grid_for(n, 256, 1u << 16), 256, 0, st>>>(src, n, bits, start);
+    GBSA_LAUNCHED();
+    uint64_t* large = ws.get<uint64_t>(n_groups + 1);   // a large group's size, then the offsets
+    uint32_t* medium = ws.get<uint32_t>(n_groups + 1);  // the groups for a block each, their number last
+    uint32_t* n_medium = medium + n_groups;
+    GBSA_CUDA(cudaMemsetAsync(n_medium, 0, 4, st));
+    k_sort_groups<<<grid_for(n_groups, kGroupWarps, 32 * device_sm_count()), 32 * kGroupWarps, 0, st>>>(
+        src, start, n_groups, bits, large, n_medium, medium);
+    GBSA_LAUNCHED();
+    k_sort_medium<<<4 * device_sm_count(), kBlockGroupThreads, 0, st>>>(src, start, n_medium, medium);
+    GBSA_LAUNCHED();
+    scan_exclusive_u64(large, large, n_groups, large + n_groups, ws, st);
+    uint64_t m = 0;
+    GBSA_CUDA(cudaMemcpyAsync(&m, large + n_groups, 8, cudaMemcpyDeviceToHost, st));
+    GBSA_CUDA(cudaStreamSynchronize(st));
+    if (m == 0) return src;
+    if (2 * m > n) return all_passes(src, dst, n);
+    // the large groups' records, side by side in the free buffer, sorted among themselves:
+    // they keep the groups' order, so each goes back into its group's place
+    const unsigned blocks = grid_for(n_groups, 8, 64 * device_sm_count());
+    k_move_groups<true><<<blocks, 256, 0, st>>>(src, dst, start, large, n_groups);
+    GBSA_LAUNCHED();
+    k_move_groups<false><<<blocks, 256, 0, st>>>(src, all_passes(dst, dst + m, m), start, large, n_groups);
+    GBSA_LAUNCHED();
     return src;
 }
 

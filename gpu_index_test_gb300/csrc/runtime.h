@@ -134,6 +134,10 @@ public:
         return static_cast<T*>(get(n * sizeof(T)));
     }
     void reset() { next_ = 0; }
+    // Buffers handed out after mark() are handed out again after rewind(): for scratch of
+    // steps that follow each other in one stream.
+    size_t mark() const { return next_; }
+    void rewind(size_t mark) { next_ = mark; }
 
 private:
     std::vector<DeviceBuffer> bufs_;

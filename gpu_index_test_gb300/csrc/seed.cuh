@@ -144,13 +144,14 @@ __device__ __forceinline__ uint64_t nbits33(const uint32_t* m, uint64_t p, int n
 }
 
 // The canonical s-mer at p, s <= 16, in the low 2 s bits.
-__device__ __forceinline__ uint32_t smer16(const DevParams& P, const uint64_t* packed, uint32_t p) {
+template <class Pos>
+__device__ __forceinline__ uint32_t smer16(const DevParams& P, const uint64_t* packed, Pos p) {
     // s-mers of up to 16 bases in 32 bits: the stream seen as 32-bit groups of 16
     // bases (group g is the high half of word g/2 for even g, the low half for odd
     // g; little-endian halves sit at u32 index g ^ 1)
     const uint32_t* w32 = reinterpret_cast<const uint32_t*>(packed);
-    const uint32_t g = p >> 4;
-    uint32_t f = __funnelshift_l(w32[(g + 1) ^ 1], w32[g ^ 1], (p & 15) * 2);
+    const Pos g = p >> 4;
+    uint32_t f = __funnelshift_l(w32[(g + 1) ^ 1], w32[g ^ 1], (uint32_t)(p & 15) * 2);
     f >>= 32 - 2 * P.s;   // P.s >= 1
     uint32_t r = __brev(~f);
     r = ((r >> 1) & 0x55555555u) | ((r & 0x55555555u) << 1);
@@ -159,7 +160,7 @@ __device__ __forceinline__ uint32_t smer16(const DevParams& P, const uint64_t* p
 }
 
 __device__ __forceinline__ uint64_t smer_hash(const DevParams& P, const uint64_t* packed, uint64_t p) {
-    if (P.s <= 16) return xxh64((uint64_t)smer16(P, packed, (uint32_t)p));
+    if (P.s <= 16) return xxh64((uint64_t)smer16(P, packed, p));
     const uint64_t f = extract_bases(packed, p, P.s);
     const uint64_t r = revcomp_bits(f, P.s);
     return xxh64(f < r ? f : r);
@@ -438,20 +439,20 @@ __device__ __forceinline__ uint32_t n_query_per_dir(const DevParams& P, uint32_t
     return n > P.w_min ? n - P.w_min : 0;
 }
 
-// Syncmers of a clean read (packed by warp_pack_clean).  A window is a syncmer when its s-mer
-// number t - 1 has the least hash of the W, decided on the hashes' high words, so that a
-// window costs W words of a ring of high words and a few minima.  Where that s-mer ties
-// with the least of the others the state machine's history may count: returns 0xFFFFFFFF,
-// and the caller takes the full scan.  kW: W when known at compile time (0: P.W).  sp: the
-// first `cap` syncmers' windows; ring: 64 words (32 + W - 1 <= 64).
-template <int kW>
-__device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, const uint64_t* packed, uint32_t nwin,
-                                                        uint32_t* ring, uint32_t* sp, uint32_t cap) {
+// Syncmers of the nwin windows from packed position p0 on, where no base is ambiguous.  A
+// window is a syncmer when its s-mer number t - 1 has the least hash of the W, decided on
+// the hashes' high words, so that a window costs W words of a ring of high words and a few
+// minima.  Calls chunk(c, bits) for each 32 windows from c on.  Where that s-mer ties with
+// the least of the others the state machine's history may count: returns false, and the
+// caller takes the full scan.  kW: W when known at compile time, with s <= 16 (0: P.W).
+// ring: 64 words (32 + W - 1 <= 64).
+template <int kW, class Chunk>
+__device__ __forceinline__ bool warp_clean_scan(const DevParams& P, const uint64_t* packed, uint32_t p0, uint32_t nwin,
+                                                uint32_t* ring, Chunk&& chunk) {
     const uint32_t lane = lane_id();
     const uint32_t W = kW ? kW : (uint32_t)P.W, t = kW ? kW / 2 : (uint32_t)(P.t - 1);
-    uint32_t n = 0;
     auto high = [&](uint32_t p) {
-        return (uint32_t)((kW ? xxh64((uint64_t)smer16(P, packed, p)) : smer_hash(P, packed, p)) >> 32);
+        return (uint32_t)((kW ? xxh64((uint64_t)smer16(P, packed, p0 + p)) : smer_hash(P, packed, p0 + p)) >> 32);
     };
     if (lane < W - 1) ring[lane] = high(lane);
     for (uint32_t c = 0; c < nwin; c += 32) {
@@ -464,15 +465,29 @@ __device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, cons
         for (uint32_t d = 0; d < W; ++d)
             if (d != t) least = min(least, ring[(w + d) & 63]);
         const bool in = w < nwin;
-        if (__any_sync(0xFFFFFFFFu, in && mid == least)) return 0xFFFFFFFFu;
-        const bool sync = in && mid < least;
-        const uint32_t b = __ballot_sync(0xFFFFFFFFu, sync);
-        const uint32_t idx = n + __popc(b & lanemask_lt());
-        if (sync && idx < cap) sp[idx] = w;
-        n += __popc(b);
+        if (__any_sync(0xFFFFFFFFu, in && mid == least)) return false;
+        chunk(c, __ballot_sync(0xFFFFFFFFu, in && mid < least));
         __syncwarp();
     }
-    return n;
+    return true;
+}
+
+// Whether the scan above may be the instance for W = 5 and short s-mers.
+__device__ __forceinline__ bool clean_scan5(const DevParams& P) { return P.W == 5 && P.t == 3 && P.s <= 16; }
+
+// The first `cap` syncmers' windows of a clean read into sp; returns their number, or
+// 0xFFFFFFFF where the full scan is needed.
+__device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, const uint64_t* packed, uint32_t nwin,
+                                                        uint32_t* ring, uint32_t* sp, uint32_t cap) {
+    uint32_t n = 0;
+    auto put = [&](uint32_t c, uint32_t b) {
+        const uint32_t idx = n + __popc(b & lanemask_lt());
+        if (((b >> lane_id()) & 1u) && idx < cap) sp[idx] = c + lane_id();
+        n += __popc(b);
+    };
+    const bool ok = clean_scan5(P) ? warp_clean_scan<5>(P, packed, 0, nwin, ring, put)
+                                   : warp_clean_scan<0>(P, packed, 0, nwin, ring, put);
+    return ok ? n : 0xFFFFFFFFu;
 }
 
 // Writes the 2*nq query randstrobes of a read (forward, then reverse complement).
