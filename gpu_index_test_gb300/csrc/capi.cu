@@ -1166,6 +1166,42 @@ int gbsa_map_reads_device(gbsa_mapper* m, const char* d_seqs, const uint64_t* d_
     });
 }
 
+// The layout of find_nams' queries on the host.
+static void layout_queries_host(gbsa_mapper& m, const gbsa_query_randstrobe* queries, const uint64_t* q_offsets,
+                                uint32_t n, cudaStream_t st) {
+    const uint64_t nqt = q_offsets[n] - q_offsets[0];
+    std::vector<Query> hq(nqt + 1);
+    std::vector<ReadRec> hr(n);
+    std::vector<uint32_t> ord;
+    uint64_t o = 0;
+    for (uint32_t r = 0; r < n; ++r) {
+        const uint64_t a = q_offsets[r], b = q_offsets[r + 1];
+        ord.resize(b - a);
+        std::iota(ord.begin(), ord.end(), 0u);
+        std::stable_sort(ord.begin(), ord.end(), [&](uint32_t x, uint32_t y) {
+            const auto& qx = queries[a + x];
+            const auto& qy = queries[a + y];
+            if ((qx.is_reverse != 0) != (qy.is_reverse != 0)) return qx.is_reverse == 0;
+            return qx.start < qy.start;
+        });
+        uint32_t nf = 0;
+        for (uint32_t j = 0; j < ord.size(); ++j) {
+            const auto& q = queries[a + ord[j]];
+            hq[o + j] = Query{q.hash, q.start, q.end};
+            nf += q.is_reverse ? 0 : 1;
+        }
+        ReadRec R{};
+        R.q_off = o;
+        R.nq = nf;
+        R.nq2 = (uint32_t)(b - a);
+        hr[r] = R;
+        o += b - a;
+    }
+    if (nqt) GBSA_CUDA(cudaMemcpyAsync(m.q.as<void>(), hq.data(), sizeof(Query) * nqt, cudaMemcpyHostToDevice, st));
+    GBSA_CUDA(cudaMemcpyAsync(m.rec.as<void>(), hr.data(), sizeof(ReadRec) * n, cudaMemcpyHostToDevice, st));
+    GBSA_CUDA(cudaStreamSynchronize(st));
+}
+
 int gbsa_find_nams(gbsa_mapper* m, const gbsa_query_randstrobe* queries, const uint64_t* q_offsets, uint32_t n_reads,
                    int rescue, uint32_t rescue_cutoff, gbsa_nam* nams, uint64_t nam_capacity, uint64_t* nam_offsets,
                    float* frac) {
@@ -1185,36 +1221,28 @@ int gbsa_find_nams(gbsa_mapper* m, const gbsa_query_randstrobe* queries, const u
         }
         // Lay the queries of each read out forward-first, each orientation ordered by
         // start (stable), which is the order randstrobes_query produces and in which the
-        // reference's (query_start, ref_start) hit sort leaves them.
-        std::vector<Query> hq(nqt + 1);
-        std::vector<ReadRec> hr(n);
-        std::vector<uint32_t> ord;
-        uint64_t o = 0;
-        for (uint32_t r = 0; r < n; ++r) {
-            const uint64_t a = q_offsets[r], b = q_offsets[r + 1];
-            ord.resize(b - a);
-            std::iota(ord.begin(), ord.end(), 0u);
-            std::stable_sort(ord.begin(), ord.end(), [&](uint32_t x, uint32_t y) {
-                const auto& qx = queries[a + x];
-                const auto& qy = queries[a + y];
-                if ((qx.is_reverse != 0) != (qy.is_reverse != 0)) return qx.is_reverse == 0;
-                return qx.start < qy.start;
-            });
-            uint32_t nf = 0;
-            for (uint32_t j = 0; j < ord.size(); ++j) {
-                const auto& q = queries[a + ord[j]];
-                hq[o + j] = Query{q.hash, q.start, q.end};
-                nf += q.is_reverse ? 0 : 1;
-            }
-            ReadRec R{};
-            R.q_off = o;
-            R.nq = nf;
-            R.nq2 = (uint32_t)(b - a);
-            hr[r] = R;
-            o += b - a;
+        // reference's (query_start, ref_start) hit sort leaves them: on the device, or here
+        // when a read has very many queries that are not in that order.
+        bool rising = true;
+        for (uint32_t r = 0; r < n; ++r) rising &= q_offsets[r] <= q_offsets[r + 1];
+        uint32_t left = 1;
+        if (rising && n) {
+            const uint64_t at = (sizeof(gbsa_query_randstrobe) * nqt + 255) & ~uint64_t(255);
+            m->out_nams.resize(at + 8ull * (n + 1) + 4);   // staging; free until the gather
+            uint8_t* d = m->out_nams.as<uint8_t>();
+            uint32_t* d_left = reinterpret_cast<uint32_t*>(d + at + 8ull * (n + 1));
+            if (nqt)
+                GBSA_CUDA(cudaMemcpyAsync(d, queries + q_offsets[0], sizeof(gbsa_query_randstrobe) * nqt,
+                                          cudaMemcpyHostToDevice, st));
+            GBSA_CUDA(cudaMemcpyAsync(d + at, q_offsets, 8ull * (n + 1), cudaMemcpyHostToDevice, st));
+            GBSA_CUDA(cudaMemsetAsync(d_left, 0, 4, st));
+            launch_layout_queries(n, reinterpret_cast<const gbsa_query_randstrobe*>(d),
+                                  reinterpret_cast<const uint64_t*>(d + at), m->q.as<Query>(), m->rec.as<ReadRec>(),
+                                  d_left, st);
+            GBSA_CUDA(cudaMemcpyAsync(&left, d_left, 4, cudaMemcpyDeviceToHost, st));
+            GBSA_CUDA(cudaStreamSynchronize(st));
         }
-        if (nqt) GBSA_CUDA(cudaMemcpyAsync(m->q.as<void>(), hq.data(), sizeof(Query) * nqt, cudaMemcpyHostToDevice, st));
-        GBSA_CUDA(cudaMemcpyAsync(m->rec.as<void>(), hr.data(), sizeof(ReadRec) * n, cudaMemcpyHostToDevice, st));
+        if (left) layout_queries_host(*m, queries, q_offsets, n, st);
         const MapConfig saved = m->cfg;
         m->cfg.rescue_level = 0;          // find_nams alone, or
         m->cfg.force_rescue = rescue ? 1 : 0;   // find_nams_rescue for every read

@@ -197,6 +197,10 @@ void launch_gather_nams(uint32_t n, const ReadRec* rec, const NamState* arena, c
                         gbsa_nam* out, float* frac, uint8_t* rescued, cudaStream_t st, uint64_t out_cap = ~0ull,
                         int mode = 0, const Arenas* A = nullptr, const Counters* ctr = nullptr,
                         const BatchDesc* desc = nullptr);
+// Queries of reads [offs[r], offs[r + 1]) (counted from offs[0]) laid out for the lookup, with
+// the reads' records; *left (0 before) is set when the caller has to lay them out.
+void launch_layout_queries(uint32_t n, const gbsa_query_randstrobe* in, const uint64_t* offs, Query* out, ReadRec* rec,
+                           uint32_t* left, cudaStream_t st);
 void launch_gather_queries(uint32_t n, const ReadRec* rec, const Query* arena, const uint64_t* out_off,
                            gbsa_query_randstrobe* out, cudaStream_t st);
 void launch_find(const IndexView& I, const uint64_t* hashes, uint64_t n, uint64_t* pos, cudaStream_t st);

@@ -138,3 +138,38 @@ def test_a_table_out_of_order_is_searched_in_order():
     h = ent["hash"]
     assert (idx.find(h) == np.array([o.find(int(x)) for x in h], np.uint64)).all()
     assert same(native.Mapper(idx, max_reads=1024).map_reads(reads), o.map_reads(reads, n_threads=4))
+
+
+@pytest.mark.parametrize("rescue", [False, True])
+def test_find_nams_takes_queries_in_any_order(rescue):
+    """Reads' queries in order, shuffled, orientations mixed, none, one, and more than a warp
+    ranks (1,024) in and out of order; offsets that do not begin at 0."""
+    rng = np.random.default_rng(11)
+    g = synth.make_genome(synth.GenomeParams(seed=11, total_len=200_000, n_contigs=2, dup_frac=0.1))
+    p = native.params_from_read_length(150)
+    idx, o = native.Index.build(p, g), oracle_py.Index.build(oracle_py.params_from_read_length(150), g)
+    genome = g.seq.tobytes()
+    lens = [150, 150, 30, 300, 2600, 2600, 3000, 4000, 150, 20, 4000]
+    q, off = native.randstrobes_query(p, reads_of([genome[a: a + n] for a, n in zip(range(500, 90_000, 7000), lens)]))
+    q, off = q.copy(), off.copy()
+    for r in range(len(lens)):
+        a, b = int(off[r]), int(off[r + 1])
+        if r in (1, 3, 5, 6, 7):
+            q[a:b] = q[a:b][rng.permutation(b - a)]
+        if r == 1 and b - a > 4:   # equal starts keep their order
+            q["start"][a + 1: a + 3] = q["start"][a]
+            q["end"][a + 1: a + 3] = q["end"][a]
+    assert max(np.diff(off.astype(np.int64))) > 1024
+    laid = q.copy()   # forward first, then by start, stable
+    for r in range(len(lens)):
+        part = q[int(off[r]): int(off[r + 1])]
+        laid[int(off[r]): int(off[r + 1])] = part[np.lexsort((part["start"], part["is_reverse"] != 0))]
+    for lo in (0, 1, 8):   # (the last: all in order)
+        m = native.Mapper(idx, max_reads=64)
+        a = m.find_nams(q, off[lo:], rescue=rescue, rescue_cutoff=50)
+        b = m.find_nams(laid, off[lo:], rescue=rescue, rescue_cutoff=50)
+        assert all((x == y).all() for x, y in zip(a, b))
+        for i in range(2, len(lens) - lo):
+            part = q[int(off[lo + i]): int(off[lo + i + 1])]
+            want = o.find_nams_rescue(part, 50) if rescue else o.find_nams(part)[0]
+            assert nams_equal(a[0][int(a[1][i]): int(a[1][i + 1])], oracle_py.sort_nams(want)), (lo, i)
