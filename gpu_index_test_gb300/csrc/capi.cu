@@ -7,6 +7,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <fstream>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -119,6 +120,68 @@ void host_parallel_tasks(size_t n, const std::function<void(size_t)>& fn) {
     HostPool::get().run(n, [&](size_t b, size_t e) {
         for (size_t i = b; i < e; ++i) fn(i);
     }, 1);
+}
+
+namespace {
+// One pool a device that asked for scratch; never destroyed (the driver is, before us).
+struct ScratchPools {
+    std::mutex mu;
+    uint64_t indexes = 0;
+    std::map<int, cudaMemPool_t> pools;
+};
+ScratchPools& scratch_pools() {
+    static ScratchPools* s = new ScratchPools();
+    return *s;
+}
+void keep_at_most(cudaMemPool_t p, uint64_t bytes) {
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &bytes);
+}
+}  // namespace
+
+void* scratch_alloc(size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    GBSA_CUDA(cudaGetDevice(&dev));
+    cudaMemPool_t pool;
+    {
+        ScratchPools& S = scratch_pools();
+        std::lock_guard<std::mutex> lock(S.mu);
+        auto it = S.pools.find(dev);
+        if (it == S.pools.end()) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            GBSA_CUDA(cudaMemPoolCreate(&pool, &props));
+            // a block may pass to another stream, but no stream is made to wait for one
+            int off = 0;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &off);
+            keep_at_most(pool, S.indexes ? kScratchKept : 0);
+            it = S.pools.emplace(dev, pool).first;
+        }
+        pool = it->second;
+    }
+    void* p = nullptr;
+    GBSA_CUDA(cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, pool, st));
+    return p;
+}
+
+void scratch_free(void* p, cudaStream_t st) noexcept { cudaFreeAsync(p, st); }
+
+ScratchLease::ScratchLease() {
+    ScratchPools& S = scratch_pools();
+    std::lock_guard<std::mutex> lock(S.mu);
+    if (S.indexes++ == 0)
+        for (auto& p : S.pools) keep_at_most(p.second, kScratchKept);
+}
+
+ScratchLease::~ScratchLease() {
+    ScratchPools& S = scratch_pools();
+    std::lock_guard<std::mutex> lock(S.mu);
+    if (--S.indexes == 0)
+        for (auto& p : S.pools) {
+            keep_at_most(p.second, 0);
+            cudaMemPoolTrimTo(p.second, 0);
+        }
 }
 
 int device_sm_count() {
@@ -845,59 +908,106 @@ int gbsa_randstrobes_query(const gbsa_params* p, const char* seqs, const uint64_
     return guarded([&] {
         if (!params_valid(*p)) throw Error(GBSA_ERR_PARAM, "invalid index parameters");
         require_device();
-        gbsa_index dummy;
-        dummy.params = *p;
-        dummy.dp = make_dev_params(*p);
-        gbsa_mapper m;
-        m.idx = &dummy;
-        GBSA_CUDA(cudaStreamCreateWithFlags(&m.st, cudaStreamNonBlocking));
-        struct G {
-            cudaStream_t s;
-            ~G() { cudaStreamDestroy(s); }
-        } g{m.st};
-        Workspace ws;
+        const DevParams dp = make_dev_params(*p);
         const uint32_t n = n_reads;
-        stage_reads(m, seqs, offsets, lengths, n, m.st);
+        // as stage_reads, from the caller's memory (pinned staging for one call costs more
+        // than the copy): the span of the reads, or the reads one after another
+        const uint64_t lo = n ? offsets[0] : 0, hi = n ? offsets[n - 1] + lengths[n - 1] : 0;
+        std::atomic<bool> inside{hi >= lo};
+        std::atomic<uint64_t> total_bases{0};
+        host_parallel_for(n, [&](size_t b, size_t e) {
+            bool ok = true;
+            uint64_t t = 0;
+            for (size_t i = b; i < e; ++i) {
+                ok &= offsets[i] >= lo && offsets[i] + lengths[i] <= hi;
+                t += lengths[i];
+            }
+            if (!ok) inside.store(false);
+            total_bases.fetch_add(t);
+        });
+        const bool direct = inside.load() && hi - lo <= 2 * total_bases.load() + (1u << 20);   // no large gaps
+        const uint64_t bases = direct ? hi - lo : total_bases.load();
+        std::vector<char> flat;
+        std::vector<uint64_t> flat_offs;
+        if (!direct) {
+            flat.resize(bases + 1);
+            flat_offs.resize(n + 1);
+            for (uint32_t i = 0; i < n; ++i) flat_offs[i + 1] = flat_offs[i] + lengths[i];
+            host_parallel_for(n, [&](size_t b, size_t e) {
+                for (size_t i = b; i < e; ++i) std::memcpy(flat.data() + flat_offs[i], seqs + offsets[i], lengths[i]);
+            });
+        }
+        struct Stream {
+            cudaStream_t s = nullptr;
+            Stream() { GBSA_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
+            ~Stream() { cudaStreamDestroy(s); }
+        } own;
+        cudaStream_t st = own.s;
+        Workspace ws(st);
+        DeviceBuffer d_seqs(bases + 64, st), d_offs(8ull * (n + 1), st), d_lens(4ull * (n + 1), st);
+        DeviceBuffer d_rec(sizeof(ReadRec) * (n + 1), st), d_long(4ull * (n + 1), st), d_ctr(sizeof(Counters), st);
+        DeviceBuffer d_cnt(8ull * (n + 1), st), d_off(8ull * (n + 1), st), d_slots(0, st);
+        // query randstrobes: ~2 per 5 bases plus slack
+        Arenas A{};
+        A.q_cap = std::max<uint64_t>(4096, bases / 2 + 8ull * n);
+        DeviceBuffer d_q(sizeof(Query) * A.q_cap, st);
+        A.long_list = d_long.as<uint32_t>();
+        if (bases)
+            GBSA_CUDA(cudaMemcpyAsync(d_seqs.as<void>(), direct ? seqs + lo : flat.data(), bases,
+                                      cudaMemcpyHostToDevice, st));
+        if (n) {
+            GBSA_CUDA(cudaMemcpyAsync(d_offs.as<void>(), direct ? offsets : flat_offs.data(), 8ull * n,
+                                      cudaMemcpyHostToDevice, st));
+            GBSA_CUDA(cudaMemcpyAsync(d_lens.as<void>(), lengths, 4ull * n, cudaMemcpyHostToDevice, st));
+        }
+        // (the caller's offsets count from `lo` bases before the buffer)
+        const uint8_t* at = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(d_seqs.as<void>()) -
+                                                             (direct ? lo : 0));
+        Counters* ctr = d_ctr.as<Counters>();
+        ReadRec* rec = d_rec.as<ReadRec>();
+        uint64_t* off = d_off.as<uint64_t>();
         for (int attempt = 0; attempt < 8; ++attempt) {
-            Counters* ctr = m.ctr.as<Counters>();
-            GBSA_CUDA(cudaMemsetAsync(ctr, 0, sizeof(Counters), m.st));
-            GBSA_CUDA(cudaMemsetAsync(m.rec.as<void>(), 0, sizeof(ReadRec) * (n + 1), m.st));
-            Arenas A = arenas_of(m);
-            launch_seed(dummy.dp, m.seqs.as<uint8_t>(), m.offs.as<uint64_t>(), m.lens.as<uint32_t>(), n,
-                        m.rec.as<ReadRec>(), A, ctr, m.st);
-            launch_seed_long(dummy.dp, m.seqs.as<uint8_t>(), m.offs.as<uint64_t>(), m.lens.as<uint32_t>(),
-                             m.rec.as<ReadRec>(), A, ctr, m.long_scratch.as<uint8_t>(), m.long_warps, m.st);
+            A.q = d_q.as<Query>();
+            GBSA_CUDA(cudaMemsetAsync(ctr, 0, sizeof(Counters), st));
+            GBSA_CUDA(cudaMemsetAsync(rec, 0, sizeof(ReadRec) * (n + 1), st));
+            launch_seed(dp, at, d_offs.as<uint64_t>(), d_lens.as<uint32_t>(), n, rec, A, ctr, st);
             Counters h{};
-            GBSA_CUDA(cudaMemcpyAsync(&h, ctr, sizeof h, cudaMemcpyDeviceToHost, m.st));
-            GBSA_CUDA(cudaStreamSynchronize(m.st));
+            uint64_t total = 0;
+            auto finish = [&] {
+                const size_t mark = ws.mark();
+                launch_read_counts(n, rec, 1, d_cnt.as<uint64_t>(), st);
+                scan_exclusive_u64(d_cnt.as<uint64_t>(), off, n, off + n, ws, st);
+                ws.rewind(mark);
+                GBSA_CUDA(cudaMemcpyAsync(&h, ctr, sizeof h, cudaMemcpyDeviceToHost, st));
+                GBSA_CUDA(cudaMemcpyAsync(&total, off + n, 8, cudaMemcpyDeviceToHost, st));
+                GBSA_CUDA(cudaStreamSynchronize(st));
+            };
+            finish();
+            if (h.n_long) {   // reads that the kernel's buffers do not hold
+                const uint32_t warps = (uint32_t)std::max(8, device_sm_count()) * 2;
+                d_slots.resize((uint64_t)warps * kLongSlotBytes);
+                launch_seed_long(dp, at, d_offs.as<uint64_t>(), d_lens.as<uint32_t>(), rec, A, ctr,
+                                 d_slots.as<uint8_t>(), warps, st);
+                finish();
+            }
             if (h.status & kStatusReadTooLong)
                 throw Error(GBSA_ERR_READ_TOO_LONG, "a read is longer than GBSA_MAX_READ_LEN bases");
             if (h.status & kStatusSyncmerOverflow) throw Error(GBSA_ERR_DEVICE_STATUS, "syncmer buffer overflow");
             if (h.status & kStatusQueryOverflow) {
-                grow(m.q, m.q_cap, h.q_used, sizeof(Query));
-                m.qaux.release();
-                m.qaux.resize(4 * m.q_cap);
-                m.qpos.release();
-                m.qpos.resize(8 * m.q_cap);
+                grow(d_q, A.q_cap, h.q_used, sizeof(Query));
                 continue;
             }
-            uint64_t* cnt = m.cnt.as<uint64_t>();
-            uint64_t* off = m.out_off.as<uint64_t>();
-            launch_read_counts(n, m.rec.as<ReadRec>(), 1, cnt, m.st);
-            scan_exclusive_u64(cnt, off, n, off + n, ws, m.st);
-            GBSA_CUDA(cudaMemcpyAsync(out_offsets, off, 8ull * (n + 1), cudaMemcpyDeviceToHost, m.st));
-            GBSA_CUDA(cudaStreamSynchronize(m.st));
-            const uint64_t total = out_offsets[n];
+            GBSA_CUDA(cudaMemcpyAsync(out_offsets, off, 8ull * (n + 1), cudaMemcpyDeviceToHost, st));
             if (out_total) *out_total = total;
-            if (total > out_capacity) throw Error(GBSA_ERR_CAPACITY, "output capacity too small");
-            if (total) {
-                DeviceBuffer dout(sizeof(gbsa_query_randstrobe) * total);
-                launch_gather_queries(n, m.rec.as<ReadRec>(), m.q.as<Query>(), off,
-                                      dout.as<gbsa_query_randstrobe>(), m.st);
-                GBSA_CUDA(cudaMemcpyAsync(out, dout.as<void>(), sizeof(gbsa_query_randstrobe) * total,
-                                          cudaMemcpyDeviceToHost, m.st));
-                GBSA_CUDA(cudaStreamSynchronize(m.st));
+            DeviceBuffer d_out(0, st);
+            if (total && total <= out_capacity) {
+                d_out.resize(sizeof(gbsa_query_randstrobe) * total);
+                launch_gather_queries(n, rec, A.q, off, d_out.as<gbsa_query_randstrobe>(), st);
+                GBSA_CUDA(cudaMemcpyAsync(out, d_out.as<void>(), sizeof(gbsa_query_randstrobe) * total,
+                                          cudaMemcpyDeviceToHost, st));
             }
+            GBSA_CUDA(cudaStreamSynchronize(st));
+            if (total > out_capacity) throw Error(GBSA_ERR_CAPACITY, "output capacity too small");
             return;
         }
         throw Error(GBSA_ERR_DEVICE_STATUS, "query arena kept overflowing");

@@ -577,8 +577,7 @@ extern "C" int gbsa_extend_seeds_device(const uint8_t* d_ref_seqs, const uint64_
         cudaStream_t st = (cudaStream_t)stream;
         // the status word is allocated in stream order: a cudaFree would wait for the
         // whole device
-        unsigned int* bad = nullptr;
-        GBSA_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&bad), sizeof(unsigned int), st));
+        unsigned int* bad = static_cast<unsigned int*>(scratch_alloc(sizeof(unsigned int), st));
         unsigned int h_bad = 0;
         const cudaError_t e = [&] {
             // one wave of resident blocks (the loop strides over the NAMs)
@@ -597,7 +596,7 @@ extern "C" int gbsa_extend_seeds_device(const uint8_t* d_ref_seqs, const uint64_
             if (r != cudaSuccess) return r;
             return cudaMemcpyAsync(&h_bad, bad, sizeof h_bad, cudaMemcpyDeviceToHost, st);
         }();
-        GBSA_CUDA(cudaFreeAsync(bad, st));
+        scratch_free(bad, st);
         GBSA_CUDA(e);
         GBSA_CUDA(cudaStreamSynchronize(st));
         if (h_bad)
@@ -623,8 +622,7 @@ extern "C" int gbsa_rescue_mates_device(const uint8_t* d_ref_seqs, const uint64_
         if (k < 3 || k > 32) throw Error(GBSA_ERR_PARAM, "k must be in [3, 32]");
         if (n_nams == 0) return GBSA_OK;
         cudaStream_t st = (cudaStream_t)stream;
-        unsigned int* bad = nullptr;
-        GBSA_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&bad), sizeof(unsigned int), st));
+        unsigned int* bad = static_cast<unsigned int*>(scratch_alloc(sizeof(unsigned int), st));
         unsigned int h_bad = 0;
         const cudaError_t e = [&] {
             int per_sm = 0;
@@ -644,7 +642,7 @@ extern "C" int gbsa_rescue_mates_device(const uint8_t* d_ref_seqs, const uint64_
             if (r != cudaSuccess) return r;
             return cudaMemcpyAsync(&h_bad, bad, sizeof h_bad, cudaMemcpyDeviceToHost, st);
         }();
-        GBSA_CUDA(cudaFreeAsync(bad, st));
+        scratch_free(bad, st);
         GBSA_CUDA(e);
         GBSA_CUDA(cudaStreamSynchronize(st));
         if (h_bad)
@@ -734,12 +732,11 @@ extern "C" int gbsa_run_align_steps_device(const uint8_t* d_ref_seqs, const uint
         const size_t b_u32 = (4ull * n_steps + 255) & ~size_t(255);
         const size_t b_u64 = (8ull * n_steps + 255) & ~size_t(255);
         const size_t b_res = (sizeof(gbsa_mate_rescue) * n_steps + 255) & ~size_t(255);
-        uint8_t* sc = nullptr;
-        GBSA_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&sc), 2 * b_nams + 2 * b_u32 + b_u64 + b_res + 256, st));
+        uint8_t* sc = static_cast<uint8_t*>(scratch_alloc(2 * b_nams + 2 * b_u32 + b_u64 + b_res + 256, st));
         struct Free {
             uint8_t* p;
             cudaStream_t s;
-            ~Free() { cudaFreeAsync(p, s); }
+            ~Free() { scratch_free(p, s); }
         } release{sc, st};
         gbsa_nam* step_nams = reinterpret_cast<gbsa_nam*>(sc);
         uint32_t* step_reads = reinterpret_cast<uint32_t*>(sc + b_nams);

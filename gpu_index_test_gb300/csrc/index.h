@@ -21,6 +21,7 @@ struct gbsa_index {
     uint64_t n = 0;
     gbsa_index_info info{};
     int device = 0;
+    gbsa::ScratchLease lease;
     gbsa::DeviceBuffer rs;       // gbsa_ref_randstrobe[n]
     gbsa::DeviceBuffer starts;   // uint64_t[2^bits + 1]
     gbsa::DeviceBuffer buckets;  // Bucket[2^bits + 1] read by the kernels when n < 2^32

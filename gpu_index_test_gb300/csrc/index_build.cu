@@ -296,20 +296,20 @@ static void finish_stats(gbsa_index& ix, const std::vector<unsigned long long>& 
 void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, const uint64_t* lengths,
                  uint32_t n_contigs, float f) {
     const DevParams P = ix.dp;
-    Workspace ws;
     cudaStream_t st;
     GBSA_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     struct StreamGuard {
         cudaStream_t s;
         ~StreamGuard() { cudaStreamDestroy(s); }
     } guard{st};
+    Workspace ws(st);
 
     // ---- genome upload + packing -------------------------------------------
     std::vector<uint64_t> cbase(n_contigs + 1, 0);
     for (uint32_t c = 0; c < n_contigs; ++c) cbase[c + 1] = cbase[c] + lengths[c];
     const uint64_t total = cbase[n_contigs];
     const uint64_t nwords = (total + 31) / 32 + 4;
-    DeviceBuffer d_g(nwords * 32 + 64);
+    DeviceBuffer d_g(nwords * 32 + 64, st);
     GBSA_CUDA(cudaMemsetAsync(d_g.as<uint8_t>(), 'N', nwords * 32 + 64, st));
     {
         // contiguous input → one copy; otherwise one copy per contig
@@ -324,7 +324,7 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
                                               cudaMemcpyHostToDevice, st));
         }
     }
-    DeviceBuffer d_packed(nwords * 8 + 64), d_nmask(nwords * 4 + 64);
+    DeviceBuffer d_packed(nwords * 8 + 64, st), d_nmask(nwords * 4 + 64, st);
     k_pack_genome<<<grid_for(nwords, 256, 65535), 256, 0, st>>>(d_g.as<uint8_t>(), nwords, d_packed.as<uint64_t>(),
                                                                 d_nmask.as<uint32_t>());
     GBSA_LAUNCHED();
@@ -346,8 +346,8 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     }
     cfirst_seg[n_contigs] = seg_c.size();
     const uint32_t n_seg = (uint32_t)seg_c.size();
-    DeviceBuffer d_segc(4 * (n_seg + 1)), d_segw0(4 * (n_seg + 1)), d_segw1(4 * (n_seg + 1));
-    DeviceBuffer d_cbase(8 * (n_contigs + 1)), d_cnwin(4 * (n_contigs + 1));
+    DeviceBuffer d_segc(4 * (n_seg + 1), st), d_segw0(4 * (n_seg + 1), st), d_segw1(4 * (n_seg + 1), st);
+    DeviceBuffer d_cbase(8 * (n_contigs + 1), st), d_cnwin(4 * (n_contigs + 1), st);
     if (n_seg) {
         GBSA_CUDA(cudaMemcpyAsync(d_segc.as<void>(), seg_c.data(), 4 * n_seg, cudaMemcpyHostToDevice, st));
         GBSA_CUDA(cudaMemcpyAsync(d_segw0.as<void>(), seg_w0.data(), 4 * n_seg, cudaMemcpyHostToDevice, st));
@@ -359,8 +359,8 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     SegTables T{d_segc.as<uint32_t>(), d_segw0.as<uint32_t>(), d_segw1.as<uint32_t>(), d_cbase.as<uint64_t>(),
                 d_cnwin.as<uint32_t>()};
 
-    DeviceBuffer d_segcnt(8 * (n_seg + 1)), d_segoff(8 * (n_seg + 1)), d_cseg(8 * (n_contigs + 1));
-    DeviceBuffer d_bits(4ull * kSegWords * (n_seg + 1)), d_csm(8 * (n_contigs + 1));
+    DeviceBuffer d_segcnt(8 * (n_seg + 1), st), d_segoff(8 * (n_seg + 1), st), d_cseg(8 * (n_contigs + 1), st);
+    DeviceBuffer d_bits(4ull * kSegWords * (n_seg + 1), st), d_csm(8 * (n_contigs + 1), st);
     const unsigned seg_blocks = grid_for(n_seg, kSegWarps, 1u << 20);
     std::vector<uint64_t> csm(n_contigs + 1, 0);   // first syncmer of every contig, and their number
     if (n_seg) {
@@ -377,7 +377,7 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
         GBSA_CUDA(cudaStreamSynchronize(st));
     }
     const uint64_t n_sm = csm[n_contigs];
-    DeviceBuffer d_sh(8 * (n_sm + 1)), d_sp(4 * (n_sm + 1));
+    DeviceBuffer d_sh(8 * (n_sm + 1), st), d_sp(4 * (n_sm + 1), st);
     if (n_seg) {
         k_write_syncmers<<<seg_blocks, 32 * kSegWarps, 0, st>>>(P, d_packed.as<uint64_t>(), T, n_seg,
                                                                 d_segoff.as<uint64_t>(), d_bits.as<uint32_t>(),
@@ -400,16 +400,21 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     cref[n_contigs] = n_rs;
     ix.n = n_rs;
     ix.info.tot_strobemer_count = n_rs;
-    DeviceBuffer d_cref(8 * (n_contigs + 1)), d_clen(8 * (n_contigs + 1));
+    DeviceBuffer d_cref(8 * (n_contigs + 1), st), d_clen(8 * (n_contigs + 1), st);
     GBSA_CUDA(cudaMemcpyAsync(d_cref.as<void>(), cref.data(), 8 * (n_contigs + 1), cudaMemcpyHostToDevice, st));
     GBSA_CUDA(cudaMemcpyAsync(d_clen.as<void>(), clen.data(), 8 * (n_contigs + 1), cudaMemcpyHostToDevice, st));
 
-    DeviceBuffer d_a(16 * (n_rs + 1)), d_b(16 * (n_rs + 1));
-    GBSA_CUDA(cudaMemsetAsync(d_a.as<void>(), 0, 16 * (n_rs + 1), st));
+    // the sort's passes go back and forth between the table and scratch; they end in the table
+    ix.rs.resize(16 * (n_rs + 1));
+    DeviceBuffer d_rs(16 * (n_rs + 1), st);
+    gbsa_ref_randstrobe* from = ix.rs.as<gbsa_ref_randstrobe>();
+    gbsa_ref_randstrobe* to = d_rs.as<gbsa_ref_randstrobe>();
+    if (sort_passes(n_rs) % 2) std::swap(from, to);
+    GBSA_CUDA(cudaMemsetAsync(from, 0, 16 * (n_rs + 1), st));
     if (n_sm) {
         k_ref_randstrobes<<<grid_for(n_sm, 256, 1u << 20), 256, 0, st>>>(
             P, d_sh.as<uint64_t>(), d_sp.as<uint32_t>(), n_sm, d_csm.as<uint64_t>(), n_contigs, d_cref.as<uint64_t>(),
-            d_clen.as<uint64_t>(), d_a.as<gbsa_ref_randstrobe>());
+            d_clen.as<uint64_t>(), from);
         GBSA_LAUNCHED();
     }
     d_sh.release();
@@ -418,20 +423,17 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     d_nmask.release();
 
     // ---- sort --------------------------------------------------------------------
-    gbsa_ref_randstrobe* sorted =
-        sort_ref_randstrobes(d_a.as<gbsa_ref_randstrobe>(), d_b.as<gbsa_ref_randstrobe>(), n_rs, max_position, ws, st);
-    if (sorted == d_a.as<gbsa_ref_randstrobe>()) {
-        ix.rs = std::move(d_a);
-    } else {
-        ix.rs = std::move(d_b);
-    }
+    const gbsa_ref_randstrobe* sorted = sort_ref_randstrobes(from, to, n_rs, max_position, ws, st);
+    const gbsa_ref_randstrobe* rs = ix.rs.as<gbsa_ref_randstrobe>();
+    if (sorted != rs)   // (a table of repeats, sorted by all bytes)
+        GBSA_CUDA(cudaMemcpyAsync(ix.rs.as<void>(), sorted, 16 * n_rs, cudaMemcpyDeviceToDevice, st));
+    d_rs.release();
 
     // ---- bucket tables, run-length statistics → filter_cutoff -----------------------
     const uint64_t nb = (1ULL << ix.bits) + 1;
     ix.starts.resize(8 * nb);
     const bool tagged = n_rs < (1ull << 32);
     if (tagged) ix.buckets.resize(sizeof(Bucket) * nb);
-    const gbsa_ref_randstrobe* rs = ix.rs.as<gbsa_ref_randstrobe>();
     std::vector<unsigned long long> H(102, 0);
     if (n_rs == 0) {
         GBSA_CUDA(cudaMemsetAsync(ix.starts.as<void>(), 0, 8 * nb, st));

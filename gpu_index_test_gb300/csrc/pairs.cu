@@ -550,9 +550,7 @@ extern "C" int gbsa_nam_pairs_device(const gbsa_nam* d_nams, const uint64_t* d_n
         const size_t b_flags = pad(total + 1), b_compact = pad(sizeof(CompactNam) * (total + 1));
         const size_t b_blocks = pad(sizeof(PairBlock) * ((total >> 5) + 2ull * n_pairs + 2));
         const size_t b_lists = pad(sizeof(gbsa_nam_pair) * slots);
-        uint8_t* scratch = nullptr;
-        GBSA_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&scratch),
-                                  b_flags + b_compact + b_blocks + b_lists + 8 * slots, st));
+        uint8_t* scratch = static_cast<uint8_t*>(scratch_alloc(b_flags + b_compact + b_blocks + b_lists + 8 * slots, st));
         uint8_t* s_compact = scratch + b_flags;
         uint8_t* s_blocks = s_compact + b_compact;
         uint8_t* s_lists = s_blocks + b_blocks;
@@ -563,7 +561,7 @@ extern "C" int gbsa_nam_pairs_device(const gbsa_nam* d_nams, const uint64_t* d_n
             reinterpret_cast<CompactNam*>(s_compact), reinterpret_cast<PairBlock*>(s_blocks),
             reinterpret_cast<gbsa_nam_pair*>(s_lists), reinterpret_cast<int*>(s_lists + b_lists), d_pairs, d_counts);
         const cudaError_t launch = cudaGetLastError();
-        GBSA_CUDA(cudaFreeAsync(scratch, st));
+        scratch_free(scratch, st);
         GBSA_CUDA(launch);
         GBSA_LAUNCHED();
         return GBSA_OK;
@@ -817,14 +815,13 @@ extern "C" int gbsa_plan_pairs_device(const gbsa_nam* d_nams, const uint64_t* d_
         cudaStream_t st = (cudaStream_t)stream;
         // scratch in stream order: step counts (then offsets) per pair, the status word
         const size_t b_cnt = (8ull * (n_pairs + 1) + 255) & ~size_t(255);
-        uint8_t* scratch = nullptr;
-        GBSA_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&scratch), b_cnt + 256, st));
+        uint8_t* scratch = static_cast<uint8_t*>(scratch_alloc(b_cnt + 256, st));
         uint64_t* counts = reinterpret_cast<uint64_t*>(scratch);
         unsigned int* bad = reinterpret_cast<unsigned int*>(scratch + b_cnt);
         struct Free {
             uint8_t* p;
             cudaStream_t s;
-            ~Free() { cudaFreeAsync(p, s); }
+            ~Free() { scratch_free(p, s); }
         } release{scratch, st};
         GBSA_CUDA(cudaMemsetAsync(bad, 0, 4, st));
         const unsigned grid = grid_for(n_pairs, kPairWarps), block = 32 * kPairWarps;
@@ -832,7 +829,7 @@ extern "C" int gbsa_plan_pairs_device(const gbsa_nam* d_nams, const uint64_t* d_
                                                     d_pair_counts, max_tries, dropoff, counts, nullptr, nullptr, 0,
                                                     nullptr);
         GBSA_LAUNCHED();
-        Workspace ws;
+        Workspace ws(st);
         scan_exclusive_u64(counts, counts, n_pairs, counts + n_pairs, ws, st);
         k_plan_pairs<true><<<grid, block, 0, st>>>(d_nams, d_nam_offsets, n_pairs, layout, d_types, d_pairs,
                                                    d_pair_counts, max_tries, dropoff, counts, d_plans, d_steps,
@@ -842,7 +839,7 @@ extern "C" int gbsa_plan_pairs_device(const gbsa_nam* d_nams, const uint64_t* d_
         unsigned int h_bad = 0;
         GBSA_CUDA(cudaMemcpyAsync(&total, counts + n_pairs, 8, cudaMemcpyDeviceToHost, st));
         GBSA_CUDA(cudaMemcpyAsync(&h_bad, bad, 4, cudaMemcpyDeviceToHost, st));
-        GBSA_CUDA(cudaStreamSynchronize(st));   // the scan's workspace is freed on return
+        GBSA_CUDA(cudaStreamSynchronize(st));
         if (n_steps) *n_steps = total;
         if (h_bad) throw Error(GBSA_ERR_PARAM, "a NAM pair with neither NAM");
         if (total > step_capacity) throw Error(GBSA_ERR_CAPACITY, "step capacity too small");

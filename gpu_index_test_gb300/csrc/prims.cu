@@ -360,6 +360,13 @@ static void radix_pass(const gbsa_ref_randstrobe* src, gbsa_ref_randstrobe* dst,
     GBSA_LAUNCHED();
 }
 
+int sort_passes(size_t n) {
+    if (n <= 1) return 0;
+    int bytes = 1;
+    while (bytes < 3 && (n >> (8 * bytes)) >= kGroupMean) ++bytes;
+    return bytes;
+}
+
 gbsa_ref_randstrobe* sort_ref_randstrobes(gbsa_ref_randstrobe* a, gbsa_ref_randstrobe* b, size_t n, uint32_t max_position,
                                           Workspace& ws, cudaStream_t st) {
     if (n <= 1) return a;
@@ -375,8 +382,7 @@ gbsa_ref_randstrobe* sort_ref_randstrobes(gbsa_ref_randstrobe* a, gbsa_ref_rands
     };
     // groups by the hash's top bits: of up to kGroupMean records on average while that saves
     // a pass, else of 24 to 48
-    int bytes = 1;
-    while (bytes < 3 && (n >> (8 * bytes)) >= kGroupMean) ++bytes;
+    const int bytes = sort_passes(n);
     int bits = 8 * bytes;
     while (bits > 8 && (n >> bits) < 24) --bits;
     gbsa_ref_randstrobe* src = a;
