@@ -82,17 +82,21 @@ __global__ void __launch_bounds__(32 * kSegWarps) k_mark_syncmers(DevParams P, c
         uint32_t any_n = P.W > 32 ? 1u : 0u;
         for (uint32_t i = lane; i < words; i += 32) any_n |= nmask[(g >> 5) + i];
         uint32_t n = 0;
-        auto put = [&](uint32_t at, uint32_t b) {
-            if (lane == 0) own[at >> 5] = b;
+        const uint32_t shift = (uint32_t)(P.W - 1);
+        auto put = [&](uint32_t at, uint32_t b) {   // bit l: window at + l - shift
+            if (lane == 0) {
+                if (at && shift) own[(at >> 5) - 1] |= b << (32 - shift);
+                if (at < w1 - w0) own[at >> 5] = b >> shift;
+            }
             n += __popc(b);
         };
         bool ok = !__any_sync(0xFFFFFFFFu, any_n != 0);
         if (ok) {
-            uint32_t* ring = reinterpret_cast<uint32_t*>(hbuf);
+            uint32_t* buf = reinterpret_cast<uint32_t*>(hbuf);
             const uint64_t* pk = packed + (g >> 5);
             const uint32_t p0 = (uint32_t)(g & 31);
-            ok = clean_scan5(P) ? warp_clean_scan<5>(P, pk, p0, w1 - w0, ring, put)
-                                : warp_clean_scan<0>(P, pk, p0, w1 - w0, ring, put);
+            ok = clean_scan5(P) ? warp_clean_scan<5>(P, pk, p0, w1 - w0, buf, put)
+                                : warp_clean_scan<0>(P, pk, p0, w1 - w0, buf, put);
             __syncwarp();
         }
         if (!ok) {

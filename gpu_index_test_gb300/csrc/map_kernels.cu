@@ -381,25 +381,27 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_lookup_long(IndexView I
 // downwards; the distance between two syncmers is the same either way), a query goes from
 // the lane that selects it straight into the index, and what is left of it for the hits (its
 // interval, the run's place and first entry) lies in the warp's scratch slot, which stays in
-// L2, instead of passing query, position and count through the arena: 2,290 warp
+// L2, instead of passing query, position and count through the arena: 2,150 warp
 // instructions a read of 150 bp (2,710 by the steps), both bound by integer issue; with the
-// tags and with one atomic a piece (WarpRoom, items_per_take) 2M reads 6.05 -> 4.5 ms, 100k
+// tags and with one atomic a piece (WarpRoom, items_per_take) 2M reads 6.05 -> 4.4 ms, 100k
 // reads of 300 bp 1.12 -> 1.00 ms, of 400 bp 1.36 -> 1.10 ms.
 constexpr uint32_t kFastQueries = 256;
+constexpr uint32_t kFastPad = 24;      // words before and behind the list: the most strobes ahead
+constexpr uint32_t kFastShift = 256;   // added to positions: more than any max_dist
 
 __host__ __device__ __forceinline__ bool fast_seed(const DevParams& P, const IndexView& I, const MapConfig& C) {
-    return P.q <= 0xFF && P.W <= 32 && I.buckets != nullptr && I.filter_cutoff <= 255 && !C.force_rescue && !C.count_bytes;
+    return P.q <= 0xFF && P.W <= 32 && P.w_max <= kFastPad && I.buckets != nullptr && I.filter_cutoff <= 255 && !C.force_rescue && !C.count_bytes;
 }
 
 __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I, const MapConfig& C,
                                           const uint8_t* __restrict__ seq, uint32_t L, uint32_t r,
                                           ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr, uint64_t* pk,
-                                          uint32_t* ring, uint64_t* sh, uint32_t* sp, uint32_t cap, WarpRoom& room,
+                                          uint32_t* buf, uint64_t* sh, uint32_t* sp, uint32_t cap, WarpRoom& room,
                                           uint32_t& direct) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = lane_id();
     if (L < (uint32_t)P.k || !warp_pack_clean(seq, L, pk)) return false;
-    const uint32_t n = warp_clean_syncmers(P, pk, L - (uint32_t)P.k + 1, ring, sp, cap);
+    const uint32_t n = warp_clean_syncmers(P, pk, L - (uint32_t)P.k + 1, buf, sp, cap);
     if (n > cap) return false;   // (ties too)
     const uint32_t nq = n_query_per_dir(P, n, L), nq2 = 2 * nq;
     if (nq2 > kFastQueries) return false;
@@ -408,10 +410,15 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
         const uint32_t w = sp[i];
         const uint64_t h = kmer_hash(P, pk, w);
         sh[i] = h;
-        sp[i] = (w << 8) | ((uint32_t)h & 0xFFu);
+        sp[i] = ((w + kFastShift) << 8) | ((uint32_t)h & (uint32_t)P.q);
+    }
+    // beside the list positions that are too far from any: the selection needs no bounds
+    if (lane < kFastPad) {
+        sp[(int)lane - (int)kFastPad] = 0;
+        sp[n + lane] = 0xFFFFFFFFu;
     }
     __syncwarp();
-    const uint32_t q8 = (uint32_t)P.q, k = (uint32_t)P.k;
+    const uint32_t k = (uint32_t)P.k;
     // per found query: its interval, the run's place, the run's first entry
     uint4* found = reinterpret_cast<uint4*>(A.slots + (uint64_t)warp_global_id() * A.slot_bytes);
     uint64_t hits = 0;   // a byte a round
@@ -426,17 +433,20 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
             const bool rev = i >= nq;
             const uint32_t j = rev ? i - nq : i;
             const int i1 = (int)(rev ? n - 1 - j : j), dir = rev ? -1 : 1;
-            const uint32_t v1 = sp[i1], p1 = v1 >> 8;
-            const uint32_t last = min(P.w_max, n - 1 - j);
+            // a strobe at most max_dist away: no larger than `limit`, bits inverted for the
+            // reverse strand, whose strobes lie at smaller positions
+            const uint32_t v1 = sp[i1], flip = rev ? 0xFFFFFFFFu : 0u;
+            const uint32_t limit = ((v1 ^ flip) | 0xFFu) + (P.max_dist << 8);
+            const uint32_t* strobe = sp + i1 + dir * (int)P.w_min;
             uint32_t best = 0xFFFFFFFFu;
-            for (uint32_t x = P.w_min; x <= last; ++x) {
-                const uint32_t v = sp[i1 + dir * (int)x];
-                const uint32_t dist = rev ? p1 - (v >> 8) : (v >> 8) - p1;
-                if (dist > P.max_dist) break;
-                best = min(best, ((uint32_t)__popc((v ^ v1) & q8) << 16) | x);   // the first of the least
+#pragma unroll 4
+            for (uint32_t x = P.w_min; x <= P.w_max; ++x, strobe += dir) {
+                const uint32_t v = *strobe;
+                const uint32_t of = ((uint32_t)__popc((v ^ v1) & 0xFFu) << 16) | x;   // the first of the least
+                if ((v ^ flip) <= limit) best = min(best, of);
             }
             const int i2 = best == 0xFFFFFFFFu ? i1 : i1 + dir * (int)(best & 0xFFFFu);
-            const uint32_t p2 = sp[i2] >> 8;
+            const uint32_t p1 = (v1 >> 8) - kFastShift, p2 = (sp[i2] >> 8) - kFastShift;
             const uint32_t s1 = rev ? L - p1 - k : p1, e2 = rev ? L - p2 : p2 + k;
             p = index_probe(I, sh[i1] + sh[i2], (int)(e2 - s1));
             if (p.pos != kMissing) {
@@ -590,7 +600,7 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
     __shared__ uint32_t s_nm[kSeedWarps][kFusedMaxLen / 32 + 4];
     __shared__ uint64_t s_hb[kSeedWarps][64];
     __shared__ uint64_t s_sh[kSeedWarps][kFusedSyncmers];
-    __shared__ uint32_t s_sp[kSeedWarps][kFusedSyncmers];
+    __shared__ uint32_t s_sp[kSeedWarps][kFusedSyncmers + 2 * kFastPad];
     const uint32_t w = threadIdx.x >> 5;
     const uint32_t per = items_per_take(n);
     WarpRoom room, queries;
@@ -609,7 +619,7 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
         if (kFast) {
             if (L > kFusedMaxLen ||
                 !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], reinterpret_cast<uint32_t*>(s_hb[w]),
-                           s_sh[w], s_sp[w], kFusedSyncmers, room, direct))
+                           s_sh[w], s_sp[w] + kFastPad, kFusedSyncmers, room, direct))
                 slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
                           kFusedMaxLen, kFusedSyncmers);
         } else {
@@ -638,7 +648,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
     __shared__ uint32_t s_nm[kWarps][kMaxLen / 32 + 4];
     __shared__ uint64_t s_hb[kWarps][64];
     __shared__ uint64_t s_sh[kWarps][kSyncmers];
-    __shared__ uint32_t s_sp[kWarps][kSyncmers];
+    __shared__ uint32_t s_sp[kWarps][kSyncmers + 2 * kFastPad];
     const uint32_t w = threadIdx.x >> 5;
     const uint8_t* __restrict__ seqs = desc->seqs;
     const uint64_t* __restrict__ offs = desc->offs;
@@ -667,7 +677,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
             if (kFast) {
                 if (L > kMaxLen ||
                     !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w],
-                               reinterpret_cast<uint32_t*>(s_hb[w]), s_sh[w], s_sp[w], kSyncmers, room, direct))
+                               reinterpret_cast<uint32_t*>(s_hb[w]), s_sh[w], s_sp[w] + kFastPad, kSyncmers, room, direct))
                     slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
                               kMaxLen, kSyncmers);
             } else {

@@ -112,26 +112,31 @@ __device__ __forceinline__ bool warp_pack_clean(const uint8_t* seq, uint32_t L, 
     const uintptr_t a0 = reinterpret_cast<uintptr_t>(seq);
     const uint32_t mis = (uint32_t)(a0 & 3);
     const uint32_t* words = reinterpret_cast<const uint32_t*>(a0 - mis);
-    uint8_t* out = reinterpret_cast<uint8_t*>(packed);
-    bool clean = true;
-    for (uint32_t g = lane; g < 8 * nw; g += 32) {   // group g: bases 4 g .. 4 g + 3
-        const uint32_t p0 = 4 * g;
-        uint32_t code8 = 0;
+    uint16_t* out = reinterpret_cast<uint16_t*>(packed);
+    uint32_t bad = 0;
+    // codes of the nv lowest bytes of w, as 8 bits, the first base highest
+    auto code8 = [&](uint32_t w, uint32_t nv) {
+        const uint32_t c4 = ((w >> 1) ^ (w >> 2)) & 0x03030303u;
+        const uint32_t t = (c4 | (c4 >> 4)) & 0x00FF00FFu;
+        const uint32_t vmask = nv >= 4 ? 0xFFFFFFFFu : (1u << (8 * nv)) - 1;
+        bad |= ((w & 0xDFDFDFDFu) ^ __byte_perm(0x54474341u, 0u, (t | (t >> 8)) & 0xFFFFu)) & vmask;
+        return ((c4 & vmask) * 0x40100401u) >> 24;
+    };
+    for (uint32_t g = lane; g < 4 * nw; g += 32) {   // group g: bases 8 g .. 8 g + 7
+        const uint32_t p0 = 8 * g;
+        uint32_t code = 0;
         if (p0 < L) {
-            const uint32_t lo = words[g];
-            const uint32_t hi = (mis != 0 && (g + 1) * 4 - mis < L) ? words[g + 1] : 0u;
-            const uint32_t w = __funnelshift_r(lo, hi, 8 * mis);   // base p0 in the low byte
-            const uint32_t c4 = ((w >> 1) ^ (w >> 2)) & 0x03030303u;
-            const uint32_t t = (c4 | (c4 >> 4)) & 0x00FF00FFu;
-            const uint32_t nv = min(L - p0, 4u);   // bases of the read among the 4
-            const uint32_t vmask = nv == 4 ? 0xFFFFFFFFu : (1u << (8 * nv)) - 1;
-            clean &= (((w & 0xDFDFDFDFu) ^ __byte_perm(0x54474341u, 0u, (t | (t >> 8)) & 0xFFFFu)) & vmask) == 0;
-            code8 = ((c4 & vmask) * 0x40100401u) >> 24;   // the first base highest
+            const uint32_t n = L - p0;   // bases of the read from here on
+            const uint32_t w0 = words[2 * g];
+            const uint32_t w1 = 4 < n + mis ? words[2 * g + 1] : 0u;
+            const uint32_t w2 = mis != 0 && 8 < n + mis ? words[2 * g + 2] : 0u;
+            code = code8(__funnelshift_r(w0, w1, 8 * mis), n) << 8;   // base p0 in the low byte
+            if (n > 4) code |= code8(__funnelshift_r(w1, w2, 8 * mis), n - 4);
         }
-        out[g ^ 7] = (uint8_t)code8;
+        out[g ^ 3] = (uint16_t)code;
     }
     __syncwarp();
-    return __all_sync(0xFFFFFFFFu, clean);
+    return !__any_sync(0xFFFFFFFFu, bad != 0);
 }
 
 // n (<= 33) bits of an LSB-first u32 bitmask stream starting at bit p (two words
@@ -441,34 +446,40 @@ __device__ __forceinline__ uint32_t n_query_per_dir(const DevParams& P, uint32_t
 
 // Syncmers of the nwin windows from packed position p0 on, where no base is ambiguous.  A
 // window is a syncmer when its s-mer number t - 1 has the least hash of the W, decided on
-// the hashes' high words, so that a window costs W words of a ring of high words and a few
-// minima.  Calls chunk(c, bits) for each 32 windows from c on.  Where that s-mer ties with
-// the least of the others the state machine's history may count: returns false, and the
-// caller takes the full scan.  kW: W when known at compile time, with s <= 16 (0: P.W).
-// ring: 64 words (32 + W - 1 <= 64).
+// the hashes' high words.  The warp goes over the s-mers, 32 a step, the high words of a
+// step and of the W - 1 s-mers before it side by side in `buf` (32 + W - 1 <= 64 words), so
+// that a window costs W loads at fixed places and a few minima.  Calls chunk(c, bits) for
+// each step: bit l is window c + l - (W - 1).  Where that s-mer ties with the least of the
+// others the state machine's history may count: returns false, and the caller takes the
+// full scan.  kW: W when known at compile time, with s <= 16 (0: P.W).
 template <int kW, class Chunk>
 __device__ __forceinline__ bool warp_clean_scan(const DevParams& P, const uint64_t* packed, uint32_t p0, uint32_t nwin,
-                                                uint32_t* ring, Chunk&& chunk) {
+                                                uint32_t* buf, Chunk&& chunk) {
     const uint32_t lane = lane_id();
     const uint32_t W = kW ? kW : (uint32_t)P.W, t = kW ? kW / 2 : (uint32_t)(P.t - 1);
-    auto high = [&](uint32_t p) {
-        return (uint32_t)((kW ? xxh64((uint64_t)smer16(P, packed, p0 + p)) : smer_hash(P, packed, p0 + p)) >> 32);
-    };
-    if (lane < W - 1) ring[lane] = high(lane);
-    for (uint32_t c = 0; c < nwin; c += 32) {
-        const uint32_t w = c + lane;
-        ring[(w + W - 1) & 63] = high(w + W - 1);
+    const uint32_t n = nwin + W - 1;
+    uint32_t* mine = buf + lane;
+    for (uint32_t c = 0; c < n; c += 32) {
+        const uint32_t p = p0 + c + lane;
+        const uint32_t h = (uint32_t)((kW ? xxh64((uint64_t)smer16(P, packed, p)) : smer_hash(P, packed, p)) >> 32);
+        const uint32_t before = lane < W - 1 ? mine[32] : 0u;
         __syncwarp();
-        const uint32_t mid = ring[(w + t) & 63];
-        uint32_t least = 0xFFFFFFFFu;
+        if (lane < W - 1) mine[0] = before;
+        mine[W - 1] = h;
+        __syncwarp();
+        uint32_t mid = h, least = 0xFFFFFFFFu;
 #pragma unroll 4
-        for (uint32_t d = 0; d < W; ++d)
-            if (d != t) least = min(least, ring[(w + d) & 63]);
+        for (uint32_t d = 0; d < W; ++d) {
+            const uint32_t v = mine[d];
+            if (d == t) mid = v;
+            else least = min(least, v);
+        }
+        const uint32_t w = c + lane - (W - 1);   // (wraps below the first window)
         const bool in = w < nwin;
         if (__any_sync(0xFFFFFFFFu, in && mid == least)) return false;
         chunk(c, __ballot_sync(0xFFFFFFFFu, in && mid < least));
-        __syncwarp();
     }
+    __syncwarp();
     return true;
 }
 
@@ -478,15 +489,16 @@ __device__ __forceinline__ bool clean_scan5(const DevParams& P) { return P.W == 
 // The first `cap` syncmers' windows of a clean read into sp; returns their number, or
 // 0xFFFFFFFF where the full scan is needed.
 __device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, const uint64_t* packed, uint32_t nwin,
-                                                        uint32_t* ring, uint32_t* sp, uint32_t cap) {
+                                                        uint32_t* buf, uint32_t* sp, uint32_t cap) {
     uint32_t n = 0;
+    const uint32_t first = lane_id() - (uint32_t)(P.W - 1);
     auto put = [&](uint32_t c, uint32_t b) {
         const uint32_t idx = n + __popc(b & lanemask_lt());
-        if (((b >> lane_id()) & 1u) && idx < cap) sp[idx] = c + lane_id();
+        if (((b >> lane_id()) & 1u) && idx < cap) sp[idx] = c + first;
         n += __popc(b);
     };
-    const bool ok = clean_scan5(P) ? warp_clean_scan<5>(P, packed, 0, nwin, ring, put)
-                                   : warp_clean_scan<0>(P, packed, 0, nwin, ring, put);
+    const bool ok = clean_scan5(P) ? warp_clean_scan<5>(P, packed, 0, nwin, buf, put)
+                                   : warp_clean_scan<0>(P, packed, 0, nwin, buf, put);
     return ok ? n : 0xFFFFFFFFu;
 }
 
