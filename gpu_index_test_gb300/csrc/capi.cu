@@ -578,8 +578,8 @@ static uint64_t run_pipeline(gbsa_mapper& m, const uint8_t* d_seqs, const uint64
     throw Error(GBSA_ERR_DEVICE_STATUS, "work areas kept overflowing");
 }
 
-// L2 access-policy window over the index's bucket table (64 MB for 2^23 buckets), read by every probe of the lookup: held persisting
-// in L2 so that the entry gathers do not evict it.  Used when the table fits the
+// L2 access-policy window over the index's bucket table (16 MB for 2^20 buckets), read by
+// every probe of the lookup: held persisting in L2 so that the entry gathers do not evict it.  Used when the table fits the
 // device's largest window; the hit ratio is the part of the table the persisting L2
 // set-aside can hold.  The set-aside (cudaLimitPersistingL2CacheSize) is a limit of
 // this process's context: it is raised to the largest window of the live mappers and
@@ -605,7 +605,7 @@ void l2_window_attach(gbsa_mapper& m, bool on) {
     }
     const gbsa_index& ix = *m.idx;
     const void* base = ix.buckets.size() ? ix.buckets.as<void>() : ix.starts.as<void>();
-    const uint64_t bytes = ((1ull << ix.bits) + 1) * 8;
+    const uint64_t bytes = ((1ull << ix.bits) + 1) * (ix.buckets.size() ? sizeof(Bucket) : 8);
     int max_window = 0, persist_max = 0;
     GBSA_CUDA(cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, dev));
     GBSA_CUDA(cudaDeviceGetAttribute(&persist_max, cudaDevAttrMaxPersistingL2CacheSize, dev));

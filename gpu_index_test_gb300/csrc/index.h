@@ -29,13 +29,16 @@ struct gbsa_index {
 
 namespace gbsa {
 
-// A bucket as the lookup reads it: its start, and a tag (8 bits of the hash, hash_tag) of
-// each of its first four entries.  Two thirds of a read's queries are not in the index (its
-// other strand, and seeds with a sequencing error): the tags answer nearly all of those
-// from the bucket's own sector, without the dependent fetch of an entry.
-struct Bucket {
+// A bucket as the lookup reads it, in one 16-byte load: its start, its size (255: or more,
+// see the next bucket's start), and a tag (8 bits of the hash, hash_tag) of each of its first
+// kBucketTags entries.  Two thirds of a read's queries are not in the index (its other
+// strand, and seeds with a sequencing error): the tags answer nearly all of those without
+// the dependent fetch of an entry.  Buckets hold up to 5 entries on average (3.8 at 20 Mbp);
+// with 4 tags a third of them had to be searched (551 of 2,150 warp instructions a read).
+constexpr uint32_t kBucketTags = 11;
+struct __align__(16) Bucket {
     uint32_t start;
-    uint32_t tags;   // entry i's in byte i (0 past the bucket's end)
+    uint32_t w[3];   // the size in byte 0, entry i's tag in byte i + 1 (0 past the bucket's end)
 };
 
 // Read-only view of the index used by device code.

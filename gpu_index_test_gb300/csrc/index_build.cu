@@ -199,18 +199,20 @@ __device__ __forceinline__ uint64_t second_run(const gbsa_ref_randstrobe* __rest
     return hi;
 }
 
-// Bucket b's start and tags, its first entry being `at`.
+// Bucket b's form for the lookup, its first entry being `at` of n.
 __device__ __forceinline__ Bucket bucket_at(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, int bits,
                                             uint64_t b, uint64_t at) {
-    Bucket k;
-    k.start = (uint32_t)at;
-    k.tags = 0;
-    for (int j = 0; j < 4 && at + j < n; ++j) {
-        const uint64_t h = rs[at + j].hash;
+    uint32_t size = 0;
+    uint64_t lo = 0;
+    uint32_t hi = 0;   // bytes 0..7 and 8..11
+    for (; size < 255 && at + size < n; ++size) {
+        const uint64_t h = rs[at + size].hash;
         if ((h >> (64 - bits)) != b) break;
-        k.tags |= hash_tag(h) << (8 * j);
+        if (size < 7) lo |= (uint64_t)hash_tag(h) << (8 * (size + 1));
+        else if (size < kBucketTags) hi |= hash_tag(h) << (8 * (size - 7));
     }
-    return k;
+    lo |= size;
+    return Bucket{(uint32_t)at, {(uint32_t)lo, (uint32_t)(lo >> 32), hi}};
 }
 
 // The bucket table (the reference's first-bucket rule: the buckets up to the first entry's
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(256) k_tables(const gbsa_ref_randstrobe* __res
     auto put = [&](uint64_t b0, uint64_t b1, uint64_t at, uint64_t own) {   // [b0, b1), `own`: where at's entries lie
         for (uint64_t b = b0; b < b1; ++b) {
             starts[b] = at;
-            if (buckets) buckets[b] = b == own ? bucket_at(rs, n, bits, b, at) : Bucket{(uint32_t)at, 0u};
+            if (buckets) buckets[b] = b == own ? bucket_at(rs, n, bits, b, at) : Bucket{(uint32_t)at, {0, 0, 0}};
         }
     };
     uint32_t once = 0;
@@ -469,7 +471,7 @@ __global__ void k_make_buckets(const uint64_t* __restrict__ starts, const gbsa_r
         const bool good = a <= n && e <= n &&
                           (a >= e || ((rs[a].hash >> (64 - bits)) == i && (rs[e - 1].hash >> (64 - bits)) == i));
         if (!good) *odd = 1;
-        out[i] = good && a < e ? bucket_at(rs, e, bits, i, a) : Bucket{(uint32_t)a, 0u};
+        out[i] = good && a < e ? bucket_at(rs, e, bits, i, a) : Bucket{(uint32_t)a, {0, 0, 0}};
     }
     for (uint64_t i = 1 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         if (rs[i - 1].hash > rs[i].hash) *odd = 1;

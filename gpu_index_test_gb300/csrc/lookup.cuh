@@ -104,27 +104,46 @@ struct Probe {
     uint32_t position, packed;
 };
 
-// Candidates are the entries of the bucket whose tag matches; a bucket of more than four is
-// searched as a whole.  `len` is the query's length.
-__device__ __forceinline__ Probe index_probe(const IndexView& I, uint64_t key, int len) {
+// What the bucket alone says of a key: the entries that may equal it.  None (`match` 0): the
+// key is not in the index.
+struct Candidates {
+    uint32_t start;
+    uint32_t size;    // 255: or more
+    uint32_t match;   // bit i: entry i's tag agrees (kBucketTags or fewer entries), else bit 0
+};
+__device__ __forceinline__ uint4 load_bucket(const IndexView& I, uint64_t key) {
+    return __ldg(reinterpret_cast<const uint4*>(I.buckets) + (uint32_t)(key >> (64 - I.bits)));
+}
+__device__ __forceinline__ Candidates bucket_candidates(const uint4& b, uint64_t key) {
+    const uint32_t tag = hash_tag(key) * 0x01010101u;
+    // a bit for each byte that agrees, gathered in bits 24..27
+    auto bits = [&](uint32_t w, uint32_t bytes) { return (__vcmpeq4(w, tag) & bytes) * 0x01020408u; };
+    Candidates c;
+    c.start = b.x;
+    c.size = b.y & 0xFFu;
+    c.match = (bits(b.y, 0x01010100u) >> 25) & 0x7u;
+    c.match |= (bits(b.z, 0x01010101u) >> 21) & 0x78u;
+    c.match |= (bits(b.w, 0x01010101u) >> 17) & 0x780u;
+    c.match &= (1u << min(c.size, kBucketTags)) - 1;
+    if (c.size > kBucketTags) c.match = 1;
+    return c;
+}
+
+// The answer for a key with candidates: those entries in order, or a bucket of more than
+// kBucketTags searched as a whole.  `len` is the query's length.
+__device__ __forceinline__ Probe probe_candidates(const IndexView& I, uint64_t key, int len, const Candidates& c) {
     Probe p;
     p.pos = kMissing;
     p.filtered = false;
     p.n_hits = 0;
     p.position = p.packed = 0;
-    const uint32_t top = (uint32_t)(key >> (64 - I.bits));
-    const uint2 bk = __ldg(reinterpret_cast<const uint2*>(I.buckets) + top);
-    const uint32_t end = __ldg(&I.buckets[top + 1].start);
-    const uint32_t a = bk.x, cnt = end > a ? end - a : 0u;
-    if (cnt == 0) return p;
+    const uint32_t a = c.start;
+    uint32_t end = a + c.size;
     Entry e;
-    // bit 8 i: entry i's tag matches (of a bucket of up to four)
-    const uint32_t match = __vcmpeq4(bk.y, hash_tag(key) * 0x01010101u) & (cnt < 4 ? (1u << (8 * cnt)) - 1 : 0xFFFFFFFFu) &
-                           0x01010101u;
-    if (cnt <= 4) {
-        for (uint32_t m = match;; m &= m - 1) {
+    if (c.size <= kBucketTags) {
+        for (uint32_t m = c.match;; m &= m - 1) {
             if (!m) return p;
-            const uint32_t i = (uint32_t)(__ffs(m) - 1) >> 3;
+            const uint32_t i = (uint32_t)__ffs(m) - 1;
             e = load_entry(I, a + i);
             if (e.hash == key) {
                 p.pos = a + i;
@@ -132,6 +151,7 @@ __device__ __forceinline__ Probe index_probe(const IndexView& I, uint64_t key, i
             }
         }
     } else {
+        if (c.size == 255) end = __ldg(&I.buckets[(uint32_t)(key >> (64 - I.bits)) + 1].start);
         const uint64_t x = find_in(I, key, a, end);
         if (x == kNotFound) return p;
         p.pos = (uint32_t)x;
@@ -148,7 +168,7 @@ __device__ __forceinline__ Probe index_probe(const IndexView& I, uint64_t key, i
     int least = len - ((int)(e.packed & 0xFF) + I.k);
     least = least < 0 ? -least : least;
     for (uint32_t x = p.pos + 1; x < end; ++x) {
-        if (cnt <= 4 && !((match >> (8 * (x - a))) & 1u)) break;
+        if (c.size <= kBucketTags && !((c.match >> (x - a)) & 1u)) break;
         const Entry f = load_entry(I, x);
         if (f.hash != key) break;
         int diff = len - ((int)(f.packed & 0xFF) + I.k);
@@ -158,6 +178,17 @@ __device__ __forceinline__ Probe index_probe(const IndexView& I, uint64_t key, i
             ++p.n_hits;
         }
     }
+    return p;
+}
+
+__device__ __forceinline__ Probe index_probe(const IndexView& I, uint64_t key, int len) {
+    const Candidates c = bucket_candidates(load_bucket(I, key), key);
+    if (c.match) return probe_candidates(I, key, len, c);
+    Probe p;
+    p.pos = kMissing;
+    p.filtered = false;
+    p.n_hits = 0;
+    p.position = p.packed = 0;
     return p;
 }
 

@@ -48,6 +48,30 @@ __device__ __forceinline__ uint32_t warp_next(unsigned int* head) { return warp_
 // round trip, and they queue at one address): four while there are many for each warp.
 __device__ __forceinline__ uint32_t items_per_take(uint32_t n) { return n >= 32 * warp_count() ? 4u : 1u; }
 
+// Work items of a kernel whose warps share a counter.  About half of them are dealt out
+// beforehand (at most eight a warp), the others taken from the counter, up to four at a time
+// while there are many: one address takes about one atomic a nanosecond, so that 100,000
+// takes of one item alone took 80 us.
+struct WarpItems {
+    uint32_t n, base, at, left, per;
+    __device__ __forceinline__ explicit WarpItems(uint32_t n_items) : n(n_items) {
+        const uint32_t warps = warp_count();
+        left = min(max(n / (2 * warps), 1u), 8u);
+        at = warp_global_id() * left;
+        base = min((uint64_t)left * warps, (uint64_t)n);
+        per = min(max((n - base) / (16 * warps), 1u), 4u);
+    }
+    // The next item, or n and above at the end.
+    __device__ __forceinline__ uint32_t next(unsigned int* head) {
+        if (left == 0) {
+            at = base + warp_take(head, per);
+            left = per;
+        }
+        --left;
+        return at++;
+    }
+};
+
 // Room in an arena whose bump counter all warps share, taken ahead in pieces of up to
 // `piece` entries: a warp's requests come from its piece while they fit.  What is left
 // unused of the pieces is counted (`spare`), so that the counters still tell what was used.
@@ -113,15 +137,9 @@ __global__ void __launch_bounds__(32 * kSeedWarps, 5) k_seed_smem(DevParams P, c
     __shared__ uint64_t s_sh[kSeedWarps][kSmemSyncmers];
     __shared__ uint32_t s_sp[kSeedWarps][kSmemSyncmers];
     const uint32_t w = threadIdx.x >> 5;
-    const uint32_t per = items_per_take(n);
+    WarpItems items(n);
     WarpRoom room;
-    uint32_t left = 0, r = 0;
-    for (;; ++r, --left) {
-        if (left == 0) {
-            r = warp_take(&ctr->queue_head, per);
-            left = per;
-        }
-        if (r >= n) break;
+    for (uint32_t r; (r = items.next(&ctr->queue_head)) < n;) {
         const uint32_t L = lens[r];
         ReadRec& R = rec[r];
         if (L > GBSA_MAX_READ_LEN) {
@@ -346,15 +364,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_lookup(IndexView I, Map
                                                                  ReadRec* __restrict__ rec, Arenas A, Counters* ctr,
                                                                  const BatchDesc* desc) {
     if (desc) n = min(n, desc->n_reads);   // batched form: n is the work areas' capacity
-    const uint32_t per = items_per_take(n);
+    WarpItems items(n);
     WarpRoom room;
-    uint32_t left = 0, r = 0;
-    for (;; ++r, --left) {
-        if (left == 0) {
-            r = warp_take(&ctr->queue_head2, per);
-            left = per;
-        }
-        if (r >= n) break;
+    for (uint32_t r; (r = items.next(&ctr->queue_head2)) < n;) {
         lookup_read<kCount>(I, C, r, rec, A, ctr, room);
     }
     room.done(&ctr->hit_spare);
@@ -381,11 +393,20 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_lookup_long(IndexView I
 // downwards; the distance between two syncmers is the same either way), a query goes from
 // the lane that selects it straight into the index, and what is left of it for the hits (its
 // interval, the run's place and first entry) lies in the warp's scratch slot, which stays in
-// L2, instead of passing query, position and count through the arena: 2,150 warp
-// instructions a read of 150 bp (2,710 by the steps), both bound by integer issue; with the
-// tags and with one atomic a piece (WarpRoom, items_per_take) 2M reads 6.05 -> 4.4 ms, 100k
-// reads of 300 bp 1.12 -> 1.00 ms, of 400 bp 1.36 -> 1.10 ms.
+// L2, instead of passing query, position and count through the arena.  A third of the
+// queries have a candidate in their bucket: those are collected and looked at 32 at a time,
+// so that the entries' part runs about once a read and not with a few lanes in each round.
+// 1,880 warp instructions a read of 150 bp (2,710 by the steps), both bound by integer
+// issue: packing 190, syncmers 650, their k-mer hashes 190, selection 440, buckets 110,
+// entries 290, hits 150.  With the tags and with few atomics (WarpRoom, WarpItems) 2M reads
+// 6.05 -> 4.3 ms, 100k pairs of 300 bp 1.12 -> 0.86 ms, of 400 bp 1.36 -> 0.99 ms.
 constexpr uint32_t kFastQueries = 256;
+// Queries of a warp's read that wait for a look at the entries.
+struct FastQueue {
+    uint64_t key[64];
+    uint32_t start[64], what[64], se[64];   // the bucket's start; match | size << 16; the query
+    uint8_t hits[32];
+};
 constexpr uint32_t kFastPad = 24;      // words before and behind the list: the most strobes ahead
 constexpr uint32_t kFastShift = 256;   // added to positions: more than any max_dist
 
@@ -396,8 +417,8 @@ __host__ __device__ __forceinline__ bool fast_seed(const DevParams& P, const Ind
 __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I, const MapConfig& C,
                                           const uint8_t* __restrict__ seq, uint32_t L, uint32_t r,
                                           ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr, uint64_t* pk,
-                                          uint32_t* buf, uint64_t* sh, uint32_t* sp, uint32_t cap, WarpRoom& room,
-                                          uint32_t& direct) {
+                                          uint32_t* buf, uint64_t* sh, uint32_t* sp, uint32_t cap, FastQueue& Q,
+                                          WarpRoom& room, uint32_t& direct) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = lane_id();
     if (L < (uint32_t)P.k || !warp_pack_clean(seq, L, pk)) return false;
@@ -419,45 +440,104 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
     }
     __syncwarp();
     const uint32_t k = (uint32_t)P.k;
-    // per found query: its interval, the run's place, the run's first entry
+    // per found query, in order: start | end << 10 | query << 20, the run's place, the run's
+    // first entry
     uint4* found = reinterpret_cast<uint4*>(A.slots + (uint64_t)warp_global_id() * A.slot_bytes);
-    uint64_t hits = 0;   // a byte a round
-    uint32_t tot = 0, good = 0, sum = 0, is_found = 0;   // is_found: a bit a round
+    uint64_t hits = 0;   // a byte for each 32 found queries: the hits of the one that is this lane's
+    uint32_t tot = 0, good = 0, sum = 0, pending = 0;
+    // query i's strobes: its key, and its interval and number
+    auto select = [&](uint32_t i, uint64_t& key, uint32_t& se) {
+        const bool rev = i >= nq;
+        const uint32_t j = rev ? i - nq : i;
+        const int i1 = (int)(rev ? n - 1 - j : j), dir = rev ? -1 : 1;
+        // a strobe at most max_dist away: no larger than `limit`, bits inverted for the
+        // reverse strand, whose strobes lie at smaller positions
+        const uint32_t v1 = sp[i1], flip = rev ? 0xFFFFFFFFu : 0u;
+        const uint32_t limit = ((v1 ^ flip) | 0xFFu) + (P.max_dist << 8);
+        const uint32_t* strobe = sp + i1 + dir * (int)P.w_min;
+        uint32_t best = 0xFFFFFFFFu;
+#pragma unroll 4
+        for (uint32_t x = P.w_min; x <= P.w_max; ++x, strobe += dir) {
+            const uint32_t v = *strobe;
+            const uint32_t of = ((uint32_t)__popc((v ^ v1) & 0xFFu) << 16) | x;   // the first of the least
+            if ((v ^ flip) <= limit) best = min(best, of);
+        }
+        const int i2 = best == 0xFFFFFFFFu ? i1 : i1 + dir * (int)(best & 0xFFFFu);
+        const uint32_t p1 = (v1 >> 8) - kFastShift, p2 = (sp[i2] >> 8) - kFastShift;
+        const uint32_t s1 = rev ? L - p1 - k : p1, e2 = rev ? L - p2 : p2 + k;
+        se = s1 | (e2 << 10) | (i << 20);
+        key = sh[i1] + sh[i2];
+    };
     for (uint32_t round = 0; 32 * round < nq2; ++round) {
         const uint32_t i = 32 * round + lane;
-        Probe p;
-        p.pos = kMissing;
-        p.filtered = false;
-        p.n_hits = 0;
+        Candidates c;
+        c.match = 0;
+        uint64_t key = 0;
+        uint32_t se = 0;
         if (i < nq2) {
-            const bool rev = i >= nq;
-            const uint32_t j = rev ? i - nq : i;
-            const int i1 = (int)(rev ? n - 1 - j : j), dir = rev ? -1 : 1;
-            // a strobe at most max_dist away: no larger than `limit`, bits inverted for the
-            // reverse strand, whose strobes lie at smaller positions
-            const uint32_t v1 = sp[i1], flip = rev ? 0xFFFFFFFFu : 0u;
-            const uint32_t limit = ((v1 ^ flip) | 0xFFu) + (P.max_dist << 8);
-            const uint32_t* strobe = sp + i1 + dir * (int)P.w_min;
-            uint32_t best = 0xFFFFFFFFu;
-#pragma unroll 4
-            for (uint32_t x = P.w_min; x <= P.w_max; ++x, strobe += dir) {
-                const uint32_t v = *strobe;
-                const uint32_t of = ((uint32_t)__popc((v ^ v1) & 0xFFu) << 16) | x;   // the first of the least
-                if ((v ^ flip) <= limit) best = min(best, of);
-            }
-            const int i2 = best == 0xFFFFFFFFu ? i1 : i1 + dir * (int)(best & 0xFFFFu);
-            const uint32_t p1 = (v1 >> 8) - kFastShift, p2 = (sp[i2] >> 8) - kFastShift;
-            const uint32_t s1 = rev ? L - p1 - k : p1, e2 = rev ? L - p2 : p2 + k;
-            p = index_probe(I, sh[i1] + sh[i2], (int)(e2 - s1));
-            if (p.pos != kMissing) {
-                found[i] = make_uint4(s1 | (e2 << 16), p.pos, p.position, p.packed);
-                is_found |= 1u << round;
-                hits |= (uint64_t)p.n_hits << (8 * round);
-                sum += p.n_hits;
-            }
+            select(i, key, se);
+            c = bucket_candidates(load_bucket(I, key), key);
         }
-        tot += __popc(__ballot_sync(kFull, p.pos != kMissing));
-        good += __popc(__ballot_sync(kFull, p.pos != kMissing && !p.filtered));
+        // queries with candidates wait until there are 32 of them (or no more to come)
+        const uint32_t some = __ballot_sync(kFull, c.match != 0);
+        if (c.match) {
+            const uint32_t at = pending + __popc(some & lanemask_lt());
+            Q.key[at] = key;
+            Q.start[at] = c.start;
+            Q.what[at] = c.match | (c.size << 16);
+            Q.se[at] = se;
+        }
+        pending += __popc(some);
+        __syncwarp();
+        while (pending >= 32 || (pending && 32 * (round + 1) >= nq2)) {
+            const uint32_t m = min(pending, 32u);
+            Probe p;
+            p.pos = kMissing;
+            p.filtered = false;
+            uint32_t x = 0;
+            if (lane < m) {
+                Candidates d;
+                d.start = Q.start[lane];
+                d.match = Q.what[lane] & 0xFFFFu;
+                d.size = Q.what[lane] >> 16;
+                x = Q.se[lane];
+                p = probe_candidates(I, Q.key[lane], (int)((x >> 10) & 0x3FFu) - (int)(x & 0x3FFu), d);
+            }
+            const uint32_t is = __ballot_sync(kFull, p.pos != kMissing);
+            good += __popc(__ballot_sync(kFull, p.pos != kMissing && !p.filtered));
+            // the found ones to their places, their hits' number to the lane that writes them
+            if (p.pos != kMissing) {
+                const uint32_t at = tot + __popc(is & lanemask_lt());
+                found[at] = make_uint4(x, p.pos, p.position, p.packed);
+                Q.hits[at & 31] = (uint8_t)p.n_hits;
+            }
+            __syncwarp();
+            const uint32_t mine = tot + ((lane - tot) & 31u);
+            if (mine < tot + __popc(is)) {
+                const uint32_t nh = Q.hits[lane];
+                hits |= (uint64_t)nh << (8 * (mine >> 5));
+                sum += nh;
+            }
+            tot += __popc(is);
+            pending -= m;
+            // what is left moves to the front (fewer than 32)
+            uint64_t rk = 0;
+            uint32_t r0 = 0, r1 = 0, r2 = 0;
+            if (lane < pending) {
+                rk = Q.key[32 + lane];
+                r0 = Q.start[32 + lane];
+                r1 = Q.what[32 + lane];
+                r2 = Q.se[32 + lane];
+            }
+            __syncwarp();
+            if (lane < pending) {
+                Q.key[lane] = rk;
+                Q.start[lane] = r0;
+                Q.what[lane] = r1;
+                Q.se[lane] = r2;
+            }
+            __syncwarp();
+        }
     }
     ReadRec& R = rec[r];
     // nonrepetitive_fraction (step2/nam.cu:892) and the rescue trigger, as in lookup_read
@@ -480,16 +560,13 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
             R.nq = nq;
             R.nq2 = nq2;
         }
-        for (uint32_t round = 0; 32 * round < nq2; ++round) {
-            const uint32_t i = 32 * round + lane;
-            if (i >= nq2) continue;
-            uint64_t pos = kNotFound;
-            if ((is_found >> round) & 1u) {
-                const uint4 f = found[i];
-                pos = f.y;
-                A.q[off + i] = Query{0, f.x & 0xFFFFu, f.x >> 16};
-            }
-            A.q_pos[off + i] = pos;
+        for (uint32_t i = lane; i < nq2; i += 32) A.q_pos[off + i] = kNotFound;
+        __syncwarp();
+        for (uint32_t f = lane; f < tot; f += 32) {
+            const uint4 v = found[f];
+            const uint32_t i = v.x >> 20;
+            A.q[off + i] = Query{0, v.x & 0x3FFu, (v.x >> 10) & 0x3FFu};
+            A.q_pos[off + i] = v.y;
         }
         __syncwarp();
         enlist_rescue(I, C, r, R, A, ctr, good < tot);
@@ -506,8 +583,7 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
     // the hits in generation order (query order, then run order)
     HitPacked* out = A.hits + hoff;
     uint32_t at = 0;
-    for (uint32_t round = 0; 32 * round < nq2; ++round) {
-        const uint32_t i = 32 * round + lane;
+    for (uint32_t round = 0; 32 * round < tot; ++round) {
         const uint32_t nh = (uint32_t)(hits >> (8 * round)) & 0xFFu;
         const uint32_t any = __ballot_sync(kFull, nh != 0);
         if (!any) continue;
@@ -520,9 +596,9 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
             at += __popc(any);
         }
         if (nh) {
-            const uint4 f = found[i];
-            const uint32_t rc = i >= nq ? 0x80000000u : 0u;
-            const int qs = (int)(f.x & 0xFFFFu), qe = (int)(f.x >> 16);
+            const uint4 f = found[32 * round + lane];
+            const uint32_t rc = (f.x >> 20) >= nq ? 0x80000000u : 0u;
+            const int qs = (int)(f.x & 0x3FFu), qe = (int)((f.x >> 10) & 0x3FFu);
             if (nh == 1) {
                 out[to] = pack_hit(rc | (f.w >> 8), qs, qe, (int)f.z, (int)(f.z + (f.w & 0xFFu) + k));
             } else {
@@ -583,11 +659,12 @@ __device__ __noinline__ void slow_read(const DevParams& P, const IndexView& I, c
 // an SM interleave the two: while some wait on gathers, others hash.  Reads that do
 // not fit the shared-memory buffers go to the long list (k_seed_long, then
 // k_lookup_long).
-// 6 blocks of 8 warps per SM (48 warps: the lookup's gathers need the warps in flight;
-// 40 registers) and per-warp buffers for reads up to 512 bases and 160 syncmers (21 KB
-// per block, leaving the rest of the SM's unified L1 to cache index entries); longer
-// reads take the long path.
-constexpr int kFusedBlocksPerSm = 6;
+// 4 blocks of 8 warps per SM: 64 registers, with which nothing spills (6 blocks, 40
+// registers: 10% more instructions; 2M reads 9.03 ms a batch, 5 blocks 8.78, 4 blocks 8.83,
+// uneven lengths 1.44 / 1.45 / 1.43), and per-warp buffers for reads up to 512 bases and 160
+// syncmers (33 KB per block, leaving the rest of the SM's unified L1 to cache index
+// entries); longer reads take the long path.
+constexpr int kFusedBlocksPerSm = 4;
 constexpr uint32_t kFusedMaxLen = 512;
 constexpr uint32_t kFusedSyncmers = 160;
 
@@ -601,16 +678,12 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
     __shared__ uint64_t s_hb[kSeedWarps][64];
     __shared__ uint64_t s_sh[kSeedWarps][kFusedSyncmers];
     __shared__ uint32_t s_sp[kSeedWarps][kFusedSyncmers + 2 * kFastPad];
+    __shared__ FastQueue s_q[kFast ? kSeedWarps : 1];
     const uint32_t w = threadIdx.x >> 5;
-    const uint32_t per = items_per_take(n);
+    WarpItems items(n);
     WarpRoom room, queries;
-    uint32_t direct = 0, left = 0, r = 0;
-    for (;; ++r, --left) {
-        if (left == 0) {
-            r = warp_take(&ctr->queue_head, per);
-            left = per;
-        }
-        if (r >= n) break;
+    uint32_t direct = 0;
+    for (uint32_t r; (r = items.next(&ctr->queue_head)) < n;) {
         const uint32_t L = lens[r];
         if (L > GBSA_MAX_READ_LEN) {
             warp_fail(rec[r], ctr, kStatusReadTooLong);
@@ -619,7 +692,7 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
         if (kFast) {
             if (L > kFusedMaxLen ||
                 !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], reinterpret_cast<uint32_t*>(s_hb[w]),
-                           s_sh[w], s_sp[w] + kFastPad, kFusedSyncmers, room, direct))
+                           s_sh[w], s_sp[w] + kFastPad, kFusedSyncmers, s_q[kFast ? w : 0], room, direct))
                 slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
                           kFusedMaxLen, kFusedSyncmers);
         } else {
@@ -649,21 +722,17 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
     __shared__ uint64_t s_hb[kWarps][64];
     __shared__ uint64_t s_sh[kWarps][kSyncmers];
     __shared__ uint32_t s_sp[kWarps][kSyncmers + 2 * kFastPad];
+    __shared__ FastQueue s_q[kFast ? kWarps : 1];
     const uint32_t w = threadIdx.x >> 5;
     const uint8_t* __restrict__ seqs = desc->seqs;
     const uint64_t* __restrict__ offs = desc->offs;
     const uint32_t* __restrict__ lens = desc->lens;
     const uint32_t* __restrict__ items = desc->items;
     const uint32_t n_items = items ? desc->n_items : desc->n_reads;
-    const uint32_t per = items_per_take(n_items);
+    WarpItems queue(n_items);
     WarpRoom room, queries;
-    uint32_t direct = 0, left = 0, it = 0;
-    for (;; ++it, --left) {
-        if (left == 0) {
-            it = warp_take(&ctr->queue_head, per);
-            left = per;
-        }
-        if (it >= n_items) break;
+    uint32_t direct = 0;
+    for (uint32_t it; (it = queue.next(&ctr->queue_head)) < n_items;) {
         // item bounds outside [0, n_reads] are clamped (reads no item covers stay empty)
         const uint32_t n_reads = desc->n_reads;
         const uint32_t r0 = min(items ? items[it] : it, n_reads);
@@ -677,7 +746,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
             if (kFast) {
                 if (L > kMaxLen ||
                     !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w],
-                               reinterpret_cast<uint32_t*>(s_hb[w]), s_sh[w], s_sp[w] + kFastPad, kSyncmers, room, direct))
+                               reinterpret_cast<uint32_t*>(s_hb[w]), s_sh[w], s_sp[w] + kFastPad, kSyncmers, s_q[kFast ? w : 0], room, direct))
                     slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
                               kMaxLen, kSyncmers);
             } else {
@@ -2521,7 +2590,7 @@ void launch_seed_long(const DevParams& P, const uint8_t* seqs, const uint64_t* o
 // Variant 0 is the plain form's fused kernel shape.
 SeedVariant seed_variant(int v) {
     static const SeedVariant table[kSeedVariants] = {
-        {8, 6, 512, 160}, {8, 5, 512, 160}, {4, 12, 512, 160}, {8, 7, 256, 96}, {16, 3, 512, 160}, {8, 6, 256, 96},
+        {8, 4, 512, 160}, {8, 5, 512, 160}, {4, 12, 512, 160}, {8, 7, 256, 96}, {16, 2, 512, 160}, {8, 6, 256, 96},
     };
     return table[v < 0 || v >= kSeedVariants ? 0 : v];
 }
@@ -2543,9 +2612,9 @@ static void launch_q_variant(int v, const DevParams& P, const IndexView& I, cons
         case 1: launch_q<kCount, kLookup, kFast, 8, 5, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
         case 2: launch_q<kCount, kLookup, kFast, 4, 12, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
         case 3: launch_q<kCount, kLookup, kFast, 8, 7, 256, 96>(P, I, C, desc, rec, A, ctr, cap, st); break;
-        case 4: launch_q<kCount, kLookup, kFast, 16, 3, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
+        case 4: launch_q<kCount, kLookup, kFast, 16, 2, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
         case 5: launch_q<kCount, kLookup, kFast, 8, 6, 256, 96>(P, I, C, desc, rec, A, ctr, cap, st); break;
-        default: launch_q<kCount, kLookup, kFast, 8, 6, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
+        default: launch_q<kCount, kLookup, kFast, 8, 4, 512, 160>(P, I, C, desc, rec, A, ctr, cap, st); break;
     }
 }
 

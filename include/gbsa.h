@@ -252,9 +252,9 @@ int gbsa_mapper_set_pipeline(gbsa_mapper* m, uint32_t chunks);
  * (gpu_index_test_gb300/autotune.py) and committed as gpu_index_test_gb300/tuned.json,
  * which the library reads from its own directory.  The results do not depend on it. */
 typedef struct gbsa_batch_config {
-    int32_t  seed_variant;   /* persistent seeding + lookup kernel: 0 8 warps x 6 blocks/SM, reads up to
+    int32_t  seed_variant;   /* persistent seeding + lookup kernel: 0 8 warps x 4 blocks/SM, reads up to
                                 512 bases in shared memory; 1 8 x 5; 2 4 x 12; 3 8 x 7, 256 bases;
-                                4 16 x 3; 5 8 x 6, 256 bases (longer reads take the long-read path) */
+                                4 16 x 2; 5 8 x 6, 256 bases (longer reads take the long-read path) */
     uint32_t lane_max_hits;  /* 1-160; without effect (one NAM merge serves every value) */
     int32_t  sort_variant;   /* block size of the sort of rescued reads with many NAMs: 0 256, 1 512 */
     uint32_t chunk_reads;    /* reads per batch of the host entry point (three batches in flight) */
@@ -642,7 +642,7 @@ int gbsa_mapper_fused_lookup(const gbsa_mapper* m);
 int gbsa_mapper_set_fuse_limit(gbsa_mapper* m, uint64_t index_bytes);
 /* Hold the index's bucket table in L2 during the probing kernels (on = 1, the
  * default) through an access-policy window marked persisting, when the table fits
- * the device's largest window (the 32-bit table of up to 2^25 buckets); the
+ * the device's largest window (16 bytes a bucket); the
  * process's persisting L2 set-aside is raised for it while such mappers live.
  * *window_bytes (may be NULL) receives the window's size, 0 when none is used.  The
  * results are the same either way.  No reference counterpart. */
