@@ -2409,6 +2409,26 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(256)
     }
 }
 
+// Writes the records x of the first m lanes to out[0 .. m).  A record has 11 words: written
+// by each lane for itself, a store touches up to 44 sectors for 4 bytes of each; through
+// `words` (32 records of shared memory) they leave in whole sectors (the two gathers of
+// 100,000 reads 93 -> 60 us, of 2M reads 0.90 -> 0.60 ms with the first of them alone).
+static_assert(sizeof(gbsa_nam) == 44, "a record is 11 words");
+__device__ __forceinline__ void write_records(uint32_t* words, const gbsa_nam& x, uint32_t m, gbsa_nam* out) {
+    const uint32_t lane = lane_id();
+    if (lane < m) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(&x);
+#pragma unroll
+        for (uint32_t i = 0; i < 11; ++i) words[11 * lane + i] = w[i];
+    }
+    __syncwarp();
+    uint32_t* to = reinterpret_cast<uint32_t*>(out);
+#pragma unroll
+    for (uint32_t i = 0; i < 11; ++i)
+        if (32 * i + lane < 11 * m) to[32 * i + lane] = words[32 * i + lane];
+    __syncwarp();
+}
+
 // Records at or beyond out_cap are not written (the caller sized out from an estimate
 // and gathers again when the total turns out larger).
 // mode 0: every read; 1: the reads that were not rescued (fractions and rescue flags
@@ -2418,6 +2438,9 @@ __global__ void k_gather_nams(uint32_t n, const ReadRec* __restrict__ rec, const
                               const uint64_t* __restrict__ out_off, gbsa_nam* __restrict__ out, uint64_t out_cap,
                               float* frac, uint8_t* rescued, int mode, Arenas A, const Counters* ctr,
                               const BatchDesc* desc) {
+    __shared__ uint32_t s_words[kWarpsPerBlock][32 * 11];
+    uint32_t* words = s_words[threadIdx.x >> 5];
+    const uint32_t lane = lane_id();
     uint64_t* copy_off = nullptr;
     if (desc) {
         const uint32_t cap = n;
@@ -2440,40 +2463,54 @@ __global__ void k_gather_nams(uint32_t n, const ReadRec* __restrict__ rec, const
             const uint32_t r = t < n_light ? A.rescue_list[t] : A.rescue_list[A.rescue_cap - 1 - (t - n_light)];
             const ReadRec R = rec[r];
             const uint64_t o = out_off[r];
-            for (uint32_t j = threadIdx.x; j < R.n_nams; j += blockDim.x)
-                if (o + j < out_cap) to_gbsa_nam(arena[R.nam_off + j], (int)j, out[o + j]);
+            const uint32_t m = o >= out_cap ? 0u : (uint32_t)min((uint64_t)R.n_nams, out_cap - o);
+            for (uint32_t j = 32 * (threadIdx.x >> 5); j < m; j += blockDim.x) {
+                gbsa_nam x;
+                if (j + lane < m) to_gbsa_nam(arena[R.nam_off + j + lane], (int)(j + lane), x);
+                write_records(words, x, min(m - j, 32u), out + o + j);
+            }
         }
         return;
     }
-    // 16 lanes a read (most hold about ten NAMs), the next read's record on its way
-    const uint32_t sub = threadIdx.x & 15u;
-    const uint32_t stride = 2 * warp_count();
-    uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
-    ReadRec R{};
-    uint64_t o = 0;
-    if (r < n) {
-        R = rec[r];
-        o = out_off[r];
-    }
-    while (r < n) {
-        const uint32_t rn = r + stride;
-        ReadRec Rn{};
-        uint64_t on = 0;
-        if (rn < n) {
-            Rn = rec[rn];
-            on = out_off[rn];
-        }
-        const bool skip = mode == 1 && (R.flags & kReadRescue);
-        for (uint32_t j = sub; j < (skip ? 0u : R.n_nams); j += 16)
-            if (o + j < out_cap) to_gbsa_nam(arena[R.nam_off + j], (int)j, out[o + j]);
-        if (sub == 0) {
+    // up to 32 reads in turn a warp, their NAMs side by side over the lanes
+    const uint32_t group = min(max(n / warp_count(), 1u), 32u);
+    for (uint32_t r0 = warp_global_id() * group; r0 < n; r0 += warp_count() * group) {
+        const uint32_t r = r0 + lane;
+        uint32_t count = 0;
+        uint64_t from = 0, o = 0;   // the read's first NAM, its first record
+        if (lane < group && r < n) {
+            const ReadRec& R = rec[r];
+            const bool resc = (R.flags & kReadRescue) != 0;
+            count = mode == 1 && resc ? 0u : R.n_nams;
+            from = R.nam_off;
+            o = out_off[r];
             if (frac) frac[r] = R.frac;
-            if (rescued) rescued[r] = (R.flags & kReadRescue) ? 1 : 0;
+            if (rescued) rescued[r] = resc ? 1 : 0;
             if (copy_off) copy_off[r] = o;
         }
-        r = rn;
-        R = Rn;
-        o = on;
+        const uint32_t upto = warp_inclusive_sum(count);
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, upto, 31);
+        from -= upto - count;
+        o -= upto - count;
+        const uint32_t before = upto - count;
+        for (uint32_t c = 0; c < total; c += 32) {
+            const uint32_t t = c + lane;
+            // the read of NAM t: the first whose NAMs end behind it
+            uint32_t at = 0;
+#pragma unroll
+            for (uint32_t step = 16; step; step /= 2)
+                if (__shfl_sync(0xFFFFFFFFu, upto, at + step - 1) <= t) at += step;
+            const uint64_t src = __shfl_sync(0xFFFFFFFFu, from, at) + t;
+            const uint64_t dst = __shfl_sync(0xFFFFFFFFu, o, at) + t;
+            const uint32_t id = t - __shfl_sync(0xFFFFFFFFu, before, at);
+            const bool in = t < total && dst < out_cap;
+            const uint64_t first = __shfl_sync(0xFFFFFFFFu, dst, 0);
+            const uint32_t m = __popc(__ballot_sync(0xFFFFFFFFu, in));
+            gbsa_nam x;
+            if (in) to_gbsa_nam(arena[src], (int)id, x);
+            if (__all_sync(0xFFFFFFFFu, !in || dst == first + lane)) write_records(words, x, m, out + first);
+            else if (in) out[dst] = x;
+        }
     }
 }
 
