@@ -623,10 +623,10 @@ __device__ __forceinline__ void step_read(const DevParams& P, const IndexView& I
                                           const uint8_t* seq, uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A,
                                           Counters* ctr, uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh,
                                           uint32_t* sp, uint32_t max_len, uint32_t cap, WarpRoom& queries,
-                                          WarpRoom& hits) {
+                                          WarpRoom& hits, bool try_clean = true) {
     ReadRec& R = rec[r];
     uint32_t ns = 0xFFFFFFFFu;
-    if (L <= max_len) ns = warp_read_syncmers(P, seq, L, pk, nm, hb, sh, sp, cap);
+    if (L <= max_len) ns = warp_read_syncmers(P, seq, L, pk, nm, hb, sh, sp, cap, try_clean);
     if (ns == 0xFFFFFFFFu) {
         if (lane_id() == 0) {
             R.flags |= kReadLong;
@@ -648,7 +648,7 @@ __device__ __noinline__ void slow_read(const DevParams& P, const IndexView& I, c
                                        uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh, uint32_t* sp,
                                        uint32_t max_len, uint32_t cap) {
     WarpRoom queries, hits;
-    step_read<false, true>(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, max_len, cap, queries, hits);
+    step_read<false, true>(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, max_len, cap, queries, hits, false);
     queries.done(&ctr->q_spare);
     hits.done(&ctr->hit_spare);
 }

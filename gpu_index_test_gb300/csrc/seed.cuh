@@ -412,31 +412,6 @@ struct Query {
     uint32_t end;
 };
 
-// Seeds one read with the warp: packs it into pk/nm (capacity for L bases), finds
-// its syncmers into sh/sp (capacity cap) and returns the syncmer count, or
-// 0xFFFFFFFF when more than cap syncmers exist.
-__device__ __forceinline__ uint32_t warp_read_syncmers(const DevParams& P, const uint8_t* seq, uint32_t L, uint64_t* pk,
-                                                       uint32_t* nm, uint64_t* hbuf, uint64_t* sh, uint32_t* sp,
-                                                       uint32_t cap) {
-    if (L < (uint32_t)P.k) return 0;
-    const bool has_n = warp_pack_read(seq, L, pk, nm);
-    const uint32_t nwin = L - (uint32_t)P.k + 1;
-    auto emit = [&](uint32_t idx, uint32_t w) {
-        if (idx < cap) sp[idx] = w;
-    };
-    // reads without N (nearly all) skip the per-window N checks; the common window
-    // width (5 s-mers: k - s = 4) is unrolled at compile time
-    uint32_t n;
-    if (has_n) n = warp_syncmer_scan(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
-    else if (P.W == 5) n = warp_syncmer_scan<5, true>(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
-    else n = warp_syncmer_scan<0, true>(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
-    if (n > cap) return 0xFFFFFFFFu;
-    __syncwarp();
-    for (uint32_t i = lane_id(); i < n; i += 32) sh[i] = kmer_hash(P, pk, sp[i]);
-    __syncwarp();
-    return n;
-}
-
 // Number of query randstrobes per orientation for n syncmers of a read of length L
 // (randstrobes_query returns none when L < w_max, step2/randstrobes.cu:197).
 __device__ __forceinline__ uint32_t n_query_per_dir(const DevParams& P, uint32_t n, uint32_t L) {
@@ -500,6 +475,36 @@ __device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, cons
     const bool ok = clean_scan5(P) ? warp_clean_scan<5>(P, packed, 0, nwin, buf, put)
                                    : warp_clean_scan<0>(P, packed, 0, nwin, buf, put);
     return ok ? n : 0xFFFFFFFFu;
+}
+
+// Seeds one read with the warp: packs it into pk/nm (capacity for L bases), finds
+// its syncmers into sh/sp (capacity cap) and returns the syncmer count, or
+// 0xFFFFFFFF when more than cap syncmers exist.
+__device__ __forceinline__ uint32_t warp_read_syncmers(const DevParams& P, const uint8_t* seq, uint32_t L, uint64_t* pk,
+                                                       uint32_t* nm, uint64_t* hbuf, uint64_t* sh, uint32_t* sp,
+                                                       uint32_t cap, bool try_clean = true) {
+    if (L < (uint32_t)P.k) return 0;
+    const bool has_n = warp_pack_read(seq, L, pk, nm);
+    const uint32_t nwin = L - (uint32_t)P.k + 1;
+    auto emit = [&](uint32_t idx, uint32_t w) {
+        if (idx < cap) sp[idx] = w;
+    };
+    // reads without N (nearly all) and without a tied window take the scan without state;
+    // else those without N skip the per-window N checks, and the common window width (5
+    // s-mers: k - s = 4) is unrolled at compile time
+    uint32_t n = 0xFFFFFFFFu;
+    if (try_clean && !has_n && P.W <= 32)
+        n = warp_clean_syncmers(P, pk, nwin, reinterpret_cast<uint32_t*>(hbuf), sp, cap);
+    if (n == 0xFFFFFFFFu) {
+        if (has_n) n = warp_syncmer_scan(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
+        else if (P.W == 5) n = warp_syncmer_scan<5, true>(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
+        else n = warp_syncmer_scan<0, true>(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
+    }
+    if (n > cap) return 0xFFFFFFFFu;
+    __syncwarp();
+    for (uint32_t i = lane_id(); i < n; i += 32) sh[i] = kmer_hash(P, pk, sp[i]);
+    __syncwarp();
+    return n;
 }
 
 // Writes the 2*nq query randstrobes of a read (forward, then reverse complement).
