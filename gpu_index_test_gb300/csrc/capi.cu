@@ -123,7 +123,7 @@ void host_parallel_tasks(size_t n, const std::function<void(size_t)>& fn) {
 }
 
 namespace {
-// One pool a device that asked for scratch; never destroyed (the driver is, before us).
+// One pool a device that asked for scratch; never destroyed (CUDA ends before us).
 struct ScratchPools {
     std::mutex mu;
     uint64_t indexes = 0;

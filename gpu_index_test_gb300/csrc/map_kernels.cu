@@ -2702,7 +2702,7 @@ void launch_lookup(const IndexView& I, const MapConfig& C, uint32_t n, ReadRec* 
 // other and need most of an SM's shared memory together (rescue 2 x 97 KB, group merge
 // 17 KB a block): they ask for the largest shared-memory carveout, so that the SM keeps
 // that configuration through the phase instead of switching it as each kernel's blocks
-// arrive (left to the driver, an earlier merge took 5.0 instead of 3.3 ms on the C2 batch
+// arrive (left to CUDA, an earlier merge took 5.0 instead of 3.3 ms on the C2 batch
 // inside the batch graph).  The seeding + lookup kernels keep the default: they use the
 // rest of the unified L1 to cache index entries.  Set once per device.
 void nam_phase_carveout() {

@@ -47,10 +47,10 @@ extern std::atomic<uint64_t> g_launches;
 // Scratch of a call, in the order of the stream that uses it, from a memory pool that the
 // library keeps for each device.  The pool holds on to at most kScratchKept bytes, and only
 // while an index lives (ScratchLease): with the last index its memory goes back, and
-// without one it returns whatever is free at each synchronisation, as the driver's own pool
+// without one it returns whatever is free at each synchronisation, as CUDA's default pool
 // does.  (An allocation from memory that the pool holds takes 1 us; mapping new memory and
 // giving it back 70 + 50 us for a status word, 130 + 60 us and a wait for the whole device
-// with cudaMalloc and cudaFree.)  Safe with several threads and streams: the driver hands a
+// with cudaMalloc and cudaFree.)  Safe with several threads and streams: CUDA hands a
 // block on only when the stream that freed it has passed that point.
 constexpr uint64_t kScratchKept = 256ull << 20;
 void* scratch_alloc(size_t bytes, cudaStream_t st);
