@@ -1754,7 +1754,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 3)
 // reference start, ...) the NAMs of one read need few bits a field, and they are created in
 // (orientation, query start, reference start) order, so their number stands for what comes
 // after the query end: score | orientation | reference | query start | query end | number
-// makes one 64-bit word without ties.  Up to 8192 such words sort in a block's registers
+// makes one 64-bit word without ties: no two NAMs agree in orientation, reference, query
+// start and reference start (queries with the same start and hash can open such NAMs, and
+// these go to the sorts below).  Up to 8192 such words sort in a block's registers
 // (bitonic; partners in other lanes by shuffles, in other warps through shared memory),
 // with nothing but the word to move; a read whose fields do not fit, or whose NAMs are not
 // in that order, goes to the sorts below.  Those move a key word and an index through
@@ -1823,10 +1825,11 @@ __device__ __noinline__ bool pack_sort(const SortJob& job, ReadRec& R, const Are
         ms = max(ms, (uint32_t)nam_score_int(a));
         mr = max(mr, a.ref_rc & 0x7FFFFFFFu);
         mq = max(mq, (uint32_t)a.qe);
-        if (i + 1 < n) {   // created in (orientation, query start, reference start) order
+        if (i + 1 < n) {   // created in (orientation, query start, reference start, reference) order
             const NamState b = closed[i + 1];
             const uint32_t oa = a.ref_rc >> 31, ob = b.ref_rc >> 31;
-            ok &= oa != ob ? oa < ob : (a.qs != b.qs ? a.qs < b.qs : a.rs <= b.rs);
+            ok &= oa != ob ? oa < ob
+                           : (a.qs != b.qs ? a.qs < b.qs : (a.rs != b.rs ? a.rs < b.rs : a.ref_rc < b.ref_rc));
         }
     }
     ms = __reduce_max_sync(0xFFFFFFFFu, ms);
