@@ -461,15 +461,17 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
 }
 
 // As bucket_at, for a table that was not built here: `odd` is set when the entries are
-// not in order or a bucket holds one that belongs elsewhere, for then a tag could answer
-// differently from the search in order.
+// not in order, a bucket holds one that belongs elsewhere, or one ends before the last entry
+// that belongs to it (start indices that stop short of the table's end), for then a tag or a
+// bucket's end could answer differently from the search in order and the walk of a run.
 __global__ void k_make_buckets(const uint64_t* __restrict__ starts, const gbsa_ref_randstrobe* __restrict__ rs,
                                uint64_t n, int bits, Bucket* __restrict__ out, uint32_t* __restrict__ odd) {
     const uint64_t nb = 1ULL << bits;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i <= nb; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t a = starts[i], e = i < nb ? starts[i + 1] : a;
+        auto top = [&](uint64_t at) { return rs[at].hash >> (64 - bits); };
         const bool good = a <= n && e <= n &&
-                          (a >= e || ((rs[a].hash >> (64 - bits)) == i && (rs[e - 1].hash >> (64 - bits)) == i));
+                          (a >= e || (top(a) == i && top(e - 1) == i && (e == n || top(e) != i)));
         if (!good) *odd = 1;
         out[i] = good && a < e ? bucket_at(rs, e, bits, i, a) : Bucket{(uint32_t)a, {0, 0, 0}};
     }

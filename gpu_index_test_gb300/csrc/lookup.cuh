@@ -232,12 +232,12 @@ __device__ __forceinline__ uint32_t index_get_count(const IndexView& I, uint64_t
 // to the query is <= the running minimum.  Stops at the end of the table.
 template <class Emit>
 __device__ __forceinline__ uint32_t walk_hit_run(const IndexView& I, int qs, int qe, uint64_t pos, Emit&& emit,
-                                                 uint32_t* run_len = nullptr) {
+                                                 uint32_t* run_len = nullptr, uint32_t most = 0xFFFFFFFFu) {
     int min_diff = 0x7FFFFFFF;
     const uint64_t key = get_hash(I, pos);
     const uint64_t p0 = pos;
     uint32_t n = 0;
-    for (; pos < I.n; ++pos) {
+    for (; pos < I.n && n < most; ++pos) {
         const gbsa_ref_randstrobe e = I.rs[pos];
         if (e.hash != key) break;
         const int rs = (int)e.position;

@@ -352,7 +352,7 @@ __device__ __forceinline__ void lookup_read(const IndexView& I, const MapConfig&
         const int qs = (int)Q[i].start, qe = (int)Q[i].end;
         walk_hit_run(I, qs, qe, pos, [&](uint32_t ref, int rs, int re) {
             out[k++] = pack_hit((dir << 31) | ref, qs, qe, rs, re);
-        });
+        }, nullptr, next - aux[i]);
     }
     if (lane == 0) {
         R.hit_off = hoff;
@@ -605,7 +605,7 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
             } else {
                 walk_hit_run(I, qs, qe, f.y, [&](uint32_t ref, int rs, int re) {
                     out[to++] = pack_hit(rc | ref, qs, qe, rs, re);
-                });
+                }, nullptr, nh);
             }
         }
     }
