@@ -387,8 +387,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_lookup_long(IndexView I
 
 // Seeding and lookup of a read in one go, for the reads nearly all batches are made of: only
 // A, C, G and T, no tied syncmer window, at most kFastQueries queries, and parameters and
-// an index for which fast_seed() holds (all profiles of read lengths).  Returns false, with
-// nothing written, for any other read (the caller then takes the steps one by one).
+// an index for which fast_seed() holds (all profiles of read lengths).  Any other read is left
+// to the steps one by one, with nothing written for it.
 //
 // Both orientations' randstrobes run through one loop (the reverse ones walk the syncmers
 // downwards; the distance between two syncmers is the same either way), a query goes from
@@ -415,18 +415,22 @@ __host__ __device__ __forceinline__ bool fast_seed(const DevParams& P, const Ind
     return P.q <= 0xFF && P.W <= 32 && P.w_max <= kFastPad && I.buckets != nullptr && I.filter_cutoff <= 255 && !C.force_rescue && !C.count_bytes;
 }
 
-__device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I, const MapConfig& C,
-                                          const uint8_t* __restrict__ seq, uint32_t L, uint32_t r,
-                                          ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr, uint64_t* pk,
-                                          uint32_t* buf, uint64_t* sh, uint32_t* sp, uint32_t cap, FastQueue& Q,
-                                          WarpRoom& room, uint32_t& direct) {
+// What fast_read says of a read: done, or left because of a base other than A, C, G and T, or
+// (all such bases, whatever the steps then find) for a tied window or its size.
+enum FastRead { kFastDone, kFastOdd, kFastTied };
+
+__device__ __forceinline__ FastRead fast_read(const DevParams& P, const IndexView& I, const MapConfig& C,
+                                              const uint8_t* __restrict__ seq, uint32_t L, uint32_t r,
+                                              ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr, uint64_t* pk,
+                                              uint32_t* buf, uint64_t* sh, uint32_t* sp, uint32_t cap, FastQueue& Q,
+                                              WarpRoom& room, uint32_t& direct) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = lane_id();
-    if (L < (uint32_t)P.k || !warp_pack_clean(seq, L, pk)) return false;
+    if (L < (uint32_t)P.k || !warp_pack_clean(seq, L, pk)) return kFastOdd;
     const uint32_t n = warp_clean_syncmers(P, pk, L - (uint32_t)P.k + 1, buf, sp, cap);
-    if (n > cap) return false;   // (ties too)
+    if (n > cap) return kFastTied;   // (or more syncmers)
     const uint32_t nq = n_query_per_dir(P, n, L), nq2 = 2 * nq;
-    if (nq2 > kFastQueries) return false;
+    if (nq2 > kFastQueries) return kFastTied;
     // the syncmers' hashes; their positions and the hash bits that the selection compares
     for (uint32_t i = lane; i < n; i += 32) {
         const uint32_t w = sp[i];
@@ -554,7 +558,7 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
         if (off + nq2 > A.q_cap) {
             warp_fail(R, ctr, kStatusQueryOverflow);
             if (lane == 0) R.nq = R.nq2 = 0;
-            return true;
+            return kFastDone;
         }
         if (lane == 0) {
             R.q_off = off;
@@ -572,14 +576,14 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
         __syncwarp();
         enlist_rescue(I, C, r, R, A, ctr, good < tot);
         __syncwarp();
-        return true;
+        return kFastDone;
     }
     const uint32_t H = __reduce_add_sync(kFull, sum);
     direct += nq2;
     const uint64_t hoff = room.take(&ctr->hit_used, H, arena_piece(A.hit_cap));
     if (hoff + H > A.hit_cap) {
         warp_fail(R, ctr, kStatusHitOverflow);
-        return true;
+        return kFastDone;
     }
     // the hits in generation order (query order, then run order)
     HitPacked* out = A.hits + hoff;
@@ -614,7 +618,7 @@ __device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I
         R.n_hits = H;
     }
     __syncwarp();
-    return true;
+    return kFastDone;
 }
 
 // The same read by the steps: seeding into the query arena, then lookup_read.  Reads that do
@@ -643,15 +647,39 @@ __device__ __forceinline__ void step_read(const DevParams& P, const IndexView& I
     }
 }
 
-// step_read beside the fast path: out of line, for the few reads that need it.
-__device__ __noinline__ void slow_read(const DevParams& P, const IndexView& I, const MapConfig& C, const uint8_t* seq,
-                                       uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A, Counters* ctr,
-                                       uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh, uint32_t* sp,
-                                       uint32_t max_len, uint32_t cap) {
+// A warp's room in the query and the hit arena.
+struct ReadRooms {
     WarpRoom queries, hits;
-    step_read<false, true>(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, max_len, cap, queries, hits, false);
-    queries.done(&ctr->q_spare);
-    hits.done(&ctr->hit_spare);
+};
+
+// step_read beside the fast path: out of line, for the reads that need it.  The warp's rooms
+// pass through by value, so that they stay in registers otherwise.  (With rooms of its own each
+// such read took a piece of both arenas, up to 512 entries of which it used some 50, and four
+// atomics: the first batch of 500k reads of 150 bp that all hold an N overflowed them and took
+// 12.6 ms; with the warp's 8.0.)
+__device__ __noinline__ ReadRooms slow_read(const DevParams& P, const IndexView& I, const MapConfig& C,
+                                            const uint8_t* seq, uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A,
+                                            Counters* ctr, uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh,
+                                            uint32_t* sp, uint32_t max_len, uint32_t cap, bool try_clean,
+                                            ReadRooms rooms) {
+    step_read<false, true>(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, max_len, cap, rooms.queries, rooms.hits,
+                           try_clean);
+    return rooms;
+}
+
+// A read of the fast kernels: in one go, else by the steps.
+template <uint32_t kMaxLen, uint32_t kSyncmers>
+__device__ __forceinline__ void fast_or_slow_read(const DevParams& P, const IndexView& I, const MapConfig& C,
+                                                  const uint8_t* seq, uint32_t L, uint32_t r, ReadRec* rec,
+                                                  const Arenas& A, Counters* ctr, uint64_t* pk, uint32_t* nm,
+                                                  uint64_t* hb, uint64_t* sh, uint32_t* sp, FastQueue& Q,
+                                                  ReadRooms& rooms, uint32_t& direct) {
+    FastRead f = kFastOdd;
+    if (L <= kMaxLen)
+        f = fast_read(P, I, C, seq, L, r, rec, A, ctr, pk, reinterpret_cast<uint32_t*>(hb), sh, sp + kFastPad, kSyncmers,
+                      Q, rooms.hits, direct);
+    if (f != kFastDone)
+        rooms = slow_read(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, kMaxLen, kSyncmers, f == kFastOdd, rooms);
 }
 
 // Seeding and lookup of a read by one warp (the main path): randstrobes_query, then
@@ -682,7 +710,7 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
     __shared__ FastQueue s_q[kFast ? kSeedWarps : 1];
     const uint32_t w = threadIdx.x >> 5;
     WarpItems items(n);
-    WarpRoom room, queries;
+    ReadRooms rooms;
     uint32_t direct = 0;
     for (uint32_t r; (r = items.next(&ctr->queue_head)) < n;) {
         const uint32_t L = lens[r];
@@ -690,19 +718,16 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
             warp_fail(rec[r], ctr, kStatusReadTooLong);
             continue;
         }
-        if (kFast) {
-            if (L > kFusedMaxLen ||
-                !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], reinterpret_cast<uint32_t*>(s_hb[w]),
-                           s_sh[w], s_sp[w] + kFastPad, kFusedSyncmers, s_q[kFast ? w : 0], room, direct))
-                slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
-                          kFusedMaxLen, kFusedSyncmers);
-        } else {
+        if (kFast)
+            fast_or_slow_read<kFusedMaxLen, kFusedSyncmers>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w],
+                                                            s_nm[w], s_hb[w], s_sh[w], s_sp[w], s_q[kFast ? w : 0],
+                                                            rooms, direct);
+        else
             step_read<kCount, true>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w],
-                                    s_sp[w], kFusedMaxLen, kFusedSyncmers, queries, room);
-        }
+                                    s_sp[w], kFusedMaxLen, kFusedSyncmers, rooms.queries, rooms.hits);
     }
-    room.done(&ctr->hit_spare);
-    if (!kFast) queries.done(&ctr->q_spare);
+    rooms.hits.done(&ctr->hit_spare);
+    rooms.queries.done(&ctr->q_spare);
     if (direct && lane_id() == 0) atomicAdd(&ctr->q_direct, (unsigned long long)direct);
 }
 
@@ -731,7 +756,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
     const uint32_t* __restrict__ items = desc->items;
     const uint32_t n_items = items ? desc->n_items : desc->n_reads;
     WarpItems queue(n_items);
-    WarpRoom room, queries;
+    ReadRooms rooms;
     uint32_t direct = 0;
     for (uint32_t it; (it = queue.next(&ctr->queue_head)) < n_items;) {
         // item bounds outside [0, n_reads] are clamped (reads no item covers stay empty)
@@ -744,20 +769,16 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
                 warp_fail(rec[r], ctr, kStatusReadTooLong);
                 continue;
             }
-            if (kFast) {
-                if (L > kMaxLen ||
-                    !fast_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w],
-                               reinterpret_cast<uint32_t*>(s_hb[w]), s_sh[w], s_sp[w] + kFastPad, kSyncmers, s_q[kFast ? w : 0], room, direct))
-                    slow_read(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w], s_sp[w],
-                              kMaxLen, kSyncmers);
-            } else {
+            if (kFast)
+                fast_or_slow_read<kMaxLen, kSyncmers>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w],
+                                                      s_hb[w], s_sh[w], s_sp[w], s_q[kFast ? w : 0], rooms, direct);
+            else
                 step_read<kCount, kLookup>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w],
-                                           s_sh[w], s_sp[w], kMaxLen, kSyncmers, queries, room);
-            }
+                                           s_sh[w], s_sp[w], kMaxLen, kSyncmers, rooms.queries, rooms.hits);
         }
     }
-    room.done(&ctr->hit_spare);
-    if (!kFast) queries.done(&ctr->q_spare);
+    rooms.hits.done(&ctr->hit_spare);
+    rooms.queries.done(&ctr->q_spare);
     if (direct && lane_id() == 0) atomicAdd(&ctr->q_direct, (unsigned long long)direct);
 }
 
