@@ -76,12 +76,14 @@ struct WarpItems {
 // Room in an arena whose bump counter all warps share, taken ahead in pieces of up to
 // `piece` entries: a warp's requests come from its piece while they fit.  What is left
 // unused of the pieces is counted (`spare`), so that the counters still tell what was used.
+// most 0: no pieces, each request takes what it needs.
 struct WarpRoom {
     uint64_t at = 0;
-    uint32_t left = 0, spare = 0;
+    uint32_t left = 0, spare = 0, most = 512;
     __device__ __forceinline__ uint64_t take(unsigned long long* used, uint64_t n, uint32_t piece) {
         if (n > left) {
             spare += left;
+            piece = min(piece, most);
             const uint64_t want = n > piece ? n : piece;
             at = warp_bump(used, want);
             left = (uint32_t)(want - n);
@@ -385,10 +387,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_lookup_long(IndexView I
     room.done(&ctr->hit_spare);
 }
 
-// Seeding and lookup of a read in one go, for the reads nearly all batches are made of: only
-// A, C, G and T, no tied syncmer window, at most kFastQueries queries, and parameters and
-// an index for which fast_seed() holds (all profiles of read lengths).  Any other read is left
-// to the steps one by one, with nothing written for it.
+// Seeding and lookup of a read in one go, for reads of at most kFastQueries queries and `cap`
+// syncmers with parameters and an index for which fast_seed() holds (all profiles of read
+// lengths).  Returns false, with nothing written, for any other read (the caller then takes
+// the steps one by one).  Reads of only A, C, G and T without a tied syncmer window, nearly
+// all, take the scan without state in line; the syncmers of one with an N, other letters or a
+// tied window come from odd_syncmers, and it goes on here: left to the steps, 500k reads of
+// 150 bp that all hold an N, or U for T, spent 2.7 and 3.0 ms in this kernel (1.7 and 1.6
+// before there was a fast path), now 1.3 and 1.5.
 //
 // Both orientations' randstrobes run through one loop (the reverse ones walk the syncmers
 // downwards; the distance between two syncmers is the same either way), a query goes from
@@ -415,22 +421,31 @@ __host__ __device__ __forceinline__ bool fast_seed(const DevParams& P, const Ind
     return P.q <= 0xFF && P.W <= 32 && P.w_max <= kFastPad && I.buckets != nullptr && I.filter_cutoff <= 255 && !C.force_rescue && !C.count_bytes;
 }
 
-// What fast_read says of a read: done, or left because of a base other than A, C, G and T, or
-// (all such bases, whatever the steps then find) for a tied window or its size.
-enum FastRead { kFastDone, kFastOdd, kFastTied };
+// Syncmers of a read with other letters than A, C, G and T (packed again, with its N bits) or
+// (acgt, packed) with a tied window, which takes the scan with state.  Out of line.
+__device__ __noinline__ uint32_t odd_syncmers(const DevParams& P, const uint8_t* seq, uint32_t L, bool acgt,
+                                              uint64_t* pk, uint32_t* nm, uint64_t* hb, uint32_t* sp, uint32_t cap) {
+    const uint32_t nwin = L - (uint32_t)P.k + 1;
+    const bool has_n = !acgt && warp_pack_read(seq, L, pk, nm);
+    uint32_t n = 0xFFFFFFFFu;
+    if (!acgt) n = warp_clean_syncmers(P, pk, nwin, reinterpret_cast<uint32_t*>(hb), sp, cap, has_n ? nm : nullptr);
+    return n != 0xFFFFFFFFu ? n : warp_state_syncmers(P, pk, nm, has_n, nwin, hb, sp, cap);
+}
 
-__device__ __forceinline__ FastRead fast_read(const DevParams& P, const IndexView& I, const MapConfig& C,
-                                              const uint8_t* __restrict__ seq, uint32_t L, uint32_t r,
-                                              ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr, uint64_t* pk,
-                                              uint32_t* buf, uint64_t* sh, uint32_t* sp, uint32_t cap, FastQueue& Q,
-                                              WarpRoom& room, uint32_t& direct) {
+__device__ __forceinline__ bool fast_read(const DevParams& P, const IndexView& I, const MapConfig& C,
+                                          const uint8_t* __restrict__ seq, uint32_t L, uint32_t r,
+                                          ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr, uint64_t* pk,
+                                          uint32_t* nm, uint64_t* hb, uint64_t* sh, uint32_t* sp, uint32_t cap,
+                                          FastQueue& Q, WarpRoom& room, uint32_t& direct) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t lane = lane_id();
-    if (L < (uint32_t)P.k || !warp_pack_clean(seq, L, pk)) return kFastOdd;
-    const uint32_t n = warp_clean_syncmers(P, pk, L - (uint32_t)P.k + 1, buf, sp, cap);
-    if (n > cap) return kFastTied;   // (or more syncmers)
+    if (L < (uint32_t)P.k) return false;
+    const bool acgt = warp_pack_clean(seq, L, pk);
+    uint32_t n = 0xFFFFFFFFu;
+    if (acgt) n = warp_clean_syncmers(P, pk, L - (uint32_t)P.k + 1, reinterpret_cast<uint32_t*>(hb), sp, cap);
+    if (n == 0xFFFFFFFFu) n = odd_syncmers(P, seq, L, acgt, pk, nm, hb, sp, cap);
     const uint32_t nq = n_query_per_dir(P, n, L), nq2 = 2 * nq;
-    if (nq2 > kFastQueries) return kFastTied;
+    if (n > cap || nq2 > kFastQueries) return false;
     // the syncmers' hashes; their positions and the hash bits that the selection compares
     for (uint32_t i = lane; i < n; i += 32) {
         const uint32_t w = sp[i];
@@ -558,7 +573,7 @@ __device__ __forceinline__ FastRead fast_read(const DevParams& P, const IndexVie
         if (off + nq2 > A.q_cap) {
             warp_fail(R, ctr, kStatusQueryOverflow);
             if (lane == 0) R.nq = R.nq2 = 0;
-            return kFastDone;
+            return true;
         }
         if (lane == 0) {
             R.q_off = off;
@@ -576,14 +591,14 @@ __device__ __forceinline__ FastRead fast_read(const DevParams& P, const IndexVie
         __syncwarp();
         enlist_rescue(I, C, r, R, A, ctr, good < tot);
         __syncwarp();
-        return kFastDone;
+        return true;
     }
     const uint32_t H = __reduce_add_sync(kFull, sum);
     direct += nq2;
     const uint64_t hoff = room.take(&ctr->hit_used, H, arena_piece(A.hit_cap));
     if (hoff + H > A.hit_cap) {
         warp_fail(R, ctr, kStatusHitOverflow);
-        return kFastDone;
+        return true;
     }
     // the hits in generation order (query order, then run order)
     HitPacked* out = A.hits + hoff;
@@ -618,7 +633,7 @@ __device__ __forceinline__ FastRead fast_read(const DevParams& P, const IndexVie
         R.n_hits = H;
     }
     __syncwarp();
-    return kFastDone;
+    return true;
 }
 
 // The same read by the steps: seeding into the query arena, then lookup_read.  Reads that do
@@ -628,10 +643,10 @@ __device__ __forceinline__ void step_read(const DevParams& P, const IndexView& I
                                           const uint8_t* seq, uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A,
                                           Counters* ctr, uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh,
                                           uint32_t* sp, uint32_t max_len, uint32_t cap, WarpRoom& queries,
-                                          WarpRoom& hits, bool try_clean = true) {
+                                          WarpRoom& hits) {
     ReadRec& R = rec[r];
     uint32_t ns = 0xFFFFFFFFu;
-    if (L <= max_len) ns = warp_read_syncmers(P, seq, L, pk, nm, hb, sh, sp, cap, try_clean);
+    if (L <= max_len) ns = warp_read_syncmers(P, seq, L, pk, nm, hb, sh, sp, cap);
     if (ns == 0xFFFFFFFFu) {
         if (lane_id() == 0) {
             R.flags |= kReadLong;
@@ -647,24 +662,16 @@ __device__ __forceinline__ void step_read(const DevParams& P, const IndexView& I
     }
 }
 
-// A warp's room in the query and the hit arena.
-struct ReadRooms {
+// step_read beside the fast path: out of line, for the few reads that need it, which take just
+// the arena room that they use (a piece each, of which a read leaves nine tenths, made batches
+// of many such reads outgrow the arenas).
+__device__ __noinline__ void slow_read(const DevParams& P, const IndexView& I, const MapConfig& C, const uint8_t* seq,
+                                       uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A, Counters* ctr,
+                                       uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh, uint32_t* sp,
+                                       uint32_t max_len, uint32_t cap) {
     WarpRoom queries, hits;
-};
-
-// step_read beside the fast path: out of line, for the reads that need it.  The warp's rooms
-// pass through by value, so that they stay in registers otherwise.  (With rooms of its own each
-// such read took a piece of both arenas, up to 512 entries of which it used some 50, and four
-// atomics: the first batch of 500k reads of 150 bp that all hold an N overflowed them and took
-// 12.6 ms; with the warp's 8.0.)
-__device__ __noinline__ ReadRooms slow_read(const DevParams& P, const IndexView& I, const MapConfig& C,
-                                            const uint8_t* seq, uint32_t L, uint32_t r, ReadRec* rec, const Arenas& A,
-                                            Counters* ctr, uint64_t* pk, uint32_t* nm, uint64_t* hb, uint64_t* sh,
-                                            uint32_t* sp, uint32_t max_len, uint32_t cap, bool try_clean,
-                                            ReadRooms rooms) {
-    step_read<false, true>(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, max_len, cap, rooms.queries, rooms.hits,
-                           try_clean);
-    return rooms;
+    queries.most = hits.most = 0;
+    step_read<false, true>(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, max_len, cap, queries, hits);
 }
 
 // A read of the fast kernels: in one go, else by the steps.
@@ -673,13 +680,10 @@ __device__ __forceinline__ void fast_or_slow_read(const DevParams& P, const Inde
                                                   const uint8_t* seq, uint32_t L, uint32_t r, ReadRec* rec,
                                                   const Arenas& A, Counters* ctr, uint64_t* pk, uint32_t* nm,
                                                   uint64_t* hb, uint64_t* sh, uint32_t* sp, FastQueue& Q,
-                                                  ReadRooms& rooms, uint32_t& direct) {
-    FastRead f = kFastOdd;
-    if (L <= kMaxLen)
-        f = fast_read(P, I, C, seq, L, r, rec, A, ctr, pk, reinterpret_cast<uint32_t*>(hb), sh, sp + kFastPad, kSyncmers,
-                      Q, rooms.hits, direct);
-    if (f != kFastDone)
-        rooms = slow_read(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, kMaxLen, kSyncmers, f == kFastOdd, rooms);
+                                                  WarpRoom& room, uint32_t& direct) {
+    if (L > kMaxLen ||
+        !fast_read(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp + kFastPad, kSyncmers, Q, room, direct))
+        slow_read(P, I, C, seq, L, r, rec, A, ctr, pk, nm, hb, sh, sp, kMaxLen, kSyncmers);
 }
 
 // Seeding and lookup of a read by one warp (the main path): randstrobes_query, then
@@ -710,7 +714,7 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
     __shared__ FastQueue s_q[kFast ? kSeedWarps : 1];
     const uint32_t w = threadIdx.x >> 5;
     WarpItems items(n);
-    ReadRooms rooms;
+    WarpRoom room, queries;
     uint32_t direct = 0;
     for (uint32_t r; (r = items.next(&ctr->queue_head)) < n;) {
         const uint32_t L = lens[r];
@@ -721,13 +725,13 @@ __global__ void __launch_bounds__(32 * kSeedWarps, kFusedBlocksPerSm)
         if (kFast)
             fast_or_slow_read<kFusedMaxLen, kFusedSyncmers>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w],
                                                             s_nm[w], s_hb[w], s_sh[w], s_sp[w], s_q[kFast ? w : 0],
-                                                            rooms, direct);
+                                                            room, direct);
         else
             step_read<kCount, true>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w], s_sh[w],
-                                    s_sp[w], kFusedMaxLen, kFusedSyncmers, rooms.queries, rooms.hits);
+                                    s_sp[w], kFusedMaxLen, kFusedSyncmers, queries, room);
     }
-    rooms.hits.done(&ctr->hit_spare);
-    rooms.queries.done(&ctr->q_spare);
+    room.done(&ctr->hit_spare);
+    if (!kFast) queries.done(&ctr->q_spare);
     if (direct && lane_id() == 0) atomicAdd(&ctr->q_direct, (unsigned long long)direct);
 }
 
@@ -756,7 +760,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
     const uint32_t* __restrict__ items = desc->items;
     const uint32_t n_items = items ? desc->n_items : desc->n_reads;
     WarpItems queue(n_items);
-    ReadRooms rooms;
+    WarpRoom room, queries;
     uint32_t direct = 0;
     for (uint32_t it; (it = queue.next(&ctr->queue_head)) < n_items;) {
         // item bounds outside [0, n_reads] are clamped (reads no item covers stay empty)
@@ -771,14 +775,14 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
             }
             if (kFast)
                 fast_or_slow_read<kMaxLen, kSyncmers>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w],
-                                                      s_hb[w], s_sh[w], s_sp[w], s_q[kFast ? w : 0], rooms, direct);
+                                                      s_hb[w], s_sh[w], s_sp[w], s_q[kFast ? w : 0], room, direct);
             else
                 step_read<kCount, kLookup>(P, I, C, seqs + offs[r], L, r, rec, A, ctr, s_pk[w], s_nm[w], s_hb[w],
-                                           s_sh[w], s_sp[w], kMaxLen, kSyncmers, rooms.queries, rooms.hits);
+                                           s_sh[w], s_sp[w], kMaxLen, kSyncmers, queries, room);
         }
     }
-    rooms.hits.done(&ctr->hit_spare);
-    rooms.queries.done(&ctr->q_spare);
+    room.done(&ctr->hit_spare);
+    if (!kFast) queries.done(&ctr->q_spare);
     if (direct && lane_id() == 0) atomicAdd(&ctr->q_direct, (unsigned long long)direct);
 }
 

@@ -419,8 +419,9 @@ __device__ __forceinline__ uint32_t n_query_per_dir(const DevParams& P, uint32_t
     return n > P.w_min ? n - P.w_min : 0;
 }
 
-// Syncmers of the nwin windows from packed position p0 on, where no base is ambiguous.  A
-// window is a syncmer when its s-mer number t - 1 has the least hash of the W, decided on
+// Syncmers of the nwin windows from packed position p0 on, where no base is ambiguous, or of
+// those without an N when nmask is set (p0 0; an N restarts the state machine).  A window is
+// a syncmer when its s-mer number t - 1 has the least hash of the W, decided on
 // the hashes' high words.  The warp goes over the s-mers, 32 a step, the high words of a
 // step and of the W - 1 s-mers before it side by side in `buf` (32 + W - 1 <= 64 words), so
 // that a window costs W loads at fixed places and a few minima.  Calls chunk(c, bits) for
@@ -429,7 +430,7 @@ __device__ __forceinline__ uint32_t n_query_per_dir(const DevParams& P, uint32_t
 // full scan.  kW: W when known at compile time, with s <= 16 (0: P.W).
 template <int kW, class Chunk>
 __device__ __forceinline__ bool warp_clean_scan(const DevParams& P, const uint64_t* packed, uint32_t p0, uint32_t nwin,
-                                                uint32_t* buf, Chunk&& chunk) {
+                                                uint32_t* buf, Chunk&& chunk, const uint32_t* nmask = nullptr) {
     const uint32_t lane = lane_id();
     const uint32_t W = kW ? kW : (uint32_t)P.W, t = kW ? kW / 2 : (uint32_t)(P.t - 1);
     const uint32_t n = nwin + W - 1;
@@ -450,7 +451,8 @@ __device__ __forceinline__ bool warp_clean_scan(const DevParams& P, const uint64
             else least = min(least, v);
         }
         const uint32_t w = c + lane - (W - 1);   // (wraps below the first window)
-        const bool in = w < nwin;
+        bool in = w < nwin;
+        if (nmask) in = in && nbits33(nmask, w, P.k) == 0;
         if (__any_sync(0xFFFFFFFFu, in && mid == least)) return false;
         chunk(c, __ballot_sync(0xFFFFFFFFu, in && mid < least));
     }
@@ -461,10 +463,11 @@ __device__ __forceinline__ bool warp_clean_scan(const DevParams& P, const uint64
 // Whether the scan above may be the instance for W = 5 and short s-mers.
 __device__ __forceinline__ bool clean_scan5(const DevParams& P) { return P.W == 5 && P.t == 3 && P.s <= 16; }
 
-// The first `cap` syncmers' windows of a clean read into sp; returns their number, or
-// 0xFFFFFFFF where the full scan is needed.
+// The first `cap` syncmers' windows of a read into sp (nmask: its N bits, null for a read
+// without N); returns their number, or 0xFFFFFFFF where the full scan is needed.
 __device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, const uint64_t* packed, uint32_t nwin,
-                                                        uint32_t* buf, uint32_t* sp, uint32_t cap) {
+                                                        uint32_t* buf, uint32_t* sp, uint32_t cap,
+                                                        const uint32_t* nmask = nullptr) {
     uint32_t n = 0;
     const uint32_t first = lane_id() - (uint32_t)(P.W - 1);
     auto put = [&](uint32_t c, uint32_t b) {
@@ -472,9 +475,22 @@ __device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, cons
         if (((b >> lane_id()) & 1u) && idx < cap) sp[idx] = c + first;
         n += __popc(b);
     };
-    const bool ok = clean_scan5(P) ? warp_clean_scan<5>(P, packed, 0, nwin, buf, put)
-                                   : warp_clean_scan<0>(P, packed, 0, nwin, buf, put);
+    const bool ok = clean_scan5(P) ? warp_clean_scan<5>(P, packed, 0, nwin, buf, put, nmask)
+                                   : warp_clean_scan<0>(P, packed, 0, nwin, buf, put, nmask);
     return ok ? n : 0xFFFFFFFFu;
+}
+
+// The same by the full scan, for any read.  Reads without N skip the per-window N checks, and
+// the common window width (5 s-mers: k - s = 4) is unrolled at compile time.
+__device__ __forceinline__ uint32_t warp_state_syncmers(const DevParams& P, const uint64_t* packed,
+                                                        const uint32_t* nmask, bool has_n, uint32_t nwin,
+                                                        uint64_t* hbuf, uint32_t* sp, uint32_t cap) {
+    auto emit = [&](uint32_t idx, uint32_t w) {
+        if (idx < cap) sp[idx] = w;
+    };
+    if (has_n) return warp_syncmer_scan(P, packed, nmask, 0, nwin, 0, nwin, 0, hbuf, emit);
+    if (P.W == 5) return warp_syncmer_scan<5, true>(P, packed, nmask, 0, nwin, 0, nwin, 0, hbuf, emit);
+    return warp_syncmer_scan<0, true>(P, packed, nmask, 0, nwin, 0, nwin, 0, hbuf, emit);
 }
 
 // Seeds one read with the warp: packs it into pk/nm (capacity for L bases), finds
@@ -482,24 +498,14 @@ __device__ __forceinline__ uint32_t warp_clean_syncmers(const DevParams& P, cons
 // 0xFFFFFFFF when more than cap syncmers exist.
 __device__ __forceinline__ uint32_t warp_read_syncmers(const DevParams& P, const uint8_t* seq, uint32_t L, uint64_t* pk,
                                                        uint32_t* nm, uint64_t* hbuf, uint64_t* sh, uint32_t* sp,
-                                                       uint32_t cap, bool try_clean = true) {
+                                                       uint32_t cap) {
     if (L < (uint32_t)P.k) return 0;
     const bool has_n = warp_pack_read(seq, L, pk, nm);
     const uint32_t nwin = L - (uint32_t)P.k + 1;
-    auto emit = [&](uint32_t idx, uint32_t w) {
-        if (idx < cap) sp[idx] = w;
-    };
-    // reads without N (nearly all) and without a tied window take the scan without state;
-    // else those without N skip the per-window N checks, and the common window width (5
-    // s-mers: k - s = 4) is unrolled at compile time
+    // reads without N (nearly all) and without a tied window take the scan without state
     uint32_t n = 0xFFFFFFFFu;
-    if (try_clean && !has_n && P.W <= 32)
-        n = warp_clean_syncmers(P, pk, nwin, reinterpret_cast<uint32_t*>(hbuf), sp, cap);
-    if (n == 0xFFFFFFFFu) {
-        if (has_n) n = warp_syncmer_scan(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
-        else if (P.W == 5) n = warp_syncmer_scan<5, true>(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
-        else n = warp_syncmer_scan<0, true>(P, pk, nm, 0, nwin, 0, nwin, 0, hbuf, emit);
-    }
+    if (!has_n && P.W <= 32) n = warp_clean_syncmers(P, pk, nwin, reinterpret_cast<uint32_t*>(hbuf), sp, cap);
+    if (n == 0xFFFFFFFFu) n = warp_state_syncmers(P, pk, nm, has_n, nwin, hbuf, sp, cap);
     if (n > cap) return 0xFFFFFFFFu;
     __syncwarp();
     for (uint32_t i = lane_id(); i < n; i += 32) sh[i] = kmer_hash(P, pk, sp[i]);
