@@ -74,22 +74,24 @@ struct WarpItems {
 };
 
 // Room in an arena whose bump counter all warps share, taken ahead in pieces of up to
-// `piece` entries: a warp's requests come from its piece while they fit.  What is left
-// unused of the pieces is counted (`spare`), so that the counters still tell what was used.
-// most 0: no pieces, each request takes what it needs.
+// `piece` entries: a warp's requests come from its piece while they fit.  A piece is given up
+// when no more than an eighth of it is left; a request that does not fit before takes just
+// what it needs (given up at any size, requests of a third of a piece and more wasted up to
+// half of it: reads with 145 hits each outgrew an arena with room for 166 a read).  What is
+// left unused of the pieces is counted (`spare`), so that the counters still tell what was
+// used.  most 0: no pieces, each request takes what it needs.
 struct WarpRoom {
     uint64_t at = 0;
     uint32_t left = 0, spare = 0, most = 512;
     __device__ __forceinline__ uint64_t take(unsigned long long* used, uint64_t n, uint32_t piece) {
         if (n > left) {
-            spare += left;
             piece = min(piece, most);
-            const uint64_t want = n > piece ? n : piece;
-            at = warp_bump(used, want);
-            left = (uint32_t)(want - n);
-        } else {
-            left -= (uint32_t)n;
+            if (n >= piece || left > piece / 8) return warp_bump(used, n);
+            spare += left;
+            at = warp_bump(used, piece);
+            left = piece;
         }
+        left -= (uint32_t)n;
         const uint64_t r = at;
         at += n;
         return r;
@@ -98,7 +100,7 @@ struct WarpRoom {
         if (lane_id() == 0 && spare + left) atomicAdd(total, (unsigned long long)(spare + left));
     }
 };
-// The pieces of all warps of the grid together take at most an eighth of the arena.
+// The pieces that the warps of the grid hold at a time take at most an eighth of the arena.
 __device__ __forceinline__ uint32_t arena_piece(uint64_t cap) {
     const uint64_t p = cap / (8ull * warp_count());
     return p < 512 ? (uint32_t)p : 512u;
