@@ -347,6 +347,7 @@ static Arenas arenas_of(gbsa_mapper& m) {
     A.nam_cap = m.nam_cap;
     A.slots = m.slots.as<uint8_t>();
     A.slot_bytes = m.slot_bytes;
+    A.n_slots = (uint32_t)(m.slots.size() / m.slot_bytes);
     A.ovf = m.ovf.as<uint8_t>();
     A.ovf_cap = m.ovf_cap;
     const size_t per = m.lists.size() / 16;   // u32 entries per list
@@ -1399,7 +1400,7 @@ int gbsa_mapper_last_counts(const gbsa_mapper* m, uint64_t* out) {
     out[3] = m->last.n_rescue + m->last.n_rescue_heavy;
     out[4] = m->last.n_long;
     out[5] = m->last.scratch_used;
-    out[6] = m->last.n_big;
+    out[6] = m->last.n_big + m->last.n_few;
     return GBSA_OK;
 }
 

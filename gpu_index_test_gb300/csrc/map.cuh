@@ -46,7 +46,9 @@ struct Counters {
     unsigned int rescue_next;  // next rescue-list entry to take (k_rescue's work counter)
     unsigned int lane_cnt[16]; // reads per hit-count bucket of the register NAM merges
     unsigned int group_next;   // next item of the group NAM kernel
-    unsigned int big_next;     // next read of the warp NAM kernel
+    unsigned int big_next;     // next read of the block NAM kernel
+    unsigned int n_few;        // reads of the block NAM kernel's list with few hits a query (from its back)
+    unsigned int few_next;     // next of them
     unsigned int queue_head;   // next read (work item) of the seeding (+ lookup) kernel
     unsigned int queue_head2;  // next read of the lookup kernel, when it runs on its own
     unsigned int rescue_block_next;  // next heavy rescued read to take a block (k_rescue)
@@ -97,19 +99,20 @@ struct Arenas {
     uint64_t nam_cap;
     uint8_t* slots;          // per-warp scratch slots of the NAM / rescue kernels
     uint64_t slot_bytes;
+    uint32_t n_slots;
     uint8_t* ovf;            // shared overflow scratch (bump-allocated)
     uint64_t ovf_cap;
     uint32_t* rescue_list;   // light reads from the front, heavy ones from the back
     uint32_t rescue_cap;
     uint32_t* long_list;
-    uint32_t* big_list;
+    uint32_t* big_list;      // reads with more NAMs than the group NAM kernel holds; those with few hits a query from the back
     uint32_t* slow_list;     // sort jobs the packed sort passed on: block sort's from the front, cluster sort's from the back
     uint32_t* lane_lists;    // kLaneBuckets lists of lane_cap reads each
     uint32_t lane_cap;
     SortJob* sort_jobs;      // small-tile jobs from the front, large-tile ones from the back
     uint32_t jobs_cap;
     uint64_t* rescue_cycles;   // optional: 8 notes per rescued read (cycles per phase, sizes)
-    uint64_t* nam_cycles;      // optional: SM cycles, hits and NAMs of each read of the warp NAM kernel
+    uint64_t* nam_cycles;      // optional: SM cycles, hits and NAMs of each read of the block NAM kernel
 };
 
 struct MapConfig {

@@ -793,7 +793,8 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks)
 // when that is full too).
 __device__ __forceinline__ uint8_t* warp_scratch(const Arenas& A, Counters* ctr, uint64_t slot_off, uint64_t bytes) {
     bytes = (bytes + 255) & ~255ull;   // keep every region 256-byte aligned
-    if (slot_off + bytes <= A.slot_bytes) return A.slots + (uint64_t)warp_global_id() * A.slot_bytes + slot_off;
+    const uint32_t slot = warp_global_id();
+    if (slot < A.n_slots && slot_off + bytes <= A.slot_bytes) return A.slots + (uint64_t)slot * A.slot_bytes + slot_off;
     const uint64_t o = warp_bump(&ctr->scratch_used, bytes);
     if (o + bytes > A.ovf_cap) return nullptr;
     return A.ovf + o;
@@ -965,11 +966,15 @@ __device__ __forceinline__ void each_row(F&& f) {
 // Merges the reads list[first ..] (one a group of G lanes, those below cnt) and writes
 // their sorted NAMs; S: the warp's shared memory.  Returns a group's read with more than
 // G * R NAMs in its lanes (its NAMs are not written), else kNoRead.
+// kLong (G 32): NAMs that can take no more hits leave full lanes for `closed` (room for the
+// read's hits), which holds all of them in creation order at the end, `n_closed`; a read with
+// more than kFewOpen NAMs left in full lanes is returned.
 constexpr uint32_t kNoRead = 0xFFFFFFFFu;
-template <int G, int R>
+constexpr uint32_t kFewOpen = 96;
+template <int G, int R, bool kLong = false>
 __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr,
                                 const uint32_t* __restrict__ list, uint32_t first, uint32_t cnt, GroupShared<R>& S,
-                                WarpRoom& room) {
+                                WarpRoom& room, NamState* closed = nullptr, uint32_t* n_closed = nullptr) {
     constexpr uint32_t kFull = 0xFFFFFFFFu;
     constexpr uint32_t kNoRef = 0xFFFFFFFFu;   // a hit's reference id has 24 bits
     const uint32_t lane = lane_id();
@@ -995,6 +1000,20 @@ __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, c
     const uint4 none = make_uint4(kNoRef - 1, 0, 0, 0);
     uint4 nx = sub < H ? __ldg(hits + sub) : none;
     bool over = false;
+    auto nam = [&](int r) {
+        NamState m;
+        m.qs = (int32_t)(qn[r] & 0xFFFFu);
+        m.qe = (int32_t)(qep[r] >> 16);
+        m.qprev = (int32_t)(qep[r] & 0xFFFFu);
+        m.rs = rs[r];
+        m.re = re[r];
+        m.rprev = rp[r];
+        m.n_hits = (int32_t)(qn[r] >> 16);
+        m.ref_rc = ref[r];
+        return m;
+    };
+    uint32_t* number = reinterpret_cast<uint32_t*>(S.k3);   // kLong: of each slot's NAM
+    uint32_t created = 0;
     for (uint32_t c = 0; c < Hm; c += G) {
         uint4* buf = S.hits[(c / G) & 1];
         buf[lane] = nx;
@@ -1045,8 +1064,54 @@ __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, c
             // a hit that no NAM took opens one in the group's next slot
             if (__any_sync(kFull, !done)) {
                 if (n == G * R) {   // (never for reads of up to G * R hits)
-                    over = true;
-                    done = true;
+                    if constexpr (kLong) {   // the NAMs that may take another hit move to the front
+                        uint32_t open = 0, to[R];
+                        each_row<R>([&](auto row_c) {
+                            constexpr int r = decltype(row_c)::value;
+                            const bool stay = (int32_t)(ref[r] ^ v.x) >= 0 && (qep[r] >> 16) >= xqs;
+                            const uint32_t b = __ballot_sync(kFull, stay);
+                            to[r] = stay ? open + __popc(b & lanemask_lt()) : kNoRef;
+                            open += __popc(b);
+                        });
+                        if (open > kFewOpen) return rd;
+                        uint32_t* word = reinterpret_cast<uint32_t*>(S.k1);
+                        auto move = [&](auto& x) {
+                            each_row<R>([&](auto row_c) {
+                                constexpr int r = decltype(row_c)::value;
+                                if (to[r] != kNoRef) word[to[r]] = (uint32_t)x[r];
+                            });
+                            __syncwarp();
+                            each_row<R>([&](auto row_c) {
+                                constexpr int r = decltype(row_c)::value;
+                                if (r * G + lane < open) x[r] = word[r * G + lane];
+                            });
+                            __syncwarp();
+                        };
+                        uint32_t at[R];
+                        each_row<R>([&](auto row_c) {
+                            constexpr int r = decltype(row_c)::value;
+                            at[r] = number[r * G + lane];
+                            if (to[r] == kNoRef) closed[at[r]] = nam(r);
+                        });
+                        move(ref);
+                        move(qep);
+                        move(qn);
+                        move(rs);
+                        move(re);
+                        move(rp);
+                        move(at);
+                        each_row<R>([&](auto row_c) {
+                            constexpr int r = decltype(row_c)::value;
+                            number[r * G + lane] = at[r];
+                            if (r * G + lane >= open) ref[r] = kNoRef;
+                        });
+                        n = open;
+                        rows = (n + G - 1) / G;
+                        live = (1u << rows) - 1;
+                    } else {
+                        over = true;
+                        done = true;
+                    }
                 }
                 const bool mine = !done && sub == (n & (G - 1));
                 each_row<R>([&](auto row_c) {
@@ -1058,8 +1123,10 @@ __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, c
                         re[r] = xre;
                         rp[r] = xrs;
                         qn[r] = (1u << 16) | xqs;
+                        if (kLong) number[r * G + lane] = created;
                     }
                 });
+                if (kLong) ++created;
                 const uint32_t row = done ? 0u : 1u << (n / G);
                 const uint32_t opened = G == 32 ? row : __reduce_or_sync(kFull, row);
                 if (!done) ++n;
@@ -1069,18 +1136,16 @@ __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, c
         }
         if (G == 32 && over) return rd;
     }
-    auto nam = [&](int r) {
-        NamState m;
-        m.qs = (int32_t)(qn[r] & 0xFFFFu);
-        m.qe = (int32_t)(qep[r] >> 16);
-        m.qprev = (int32_t)(qep[r] & 0xFFFFu);
-        m.rs = rs[r];
-        m.re = re[r];
-        m.rprev = rp[r];
-        m.n_hits = (int32_t)(qn[r] >> 16);
-        m.ref_rc = ref[r];
-        return m;
-    };
+    if constexpr (kLong) {
+        __syncwarp();
+        each_row<R>([&](auto row_c) {
+            constexpr int r = decltype(row_c)::value;
+            if (r * G + lane < n) closed[number[r * G + lane]] = nam(r);
+        });
+        __syncwarp();
+        *n_closed = created;
+        return kNoRead;
+    }
     // ranks by the first key word (a NAM's is never all ones), one byte a row
     uint64_t ranks = 0;
     each_row<R>([&](auto row_c) {
@@ -1162,6 +1227,25 @@ __device__ uint32_t group_merge(const MapConfig& C, ReadRec* __restrict__ rec, c
     return kNoRead;
 }
 
+// Lists a read with more NAMs than a warp's slots for k_nams: from the front, or, where its
+// first queries have kFewHits hits or fewer each, from the back.  A query costs a block 3,500
+// cycles whatever it brings, a hit a warp some 200, and the block sorts faster: reads of a few
+// dozen queries with many hits each were slower by the warp (100k pairs 0.77 -> 0.86 ms, 100k
+// reads of 250 bp 1.74 -> 2.15), reads of 4,000 bp by the block (see long_merge).
+constexpr uint32_t kFewHits = 4;
+__device__ __forceinline__ void list_big_read(const Arenas& A, Counters* ctr, uint32_t r, const ReadRec& R) {
+    const uint32_t lane = lane_id();
+    const uint4* hits = reinterpret_cast<const uint4*>(A.hits + R.hit_off);
+    const uint32_t m = min(R.n_hits, 160u);   // (more than 128)
+    uint32_t q = 0;
+    for (uint32_t h = lane; h < m; h += 32) q += h == 0 || __ldg(&hits[h].y) != __ldg(&hits[h - 1].y) ? 1u : 0u;
+    q = __reduce_add_sync(0xFFFFFFFFu, q);
+    if (lane == 0) {
+        if (m <= kFewHits * q) A.big_list[A.rescue_cap - 1 - atomicAdd(&ctr->n_few, 1u)] = r;
+        else A.big_list[atomicAdd(&ctr->n_big, 1u)] = r;
+    }
+}
+
 // The register merge: persistent warps take the reads by bucket from a work counter, the
 // most hits first.  Groups of 4 lanes take reads of up to 16 hits, of 8 up to 32, of 16 up
 // to 64, a warp all others; a read with more than 128 NAMs (one in a thousand) goes to
@@ -1205,7 +1289,7 @@ __global__ void __launch_bounds__(32 * kGroupWarps, kGroupBlocksPerSm)
             group_merge<16, 4>(C, rec, A, ctr, list, t, s_cnt[b], S, room);
         } else {
             const uint32_t r = group_merge<32, 4>(C, rec, A, ctr, list, t, s_cnt[b], S, room);
-            if (r != kNoRead && lane_id() == 0) A.big_list[atomicAdd(&ctr->n_big, 1u)] = r;
+            if (r != kNoRead) list_big_read(A, ctr, r, rec[r]);
             __syncwarp();
         }
     }
@@ -1951,32 +2035,116 @@ __global__ void __launch_bounds__(kPackThreads, 2)
     }
 }
 
+// A read with more than 128 NAMs of which few are open at a time (one of a thousand bases and
+// more, whose queries have a hit or two each), by the warp: the slots are given back as the
+// queries pass their NAMs, and the NAMs are sorted through scratch.  False: too many are open.
+// 10,000 reads of 4,000 bp, two thirds of them such: this stage 22.7 ms with a block a read, 2.6
+// so (3.9 with a warp and the open NAMs in memory), the call 28.4 -> 8.1 ms (10.3).
+__device__ __noinline__ bool long_merge(const MapConfig& C, ReadRec* __restrict__ rec, const Arenas& A, Counters* ctr,
+                                        uint32_t rd, GroupShared<4>& S) {
+    const uint32_t lane = lane_id();
+    ReadRec& R = rec[rd];
+    const uint32_t H = R.n_hits;
+    const uint64_t b_list = (32ull * H + 255) & ~255ull;
+    NamState* list = reinterpret_cast<NamState*>(warp_scratch(A, ctr, 0, b_list));
+    if (!list) {
+        warp_fail(R, ctr, kStatusScratchOverflow);
+        return true;
+    }
+    WarpRoom room;
+    uint32_t n = 0;
+    if (group_merge<32, 4, true>(C, rec, A, ctr, &rd, 0, 1, S, room, list, &n) != kNoRead) return false;
+    const uint32_t P = next_pow2(n);
+    uint8_t* sc = warp_scratch(A, ctr, b_list <= A.slot_bytes ? b_list : 0, 28ull * P);
+    if (!sc) {
+        warp_fail(R, ctr, kStatusScratchOverflow);
+        return true;
+    }
+    uint64_t* k2 = reinterpret_cast<uint64_t*>(sc);
+    uint64_t* k3 = k2 + P;
+    // what moves lies in shared memory where it fits
+    static_assert(sizeof(S.k1) + sizeof(S.k2) + sizeof(S.k3) >= 256 * 12, "256 keys with their numbers");
+    uint64_t* k1 = P <= 256 ? S.k1 : k3 + P;
+    uint32_t* ix = reinterpret_cast<uint32_t*>(k1 + P);
+    for (uint32_t t = lane; t < P; t += 32) {
+        NamKey k;
+        k.k1 = k.k2 = k.k3 = ~0ULL;   // padding sorts last (a NAM's first key word is never all ones)
+        if (t < n) k = nam_key(list[t], t, C.sort_mode);
+        k1[t] = k.k1;
+        ix[t] = t;
+        k2[t] = k.k2;
+        k3[t] = k.k3;
+    }
+    __syncwarp();
+    warp_sort_idx(k1, ix, k2, k3, P);
+    const uint64_t noff = warp_bump(&ctr->nam_used, n);
+    if (noff + n > A.nam_cap) {
+        warp_fail(R, ctr, kStatusNamOverflow);
+        return true;
+    }
+    for (uint32_t t = lane; t < n; t += 32) A.nams[noff + t] = list[ix[t]];
+    if (lane == 0) {
+        R.nam_off = noff;
+        R.n_nams = n;
+    }
+    __syncwarp();
+    return true;
+}
+
 // find_nams for the reads with more NAMs than k_nams_group's slots (reads in repeats, with
 // queries of dozens of hits): a block a read, a query's hits merged at once (merge_query).
 // A warp a read, hit by hit with 8 slots a lane, took 0.36 ms for the longest of 81 such
 // reads of 100k, 0.95 ms where some of 250 bp had more than 256 NAMs; here 0.12 and 0.17.
+// Before them the reads with few hits a query, a warp each (long_merge).
 constexpr int kBigThreads = kPackThreads;
+constexpr int kBigWarps = kBigThreads / 32;
 constexpr uint32_t kBigHits = 512;   // hits of one query in shared memory
+union BigShared {
+    uint32_t hits[rescue_hit_words(kBigHits)];
+    uint64_t sort[4 * kPackThreads];   // also the warp sort's buffer
+    GroupShared<4> merge[kBigWarps];
+};
 
-__global__ void __launch_bounds__(kBigThreads, 2) k_nams(MapConfig C, int k, ReadRec* __restrict__ rec, Arenas A,
-                                                         Counters* ctr) {
-    __shared__ union {
-        uint32_t hits[rescue_hit_words(kBigHits)];
-        uint64_t sort[4 * kPackThreads];   // also the warp sort's buffer
-    } s;
+__global__ void __launch_bounds__(kBigThreads, 2)
+    k_nams(const __grid_constant__ MapConfig C, int k, ReadRec* __restrict__ rec, const __grid_constant__ Arenas A,
+           Counters* ctr) {
+    extern __shared__ __align__(16) uint8_t s_dyn[];
+    BigShared& s = *reinterpret_cast<BigShared*>(s_dyn);
+    __shared__ uint32_t s_left[2 * kBigWarps], s_n_left;   // reads that long_merge left
     __shared__ uint32_t s_cnt[kBigThreads / 32];
     __shared__ uint32_t s_item, s_run, s_min, s_max;
     __shared__ uint8_t* s_scratch;
     static_assert(sizeof(s) >= 7168 && kWarpSortMax <= 256, "a warp's sort entries fit");
     const uint32_t tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
-    const uint32_t n_big = *(volatile unsigned int*)&ctr->n_big;
-    for (;;) {
-        if (tid == 0) s_item = atomicAdd(&ctr->big_next, 1u);
-        __syncthreads();
-        const uint32_t b = s_item;
-        if (b >= n_big) break;
+    const uint32_t n_big = *(volatile unsigned int*)&ctr->n_big, n_few = *(volatile unsigned int*)&ctr->n_few;
+    uint32_t left = 0, left_at = 0;
+    for (bool few = n_few != 0;;) {
+        if (few && left_at == left) {   // until the list ends, or there are reads for the block
+            if (tid == 0) s_n_left = 0;
+            __syncthreads();
+            while (__shfl_sync(0xFFFFFFFFu, *(volatile uint32_t*)&s_n_left, 0) < kBigWarps) {
+                const uint32_t t = warp_next(&ctr->few_next);
+                if (t >= n_few) break;
+                const uint32_t r = A.big_list[A.rescue_cap - 1 - t];
+                if (!long_merge(C, rec, A, ctr, r, s.merge[w]) && lane == 0) s_left[atomicAdd(&s_n_left, 1u)] = r;
+                __syncwarp();
+            }
+            __syncthreads();
+            left = s_n_left;
+            left_at = 0;
+            few = left >= kBigWarps;
+        }
+        uint32_t r, b = 0xFFFFFFFFu;
+        if (left_at < left) {
+            r = s_left[left_at++];
+        } else {
+            if (tid == 0) s_item = atomicAdd(&ctr->big_next, 1u);
+            __syncthreads();
+            b = s_item;
+            if (b >= n_big) break;
+            r = A.big_list[b];
+        }
         const long long t0 = clock64();
-        const uint32_t r = A.big_list[b];
         ReadRec& R = rec[r];
         const uint32_t H = R.n_hits;
         const HitPacked* hits = A.hits + R.hit_off;
@@ -2056,7 +2224,7 @@ __global__ void __launch_bounds__(kBigThreads, 2) k_nams(MapConfig C, int k, Rea
         __syncthreads();
         if (!done && w == 0) {
             if (n <= kWarpSortMax) {
-                warp_finish_nams(C, closed, n, reinterpret_cast<uint32_t*>(&s), R, A, ctr);
+                warp_finish_nams(C, closed, n, reinterpret_cast<uint32_t*>(s_dyn), R, A, ctr);
             } else {
                 for (uint32_t t = lane; t < n; t += 32) keys[t] = nam_key(closed[t], t, C.sort_mode);
                 __syncwarp();
@@ -2071,7 +2239,7 @@ __global__ void __launch_bounds__(kBigThreads, 2) k_nams(MapConfig C, int k, Rea
                 }
             }
         }
-        if (A.nam_cycles && tid == 0) {
+        if (A.nam_cycles && tid == 0 && b < n_big) {
             uint64_t* note = A.nam_cycles + 4ull * b;   // cycles, hits, NAMs, merge cycles
             note[0] = (uint64_t)(clock64() - t0);
             note[1] = H;
@@ -2749,6 +2917,7 @@ void nam_phase_carveout() {
         GBSA_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared));
     GBSA_CUDA(cudaFuncSetAttribute(k_rescue, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RescueShared)));
+    GBSA_CUDA(cudaFuncSetAttribute(k_nams, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BigShared)));
     done[dev] = 1;
 }
 
@@ -2768,10 +2937,12 @@ void launch_bucket_reads(uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cuda
 
 void launch_nams_warp(const MapConfig& C, int k, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
     if (!n) return;
-    // a scratch slot a block (its first warp's; at most nam_kernel_warps(n) warps)
-    const unsigned blocks = (unsigned)std::min<uint64_t>((uint64_t)device_sm_count() * 2,
-                                                         (n + kBigThreads / 32 - 1) / (kBigThreads / 32));
-    k_nams<<<blocks, kBigThreads, 0, st>>>(C, k, rec, A, ctr);
+    nam_phase_carveout();
+    // a block for 16 reads, 64 at least (a hundred reads of 4,000 bp went through 7 blocks); a
+    // warp without a scratch slot takes the overflow arena's room
+    const unsigned blocks =
+        std::min<unsigned>((unsigned)device_sm_count() * 2, std::min(n, std::max(64u, (n + 15) / 16)));
+    k_nams<<<blocks, kBigThreads, sizeof(BigShared), st>>>(C, k, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 

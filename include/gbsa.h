@@ -623,7 +623,7 @@ int gbsa_mapper_stage_ms(const gbsa_mapper* m, float* ms, int n);
  * path, [2] NAM-state arena slots taken by the merges (the room they reserve, not the NAMs
  * output, which the call returns), [3] rescued reads,
  * [4] reads seeded by the long-read kernel,
- * [5] overflow scratch bytes, [6] reads merged by the warp-cooperative NAM kernel.
+ * [5] overflow scratch bytes, [6] reads with more NAMs than the register merge holds.
  * out must hold 7 values.  No reference counterpart. */
 int gbsa_mapper_last_counts(const gbsa_mapper* m, uint64_t* out);
 /* Batches this mapper ran again because a work area (queries, hits, NAMs, overflow
@@ -663,7 +663,7 @@ int gbsa_mapper_set_rescue_block(gbsa_mapper* m, uint32_t hits);
  * to cap values.  No reference counterpart. */
 int gbsa_mapper_rescue_cycles(const gbsa_mapper* m, uint64_t* out, uint32_t cap, uint32_t* n_out);
 
-/* With profiling on: per read of the last batch's warp-per-read find_nams kernel,
+/* With profiling on: per read of the last batch's block-per-read find_nams merge,
  * four values (SM cycles in total, hits, NAMs, SM cycles of the merge); n_out[0]
  * receives the read count; out holds up to cap values.  No reference counterpart. */
 int gbsa_mapper_nam_cycles(const gbsa_mapper* m, uint64_t* out, uint32_t cap, uint32_t* n_out);
