@@ -461,28 +461,34 @@ __global__ void __launch_bounds__(32 * kPairWarps)
         gbsa_nam_pair* to = out + p * max_tries;
         __syncwarp();
         // rank of every entry by the comparator; entries it does not order need the
-        // reference's steps
+        // reference's steps, so the ranking ends at the first such (the thousands of copies'
+        // NAMs of reads in repeats: 2,000 pairs of 764 NAMs an end, nearly all time in those
+        // steps, took 1,034 ms with the ranks of all, 929 with a thread a pair, now 697)
         uint64_t* keys = reinterpret_cast<uint64_t*>(stacks + 2 * base);
         bool tie = false;
         for (int i = lane; i < len; i += 32) keys[i] = nam_pair_key(list[i], n1, tie);
-        __syncwarp();
-        for (int e = lane; e < len; e += 32) {
-            const uint64_t ke = keys[e];
-            const gbsa_nam_pair pe = list[e];
-            uint32_t rank = 0;
-            for (int f = 0; f < len; ++f) {
-                const uint64_t kf = keys[f];
-                if (kf < ke) {
-                    ++rank;
-                } else if (kf == ke && f != e) {
-                    const gbsa_nam_pair pf = list[f];
-                    if (nam_pair_before(pf, pe, n1, n2)) ++rank;
-                    else tie |= !nam_pair_before(pe, pf, n1, n2);
-                }
-            }
-            if (rank < k) to[rank] = pe;
-        }
         tie = __any_sync(kAll, tie);
+        for (int b = 0; b < len && !tie; b += 32) {
+            const int e = b + lane;
+            const uint64_t ke = e < len ? keys[e] : 0;   // (no key is below 0 or equal to it)
+            const gbsa_nam_pair pe = list[min(e, len - 1)];
+            uint32_t rank = 0;
+            for (int c = 0; c < len && !tie; c += 64) {
+                const int end = min(c + 64, len);
+                for (int f = c; f < end; ++f) {
+                    const uint64_t kf = keys[f];
+                    if (kf < ke) {
+                        ++rank;
+                    } else if (kf == ke && f != e) {
+                        const gbsa_nam_pair pf = list[f];
+                        if (nam_pair_before(pf, pe, n1, n2)) ++rank;
+                        else tie |= !nam_pair_before(pe, pf, n1, n2);
+                    }
+                }
+                tie = __any_sync(kAll, tie);
+            }
+            if (e < len && rank < k) to[rank] = pe;
+        }
         __syncwarp();
         if (tie && lane == 0) {
             // quick_sort_iterative (main.cu:317-358): Lomuto partition around the last
