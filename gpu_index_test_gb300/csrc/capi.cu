@@ -1332,12 +1332,18 @@ int gbsa_find_nams(gbsa_mapper* m, const gbsa_query_randstrobe* queries, const u
         }
         // Lay the queries of each read out forward-first, each orientation ordered by
         // start (stable), which is the order randstrobes_query produces and in which the
-        // reference's (query_start, ref_start) hit sort leaves them: on the device, or here
-        // when a read has very many queries that are not in that order.
+        // reference's (query_start, ref_start) hit sort leaves them: on the device, or here when
+        // there are few of them in all, or a read has very many that are not in that order.
+        // (Through the device, and with its answer awaited, one read took 142 us a call, now 133;
+        // above some 500 queries the device is the faster: 846 of them 179 us by the host, 139.)
         bool rising = true;
-        for (uint32_t r = 0; r < n; ++r) rising &= q_offsets[r] <= q_offsets[r + 1];
+        uint64_t most = 0;   // queries of a read
+        for (uint32_t r = 0; r < n; ++r) {
+            rising &= q_offsets[r] <= q_offsets[r + 1];
+            most = std::max(most, q_offsets[r + 1] - q_offsets[r]);
+        }
         uint32_t left = 1;
-        if (rising && n) {
+        if (rising && nqt > 512) {
             const uint64_t at = (sizeof(gbsa_query_randstrobe) * nqt + 255) & ~uint64_t(255);
             m->out_nams.resize(at + 8ull * (n + 1) + 4);   // staging; free until the gather
             uint8_t* d = m->out_nams.as<uint8_t>();
@@ -1346,12 +1352,16 @@ int gbsa_find_nams(gbsa_mapper* m, const gbsa_query_randstrobe* queries, const u
                 GBSA_CUDA(cudaMemcpyAsync(d, queries + q_offsets[0], sizeof(gbsa_query_randstrobe) * nqt,
                                           cudaMemcpyHostToDevice, st));
             GBSA_CUDA(cudaMemcpyAsync(d + at, q_offsets, 8ull * (n + 1), cudaMemcpyHostToDevice, st));
-            GBSA_CUDA(cudaMemsetAsync(d_left, 0, 4, st));
+            left = 0;
+            if (most > kRankQueries) GBSA_CUDA(cudaMemsetAsync(d_left, 0, 4, st));
             launch_layout_queries(n, reinterpret_cast<const gbsa_query_randstrobe*>(d),
                                   reinterpret_cast<const uint64_t*>(d + at), m->q.as<Query>(), m->rec.as<ReadRec>(),
                                   d_left, st);
-            GBSA_CUDA(cudaMemcpyAsync(&left, d_left, 4, cudaMemcpyDeviceToHost, st));
-            GBSA_CUDA(cudaStreamSynchronize(st));
+            // (only then can the device leave a read to us)
+            if (most > kRankQueries) {
+                GBSA_CUDA(cudaMemcpyAsync(&left, d_left, 4, cudaMemcpyDeviceToHost, st));
+                GBSA_CUDA(cudaStreamSynchronize(st));
+            }
         }
         if (left) layout_queries_host(*m, queries, q_offsets, n, st);
         const MapConfig saved = m->cfg;

@@ -201,7 +201,9 @@ void launch_gather_nams(uint32_t n, const ReadRec* rec, const NamState* arena, c
                         int mode = 0, const Arenas* A = nullptr, const Counters* ctr = nullptr,
                         const BatchDesc* desc = nullptr);
 // Queries of reads [offs[r], offs[r + 1]) (counted from offs[0]) laid out for the lookup, with
-// the reads' records; *left (0 before) is set when the caller has to lay them out.
+// the reads' records; *left (0 before) is set when the caller has to lay them out: a read of
+// more than kRankQueries queries that are not in order.
+constexpr uint64_t kRankQueries = 1024;
 void launch_layout_queries(uint32_t n, const gbsa_query_randstrobe* in, const uint64_t* offs, Query* out, ReadRec* rec,
                            uint32_t* left, cudaStream_t st);
 void launch_gather_queries(uint32_t n, const ReadRec* rec, const Query* arena, const uint64_t* out_off,

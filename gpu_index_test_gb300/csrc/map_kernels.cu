@@ -3016,8 +3016,6 @@ void launch_gather_nams(uint32_t n, const ReadRec* rec, const NamState* arena, c
 // them) are copied; others are placed by rank, or when a read has more than kRankQueries of
 // them `left` is set and the caller lays the batch out itself.  Bound by the upload.  (On the
 // host, a sort a read: 5,000 reads of 150 bp 1.67 ms a call, now 0.31.)
-constexpr uint64_t kRankQueries = 1024;
-
 __global__ void k_layout_queries(uint32_t n, const gbsa_query_randstrobe* __restrict__ in,
                                  const uint64_t* __restrict__ offs, Query* __restrict__ out, ReadRec* __restrict__ rec,
                                  uint32_t* __restrict__ left) {
