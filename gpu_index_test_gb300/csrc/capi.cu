@@ -605,8 +605,8 @@ void l2_window_attach(gbsa_mapper& m, bool on) {
         return;
     }
     const gbsa_index& ix = *m.idx;
-    const void* base = ix.buckets.size() ? ix.buckets.as<void>() : ix.starts.as<void>();
-    const uint64_t bytes = ((1ull << ix.bits) + 1) * (ix.buckets.size() ? sizeof(Bucket) : 8);
+    const void* base = ix.tagged ? (const void*)ix.buckets() : ix.starts();
+    const uint64_t bytes = ((1ull << ix.bits) + 1) * (ix.tagged ? sizeof(Bucket) : 8);
     int max_window = 0, persist_max = 0;
     GBSA_CUDA(cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, dev));
     GBSA_CUDA(cudaDeviceGetAttribute(&persist_max, cudaDevAttrMaxPersistingL2CacheSize, dev));
@@ -789,11 +789,9 @@ int gbsa_index_load(const gbsa_params* p, const gbsa_ref_randstrobe* randstrobes
         ix->filter_cutoff = filter_cutoff;
         ix->n = n;
         GBSA_CUDA(cudaGetDevice(&ix->device));
-        ix->rs.resize(16 * (n + 1));
-        const uint64_t nb = (1ULL << bits) + 1;
-        ix->starts.resize(8 * nb);
-        if (n) GBSA_CUDA(cudaMemcpy(ix->rs.as<void>(), randstrobes, 16 * n, cudaMemcpyHostToDevice));
-        GBSA_CUDA(cudaMemcpy(ix->starts.as<void>(), start_indices, 8 * nb, cudaMemcpyHostToDevice));
+        ix->resize_tables();
+        if (n) GBSA_CUDA(cudaMemcpy(ix->rs(), randstrobes, 16 * n, cudaMemcpyHostToDevice));
+        GBSA_CUDA(cudaMemcpy(ix->starts(), start_indices, 8 * ix->n_starts(), cudaMemcpyHostToDevice));
         make_buckets(*ix, 0);
         ix->info.size = n;
         ix->info.bits = bits;
@@ -855,8 +853,8 @@ int gbsa_index_write_sti(const gbsa_index* idx, const char* path) {
     return guarded([&] {
         std::vector<gbsa_ref_randstrobe> rs(idx->n);
         std::vector<uint64_t> starts((1ULL << idx->bits) + 1);
-        if (idx->n) GBSA_CUDA(cudaMemcpy(rs.data(), idx->rs.as<void>(), 16 * idx->n, cudaMemcpyDeviceToHost));
-        GBSA_CUDA(cudaMemcpy(starts.data(), idx->starts.as<void>(), 8 * starts.size(), cudaMemcpyDeviceToHost));
+        if (idx->n) GBSA_CUDA(cudaMemcpy(rs.data(), idx->rs(), 16 * idx->n, cudaMemcpyDeviceToHost));
+        GBSA_CUDA(cudaMemcpy(starts.data(), idx->starts(), 8 * starts.size(), cudaMemcpyDeviceToHost));
         write_sti(*idx, rs, starts, path);
     });
 }
@@ -874,9 +872,9 @@ int gbsa_index_get_params(const gbsa_index* idx, gbsa_params* out) {
 int gbsa_index_export(const gbsa_index* idx, gbsa_ref_randstrobe* randstrobes, uint64_t* start_indices) {
     return guarded([&] {
         if (idx->n && randstrobes)
-            GBSA_CUDA(cudaMemcpy(randstrobes, idx->rs.as<void>(), 16 * idx->n, cudaMemcpyDeviceToHost));
+            GBSA_CUDA(cudaMemcpy(randstrobes, idx->rs(), 16 * idx->n, cudaMemcpyDeviceToHost));
         if (start_indices)
-            GBSA_CUDA(cudaMemcpy(start_indices, idx->starts.as<void>(), 8 * ((1ULL << idx->bits) + 1),
+            GBSA_CUDA(cudaMemcpy(start_indices, idx->starts(), 8 * ((1ULL << idx->bits) + 1),
                                  cudaMemcpyDeviceToHost));
     });
 }

@@ -13,6 +13,10 @@
 #include "common.cuh"
 #include "runtime.h"
 
+namespace gbsa {
+struct Bucket;
+}
+
 struct gbsa_index {
     gbsa_params params{};
     gbsa::DevParams dp{};
@@ -22,9 +26,22 @@ struct gbsa_index {
     gbsa_index_info info{};
     int device = 0;
     gbsa::ScratchLease lease;
-    gbsa::DeviceBuffer rs;       // gbsa_ref_randstrobe[n]
-    gbsa::DeviceBuffer starts;   // uint64_t[2^bits + 1]
-    gbsa::DeviceBuffer buckets;  // Bucket[2^bits + 1] read by the kernels when n < 2^32
+    // One allocation: gbsa_ref_randstrobe[n], uint64_t[2^bits + 1], and when n < 2^32 and the
+    // table is in order (`tagged`) Bucket[2^bits + 1], which the kernels read.  (Three of them
+    // took 95 us more to load an index of 1 Mbp.)
+    gbsa::DeviceBuffer tables;
+    bool tagged = false;
+
+    void resize_tables() {
+        tagged = n < (1ull << 32);
+        tables.resize(buckets_at() + (tagged ? 16 * n_starts() : 0));
+    }
+    uint64_t n_starts() const { return (1ull << bits) + 1; }
+    uint64_t starts_at() const { return (16 * (n + 1) + 255) & ~255ull; }
+    uint64_t buckets_at() const { return (starts_at() + 8 * n_starts() + 255) & ~255ull; }
+    gbsa_ref_randstrobe* rs() const { return tables.as<gbsa_ref_randstrobe>(); }
+    uint64_t* starts() const { return reinterpret_cast<uint64_t*>(tables.as<uint8_t>() + starts_at()); }
+    gbsa::Bucket* buckets() const;   // null when not `tagged`
 };
 
 namespace gbsa {
@@ -41,6 +58,14 @@ struct __align__(16) Bucket {
     uint32_t w[3];   // the size in byte 0, entry i's tag in byte i + 1 (0 past the bucket's end)
 };
 
+}  // namespace gbsa
+
+inline gbsa::Bucket* gbsa_index::buckets() const {
+    return tagged ? reinterpret_cast<gbsa::Bucket*>(tables.as<uint8_t>() + buckets_at()) : nullptr;
+}
+
+namespace gbsa {
+
 // Read-only view of the index used by device code.
 struct IndexView {
     const gbsa_ref_randstrobe* rs;
@@ -53,9 +78,7 @@ struct IndexView {
 };
 
 inline IndexView view_of(const gbsa_index& ix) {
-    return IndexView{ix.rs.as<gbsa_ref_randstrobe>(), ix.starts.as<uint64_t>(),
-                     ix.buckets.size() ? ix.buckets.as<Bucket>() : nullptr, ix.n, ix.bits, ix.filter_cutoff,
-                     ix.params.k};
+    return IndexView{ix.rs(), ix.starts(), ix.buckets(), ix.n, ix.bits, ix.filter_cutoff, ix.params.k};
 }
 
 // Builds the lookup's bucket table of a loaded index, when every start fits 32 bits

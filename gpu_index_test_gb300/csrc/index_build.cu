@@ -411,9 +411,9 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
     GBSA_CUDA(cudaMemcpyAsync(d_clen.as<void>(), clen.data(), 8 * (n_contigs + 1), cudaMemcpyHostToDevice, st));
 
     // the sort's passes go back and forth between the table and scratch; they end in the table
-    ix.rs.resize(16 * (n_rs + 1));
+    ix.resize_tables();
     DeviceBuffer d_rs(16 * (n_rs + 1), st);
-    gbsa_ref_randstrobe* from = ix.rs.as<gbsa_ref_randstrobe>();
+    gbsa_ref_randstrobe* from = ix.rs();
     gbsa_ref_randstrobe* to = d_rs.as<gbsa_ref_randstrobe>();
     if (sort_passes(n_rs) % 2) std::swap(from, to);
     GBSA_CUDA(cudaMemsetAsync(from, 0, 16 * (n_rs + 1), st));
@@ -430,25 +430,20 @@ void build_index(gbsa_index& ix, const char* seqs, const uint64_t* offsets, cons
 
     // ---- sort --------------------------------------------------------------------
     const gbsa_ref_randstrobe* sorted = sort_ref_randstrobes(from, to, n_rs, max_position, ws, st);
-    const gbsa_ref_randstrobe* rs = ix.rs.as<gbsa_ref_randstrobe>();
+    const gbsa_ref_randstrobe* rs = ix.rs();
     if (sorted != rs)   // (a table of repeats, sorted by all bytes)
-        GBSA_CUDA(cudaMemcpyAsync(ix.rs.as<void>(), sorted, 16 * n_rs, cudaMemcpyDeviceToDevice, st));
+        GBSA_CUDA(cudaMemcpyAsync(ix.rs(), sorted, 16 * n_rs, cudaMemcpyDeviceToDevice, st));
     d_rs.release();
 
     // ---- bucket tables, run-length statistics → filter_cutoff -----------------------
-    const uint64_t nb = (1ULL << ix.bits) + 1;
-    ix.starts.resize(8 * nb);
-    const bool tagged = n_rs < (1ull << 32);
-    if (tagged) ix.buckets.resize(sizeof(Bucket) * nb);
     std::vector<unsigned long long> H(102, 0);
     if (n_rs == 0) {
-        GBSA_CUDA(cudaMemsetAsync(ix.starts.as<void>(), 0, 8 * nb, st));
-        GBSA_CUDA(cudaMemsetAsync(ix.buckets.as<void>(), 0, sizeof(Bucket) * nb, st));
+        GBSA_CUDA(cudaMemsetAsync(ix.starts(), 0, ix.tables.size() - ix.starts_at(), st));
     } else {
         unsigned long long* d_h = ws.get<unsigned long long>(102);
         GBSA_CUDA(cudaMemsetAsync(d_h, 0, 102 * 8, st));
-        k_tables<<<grid_for(n_rs, 256, 16 * device_sm_count()), 256, 0, st>>>(rs, n_rs, ix.bits, ix.starts.as<uint64_t>(),
-                                                                tagged ? ix.buckets.as<Bucket>() : nullptr, d_h);
+        k_tables<<<grid_for(n_rs, 256, 16 * device_sm_count()), 256, 0, st>>>(rs, n_rs, ix.bits, ix.starts(),
+                                                                              ix.buckets(), d_h);
         GBSA_LAUNCHED();
         GBSA_CUDA(cudaMemcpyAsync(H.data(), d_h, 102 * 8, cudaMemcpyDeviceToHost, st));
     }
@@ -480,19 +475,16 @@ __global__ void k_make_buckets(const uint64_t* __restrict__ starts, const gbsa_r
 }
 
 void make_buckets(gbsa_index& ix, cudaStream_t st) {
-    if (ix.n >= (1ull << 32)) return;
-    const uint64_t nb = 1ULL << ix.bits;
-    ix.buckets.resize(sizeof(Bucket) * (nb + 1));
-    DeviceBuffer d_odd(4);
+    if (!ix.tagged) return;
+    DeviceBuffer d_odd(4, st);
     uint32_t odd = 0;
     GBSA_CUDA(cudaMemsetAsync(d_odd.as<void>(), 0, 4, st));
-    k_make_buckets<<<grid_for(nb + 1, 256, 1u << 20), 256, 0, st>>>(ix.starts.as<uint64_t>(),
-                                                                    ix.rs.as<gbsa_ref_randstrobe>(), ix.n, ix.bits,
-                                                                    ix.buckets.as<Bucket>(), d_odd.as<uint32_t>());
+    k_make_buckets<<<grid_for(ix.n_starts(), 256, 1u << 20), 256, 0, st>>>(ix.starts(), ix.rs(), ix.n, ix.bits,
+                                                                           ix.buckets(), d_odd.as<uint32_t>());
     GBSA_LAUNCHED();
     GBSA_CUDA(cudaMemcpyAsync(&odd, d_odd.as<void>(), 4, cudaMemcpyDeviceToHost, st));
     GBSA_CUDA(cudaStreamSynchronize(st));
-    if (odd) ix.buckets.release();
+    if (odd) ix.tagged = false;
 }
 
 }  // namespace gbsa
