@@ -471,24 +471,36 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
             side2 = m.side2_lo;
         }
     }
-    GBSA_CUDA(cudaEventRecord(m.fork_ev, st));
-    GBSA_CUDA(cudaStreamWaitEvent(side, m.fork_ev, 0));
-    Arenas As = A;
-    As.slots = m.side_slots.as<uint8_t>();
-    launch_rescue(I, C, n, m.rec.as<ReadRec>(), As, ctr, side);
-    GBSA_CUDA(cudaEventRecord(m.rescue_ev, side));
-    if (m.profile) record_stage(m.ev[6], side);
-    // what the packed sort passes on: the block sorts and the cluster sorts take different
-    // reads, beside each other
-    if (n) launch_sort_packed(C, m.rec.as<ReadRec>(), As, ctr, side);
-    GBSA_CUDA(cudaEventRecord(m.join2_ev, side));
-    GBSA_CUDA(cudaStreamWaitEvent(side2, m.join2_ev, 0));
-    if (n) launch_sort_jobs(C, m.rec.as<ReadRec>(), As, ctr, side);
-    if (n) launch_sort_jobs_cluster(C, m.rec.as<ReadRec>(), As, ctr, side2);
-    GBSA_CUDA(cudaEventRecord(m.join2_ev, side2));
-    GBSA_CUDA(cudaStreamWaitEvent(side, m.join2_ev, 0));
-    if (m.profile) record_stage(m.ev[7], side);
-    GBSA_CUDA(cudaEventRecord(m.join_ev, side));
+    const bool rescues = C.force_rescue || C.rescue_level > 1;   // else no read is on the list
+    if (rescues) {
+        GBSA_CUDA(cudaEventRecord(m.fork_ev, st));
+        GBSA_CUDA(cudaStreamWaitEvent(side, m.fork_ev, 0));
+        Arenas As = A;
+        As.slots = m.side_slots.as<uint8_t>();
+        launch_rescue(I, C, n, m.rec.as<ReadRec>(), As, ctr, side);
+        GBSA_CUDA(cudaEventRecord(m.rescue_ev, side));
+        if (m.profile) record_stage(m.ev[6], side);
+        // What the packed sort passes on: the block sorts and the cluster sorts take different
+        // reads, beside each other in the orders that it does not sort (a stream and two events
+        // for them cost a call with one read 3 of 128 us).
+        const bool apart = C.sort_mode != GBSA_SORT_SCORE && n > 64;
+        if (n) launch_sort_packed(C, n, m.rec.as<ReadRec>(), As, ctr, side);
+        if (apart) {
+            GBSA_CUDA(cudaEventRecord(m.join2_ev, side));
+            GBSA_CUDA(cudaStreamWaitEvent(side2, m.join2_ev, 0));
+        }
+        if (n) launch_sort_jobs(C, n, m.rec.as<ReadRec>(), As, ctr, side);
+        if (n) launch_sort_jobs_cluster(C, n, m.rec.as<ReadRec>(), As, ctr, apart ? side2 : side);
+        if (apart) {
+            GBSA_CUDA(cudaEventRecord(m.join2_ev, side2));
+            GBSA_CUDA(cudaStreamWaitEvent(side, m.join2_ev, 0));
+        }
+        if (m.profile) record_stage(m.ev[7], side);
+        GBSA_CUDA(cudaEventRecord(m.join_ev, side));
+    } else if (m.profile) {
+        record_stage(m.ev[6], st);
+        record_stage(m.ev[7], st);
+    }
     launch_bucket_reads(n, m.rec.as<ReadRec>(), A, ctr, st, desc);
     launch_nams(C, n, m.rec.as<ReadRec>(), A, ctr, st);
     mark(4);
@@ -498,7 +510,7 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
     // it only order NAMs): per-read counts → offsets, and the records of the reads that
     // were not rescued, while the side stream may still sort; the rescued reads' records
     // after the join.  (Meaningless when an arena overflowed; the batch then runs again.)
-    GBSA_CUDA(cudaStreamWaitEvent(st, m.rescue_ev, 0));
+    if (rescues) GBSA_CUDA(cudaStreamWaitEvent(st, m.rescue_ev, 0));
     uint64_t* cnt = m.cnt.as<uint64_t>();
     uint64_t* off = m.out_off.as<uint64_t>();
     launch_read_counts(n, m.rec.as<ReadRec>(), 0, cnt, st, desc);
@@ -507,8 +519,8 @@ void enqueue_batch(gbsa_mapper& m, const uint8_t* d_seqs, const uint64_t* d_offs
         launch_gather_nams(n, m.rec.as<ReadRec>(), m.nams.as<NamState>(), off, gt ? gt->nams : nullptr,
                            gt ? gt->frac : nullptr, gt ? gt->resc : nullptr, st, gt ? gt->cap : 0, 1, nullptr,
                            nullptr, desc);
-    GBSA_CUDA(cudaStreamWaitEvent(st, m.join_ev, 0));
-    if (gt || desc)
+    if (rescues) GBSA_CUDA(cudaStreamWaitEvent(st, m.join_ev, 0));
+    if (rescues && (gt || desc))
         launch_gather_nams(n, m.rec.as<ReadRec>(), m.nams.as<NamState>(), off, gt ? gt->nams : nullptr, nullptr,
                            nullptr, st, gt ? gt->cap : 0, 2, &A, ctr, desc);
     GBSA_CUDA(cudaMemcpyAsync(m.h_status.as<void>(), ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));

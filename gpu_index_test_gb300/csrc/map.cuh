@@ -188,9 +188,10 @@ void launch_bucket_reads(uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cuda
 void launch_nams_warp(const MapConfig& C, int k, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 void launch_rescue(const IndexView& I, const MapConfig& C, uint32_t n_reads, ReadRec* rec, Arenas A, Counters* ctr,
                    cudaStream_t st);
-void launch_sort_packed(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
-void launch_sort_jobs(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
-void launch_sort_jobs_cluster(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
+// n: reads at most
+void launch_sort_packed(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
+void launch_sort_jobs(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
+void launch_sort_jobs_cluster(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st);
 // mode 0: every read; 1: the reads that were not rescued; 2: the rescued reads (A and
 // ctr give the rescue list; needed for mode 2 only).
 // With desc (batched form): n is the work areas' read capacity, the batch's read count,

@@ -2977,26 +2977,27 @@ static void sort_smem_limit() {
     done[dev] = 1;
 }
 
-void launch_sort_packed(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
+// The sorts' grids: resident blocks, no more than there can be jobs.
+void launch_sort_packed(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
     sort_smem_limit();
-    k_sort_packed<<<(unsigned)device_sm_count() * 2, kPackThreads, 8 * kPackMax, st>>>(C, rec, A, ctr);
+    k_sort_packed<<<std::min(n, (unsigned)device_sm_count() * 2), kPackThreads, 8 * kPackMax, st>>>(C, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 
-void launch_sort_jobs(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
+void launch_sort_jobs(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
     sort_smem_limit();
     const unsigned sms = (unsigned)device_sm_count();
     if (C.sort_variant == 1)
-        k_sort_jobs<2 * kSortThreads, kSortTile><<<sms * 3, 2 * kSortThreads, kSortSmem, st>>>(C, rec, A, ctr);
+        k_sort_jobs<2 * kSortThreads, kSortTile><<<std::min(n, sms * 3), 2 * kSortThreads, kSortSmem, st>>>(C, rec, A, ctr);
     else
-        k_sort_jobs<kSortThreads, kSortTile><<<sms * 4, kSortThreads, kSortSmem, st>>>(C, rec, A, ctr);
+        k_sort_jobs<kSortThreads, kSortTile><<<std::min(n, sms * 4), kSortThreads, kSortSmem, st>>>(C, rec, A, ctr);
     GBSA_LAUNCHED();
 }
 
-void launch_sort_jobs_cluster(const MapConfig& C, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
+void launch_sort_jobs_cluster(const MapConfig& C, uint32_t n, ReadRec* rec, Arenas A, Counters* ctr, cudaStream_t st) {
     sort_smem_limit();
     // SMs / 2 clusters of kClusterCtas CTAs
-    const unsigned clusters = std::max(1u, (unsigned)device_sm_count() / 2);
+    const unsigned clusters = std::min(n, std::max(1u, (unsigned)device_sm_count() / 2));
     k_sort_jobs_cluster<<<clusters * kClusterCtas, 256, kSortSmem, st>>>(C, rec, A, ctr);
     GBSA_LAUNCHED();
 }
