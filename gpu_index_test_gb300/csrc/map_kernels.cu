@@ -2638,6 +2638,8 @@ __global__ void k_gather_nams(uint32_t n, const ReadRec* __restrict__ rec, const
                               float* frac, uint8_t* rescued, int mode, Arenas A, const Counters* ctr,
                               const BatchDesc* desc) {
     __shared__ uint32_t s_words[kWarpsPerBlock][32 * 11];
+    __shared__ uint32_t s_many[kWarpsPerBlock];   // mode 2: reads for the block
+    __shared__ uint64_t s_from[kWarpsPerBlock], s_to[kWarpsPerBlock];
     uint32_t* words = s_words[threadIdx.x >> 5];
     const uint32_t lane = lane_id();
     uint64_t* copy_off = nullptr;
@@ -2654,20 +2656,41 @@ __global__ void k_gather_nams(uint32_t n, const ReadRec* __restrict__ rec, const
             if (blockIdx.x == 0 && threadIdx.x == 0) copy_off[n] = out_off[cap];
         }
     }
-    // a rescued read by the block (it may hold thousands of NAMs: by a warp, the longest took
-    // 30 us of a batch of 1000 reads)
+    // a rescued read with up to 64 NAMs by a warp, one with more by the block (it may hold
+    // thousands: by a warp, the longest took 30 us of a batch of 1000 reads; but 100,000 reads
+    // that are not in the index, a block each, 55 us); a block's reads lie apart on the list,
+    // whose heavy ones are side by side
     if (mode == 2) {
-        const uint32_t n_light = ctr->n_rescue, n_heavy = ctr->n_rescue_heavy;
-        for (uint32_t t = blockIdx.x; t < n_light + n_heavy; t += gridDim.x) {
-            const uint32_t r = t < n_light ? A.rescue_list[t] : A.rescue_list[A.rescue_cap - 1 - (t - n_light)];
-            const ReadRec R = rec[r];
-            const uint64_t o = out_off[r];
-            const uint32_t m = o >= out_cap ? 0u : (uint32_t)min((uint64_t)R.n_nams, out_cap - o);
-            for (uint32_t j = 32 * (threadIdx.x >> 5); j < m; j += blockDim.x) {
+        const uint32_t w = threadIdx.x >> 5, n_light = ctr->n_rescue, total = n_light + ctr->n_rescue_heavy;
+        auto copy = [&](uint64_t from, uint64_t o, uint32_t m, uint32_t first, uint32_t step) {
+            for (uint32_t j = first; j < m; j += step) {
                 gbsa_nam x;
-                if (j + lane < m) to_gbsa_nam(arena[R.nam_off + j + lane], (int)(j + lane), x);
+                if (j + lane < m) to_gbsa_nam(arena[from + j + lane], (int)(j + lane), x);
                 write_records(words, x, min(m - j, 32u), out + o + j);
             }
+        };
+        for (uint32_t t0 = blockIdx.x; t0 < total; t0 += gridDim.x * kWarpsPerBlock) {
+            const uint32_t t = t0 + w * gridDim.x;
+            uint64_t from = 0, o = 0;
+            uint32_t m = 0;
+            if (t < total) {
+                const uint32_t r = t < n_light ? A.rescue_list[t] : A.rescue_list[A.rescue_cap - 1 - (t - n_light)];
+                from = rec[r].nam_off;
+                o = out_off[r];
+                m = o >= out_cap ? 0u : (uint32_t)min((uint64_t)rec[r].n_nams, out_cap - o);
+            }
+            if (m <= 64) {
+                copy(from, o, m, 0, 32);
+                m = 0;
+            }
+            if (lane == 0) {
+                s_many[w] = m;
+                s_from[w] = from;
+                s_to[w] = o;
+            }
+            if (!__syncthreads_or(m != 0)) continue;
+            for (uint32_t v = 0; v < kWarpsPerBlock; ++v) copy(s_from[v], s_to[v], s_many[v], 32 * w, blockDim.x);
+            __syncthreads();
         }
         return;
     }
