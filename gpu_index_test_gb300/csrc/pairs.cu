@@ -467,14 +467,15 @@ __global__ void __launch_bounds__(32 * kPairWarps)
         uint64_t* keys = reinterpret_cast<uint64_t*>(stacks + 2 * base);
         bool tie = false;
         for (int i = lane; i < len; i += 32) keys[i] = nam_pair_key(list[i], n1, tie);
+        __syncwarp();
         tie = __any_sync(kAll, tie);
         for (int b = 0; b < len && !tie; b += 32) {
             const int e = b + lane;
             const uint64_t ke = e < len ? keys[e] : 0;   // (no key is below 0 or equal to it)
             const gbsa_nam_pair pe = list[min(e, len - 1)];
             uint32_t rank = 0;
-            for (int c = 0; c < len && !tie; c += 64) {
-                const int end = min(c + 64, len);
+            for (int c = 0; c < len && !tie; c += 256) {
+                const int end = min(c + 256, len);
                 for (int f = c; f < end; ++f) {
                     const uint64_t kf = keys[f];
                     if (kf < ke) {
