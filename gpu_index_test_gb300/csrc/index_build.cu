@@ -199,18 +199,22 @@ __device__ __forceinline__ uint64_t second_run(const gbsa_ref_randstrobe* __rest
     return hi;
 }
 
-// Bucket b's form for the lookup, its first entry being `at` of n.
+// Bucket b's form for the lookup, its first entry being `at` of n.  kWhole: all entries from
+// `at` on are the bucket's.
+template <bool kWhole>
 __device__ __forceinline__ Bucket bucket_at(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, int bits,
                                             uint64_t b, uint64_t at) {
     uint32_t size = 0;
     uint64_t lo = 0;
     uint32_t hi = 0;   // bytes 0..7 and 8..11
-    for (; size < 255 && at + size < n; ++size) {
+    const uint32_t most = kWhole ? kBucketTags : 255;
+    for (; size < most && at + size < n; ++size) {
         const uint64_t h = rs[at + size].hash;
-        if ((h >> (64 - bits)) != b) break;
+        if (!kWhole && (h >> (64 - bits)) != b) break;
         if (size < 7) lo |= (uint64_t)hash_tag(h) << (8 * (size + 1));
         else if (size < kBucketTags) hi |= hash_tag(h) << (8 * (size - 7));
     }
+    if (kWhole) size = (uint32_t)(n - at < 255 ? n - at : 255);
     lo |= size;
     return Bucket{(uint32_t)at, {(uint32_t)lo, (uint32_t)(lo >> 32), hi}};
 }
@@ -218,29 +222,47 @@ __device__ __forceinline__ Bucket bucket_at(const gbsa_ref_randstrobe* __restric
 // The bucket table (the reference's first-bucket rule: the buckets up to the first entry's
 // start at the second run), where `buckets` is set the lookup's form of it, and the
 // histogram of the runs' lengths (bins 1..100 exact, bin 101: longer), in one pass: an entry
-// that opens a bucket writes it and the empty ones before it, one that opens a run walks it
-// (102 entries at most).
+// that opens a bucket writes it and the empty ones before it (its warp, where there are more
+// than 16: a table of few entries for its buckets, 2,000 for 2^24, took 5.3 ms by the entry
+// alone, and 2.5 without the tags; now 1.6), one that opens a run walks it (102
+// entries at most).
 __global__ void __launch_bounds__(256) k_tables(const gbsa_ref_randstrobe* __restrict__ rs, uint64_t n, int bits,
                                                 uint64_t* __restrict__ starts, Bucket* __restrict__ buckets,
                                                 unsigned long long* __restrict__ hist) {
     __shared__ unsigned int h[102];
     for (int i = threadIdx.x; i < 102; i += blockDim.x) h[i] = 0;
     __syncthreads();
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint64_t nb = 1ULL << bits;
-    auto put = [&](uint64_t b0, uint64_t b1, uint64_t at, uint64_t own) {   // [b0, b1), `own`: where at's entries lie
-        for (uint64_t b = b0; b < b1; ++b) {
-            starts[b] = at;
-            if (buckets) buckets[b] = b == own ? bucket_at(rs, n, bits, b, at) : Bucket{(uint32_t)at, {0, 0, 0}};
+    auto put = [&](uint64_t b, uint64_t at, bool own) {   // own: bucket b is that of entry `at`
+        starts[b] = at;
+        if (buckets) buckets[b] = own ? bucket_at<false>(rs, n, bits, b, at) : Bucket{(uint32_t)at, {0, 0, 0}};
+    };
+    auto empty = [&](uint64_t b0, uint64_t b1, uint64_t at) {   // buckets [b0, b1), the warp's lanes each their own
+        uint32_t m = __ballot_sync(kFull, b1 > b0 + 16);
+        if (b1 <= b0 + 16)
+            for (uint64_t b = b0; b < b1; ++b) put(b, at, false);
+        for (; m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            const uint64_t to = __shfl_sync(kFull, b1, src), first = __shfl_sync(kFull, at, src);
+            for (uint64_t b = __shfl_sync(kFull, b0, src) + lane_id(); b < to; b += 32) put(b, first, false);
         }
     };
     uint32_t once = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t hash = rs[i].hash, t = hash >> (64 - bits);
-        const uint64_t before = i ? rs[i - 1].hash : ~hash;
-        if (i == 0) put(0, t + 1, second_run(rs, n), t);
-        else put((before >> (64 - bits)) + 1, t + 1, i, t);
-        if (i == n - 1) put(t + 1, nb + 1, n, nb + 1);
-        if (hash != before) {
+    for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = base + threadIdx.x;
+        uint64_t b0 = 0, b1 = 0, at = 0, hash = 0, before = 0;
+        if (i < n) {
+            hash = rs[i].hash;
+            before = i ? rs[i - 1].hash : ~hash;
+            b1 = hash >> (64 - bits);
+            b0 = i ? (before >> (64 - bits)) + 1 : 0;   // (above b1 within a bucket)
+            at = i ? i : second_run(rs, n);
+            if (b0 <= b1) put(b1, at, true);
+        }
+        empty(b0, b1, at);
+        if (base + blockDim.x >= n) empty(b1 + 1, i == n - 1 ? nb + 1 : 0, n);
+        if (i < n && hash != before) {
             uint32_t len = 1;
             while (len < 101 && i + len < n && rs[i + len].hash == hash) ++len;
             if (len == 1) ++once;
@@ -468,7 +490,7 @@ __global__ void k_make_buckets(const uint64_t* __restrict__ starts, const gbsa_r
         const bool good = a <= n && e <= n &&
                           (a >= e || (top(a) == i && top(e - 1) == i && (e == n || top(e) != i)));
         if (!good) *odd = 1;
-        out[i] = good && a < e ? bucket_at(rs, e, bits, i, a) : Bucket{(uint32_t)a, {0, 0, 0}};
+        out[i] = good && a < e ? bucket_at<true>(rs, e, bits, i, a) : Bucket{(uint32_t)a, {0, 0, 0}};
     }
     for (uint64_t i = 1 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         if (rs[i - 1].hash > rs[i].hash) *odd = 1;
@@ -479,8 +501,8 @@ void make_buckets(gbsa_index& ix, cudaStream_t st) {
     DeviceBuffer d_odd(4, st);
     uint32_t odd = 0;
     GBSA_CUDA(cudaMemsetAsync(d_odd.as<void>(), 0, 4, st));
-    k_make_buckets<<<grid_for(ix.n_starts(), 256, 1u << 20), 256, 0, st>>>(ix.starts(), ix.rs(), ix.n, ix.bits,
-                                                                           ix.buckets(), d_odd.as<uint32_t>());
+    k_make_buckets<<<grid_for(std::max(ix.n_starts(), ix.n), 256, 1u << 20), 256, 0, st>>>(
+        ix.starts(), ix.rs(), ix.n, ix.bits, ix.buckets(), d_odd.as<uint32_t>());
     GBSA_LAUNCHED();
     GBSA_CUDA(cudaMemcpyAsync(&odd, d_odd.as<void>(), 4, cudaMemcpyDeviceToHost, st));
     GBSA_CUDA(cudaStreamSynchronize(st));
