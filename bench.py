@@ -1162,7 +1162,7 @@ def main():
     main_stages = ("seed_lookup", "lookup_long", "nams", "nams_warp") if fused else ("seed", "lookup", "nams", "nams_warp")
     dom = max(main_stages, key=lambda k: stage_ms.get(k, 0.0))
     # NAMs the step outputs (the NAM-state arena's slots, counts["nam_slots"], include the
-    # room the lane merge reserves: two per hit)
+    # room the merges take)
     q, hits, nams_n = counts["queries"], counts["hits"], int(total_nams)
     packed = int(((reads.lengths.astype(np.int64) + 3) // 4).sum())
     # Algorithmic bytes as the measurement plan defines them per read: the 2-bit packed
@@ -1175,14 +1175,14 @@ def main():
         "seed_long": 0,
         "nams": 44 * nams_n, "nams_warp": 0, "rescue": 0, "rescue_sort": 0,
     }
-    # Bytes the kernels pass between their own phases through HBM / L2 (not algorithmic):
-    # query records written and read back, index positions, per-query hit counts and
-    # offsets, hit records written (seeding + lookup) and read (NAM stages), NAM states
-    # written unsorted and sorted.
+    # Bytes the kernels pass between their own phases through HBM (not algorithmic): hit
+    # records written (seeding + lookup; what it keeps of a found query stays in L2) and read
+    # (NAM stages), NAM states written sorted; in two kernels also query records written and
+    # read back, index positions, per-query hit counts and offsets.
     inter = {
-        "seed_lookup": 16 * q + 16 * q + 8 * q + 8 * q + 16 * hits,
+        "seed_lookup": 16 * hits,
         "seed": 16 * q, "lookup": 16 * q + 8 * q + 8 * q + 16 * hits,
-        "nams": 16 * hits + 64 * nams_n,
+        "nams": 16 * hits + 32 * nams_n,
     }
     peak, peak_kind = peaks()
     achieved = alg[dom] / (stage_ms[dom] / 1e3) / 1e9 if stage_ms[dom] > 0 else 0.0
@@ -1213,7 +1213,8 @@ def main():
         "kernel": lk_stage, "sectors_per_launch": int(sectors_lookup), "achieved": round(lk_gbs, 1), "unit": "GB/s",
         "peak": round(g_gbs, 1), "frac": round(lk_gbs / g_gbs, 4) if g_gbs > 0 else None,
         "peak_source": "gbsa_bench_gather_index: uniform random keys, bucket bound pair then the bucket's first "
-                       "entry (dependent) on this index's own tables, 8 probes in flight per thread",
+                       "entry (dependent) on this index's own tables, 8 probes in flight per thread; "
+                       "no upper bound for the kernel, whose bucket tags answer most probes without an entry",
         "peak_probes_per_s": round(g_probes, 1),
         "flat_buffer_gather_gbs": {"512MB": round(gather_hbm, 1), "16MB": round(gather_l2, 1)},
     }

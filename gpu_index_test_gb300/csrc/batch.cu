@@ -11,7 +11,7 @@
 //   * seeding and lookup run as one persistent kernel (a grid of SMs x resident
 //     blocks) whose warps pull work items — a single-end read, or both mates of a
 //     pair — from a device queue, so reads of uneven lengths balance over the grid;
-//   * the NAM phase (lane and warp merges on one stream, rescue and its sorts on a
+//   * the NAM phase (group and block merges on one stream, rescue and its sorts on a
 //     second) pulls its reads from the device lists the front end fills, as in the
 //     plain form, inside the same graph.
 //

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) k_gather(const uint4* __restrict__ buf, u
 }
 
 // The lookup's own access pattern on the lookup's own buffers: for a uniform random
-// key, the bucket bound pair from the index's bucket table (the 32-bit copy when it
+// key, the bucket bound pair from the index's bucket table (the lookup's tagged buckets when it
 // has one), then the first entry of the bucket, a load that depends on the first.
 // 8 probes in flight per thread.  Sectors: the bucket pair's, plus the entry's for a
 // non-empty bucket.

@@ -6,6 +6,7 @@
 //           bounds the bucket, with the reference's first-bucket rule
 //           (step2/index.cu:207-210: buckets up to the first hash's own start at the
 //           second distinct hash)
+//   buckets Bucket[2^bits + 1], the lookup's form of the table
 #pragma once
 
 #include <cstdint>

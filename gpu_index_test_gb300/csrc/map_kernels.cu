@@ -1,11 +1,12 @@
-// map_kernels.cu — kernels of the read → NAM path (plain form: one kernel per stage,
-// a warp per read, intermediates in HBM arenas).
+// map_kernels.cu — kernels of the read → NAM path (intermediates in HBM arenas).
 //
-//   k_seed_smem / k_seed_long   randstrobes_query (step2/randstrobes.cu:195-241)
-//   k_lookup                    the query loop of find_nams (step2/nam.cu:748-790):
-//                               find, is_filtered, add_to_hits_per_ref; the rescue
-//                               decision of step2/main.cu:3209-3216
-//   k_nams                      merge_hits_into_nams_forward_and_reverse(sort=true)
+//   k_seed_lookup               randstrobes_query (step2/randstrobes.cu:195-241) and the
+//                               query loop of find_nams (step2/nam.cu:748-790): find,
+//                               is_filtered, add_to_hits_per_ref; the rescue decision of
+//                               step2/main.cu:3209-3216
+//   k_seed_smem / k_seed_long, k_lookup / k_lookup_long   the same in two kernels, and for
+//                               long reads
+//   k_nams_group, k_nams        merge_hits_into_nams_forward_and_reverse(sort=true)
 //                               (step2/nam.cu:515-539, 347-513) + NAM sort
 //   k_rescue                    find_nams_rescue (step2/nam.cu:927-985) + NAM sort
 #include <algorithm>
@@ -878,9 +879,9 @@ __device__ void warp_finish_nams(const MapConfig& C, const NamState* closed, uin
 // count) takes a read, 32 / G reads a warp, with R slots a lane: NAM i is slot (row) i / G
 // of lane i % G.  Slots are never given back (a read has at most as many NAMs as hits;
 // the few reads with more NAMs than slots go to a list in memory), so slot order is
-// creation order.  Same hit-major rule as warp_find_nams: hits in (orientation,
-// query_start, position) order, each joins the first NAM in creation order that accepts
-// it, found with one ballot a row; a NAM that the query start has passed, or of the other
+// creation order.  The hit-major rule of merge_hits_into_nams (step2/nam.cu:347-513): hits
+// in (orientation, query_start, position) order, each joins the first NAM in creation order
+// that accepts it, found with one ballot a row; a NAM that the query start has passed, or of the other
 // orientation, accepts nothing, so it needs no closing (rows with no other NAM are
 // skipped).  The NAMs are then ranked by their keys through shared memory and written
 // once, in order.
@@ -891,7 +892,7 @@ __device__ void warp_finish_nams(const MapConfig& C, const NamState* closed, uin
 constexpr int kGroupWarps = 4;
 constexpr int kGroupBlocksPerSm = 8;     // 64 registers a thread
 // The rescue chain runs beside the NAM kernels on another stream; the persistent grids are
-// sized so that its block (72 KB) keeps room beside them.
+// sized so that its blocks (RescueShared, 97 KB each) keep room beside them.
 constexpr int kRescueBlocksPerSm = 2;
 
 __device__ __forceinline__ HitRec load_hit(const HitPacked* __restrict__ hits, uint32_t i, uint32_t H) {

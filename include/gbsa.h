@@ -148,7 +148,10 @@ int gbsa_pick_bits(const gbsa_params* p, uint64_t total_length);
 
 /* StrobemerIndex(references, parameters, bits) + populate(f, n_threads)
  * (step2/index.hpp:39-54; body restated from step2/index.cu:143-311).
- * Contig i is seqs[offsets[i] .. offsets[i] + lengths[i]).  bits == -1 picks bits. */
+ * Contig i is seqs[offsets[i] .. offsets[i] + lengths[i]).  bits == -1 picks bits.
+ * An index takes 16 bytes an entry and 24 a bucket on the device (8 with 2^32 entries or
+ * more): 16.4 GB at 3.1 Gbp (620M entries, 2^28 buckets).  While one lives the library keeps up
+ * to 256 MiB of scratch on its device. */
 int gbsa_index_build(const gbsa_params* p, const char* seqs, const uint64_t* offsets,
                      const uint64_t* lengths, uint32_t n_contigs, int bits, float f,
                      gbsa_index** out);
