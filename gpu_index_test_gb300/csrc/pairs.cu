@@ -474,8 +474,8 @@ __global__ void __launch_bounds__(32 * kPairWarps)
             const uint64_t ke = e < len ? keys[e] : 0;   // (no key is below 0 or equal to it)
             const gbsa_nam_pair pe = list[min(e, len - 1)];
             uint32_t rank = 0;
-            for (int c = 0; c < len && !tie; c += 256) {
-                const int end = min(c + 256, len);
+            for (int c = 0; c < len && !tie; c += 1024) {
+                const int end = min(c + 1024, len);
                 for (int f = c; f < end; ++f) {
                     const uint64_t kf = keys[f];
                     if (kf < ke) {
